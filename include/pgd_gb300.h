@@ -74,8 +74,11 @@ typedef struct {
     int64_t n;              /* vertices                                     */
     int64_t m;              /* undirected edges                             */
     float kernel_ms;        /* device time of the decomposition kernels     */
-    float hub_ms;           /* of which the hub-anchored kernel (k_hub)     */
-    float tri_ms;           /* of which the triangle pass (t of every edge) */
+    float hub_ms;           /* of which the 4-cycle pass, which runs beside
+                               the triangle passes (edge-by-edge runs of
+                               small samples: the hub-anchored kernel)      */
+    float tri_ms;           /* of which the triangle and 4-clique passes
+                               (edge-by-edge runs: t of every edge)         */
     float reserved;
 } pgd_counts;
 

@@ -111,7 +111,10 @@ extern "C" pgd_status pgd_context_create(const pgd_opts *opts, pgd_ctx **out) {
         cudaMalloc((void **)&ctx->d_ctr, 64 * sizeof(unsigned long long)) != cudaSuccess ||
         cudaEventCreate(&ctx->ev0) != cudaSuccess || cudaEventCreate(&ctx->ev1) != cudaSuccess ||
         cudaEventCreate(&ctx->evt0) != cudaSuccess || cudaEventCreate(&ctx->evt1) != cudaSuccess ||
-        cudaEventCreate(&ctx->evh0) != cudaSuccess || cudaEventCreate(&ctx->evh1) != cudaSuccess) {
+        cudaEventCreate(&ctx->evh0) != cudaSuccess || cudaEventCreate(&ctx->evh1) != cudaSuccess ||
+        cudaStreamCreateWithFlags(&ctx->side, cudaStreamNonBlocking) != cudaSuccess ||
+        cudaEventCreateWithFlags(&ctx->ev_fork, cudaEventDisableTiming) != cudaSuccess ||
+        cudaEventCreateWithFlags(&ctx->ev_join, cudaEventDisableTiming) != cudaSuccess) {
         cudaGetLastError();
         pgd_context_destroy(ctx);
         return PGD_ECUDA;
@@ -128,8 +131,12 @@ extern "C" pgd_status pgd_context_destroy(pgd_ctx *ctx) {
     if (ctx->d_ctr) cudaFree(ctx->d_ctr);
     if (ctx->ev0) cudaEventDestroy(ctx->ev0);
     if (ctx->ev1) cudaEventDestroy(ctx->ev1);
-    for (cudaEvent_t e : {ctx->evt0, ctx->evt1, ctx->evh0, ctx->evh1})
+    for (cudaEvent_t e : {ctx->evt0, ctx->evt1, ctx->evh0, ctx->evh1, ctx->ev_fork, ctx->ev_join})
         if (e) cudaEventDestroy(e);
+    if (ctx->side) {
+        cudaStreamSynchronize(ctx->side);
+        cudaStreamDestroy(ctx->side);
+    }
     if (ctx->own_stream && ctx->stream) cudaStreamDestroy(ctx->stream);
     delete ctx;
     return PGD_OK;
@@ -174,6 +181,7 @@ extern "C" pgd_status pgd_graph_destroy(pgd_graph *g) {
     pgd_graph_free(g, g->toprows, (g->top_words + 1) * sizeof(uint32_t));
     pgd_graph_free(g, g->vrec, (g->n + 1) * 32);
     pgd_graph_free(g, g->adj_rank, (2 * g->m + 1) * sizeof(int32_t));
+    pgd_rank_drop(g);
     // whatever is left (partial builds) is returned to the budget as well
     g->ctx->resident -= g->bytes;
     cudaStreamSynchronize(g->ctx->stream);

@@ -49,6 +49,7 @@
 
 #include "pgd_internal.h"
 #include "pgd_kernels.cuh"
+#include "rank_path.h"
 #include "tc_ptx.cuh"
 
 namespace {
@@ -2566,6 +2567,11 @@ static size_t hub_layout(int64_t n, int32_t nhubs, int32_t nwide, int32_t max_de
     return (size_t)((H->smem_hist ? H->hstride : 0) + bm_words) * 4;
 }
 
+// A sample of fewer than one edge in kSampleShare is decomposed edge by edge
+// (run_decompose), everything else by the passes of rank_path.cu, whose cost
+// does not depend on the number of edges asked for.
+constexpr int64_t kSampleShare = 64;
+
 // Device times of one decomposition: all kernels, the triangle pass, k_hub.
 struct StageMs {
     float total = 0, tri = 0, hub = 0;
@@ -2853,6 +2859,41 @@ static pgd_status run_decompose(pgd_ctx *ctx, const DevGraph &G, int4 *slot, int
     return PGD_OK;
 }
 
+// The rank-ordered path (rank_path.cu) on one graph; *ms gets its device times.
+static pgd_status rank_decompose(pgd_graph *g, bool micro, StageMs *ms) {
+    pgd_ctx *ctx = g->ctx;
+    cudaStream_t s = ctx->stream;
+    pgd_status st;
+    *ms = StageMs();
+    if (!g->ranked) {
+        g->ranked = new pgd_rank_graph();
+        if ((st = pgd_rank_build(g, 2 * g->m, nullptr, nullptr, g->ranked))) {
+            pgd_rank_drop(g);
+            return st;
+        }
+    }
+    pgd_rank_out o{};
+    o.ev = g->ev;
+    o.eu = g->eu;
+    o.deg = g->deg;
+    o.order = g->order;
+    o.npos = g->norder;
+    o.n = g->n;
+    o.m = g->m;
+    o.micro = micro ? g->micro : nullptr;
+    o.sums = ctx->d_sums;
+    PGD_CUDA(ctx, cudaEventRecord(ctx->ev0, s));
+    if ((st = pgd_rank_decompose(ctx, *g->ranked, o))) return st;
+    PGD_CUDA(ctx, cudaEventRecord(ctx->ev1, s));
+    PGD_CUDA(ctx, cudaEventSynchronize(ctx->ev1));
+    PGD_CUDA(ctx, cudaEventElapsedTime(&ms->total, ctx->ev0, ctx->ev1));
+    if (g->norder > 0 && g->m > 0) {
+        PGD_CUDA(ctx, cudaEventElapsedTime(&ms->tri, ctx->evt0, ctx->evt1));
+        PGD_CUDA(ctx, cudaEventElapsedTime(&ms->hub, ctx->evh0, ctx->evh1));
+    }
+    return PGD_OK;
+}
+
 pgd_status pgd_dev_decompose(pgd_graph *g, bool micro, pgd_counts *out) {
     pgd_ctx *ctx = g->ctx;
     cudaStream_t s = ctx->stream;
@@ -2860,10 +2901,15 @@ pgd_status pgd_dev_decompose(pgd_graph *g, bool micro, pgd_counts *out) {
     if (micro && !g->micro) {
         if ((st = pgd_graph_alloc(g, (void **)&g->micro, (g->m + 1) * PGD_NMICRO * sizeof(uint64_t)))) return st;
     }
-    if ((!g->has_aux || g->aux_cache_hub != ctx->cache_hub) && (st = build_aux(g))) return st;
     PGD_CUDA(ctx, cudaMemsetAsync(ctx->d_sums, 0, PGD_NSUMS * sizeof(unsigned long long), s));
     StageMs ms;
-    if ((st = run_decompose(ctx, dev_view(g, micro), (int4 *)g->slot, g->nhubs, g->nhubs_wide, g->max_degree, &ms))) return st;
+    if (g->norder >= g->m / kSampleShare) {
+        if ((st = rank_decompose(g, micro, &ms))) return st;
+    } else {
+        if ((!g->has_aux || g->aux_cache_hub != ctx->cache_hub) && (st = build_aux(g))) return st;
+        if ((st = run_decompose(ctx, dev_view(g, micro), (int4 *)g->slot, g->nhubs, g->nhubs_wide, g->max_degree, &ms)))
+            return st;
+    }
     unsigned long long h[PGD_NSUMS];
     PGD_CUDA(ctx, cudaMemcpyAsync(h, ctx->d_sums, sizeof(h), cudaMemcpyDeviceToHost, s));
     PGD_CUDA(ctx, cudaStreamSynchronize(s));

@@ -13,6 +13,8 @@ struct pgd_ctx {
     int num_sms = 0;
     cudaStream_t stream = nullptr;
     bool own_stream = false;
+    cudaStream_t side = nullptr;   // work that runs beside the stream's, forked from and joined to it by events
+    cudaEvent_t ev_fork = nullptr, ev_join = nullptr;
     uint64_t budget = 0;     // bytes graphs of this context may hold
     uint64_t resident = 0;   // bytes currently held
     std::string err;
@@ -81,6 +83,7 @@ struct pgd_graph {
     int64_t top_words = 0;
     int32_t *vrank = nullptr;         // n: rank by (degree desc, id)
     int32_t *adjp_rank = nullptr;     // m: vrank of each adjp entry
+    struct pgd_rank_graph *ranked = nullptr;   // rank-ordered copy (rank_path.cu), built on first use
     void *slot = nullptr;             // 2m * 16 B: per adjacency slot {w, vrank(w) | row flag, hubid(w), t}
 };
 
@@ -104,6 +107,7 @@ pgd_status pgd_cuda_fail(pgd_ctx *ctx, cudaError_t e, const char *what);
 // Device memory owned by a graph (counted against the context budget).
 pgd_status pgd_graph_alloc(pgd_graph *g, void **p, size_t bytes);
 void pgd_graph_free(pgd_graph *g, void *p, size_t bytes);
+void pgd_rank_drop(pgd_graph *g);   // frees g's rank-ordered copy, if any
 
 // Stream-ordered temporaries (not counted against the budget).
 pgd_status pgd_tmp_alloc(pgd_ctx *ctx, void **p, size_t bytes);

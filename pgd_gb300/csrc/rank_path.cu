@@ -1,0 +1,1433 @@
+// rank_path.cu -- per-edge graphlet counts of sparse graphs in degree-rank
+// order: triangles and 4-cliques from each vertex's up-neighbourhood, 4-cycles
+// from wedges whose highest-ranked vertex is an end.
+//
+// Replaces the OpenMP edge loop of graphlet_decomposition[_micro]
+// (graphlet_core.cpp:1408-1424 and :1549-1577) with its helpers
+// triangles_and_wedges / cycle / clique (:1069-1240).  That loop rescans the
+// neighbourhoods of both ends for every edge; here every triangle, 4-clique
+// and wedge is met once (the wedges twice) and credited to its edges.
+//
+// Vertices are renumbered by (degree descending, id descending); a row lists
+// its neighbours' ranks in ascending order, so its first entries N+(x) are the
+// neighbours above x.  With T(e) the common neighbours of an edge e's ends,
+// t = |T|, k4 the edges inside T, and c4 the induced 4-cycles through e:
+//   * triangles {a, x, y}, a the lowest: y in N+(a) n N+(x).  Pass 1 adds one to
+//     t of the three edges.  Pass 2 repeats it with the adjacency F of N+(a) as
+//     a bit matrix: |F_x & F_y| is the number of 4-cliques {a, z, x, y}, each
+//     credited to its six edges, and the other two edges' t go to
+//       D(e) = sum over w in T(e) of t of the edges from w to e's two ends.
+//   * 4-cycles: the top vertex u of a cycle meets its opposite w through
+//     wedges u - v - w with v and w below u.  For each u a counter per w counts
+//     them; a second walk adds count(w) - 1 to edges (u, v) and (v, w).  That
+//     gives C4(e), the 4-cycles through e with or without chords, and
+//       c4 = C4 - D + 2 t + 2 k4
+//     (a cycle p, q, w, x through e = (p, q) has the chord (p, w) iff w is in
+//     T, of which there are sum_T (t(w, p) - 1), likewise for x and q, and both
+//     chords 2 k4 times).
+// t, k4 and c4 are at most m < 2^31, and everything else is used modulo 2^32,
+// so all partial results are 32-bit.
+//
+// The numbers on R-MAT scale 20 (15.7 M edges): 5.65e9 wedges, 4.4e9 list
+// entries probed per triangle pass, 4.2e8 triangles -- against 4.6e10 histogram
+// entries and 9e10 list entries and bitmap words for the per-edge method of
+// decompose.cu, which stays for small samples of the edges and for the
+// allocation-free entry point.
+#include <stddef.h>
+
+#include <algorithm>
+#include <cub/cub.cuh>
+
+#include "pgd_kernels.cuh"
+#include "rank_path.h"
+
+namespace {
+
+constexpr int kThreads = 256;
+constexpr uint32_t kFull = 0xffffffffu;
+
+inline int grid_for(int64_t n, int per_block = kThreads, int cap = 1 << 20) {
+    int64_t g = (n + per_block - 1) / per_block;
+    if (g < 1) g = 1;
+    if (g > cap) g = cap;
+    return (int)g;
+}
+
+inline int bits_for(int64_t x) {   // bits that hold every value below x (at least one)
+    int b = 1;
+    while (b < 63 && (int64_t(1) << b) < x) b++;
+    return b;
+}
+
+// ---------------------------------------------------------------------------
+// work classes
+
+enum {
+    kEgoWarp = 0,    // |N+(a)| in [2, 32]: a warp per vertex
+    kEgoA,           // (32, 256]
+    kEgoB,           // (256, 512]
+    kEgoC,           // (512, 1024]
+    kEgoGlobal,      // beyond: the tables in global memory
+    kCycWarp,        // 2 .. kCycWarpMax wedges: a warp per vertex
+    kCycHash,        // .. kCycHashMax wedges: a block per vertex, hashed counters
+    kClasses         // more wedges: items of k_cycle_direct
+};
+constexpr int kEgoMax[] = {32, 256, 512, 1024};
+constexpr int kCycWarpMax = 512;
+constexpr int kCycHashMax = 4096;
+constexpr int kMaxRanges = 8192;
+constexpr int64_t kBposBytes = 4ll << 30;      // largest table of range boundaries per row
+constexpr int kDirectThreads = 1024;
+constexpr uint32_t kDirectWords = 50 * 1024;   // counter words of one item: 200 KB of shared memory
+
+// Sizes found on the device while the graph is built.
+struct RankMeta {
+    uint32_t tier[5];        // ranks below tier[i] have degree >= 65536, 256, 16, 4, 2
+    uint32_t tcode[5];       // bit address at which tier i + 1 ends (counter widths 32, 16, 8, 4, 2)
+    uint32_t max_up;
+    uint32_t entries2;       // entries of the rows of vertices of degree >= 2
+    uint32_t nlist[kClasses];
+    unsigned long long direct_wedges;   // wedges of the vertices beyond the lists
+    uint32_t bound[kMaxRanges + 1];   // range boundaries (ranks)
+};
+
+// Bit address of the counter of rank r.  A counter of w never exceeds deg(w):
+// 32, 16, 8, 4 or 2 bits by degree (wide ones first, so none straddles a word).
+__device__ __forceinline__ uint32_t code_of(const RankMeta *M, uint32_t r) {
+    uint32_t lo = 0, c = 0;
+#pragma unroll
+    for (int i = 0; i < 5; i++) {
+        const uint32_t hi = M->tier[i];
+        if (r < hi) return c + ((r - lo) << (5 - i));
+        lo = hi;
+        c = M->tcode[i];
+    }
+    return c;
+}
+
+__device__ __forceinline__ uint32_t mask_of(const RankMeta *M, uint32_t code) {
+    if (code >= M->tcode[2]) return code < M->tcode[3] ? 0xfu : 0x3u;
+    if (code >= M->tcode[1]) return 0xffu;
+    return code >= M->tcode[0] ? 0xffffu : 0xffffffffu;
+}
+
+__device__ __forceinline__ uint32_t lower_bound_u(const int32_t *a, uint32_t lo, uint32_t hi, int32_t x) {
+    while (lo < hi) {
+        const uint32_t mid = lo + ((hi - lo) >> 1);
+        if (__ldg(a + mid) < x) lo = mid + 1;
+        else hi = mid;
+    }
+    return lo;
+}
+
+// First lane whose inclusive prefix exceeds it (all 32 lanes call).
+__device__ __forceinline__ int owner_of(int incl, int it) {
+    int lo = 0;
+#pragma unroll
+    for (int step = 16; step > 0; step >>= 1) {
+        const int pre = __shfl_sync(kFull, incl, lo + step - 1);
+        if (pre <= it) lo += step;
+    }
+    return lo;
+}
+
+// Row of each slot p = p0 + lane of one warp (lanes with p >= nnz get a valid
+// row too).  Rows without entries come last in rank order, so 32 consecutive
+// slots span at most 32 rows: one 32-way search finds the first, a 5-step
+// search over the next row ends the rest.
+__device__ __forceinline__ int rows_of_warp(const uint32_t *roff, int64_t n, uint32_t p0, uint32_t p, int lane) {
+    int64_t lo = 0, hi = n;   // roff[lo] <= p0 < roff[hi]
+    while (hi - lo > 1) {
+        const int64_t step = (hi - lo + 31) / 32;
+        const int64_t at = min(lo + (lane + 1) * step, hi);
+        const unsigned m = __ballot_sync(kFull, at < hi && __ldg(roff + at) <= p0);
+        const int k = __popc(m);
+        const int64_t nlo = lo + k * step;
+        hi = min(nlo + step, hi);
+        lo = nlo;
+    }
+    const uint32_t end = __ldg(roff + min(lo + 1 + lane, n));
+    const int own = owner_of((int)min(end - p0, 0x7fffffffu), (int)(p - p0));
+    return (int)min(lo + own, n - 1);
+}
+
+// ---------------------------------------------------------------------------
+// building
+
+__global__ void k_rank_keys2(const int32_t *deg, const int32_t *vgraph, const uint8_t *vmask, int64_t n,
+                             int32_t max_degree, int vb, uint64_t *keys) {
+    for (int64_t v = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; v < n; v += (int64_t)gridDim.x * blockDim.x) {
+        const int32_t d = vmask && vmask[vgraph[v]] ? 0 : deg[v];
+        keys[v] = ((uint64_t)(uint32_t)(max_degree - d) << vb) | (uint64_t)(n - 1 - v);
+    }
+}
+
+__global__ void k_rank_scatter2(const uint64_t *sorted, int64_t n, int32_t max_degree, int vb, int32_t *vrank,
+                                int32_t *rv, uint32_t *rdeg) {
+    for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i <= n; i += (int64_t)gridDim.x * blockDim.x) {
+        if (i == n) {
+            rdeg[n] = 0;
+            continue;
+        }
+        const uint64_t k = sorted[i];
+        const int32_t v = (int32_t)(n - 1 - (int64_t)(k & ((1ull << vb) - 1)));
+        vrank[v] = (int32_t)i;
+        rv[i] = v;
+        rdeg[i] = (uint32_t)(max_degree - (int32_t)(k >> vb));
+    }
+}
+
+// The entries in rank order of their row, each as (rank of the neighbour, rank
+// of the row): stably sorted by the first, the second ones are the rows of the
+// rank-ordered graph, ascending.
+__global__ void k_rank_entries(const uint32_t *roff, const int32_t *rv, const int64_t *off, const int32_t *adj,
+                               const int32_t *vrank, int64_t n, int64_t nnz, uint32_t *key, int32_t *val) {
+    const int lane = threadIdx.x & 31;
+    const int64_t stride = (int64_t)gridDim.x * blockDim.x;
+    for (int64_t p0 = blockIdx.x * (int64_t)blockDim.x + threadIdx.x - lane; p0 < nnz; p0 += stride) {
+        const int64_t p = min(p0 + lane, nnz - 1);
+        const int r = rows_of_warp(roff, n, (uint32_t)p0, (uint32_t)p, lane);
+        if (p0 + lane < nnz) {
+            key[p] = (uint32_t)vrank[adj[off[rv[r]] + (p - (int64_t)roff[r])]];
+            val[p] = r;
+        }
+    }
+}
+
+// Degree tiers and their counter addresses (one thread).
+__global__ void k_rank_tiers(const uint32_t *rdeg, const uint32_t *roff, int64_t n, RankMeta *M) {
+    const uint32_t lim[5] = {65536, 256, 16, 4, 2};
+    uint32_t c = 0, prev = 0;
+    for (int i = 0; i < 5; i++) {
+        int64_t lo = prev, hi = n;   // first rank of degree below lim[i]
+        while (lo < hi) {
+            const int64_t mid = (lo + hi) >> 1;
+            if (rdeg[mid] >= lim[i]) lo = mid + 1;
+            else hi = mid;
+        }
+        M->tier[i] = (uint32_t)lo;
+        c += ((uint32_t)lo - prev) << (5 - i);
+        M->tcode[i] = c;
+        prev = (uint32_t)lo;
+    }
+    M->max_up = 0;
+    M->entries2 = roff[prev];
+    M->direct_wedges = 0;
+    for (int i = 0; i < kClasses; i++) M->nlist[i] = 0;
+}
+
+// Range boundaries: `ranges` parts of about equal weight, a rank's weight being
+// half its share of the entries and half its share of the counter bits (so a
+// range holds at most 2 / ranges of the bits).
+__global__ void k_rank_bounds(const uint32_t *roff, int ranges, RankMeta *M) {
+    const uint32_t n2 = M->tier[4];
+    const double fe = 0.5 / (double)max(1u, roff[n2]), fb = 0.5 / (double)max(1u, M->tcode[4]);
+    for (int k = threadIdx.x; k <= ranges; k += blockDim.x) {
+        const double want = (double)k / ranges;
+        uint32_t lo = 0, hi = n2;   // first rank whose prefix weight reaches want
+        while (lo < hi) {
+            const uint32_t mid = lo + ((hi - lo) >> 1);
+            if (fe * roff[mid] + fb * code_of(M, mid) < want) lo = mid + 1;
+            else hi = mid;
+        }
+        M->bound[k] = k == 0 ? 0 : (k == ranges ? n2 : lo);
+    }
+}
+
+// Per slot: the entry's counter address; the row's count of entries above it;
+// and, from the side of the lower end, the slots of the two directions.
+__global__ void k_rank_slots(const uint32_t *roff, const int32_t *radj, int64_t n, int64_t nnz, RankMeta *M,
+                             uint32_t *wcode, int32_t *tw, int32_t *rup) {
+    const int lane = threadIdx.x & 31;
+    const int64_t stride = (int64_t)gridDim.x * blockDim.x;
+    for (int64_t p0 = blockIdx.x * (int64_t)blockDim.x + threadIdx.x - lane; p0 < nnz; p0 += stride) {
+        const int64_t p = min(p0 + lane, nnz - 1);
+        const int r = rows_of_warp(roff, n, (uint32_t)p0, (uint32_t)p, lane);
+        if (p0 + lane >= nnz) continue;
+        const int32_t x = radj[p];
+        wcode[p] = code_of(M, (uint32_t)x);
+        if (x < r) {
+            const uint32_t s = lower_bound_u(radj, roff[x], roff[x + 1], r);
+            tw[p] = (int32_t)s;
+            tw[s] = (int32_t)p;
+            if (p + 1 == (int64_t)roff[r + 1] || radj[p + 1] > r) {
+                const uint32_t up = (uint32_t)p + 1 - roff[r];
+                rup[r] = (int32_t)up;
+                if (up > 32) atomicMax(&M->max_up, up);
+            }
+        }
+    }
+}
+
+__global__ void k_rank_eslot(const int32_t *ev, const int32_t *eu, const int32_t *vrank, const uint32_t *roff,
+                             const int32_t *rup, const int32_t *radj, const int32_t *vgraph, const uint8_t *vmask,
+                             int64_t m, int32_t *eslot) {
+    for (int64_t e = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; e < m; e += (int64_t)gridDim.x * blockDim.x) {
+        const int32_t v = ev[e];
+        if (vmask && vmask[vgraph[v]]) {
+            eslot[e] = -1;
+            continue;
+        }
+        const int32_t a = vrank[v], b = vrank[eu[e]];
+        const int32_t r = max(a, b), x = min(a, b);
+        eslot[e] = (int32_t)lower_bound_u(radj, roff[r], roff[r] + (uint32_t)rup[r], x);
+    }
+}
+
+// First entry of degree 1 of each row (the vertices of degree 1 come last).
+__global__ void k_rank_bend(const uint32_t *roff, const int32_t *radj, int n2, uint32_t *bend) {
+    for (int64_t v = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; v < n2; v += (int64_t)gridDim.x * blockDim.x)
+        bend[v] = lower_bound_u(radj, roff[v], roff[v + 1], n2);
+}
+
+// First entry of each row at or beyond each inner range boundary.
+__global__ void k_rank_bpos(const uint32_t *roff, const int32_t *radj, int n2, int ranges, const RankMeta *M,
+                            uint32_t *bpos) {
+    const int64_t total = (int64_t)n2 * (ranges - 1);
+    for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < total; i += (int64_t)gridDim.x * blockDim.x) {
+        const int k = 1 + (int)(i / n2), v = (int)(i % n2);
+        bpos[i] = lower_bound_u(radj, roff[v], roff[v + 1], (int32_t)M->bound[k]);
+    }
+}
+
+// Wedges of every top vertex u (its lower neighbours' entries below u), with
+// one atomic per warp where its slots belong to one row.
+__global__ void k_rank_wedges(const uint32_t *roff, const int32_t *radj, const int32_t *tw, const uint32_t *bend,
+                              int64_t n, int n2, int64_t nnz2, uint32_t *wd) {
+    const int lane = threadIdx.x & 31;
+    const int64_t stride = (int64_t)gridDim.x * blockDim.x;
+    for (int64_t p0 = blockIdx.x * (int64_t)blockDim.x + threadIdx.x - lane; p0 < nnz2; p0 += stride) {
+        const int64_t p = min(p0 + lane, nnz2 - 1);
+        const int u = rows_of_warp(roff, n, (uint32_t)p0, (uint32_t)p, lane);
+        uint32_t c = 0;
+        const int32_t v = radj[p];
+        if (p0 + lane < nnz2 && v > u && v < n2) c = bend[v] - (uint32_t)tw[p] - 1;
+        const int u0 = __shfl_sync(kFull, u, 0);
+        if (__all_sync(kFull, u == u0)) {
+            c = __reduce_add_sync(kFull, c);
+            if (lane == 0 && c) atomicAdd(wd + u, c);
+        } else if (c) {
+            atomicAdd(wd + u, c);
+        }
+    }
+}
+
+__device__ __forceinline__ void list_append(bool in, int32_t v, int32_t *list, uint32_t *count, int lane) {
+    const unsigned m = __ballot_sync(kFull, in);
+    if (!m) return;
+    uint32_t at = 0;
+    if (lane == 0) at = atomicAdd(count, (uint32_t)__popc(m));
+    at = __shfl_sync(kFull, at, 0);
+    if (in) list[at + __popc(m & ((1u << lane) - 1))] = v;
+}
+
+// Every vertex into the lists of its classes.
+__global__ void k_rank_lists(const int32_t *rup, const uint32_t *wd, int n2, int32_t *lists, RankMeta *M) {
+    const int lane = threadIdx.x & 31;
+    const int64_t stride = (int64_t)gridDim.x * blockDim.x;
+    unsigned long long direct = 0;
+    for (int64_t x0 = blockIdx.x * (int64_t)blockDim.x + threadIdx.x - lane; x0 < n2; x0 += stride) {
+        const int64_t x = x0 + lane;
+        const int up = x < n2 ? rup[x] : 0;
+        const uint32_t w = x < n2 ? wd[x] : 0;
+        const int ec = up < 2 ? -1 : up <= kEgoMax[0] ? 0 : up <= kEgoMax[1] ? 1 : up <= kEgoMax[2] ? 2 : up <= kEgoMax[3] ? 3 : 4;
+#pragma unroll
+        for (int c = 0; c < kCycWarp; c++) list_append(ec == c, (int32_t)x, lists + (int64_t)c * n2, &M->nlist[c], lane);
+        list_append(w >= 2 && w <= kCycWarpMax, (int32_t)x, lists + (int64_t)kCycWarp * n2, &M->nlist[kCycWarp], lane);
+        list_append(w > kCycWarpMax && w <= kCycHashMax, (int32_t)x, lists + (int64_t)kCycHash * n2, &M->nlist[kCycHash],
+                    lane);
+        if (w > kCycHashMax) direct += w;
+    }
+    direct = pgd_warp_sum(direct);
+    if (lane == 0 && direct) atomicAdd(&M->direct_wedges, direct);
+}
+
+// Ranges [k, end) of u's next item: as many as its counters and its share of
+// the wedges allow (at least one).
+__device__ __forceinline__ int next_piece(const RankMeta *M, uint32_t u, int k, int ranges, int per_item) {
+    const uint32_t c0 = code_of(M, max(M->bound[k], u + 1)) & ~31u;
+    int e = k + 1;
+    while (e < ranges && e - k < per_item && (code_of(M, M->bound[e + 1]) - c0 + 31) / 32 <= kDirectWords) e++;
+    return e;
+}
+
+// Items of the vertices with many wedges: mode 0 counts them per vertex, mode 1
+// writes them.  A vertex whose wedges exceed a fixed part of all is split by
+// ranges of the wedge's end, so that no item keeps one block busy to the end.
+__global__ void k_rank_items(const uint32_t *wd, int n2, int ranges, const RankMeta *M, int parts,
+                             uint32_t *count, const uint32_t *pos, int2 *items) {
+    const unsigned long long target = max(65536ull, M->direct_wedges / (unsigned)parts);
+    for (int64_t x = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; x <= n2; x += (int64_t)gridDim.x * blockDim.x) {
+        uint32_t c = 0;
+        if (x < n2 && wd[x] > kCycHashMax) {
+            const uint32_t u = (uint32_t)x;
+            int k = 0;   // first range that reaches beyond u
+            while (k + 1 < ranges && M->bound[k + 1] <= u + 1) k++;
+            const int split = (int)min((unsigned long long)(ranges - k), wd[x] / target + 1);
+            const int per_item = (ranges - k + split - 1) / split;
+            while (k < ranges) {
+                const int e = next_piece(M, u, k, ranges, per_item);
+                if (items) items[pos[x] + c] = make_int2((int)u, k | (e << 16));
+                c++;
+                k = e;
+            }
+        }
+        if (count) count[x] = c;
+    }
+}
+
+// ---------------------------------------------------------------------------
+// 4-cycles
+
+struct CycArgs {
+    const uint32_t *roff;
+    const int32_t *rup;
+    const int32_t *radj;
+    const uint32_t *wcode;
+    const int32_t *tw;
+    const uint32_t *bend;
+    const uint32_t *bpos;
+    int n2;
+    int ranges;
+    const RankMeta *M;
+    const int32_t *list;
+    const int2 *items;
+    uint32_t count;
+    uint32_t grab;      // k_cycle_warp: vertices a warp takes at a time
+    unsigned long long *next;
+    uint32_t *cyc;      // per slot
+};
+
+// Shared scratch of a block's walk over the rows of up to NT middle vertices.
+template <int NT>
+struct Walk {
+    int pre[NT];          // inclusive prefix sums of the rows' lengths
+    uint32_t start[NT];   // first entry taken of each row
+    uint32_t acc[NT];     // what the second walk found for (u, v)
+    int wtot[NT / 32];
+};
+
+template <int NT>
+__device__ __forceinline__ int walk_search(const int *pre, int i) {   // first t with pre[t] > i
+    int lo = 0;
+#pragma unroll
+    for (int step = NT / 2; step > 0; step >>= 1)
+        if (pre[lo + step - 1] <= i) lo += step;
+    return lo;
+}
+
+// Applies fn(code, position) to every wedge end w of u in the ranges [k0, k1):
+// the rows of NT middle vertices v at a time are concatenated and every warp
+// takes an equal contiguous share, so short and long rows keep all lanes busy.
+// fn's results are added per v and, in the second walk (ACC), written to the
+// slot u -> v.  All threads of the block call; returns behind a barrier.
+template <int NT, bool ACC, typename Fn>
+__device__ __forceinline__ void walk_wedges(const CycArgs &A, Walk<NT> &W, uint32_t u, int k0, int k1, Fn fn) {
+    const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
+    const uint32_t j0 = A.roff[u] + (uint32_t)A.rup[u];
+    const uint32_t j1 = A.bend[u];
+    for (uint32_t c0 = j0; c0 < j1; c0 += NT) {
+        const uint32_t j = c0 + threadIdx.x;
+        int len = 0;
+        uint32_t s0 = 0;
+        if (j < j1) {
+            const int32_t v = __ldg(A.radj + j);
+            s0 = (uint32_t)__ldg(A.tw + j) + 1;
+            uint32_t e0 = __ldg(A.bend + v);
+            if (A.bpos) {
+                if (k1 < A.ranges) e0 = __ldg(A.bpos + (int64_t)(k1 - 1) * A.n2 + v);
+                if (k0 > 0) s0 = max(s0, __ldg(A.bpos + (int64_t)(k0 - 1) * A.n2 + v));
+            } else {
+                if (k1 < A.ranges) e0 = lower_bound_u(A.radj, s0, max(s0, e0), (int32_t)A.M->bound[k1]);
+                if (k0 > 0) s0 = lower_bound_u(A.radj, s0, max(s0, e0), (int32_t)A.M->bound[k0]);
+            }
+            len = e0 > s0 ? (int)(e0 - s0) : 0;
+        }
+        const int incl = pgd_warp_incl_scan(len);
+        if (lane == 31) W.wtot[wid] = incl;
+        __syncthreads();
+        const int wt = lane < NT / 32 ? W.wtot[lane] : 0;
+        const int wincl = pgd_warp_incl_scan(wt);
+        const int total = __shfl_sync(kFull, wincl, 31);
+        W.pre[threadIdx.x] = __shfl_sync(kFull, wincl - wt, wid) + incl;
+        W.start[threadIdx.x] = s0;
+        if (ACC) W.acc[threadIdx.x] = 0;
+        __syncthreads();
+        const int share = (total + NT / 32 - 1) / (NT / 32);
+        const int lo = min(total, wid * share), hi = min(total, lo + share);
+        int base = lo < hi ? walk_search<NT>(W.pre, lo) : 0;
+        for (int s = lo; s < hi;) {
+            const int own_end = min(W.pre[base], hi);
+            if (own_end - s >= 64) {
+                // one row covers the next entries: straight, four per lane
+                const uint32_t row0 = W.start[base] - (uint32_t)(base ? W.pre[base - 1] : 0);
+                uint32_t a = 0;
+                for (; s + 128 <= own_end; s += 128) {
+                    const uint32_t q = row0 + (uint32_t)(s + lane);
+                    const uint32_t w0 = __ldg(A.wcode + q), w1 = __ldg(A.wcode + q + 32), w2 = __ldg(A.wcode + q + 64),
+                                   w3 = __ldg(A.wcode + q + 96);
+                    a += fn(w0, q) + fn(w1, q + 32) + fn(w2, q + 64) + fn(w3, q + 96);
+                }
+                for (; s < own_end; s += 32) {
+                    const uint32_t q = row0 + (uint32_t)(s + lane);
+                    if (s + lane < own_end) a += fn(__ldg(A.wcode + q), q);
+                }
+                s = own_end;
+                if (ACC) {
+                    a = __reduce_add_sync(kFull, a);
+                    if (lane == 0 && a) atomicAdd(&W.acc[base], a);
+                }
+                if (s < hi) base = walk_search<NT>(W.pre, s);
+                continue;
+            }
+            const int cand = base + lane < NT ? W.pre[base + lane] : 0x7fffffff;
+            const int last = __shfl_sync(kFull, cand, 31);
+            const int iA = s + lane, iB = s + 32 + lane;
+            const bool vA = iA < hi, vB = iB < hi;
+            int ownA = base + owner_of(cand, iA), ownB = base + owner_of(cand, iB);
+            if (vA && iA >= last) ownA = walk_search<NT>(W.pre, iA);
+            if (vB && iB >= last) ownB = walk_search<NT>(W.pre, iB);
+            uint32_t qA = 0, qB = 0, wA = 0, wB = 0;
+            if (vA) {
+                qA = W.start[ownA] + (uint32_t)(iA - (ownA ? W.pre[ownA - 1] : 0));
+                wA = __ldg(A.wcode + qA);
+            }
+            if (vB) {
+                qB = W.start[ownB] + (uint32_t)(iB - (ownB ? W.pre[ownB - 1] : 0));
+                wB = __ldg(A.wcode + qB);
+            }
+            if (vA) {
+                const uint32_t a = fn(wA, qA);
+                if (ACC && a) atomicAdd(&W.acc[ownA], a);
+            }
+            if (vB) {
+                const uint32_t a = fn(wB, qB);
+                if (ACC && a) atomicAdd(&W.acc[ownB], a);
+            }
+            __syncwarp();
+            s += 64;
+            if (s < hi) base = min(__shfl_sync(kFull, ownB, 31), NT - 1);
+        }
+        __syncthreads();
+        if (ACC && j < j1) {
+            const uint32_t a = W.acc[threadIdx.x];
+            if (a) atomicAdd(A.cyc + j, a);
+        }
+        __syncthreads();
+    }
+}
+
+// Many wedges: one block per (u, ranges of w), a counter per w in shared
+// memory at its bit address.
+__global__ void __launch_bounds__(kDirectThreads, 1) k_cycle_direct(CycArgs A) {
+    extern __shared__ __align__(16) uint32_t s_dyn[];
+    __shared__ Walk<kDirectThreads> W;
+    __shared__ uint32_t s_item;
+    const RankMeta *M = A.M;
+    while (true) {
+        if (threadIdx.x == 0) s_item = (uint32_t)atomicAdd(A.next, 1ull);
+        __syncthreads();
+        const uint32_t item = s_item;
+        if (item >= A.count) break;
+        const int2 it = A.items[item];
+        const uint32_t u = (uint32_t)it.x;
+        const int k0 = it.y & 0xffff, k1 = it.y >> 16;
+        const uint32_t c0 = code_of(M, max(M->bound[k0], u + 1)) & ~31u;
+        const uint32_t words = (code_of(M, M->bound[k1]) - c0 + 31) / 32;
+        for (uint32_t i = threadIdx.x; i < words; i += kDirectThreads) s_dyn[i] = 0;
+        __syncthreads();
+        walk_wedges<kDirectThreads, false>(A, W, u, k0, k1, [&](uint32_t c, uint32_t) {
+            atomicAdd(s_dyn + ((c - c0) >> 5), 1u << (c & 31));
+            return 0u;
+        });
+        const uint32_t t0 = M->tcode[0], t1 = M->tcode[1], t2 = M->tcode[2], t3 = M->tcode[3];
+        walk_wedges<kDirectThreads, true>(A, W, u, k0, k1, [&](uint32_t c, uint32_t q) {
+            const uint32_t mask = c >= t2 ? (c < t3 ? 0xfu : 0x3u) : (c >= t1 ? 0xffu : (c >= t0 ? 0xffffu : kFull));
+            const uint32_t k = ((s_dyn[(c - c0) >> 5] >> (c & 31)) & mask) - 1;
+            if (k) atomicAdd(A.cyc + q, k);
+            return k;
+        });
+        __syncthreads();
+    }
+}
+
+// Hashed counters: open addressing, at most half full.
+__device__ __forceinline__ uint32_t hash_of(uint32_t key, int shift) { return (key * 0x9E3779B1u) >> shift; }
+
+__device__ __forceinline__ uint32_t hash_find_add(uint32_t *keys, uint32_t key, uint32_t mask, int shift) {
+    uint32_t h = hash_of(key, shift);
+    while (true) {
+        const uint32_t k = keys[h];
+        if (k == key) return h;
+        if (k == kFull) {
+            const uint32_t old = atomicCAS(keys + h, kFull, key);
+            if (old == kFull || old == key) return h;
+        }
+        h = (h + 1) & mask;
+    }
+}
+
+__device__ __forceinline__ uint32_t hash_find(const uint32_t *keys, uint32_t key, uint32_t mask, int shift) {
+    uint32_t h = hash_of(key, shift);
+    while (keys[h] != key) h = (h + 1) & mask;   // the key is in the table
+    return h;
+}
+
+constexpr int kHashThreads = 512;
+constexpr int kHashSlots = 2 * kCycHashMax;
+constexpr int kHashSmem = kHashSlots * 6 + (int)sizeof(Walk<kHashThreads>);
+
+// A middling number of wedges: one block per u, hashed 16-bit counters (a
+// counter holds at most kCycHashMax).
+__global__ void __launch_bounds__(kHashThreads, 4) k_cycle_hash(CycArgs A) {
+    constexpr int kSlots = kHashSlots;
+    extern __shared__ __align__(16) uint32_t s_dyn[];
+    uint32_t *s_key = s_dyn, *s_cnt = s_dyn + kSlots;
+    Walk<kHashThreads> &W = *(Walk<kHashThreads> *)(s_dyn + kSlots + kSlots / 2);
+    __shared__ uint32_t s_item;
+    while (true) {
+        if (threadIdx.x == 0) s_item = (uint32_t)atomicAdd(A.next, 1ull);
+        __syncthreads();
+        const uint32_t item = s_item;
+        if (item >= A.count) break;
+        const uint32_t u = (uint32_t)A.list[item];
+        for (int i = threadIdx.x; i < kSlots; i += kHashThreads) s_key[i] = kFull;
+        for (int i = threadIdx.x; i < kSlots / 2; i += kHashThreads) s_cnt[i] = 0;
+        __syncthreads();
+        constexpr int shift = 32 - 13;
+        static_assert(kSlots == 1 << 13, "hash width");
+        walk_wedges<kHashThreads, false>(A, W, u, 0, A.ranges, [&](uint32_t c, uint32_t) {
+            const uint32_t h = hash_find_add(s_key, c, kSlots - 1, shift);
+            atomicAdd(s_cnt + (h >> 1), 1u << ((h & 1) << 4));
+            return 0u;
+        });
+        walk_wedges<kHashThreads, true>(A, W, u, 0, A.ranges, [&](uint32_t c, uint32_t q) {
+            const uint32_t h = hash_find(s_key, c, kSlots - 1, shift);
+            const uint32_t k = ((s_cnt[h >> 1] >> ((h & 1) << 4)) & 0xffffu) - 1;
+            if (k) atomicAdd(A.cyc + q, k);
+            return k;
+        });
+        __syncthreads();
+    }
+}
+
+constexpr int kWarpThreads = 256;
+constexpr int kWarpSlots = 2 * kCycWarpMax;
+constexpr int kWarpWords = kWarpSlots + kWarpSlots / 2 + 32;   // keys, 16-bit counters, sums per row
+constexpr int kWarpSmem = kWarpThreads / 32 * kWarpWords * 4;
+static_assert(kWarpSlots == 1 << 10, "largest table of a warp");
+
+// Few wedges: one warp per u.
+__global__ void __launch_bounds__(kWarpThreads) k_cycle_warp(CycArgs A) {
+    extern __shared__ __align__(16) uint32_t s_dyn[];
+    const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
+    uint32_t *key = s_dyn + wid * kWarpWords, *cnt = key + kWarpSlots, *acc = cnt + kWarpSlots / 2;
+    const uint32_t *bend = A.bend;
+    while (true) {
+        uint32_t i0 = 0;
+        if (lane == 0) i0 = (uint32_t)atomicAdd(A.next, (unsigned long long)A.grab);
+        i0 = __shfl_sync(kFull, i0, 0);
+        if (i0 >= A.count) break;
+        const uint32_t i1 = min(i0 + A.grab, A.count);
+        for (uint32_t i = i0; i < i1; i++) {
+            const uint32_t u = (uint32_t)A.list[i];
+            const uint32_t j0 = A.roff[u] + (uint32_t)A.rup[u], j1 = bend[u];
+            int bits = 0;   // log2 of the table's slots, 0 until the first rows are known
+            for (int pass = 0; pass < 2; pass++) {
+                for (uint32_t c0 = j0; c0 < j1; c0 += 32) {
+                    const uint32_t j = c0 + lane;
+                    int len = 0;
+                    uint32_t s0 = 0;
+                    if (j < j1) {
+                        s0 = (uint32_t)__ldg(A.tw + j) + 1;
+                        len = (int)(__ldg(bend + __ldg(A.radj + j)) - s0);
+                    }
+                    const int incl = pgd_warp_incl_scan(len);
+                    const int total = __shfl_sync(kFull, incl, 31);
+                    if (!bits) {
+                        // all wedges within these rows: a table twice their number, else the largest
+                        bits = c0 + 32 >= j1 ? max(5, 33 - __clz(max(total, 2) - 1)) : 10;
+                        for (int k = lane; k < (1 << bits); k += 32) key[k] = kFull;
+                        for (int k = lane; k < (1 << bits) / 2; k += 32) cnt[k] = 0;
+                    }
+                    acc[lane] = 0;
+                    __syncwarp();
+                    const int off0 = (int)s0 - (incl - len);   // slot = off0 + flattened index
+                    const uint32_t mask = (1u << bits) - 1;
+                    const int shift = 32 - bits;
+                    for (int b = 0; b < total; b += 32) {
+                        const int it = b + lane;
+                        const int own = owner_of(incl, it) & 31;
+                        const int o = __shfl_sync(kFull, off0, own);
+                        if (it < total) {
+                            const uint32_t q = (uint32_t)(o + it);
+                            const uint32_t c = __ldg(A.wcode + q);
+                            if (pass == 0) {
+                                const uint32_t h = hash_find_add(key, c, mask, shift);
+                                atomicAdd(cnt + (h >> 1), 1u << ((h & 1) << 4));
+                            } else {
+                                const uint32_t h = hash_find(key, c, mask, shift);
+                                const uint32_t k = ((cnt[h >> 1] >> ((h & 1) << 4)) & 0xffffu) - 1;
+                                if (k) {
+                                    atomicAdd(A.cyc + q, k);
+                                    atomicAdd(acc + own, k);
+                                }
+                            }
+                        }
+                    }
+                    __syncwarp();
+                    if (pass == 1 && j < j1 && acc[lane]) atomicAdd(A.cyc + j, acc[lane]);
+                }
+            }
+            __syncwarp();
+        }
+    }
+}
+
+// ---------------------------------------------------------------------------
+// triangles (pass 1) and 4-cliques with the sums of t (pass 2)
+
+struct EgoArgs {
+    const uint32_t *roff;
+    const int32_t *rup;
+    const int32_t *radj;
+    const int32_t *list;
+    uint32_t count;
+    uint32_t grab;              // k_ego_warp: vertices a warp takes at a time
+    unsigned long long *next;
+    uint32_t *t;                // per slot of the lower end: triangles
+    unsigned long long *dk;     // per slot of the lower end: D << 32 | k4
+    uint2 *hits;                // pass 2: triangle list of each block ({i << 16 | j, slot x -> y})
+    int64_t hits_stride;
+    uint8_t *tables;            // kEgoGlobal: tables of each block
+    int64_t tables_stride;
+};
+
+// |N+(a)| = d <= 32: a warp per vertex.  The pairs (i, j), j < i, of N+(a) are
+// dealt to the lanes; y = N+(a)[j] is searched in N+(x), x = N+(a)[i].
+template <int PASS>
+__global__ void __launch_bounds__(kWarpThreads) k_ego_warp(EgoArgs A) {
+    constexpr int kPairs = 32 * 31 / 2;
+    constexpr int kW = kWarpThreads / 32;
+    __shared__ uint16_t s_pair[kPairs];
+    __shared__ uint32_t s_a[kW][32], s_b[kW][32], s_f[kW][32], s_t[kW][32];
+    __shared__ uint32_t s_slot[PASS == 2 ? kW : 1][PASS == 2 ? kPairs : 1];
+    __shared__ uint16_t s_hit[PASS == 2 ? kW : 1][PASS == 2 ? kPairs : 1];
+    const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
+    for (int i = 1 + (int)threadIdx.x; i < 32; i += kWarpThreads)
+        for (int j = 0; j < i; j++) s_pair[i * (i - 1) / 2 + j] = (uint16_t)(i << 8 | j);
+    __syncthreads();
+    uint32_t *ca = s_a[wid], *cb = s_b[wid], *f = s_f[wid], *ta = s_t[wid];
+    while (true) {
+        uint32_t i0 = 0;
+        if (lane == 0) i0 = (uint32_t)atomicAdd(A.next, (unsigned long long)A.grab);
+        i0 = __shfl_sync(kFull, i0, 0);
+        if (i0 >= A.count) break;
+        const uint32_t i1 = min(i0 + A.grab, A.count);
+        for (uint32_t ii = i0; ii < i1; ii++) {
+            const uint32_t a = (uint32_t)A.list[ii];
+            const int d = A.rup[a];
+            const uint32_t ra = A.roff[a];
+            int32_t x = 0;
+            uint32_t rx = 0;
+            int ux = 0;
+            if (lane < d) {
+                x = __ldg(A.radj + ra + lane);
+                rx = __ldg(A.roff + x);
+                ux = __ldg(A.rup + x);
+            }
+            ca[lane] = 0;
+            if (PASS == 2) {
+                cb[lane] = 0;
+                f[lane] = 0;
+                ta[lane] = lane < d ? A.t[ra + lane] : 0;
+            }
+            __syncwarp();
+            const int np = d * (d - 1) / 2;
+            int nh = 0;
+            for (int b = 0; b < np; b += 32) {
+                const bool act = b + lane < np;
+                const int pr = act ? s_pair[b + lane] : 0x0100;
+                const int i = pr >> 8, j = pr & 255;
+                const int32_t y = __shfl_sync(kFull, x, j);
+                const uint32_t r0 = __shfl_sync(kFull, rx, i);
+                const int ui = __shfl_sync(kFull, ux, i);
+                bool hit = false;
+                uint32_t pos = 0;
+                if (act) {
+                    pos = lower_bound_u(A.radj, r0, r0 + (uint32_t)ui, y);
+                    hit = pos < r0 + (uint32_t)ui && __ldg(A.radj + pos) == y;
+                }
+                if (PASS == 1) {
+                    if (hit) {
+                        atomicAdd(A.t + pos, 1u);
+                        atomicAdd(ca + i, 1u);
+                        atomicAdd(ca + j, 1u);
+                    }
+                } else {
+                    const unsigned m = __ballot_sync(kFull, hit);
+                    if (hit) {
+                        const int at = nh + __popc(m & ((1u << lane) - 1));
+                        s_slot[wid][at] = pos;
+                        s_hit[wid][at] = (uint16_t)pr;
+                        atomicOr(f + i, 1u << j);
+                        atomicOr(f + j, 1u << i);
+                    }
+                    nh += __popc(m);
+                }
+            }
+            __syncwarp();
+            if (PASS == 1) {
+                if (lane < d && ca[lane]) atomicAdd(A.t + ra + lane, ca[lane]);
+            } else {
+                for (int h = lane; h < nh; h += 32) {
+                    const uint32_t pos = s_slot[wid][h];
+                    const int i = s_hit[wid][h] >> 8, j = s_hit[wid][h] & 255;
+                    const uint32_t c = (uint32_t)__popc(f[i] & f[j]);
+                    const uint32_t tij = A.t[pos], ti = ta[i], tj = ta[j];
+                    atomicAdd(A.dk + pos, ((unsigned long long)(ti + tj) << 32) + c);
+                    atomicAdd(ca + i, c);
+                    atomicAdd(ca + j, c);
+                    atomicAdd(cb + i, tj + tij);
+                    atomicAdd(cb + j, ti + tij);
+                }
+                __syncwarp();
+                if (lane < d && (ca[lane] | cb[lane]))
+                    atomicAdd(A.dk + ra + lane, ((unsigned long long)cb[lane] << 32) + (ca[lane] >> 1));
+            }
+            __syncwarp();
+        }
+    }
+}
+
+// Table sizes of the block kernels for up to dmax neighbours.
+__host__ __device__ __forceinline__ int ego_hash_bits(int dmax) {   // a table at least 4 times as large
+    int b = 7;
+    while ((1 << b) < 4 * dmax) b++;
+    return b;
+}
+__host__ __device__ __forceinline__ int ego_row_words(int dmax) { return ((dmax + 63) / 64) | 1; }   // odd: rows spread over banks
+inline int64_t ego_table_bytes(int dmax, bool pass2) {
+    int64_t b = ((int64_t)6 << ego_hash_bits(dmax)) + (int64_t)dmax * 4 * 4;
+    if (pass2) b += (int64_t)dmax * 4 * 2 + (int64_t)dmax * 8 * ego_row_words(dmax);
+    return (b + 127) & ~(int64_t)127;
+}
+
+// |N+(a)| = d in a block's range: a block per vertex.  N+(a) goes into a hash
+// table rank -> index; each warp takes vertices x of N+(a) and looks the
+// entries of N+(x) up.
+template <int PASS, int NT, bool GLOBAL>
+__global__ void __launch_bounds__(NT) k_ego_block(EgoArgs A, int dmax) {
+    extern __shared__ __align__(16) uint32_t s_dyn[];
+    __shared__ uint32_t s_item;
+    __shared__ uint32_t s_nhit;
+    __shared__ int s_row;
+    const int lane = threadIdx.x & 31;
+    const int hb = ego_hash_bits(dmax), shift = 32 - hb;
+    const uint32_t hmask = (1u << hb) - 1;
+    uint8_t *base = GLOBAL ? A.tables + (int64_t)blockIdx.x * A.tables_stride : (uint8_t *)s_dyn;
+    // [F rows (64-bit)] keys, positions of N+(a)'s rows, their lengths, list, counts, (sums of t, t), indices (16-bit)
+    const int WS = ego_row_words(dmax);
+    unsigned long long *F = (unsigned long long *)base;
+    uint32_t *hkey = (uint32_t *)(base + (PASS == 2 ? (int64_t)dmax * 8 * WS : 0));
+    uint32_t *rs = hkey + (1 << hb);
+    int32_t *ru = (int32_t *)(rs + dmax);
+    int32_t *ls = ru + dmax;
+    uint32_t *ck = (uint32_t *)(ls + dmax);
+    uint32_t *cd = ck + dmax;                          // pass 2
+    uint32_t *ta = cd + (PASS == 2 ? dmax : 0);        // pass 2
+    uint16_t *hidx = (uint16_t *)(PASS == 2 ? ta + dmax : cd);
+    uint2 *hits = PASS == 2 ? A.hits + (int64_t)blockIdx.x * A.hits_stride : nullptr;
+    while (true) {
+        if (threadIdx.x == 0) {
+            s_item = (uint32_t)atomicAdd(A.next, 1ull);
+            s_nhit = 0;
+        }
+        __syncthreads();
+        const uint32_t item = s_item;
+        if (item >= A.count) break;
+        const uint32_t a = (uint32_t)A.list[item];
+        const int d = A.rup[a];
+        const uint32_t ra = A.roff[a];
+        const int W = (d + 63) >> 6;
+        if (threadIdx.x == 0) s_row = d - 1;
+        for (int i = threadIdx.x; i <= (int)hmask; i += NT) hkey[i] = kFull;
+        if (PASS == 2)
+            for (int i = threadIdx.x; i < d * WS; i += NT) F[i] = 0;
+        __syncthreads();
+        for (int i = threadIdx.x; i < d; i += NT) {
+            const int32_t x = __ldg(A.radj + ra + i);
+            ls[i] = x;
+            rs[i] = __ldg(A.roff + x);
+            ru[i] = __ldg(A.rup + x);
+            ck[i] = 0;
+            if (PASS == 2) {
+                cd[i] = 0;
+                ta[i] = A.t[ra + i];
+            }
+            uint32_t h = hash_of((uint32_t)x, shift);
+            while (atomicCAS(hkey + h, kFull, (uint32_t)x) != kFull) h = (h + 1) & hmask;
+            hidx[h] = (uint16_t)i;
+        }
+        __syncthreads();
+        while (true) {
+            int i = 0;
+            if (lane == 0) i = atomicSub(&s_row, 1);
+            i = __shfl_sync(kFull, i, 0);
+            if (i < 1) break;   // the first neighbour has none of the others above it
+            const uint32_t r0 = rs[i];
+            const int len = ru[i];
+            const int32_t last = ls[i - 1];
+            uint32_t found = 0;
+            for (int b = 0; b < len; b += 32) {
+                const int32_t y = b + lane < len ? __ldg(A.radj + r0 + b + lane) : 0x7fffffff;
+                bool hit = false;
+                int jx = 0;
+                if (y <= last) {
+                    uint32_t h = hash_of((uint32_t)y, shift);
+                    uint32_t k;
+                    while ((k = hkey[h]) != (uint32_t)y && k != kFull) h = (h + 1) & hmask;
+                    if (k == (uint32_t)y) {
+                        hit = true;
+                        jx = hidx[h];
+                    }
+                }
+                const unsigned m = __ballot_sync(kFull, hit);
+                if (m) {
+                    if (PASS == 1) {
+                        if (hit) {
+                            atomicAdd(A.t + r0 + b + lane, 1u);
+                            atomicAdd(ck + jx, 1u);
+                        }
+                        found += __popc(m);
+                    } else {
+                        uint32_t at = 0;
+                        if (lane == 0) at = atomicAdd(&s_nhit, (uint32_t)__popc(m));
+                        at = __shfl_sync(kFull, at, 0);
+                        if (hit) {
+                            hits[at + __popc(m & ((1u << lane) - 1))] =
+                                make_uint2((uint32_t)i << 16 | (uint32_t)jx, r0 + (uint32_t)(b + lane));
+                            atomicOr(F + (int64_t)i * WS + (jx >> 6), 1ull << (jx & 63));
+                            atomicOr(F + (int64_t)jx * WS + (i >> 6), 1ull << (i & 63));
+                        }
+                    }
+                }
+                if (__shfl_sync(kFull, y, 31) > last) break;   // ascending: nothing more at or below last
+            }
+            if (PASS == 1 && lane == 0 && found) atomicAdd(ck + i, found);
+        }
+        __syncthreads();
+        if (PASS == 2) {
+            const uint32_t nh = s_nhit;
+            for (uint32_t h0 = threadIdx.x - lane; h0 < nh; h0 += NT) {
+                const uint32_t h = h0 + lane;
+                uint32_t c = 0, di = 0;
+                int i = -1;
+                if (h < nh) {
+                    const uint2 e = hits[h];
+                    i = (int)(e.x >> 16);
+                    const int jx = (int)(e.x & 0xffff);
+                    const unsigned long long *fi = F + (int64_t)i * WS, *fj = F + (int64_t)jx * WS;
+                    for (int w = 0; w < W; w++) c += (uint32_t)__popcll(fi[w] & fj[w]);
+                    const uint32_t tij = A.t[e.y], ti = ta[i], tj = ta[jx];
+                    atomicAdd(A.dk + e.y, ((unsigned long long)(ti + tj) << 32) + c);
+                    if (c) atomicAdd(ck + jx, c);
+                    atomicAdd(cd + jx, ti + tij);
+                    di = tj + tij;
+                }
+                // most warps hold one x: reduce its sums first
+                const int i0 = __shfl_sync(kFull, i, 0);
+                if (__all_sync(kFull, i == i0 || i < 0)) {
+                    c = __reduce_add_sync(kFull, c);
+                    di = __reduce_add_sync(kFull, di);
+                    if (lane == 0) {
+                        if (c) atomicAdd(ck + i0, c);
+                        atomicAdd(cd + i0, di);
+                    }
+                } else if (i >= 0) {
+                    if (c) atomicAdd(ck + i, c);
+                    atomicAdd(cd + i, di);
+                }
+            }
+            __syncthreads();
+        }
+        for (int i = threadIdx.x; i < d; i += NT) {
+            if (PASS == 1) {
+                if (ck[i]) atomicAdd(A.t + ra + i, ck[i]);
+            } else if (ck[i] | cd[i]) {
+                atomicAdd(A.dk + ra + i, ((unsigned long long)cd[i] << 32) + (ck[i] >> 1));
+            }
+        }
+        __syncthreads();
+    }
+}
+
+// ---------------------------------------------------------------------------
+// closing: t, k4, c4 of each position, its closed forms and its row
+
+struct CloseArgs {
+    pgd_rank_out o;
+    const int32_t *eslot;
+    const int32_t *tw;
+    const uint32_t *t;
+    const unsigned long long *dk;
+    const uint32_t *cyc;
+};
+
+__device__ __forceinline__ void flush_warp(unsigned long long *acc, unsigned long long *dst, int lane) {
+#pragma unroll
+    for (int i = 0; i < PGD_NSUMS; i++) {
+        const unsigned long long v = pgd_warp_sum(acc[i]);
+        if (lane == 0 && v) atomicAdd(dst + i, v);
+        acc[i] = 0;
+    }
+}
+
+// A warp takes a contiguous part of the positions, 32 at a time; in a batch
+// they belong to few graphs, whose sums are flushed when the graph changes.
+__global__ void __launch_bounds__(kThreads) k_rank_close(CloseArgs A) {
+    const pgd_rank_out &o = A.o;
+    const int lane = threadIdx.x & 31;
+    const int64_t nw = ((int64_t)gridDim.x * blockDim.x) >> 5;
+    const int64_t w = (blockIdx.x * (int64_t)blockDim.x + threadIdx.x) >> 5;
+    const int64_t steps = (o.npos + 31) / 32, per = (steps + nw - 1) / nw;
+    const int64_t e1 = min(o.npos, (w + 1) * per * 32);
+    unsigned long long acc[PGD_NSUMS];
+#pragma unroll
+    for (int i = 0; i < PGD_NSUMS; i++) acc[i] = 0;
+    int cur = -1;   // graph of the sums held (batch)
+    long long n = o.n, m = o.m;
+    for (int64_t e0 = w * per * 32; e0 < e1; e0 += 32) {
+        const int64_t e = e0 + lane;
+        bool act = e < e1;
+        int g = 0;
+        if (o.egraph) {
+            if (act) g = o.egraph[e];
+            if (act && o.gdense && o.gdense[g]) act = false;
+        }
+        long long dv = 0, du = 0;
+        unsigned long long t = 0, k4 = 0, c4 = 0;
+        if (act) {
+            const int32_t id = o.order[e];
+            const int32_t j = __ldg(A.eslot + id);
+            dv = __ldg(o.deg + __ldg(o.ev + id));
+            du = __ldg(o.deg + __ldg(o.eu + id));
+            const uint32_t tt = __ldg(A.t + j);
+            const unsigned long long x = __ldg(A.dk + j);
+            const uint32_t cc = __ldg(A.cyc + j) + __ldg(A.cyc + __ldg(A.tw + j));
+            t = tt;
+            k4 = (uint32_t)x;
+            c4 = cc - (uint32_t)(x >> 32) + 2 * tt + 2 * (uint32_t)x;
+        }
+        unsigned todo = __ballot_sync(kFull, act);
+        while (todo) {
+            const int g0 = o.egraph ? __shfl_sync(kFull, g, __ffs(todo) - 1) : 0;
+            if (o.egraph && g0 != cur) {
+                if (cur >= 0) flush_warp(acc, o.sums + (int64_t)cur * PGD_NSUMS, lane);
+                cur = g0;
+                n = o.gnm[2 * (int64_t)g0];
+                m = o.gnm[2 * (int64_t)g0 + 1];
+            }
+            const bool mine = act && (!o.egraph || g == g0);
+            if (mine) {
+                pgd_edge_sums(acc, dv, du, t, m, n);
+                acc[3] += k4;
+                acc[4] += c4;
+            }
+            todo &= ~__ballot_sync(kFull, mine);
+        }
+        if (act && o.micro) {
+            ulonglong2 *row = (ulonglong2 *)(o.micro + e * PGD_NMICRO);
+#pragma unroll
+            for (int c = 0; c < PGD_NMICRO; c += 2) {
+                ulonglong2 v;
+                v.x = pgd_micro_col(c, dv, du, t, k4, c4);
+                v.y = pgd_micro_col(c + 1, dv, du, t, k4, c4);
+                row[c / 2] = v;
+            }
+        }
+    }
+    if (o.egraph) {
+        if (cur >= 0) flush_warp(acc, o.sums + (int64_t)cur * PGD_NSUMS, lane);
+        return;
+    }
+    __shared__ unsigned long long red[kThreads / 32][PGD_NSUMS];
+#pragma unroll
+    for (int i = 0; i < PGD_NSUMS; i++) {
+        const unsigned long long v = pgd_warp_sum(acc[i]);
+        if (lane == 0) red[threadIdx.x >> 5][i] = v;
+    }
+    __syncthreads();
+    if (threadIdx.x < PGD_NSUMS) {
+        unsigned long long s = 0;
+        for (int i = 0; i < kThreads / 32; i++) s += red[i][threadIdx.x];
+        if (s) atomicAdd(o.sums + threadIdx.x, s);
+    }
+}
+
+// Stream-ordered temporaries released on every return path.
+struct Tmp {
+    pgd_ctx *ctx;
+    void *held[16];   // more than any caller takes
+    int k = 0;
+    explicit Tmp(pgd_ctx *c) : ctx(c) {}
+    Tmp(const Tmp &) = delete;
+    Tmp &operator=(const Tmp &) = delete;
+    ~Tmp() {
+        while (k) pgd_tmp_free(ctx, held[--k]);
+    }
+    template <typename T>
+    pgd_status alloc(T **out, size_t bytes) {
+        void *p = nullptr;
+        const pgd_status st = pgd_tmp_alloc(ctx, &p, bytes);
+        if (st == PGD_OK) {
+            held[k++] = p;
+            *out = (T *)p;
+        }
+        return st;
+    }
+};
+
+}  // namespace
+
+// ---------------------------------------------------------------------------
+
+void pgd_rank_free(pgd_graph *g, pgd_rank_graph *R) {
+    while (R->nheld) {
+        R->nheld--;
+        pgd_graph_free(g, R->held[R->nheld], R->held_bytes[R->nheld]);
+    }
+    *R = pgd_rank_graph();
+}
+
+void pgd_rank_drop(pgd_graph *g) {
+    if (!g->ranked) return;
+    pgd_rank_free(g, g->ranked);
+    delete g->ranked;
+    g->ranked = nullptr;
+}
+
+#define RB_TRY(expr)                   \
+    do {                               \
+        if ((st = (expr)) != PGD_OK) { \
+            pgd_rank_free(g, R);       \
+            return st;                 \
+        }                              \
+    } while (0)
+#define RB_CUDA(call)                                     \
+    do {                                                  \
+        const cudaError_t e__ = (call);                   \
+        if (e__ != cudaSuccess) {                         \
+            pgd_rank_free(g, R);                          \
+            return pgd_cuda_fail(ctx, e__, #call);        \
+        }                                                 \
+    } while (0)
+
+pgd_status pgd_rank_build(pgd_graph *g, int64_t nnz, const int32_t *vgraph, const uint8_t *vmask, pgd_rank_graph *R) {
+    pgd_ctx *ctx = g->ctx;
+    cudaStream_t s = ctx->stream;
+    pgd_status st;
+    const int64_t n = g->n, m = g->m;
+    *R = pgd_rank_graph();
+    R->n = n;
+    R->nnz = nnz;
+    if (nnz == 0) return PGD_OK;
+    auto keep = [&](auto **p, size_t bytes) -> pgd_status {
+        const pgd_status e = pgd_graph_alloc(g, (void **)p, bytes);
+        if (e == PGD_OK) {
+            R->held[R->nheld] = *p;
+            R->held_bytes[R->nheld++] = bytes;
+        }
+        return e;
+    };
+    RB_TRY(keep(&R->roff, (n + 1) * sizeof(uint32_t)));
+    RB_TRY(keep(&R->rup, n * sizeof(int32_t)));
+    RB_TRY(keep(&R->radj, nnz * sizeof(int32_t)));
+    RB_TRY(keep(&R->wcode, nnz * sizeof(uint32_t)));
+    RB_TRY(keep(&R->tw, nnz * sizeof(int32_t)));
+    RB_TRY(keep(&R->eslot, m * sizeof(int32_t)));
+    RB_TRY(keep(&R->meta, sizeof(RankMeta)));
+    RankMeta *M = (RankMeta *)R->meta;
+    Tmp tg(ctx);
+    uint64_t *keys = nullptr, *keys2 = nullptr;
+    int32_t *vrank = nullptr, *rv = nullptr, *val = nullptr;
+    uint32_t *rdeg = nullptr, *key = nullptr, *key2 = nullptr;
+    RB_TRY(tg.alloc(&keys, n * sizeof(uint64_t)));
+    RB_TRY(tg.alloc(&keys2, n * sizeof(uint64_t)));
+    RB_TRY(tg.alloc(&vrank, n * sizeof(int32_t)));
+    RB_TRY(tg.alloc(&rv, n * sizeof(int32_t)));
+    RB_TRY(tg.alloc(&rdeg, (n + 1) * sizeof(uint32_t)));
+    RB_TRY(tg.alloc(&key, nnz * sizeof(uint32_t)));
+    RB_TRY(tg.alloc(&key2, nnz * sizeof(uint32_t)));
+    RB_TRY(tg.alloc(&val, nnz * sizeof(int32_t)));
+    const int vb = bits_for(n), db = bits_for((int64_t)g->max_degree + 1);
+    size_t tb1 = 0, tb2 = 0, tb3 = 0;
+    cub::DeviceRadixSort::SortKeys(nullptr, tb1, keys, keys2, n, 0, vb + db, s);
+    cub::DeviceScan::ExclusiveSum(nullptr, tb2, rdeg, R->roff, n + 1, s);
+    cub::DeviceRadixSort::SortPairs(nullptr, tb3, key, key2, val, R->radj, nnz, 0, vb, s);
+    size_t tb = std::max(tb1, std::max(tb2, tb3));
+    void *tmp = nullptr;
+    RB_TRY(tg.alloc(&tmp, tb));
+    // ranks, row offsets and tiers
+    PGD_LAUNCH(ctx, k_rank_keys2, grid_for(n), kThreads, 0, g->deg, vgraph, vmask, n, g->max_degree, vb, keys);
+    RB_CUDA(cub::DeviceRadixSort::SortKeys(tmp, tb, keys, keys2, n, 0, vb + db, s));
+    PGD_LAUNCH(ctx, k_rank_scatter2, grid_for(n + 1), kThreads, 0, keys2, n, g->max_degree, vb, vrank, rv, rdeg);
+    RB_CUDA(cub::DeviceScan::ExclusiveSum(tmp, tb, rdeg, R->roff, n + 1, s));
+    PGD_LAUNCH(ctx, k_rank_tiers, 1, 1, 0, rdeg, R->roff, n, M);
+    // rows in rank order
+    PGD_LAUNCH(ctx, k_rank_entries, grid_for(nnz), kThreads, 0, R->roff, rv, g->off, g->adj, vrank, n, nnz, key, val);
+    RB_CUDA(cub::DeviceRadixSort::SortPairs(tmp, tb, key, key2, val, R->radj, nnz, 0, vb, s));
+    RB_CUDA(cudaMemsetAsync(R->rup, 0, n * sizeof(int32_t), s));
+    PGD_LAUNCH(ctx, k_rank_slots, grid_for(nnz), kThreads, 0, R->roff, R->radj, n, nnz, M, R->wcode, R->tw, R->rup);
+    PGD_LAUNCH(ctx, k_rank_eslot, grid_for(m), kThreads, 0, g->ev, g->eu, vrank, R->roff, R->rup, R->radj, vgraph,
+               vmask, m, R->eslot);
+    RankMeta h;
+    constexpr size_t kHead = offsetof(RankMeta, bound);
+    RB_CUDA(cudaMemcpyAsync(&h, M, kHead, cudaMemcpyDeviceToHost, s));
+    RB_CUDA(cudaStreamSynchronize(s));
+    R->n2 = (int32_t)h.tier[4];
+    R->max_up = (int32_t)std::max((uint32_t)kEgoMax[kEgoWarp], h.max_up);
+    if (R->n2 == 0) return PGD_OK;
+    // wedges per vertex and the work lists
+    const int n2 = R->n2;
+    uint32_t *wd = nullptr;
+    RB_TRY(tg.alloc(&wd, n2 * sizeof(uint32_t)));
+    RB_TRY(keep(&R->bend, n2 * sizeof(uint32_t)));
+    RB_TRY(keep(&R->lists, (size_t)kClasses * n2 * sizeof(int32_t)));
+    RB_CUDA(cudaMemsetAsync(wd, 0, n2 * sizeof(uint32_t), s));
+    PGD_LAUNCH(ctx, k_rank_bend, grid_for(n2), kThreads, 0, R->roff, R->radj, n2, R->bend);
+    PGD_LAUNCH(ctx, k_rank_wedges, grid_for(h.entries2), kThreads, 0, R->roff, R->radj, R->tw, R->bend, n, n2,
+               (int64_t)h.entries2, wd);
+    PGD_LAUNCH(ctx, k_rank_lists, grid_for(n2), kThreads, 0, R->rup, wd, n2, R->lists, M);
+    RB_CUDA(cudaMemcpyAsync(&h, M, kHead, cudaMemcpyDeviceToHost, s));
+    RB_CUDA(cudaStreamSynchronize(s));
+    for (int i = 0; i < kClasses; i++) R->nlist[i] = h.nlist[i];
+    if (h.direct_wedges == 0) return PGD_OK;
+    // items of the vertices with many wedges, by ranges of the wedges' ends:
+    // fine enough to balance the items, and at most half an item's counters each
+    const int64_t words = ((int64_t)h.tcode[4] + 31) / 32;
+    R->nranges = (int32_t)std::min<int64_t>(kMaxRanges, std::max<int64_t>(16, 2 * (2 * words / kDirectWords + 1)));
+    PGD_LAUNCH(ctx, k_rank_bounds, 1, 128, 0, R->roff, R->nranges, M);
+    const int64_t bpos_bytes = (int64_t)(R->nranges - 1) * n2 * (int64_t)sizeof(uint32_t);
+    if (bpos_bytes <= kBposBytes) {
+        RB_TRY(keep(&R->bpos, (size_t)bpos_bytes));
+        PGD_LAUNCH(ctx, k_rank_bpos, grid_for((int64_t)n2 * (R->nranges - 1)), kThreads, 0, R->roff, R->radj, n2,
+                   R->nranges, M, R->bpos);
+    }
+    uint32_t *count = nullptr, *pos = nullptr;
+    RB_TRY(tg.alloc(&count, ((size_t)n2 + 1) * sizeof(uint32_t)));
+    RB_TRY(tg.alloc(&pos, ((size_t)n2 + 1) * sizeof(uint32_t)));
+    const int parts = ctx->num_sms * 8;
+    PGD_LAUNCH(ctx, k_rank_items, grid_for(n2 + 1), kThreads, 0, wd, n2, R->nranges, M, parts, count,
+               (const uint32_t *)nullptr, (int2 *)nullptr);
+    RB_CUDA(cub::DeviceScan::ExclusiveSum(tmp, tb, count, pos, (int64_t)n2 + 1, s));
+    RB_CUDA(cudaMemcpyAsync(&R->nitems, pos + n2, sizeof(uint32_t), cudaMemcpyDeviceToHost, s));
+    RB_CUDA(cudaStreamSynchronize(s));
+    RB_TRY(keep(&R->items, (size_t)R->nitems * sizeof(int2)));
+    PGD_LAUNCH(ctx, k_rank_items, grid_for(n2 + 1), kThreads, 0, wd, n2, R->nranges, M, parts, (uint32_t *)nullptr,
+               (const uint32_t *)pos, R->items);
+    RB_CUDA(cudaGetLastError());
+    return PGD_OK;
+}
+
+// Vertices a warp takes from a list at a time: one while there are warps to
+// spare (a short list then spreads over the whole device), else four.
+static uint32_t grab_for(const pgd_ctx *ctx, uint32_t count) { return count > 64u * (uint32_t)ctx->num_sms ? 4 : 1; }
+
+static int warp_blocks(const pgd_ctx *ctx, uint32_t count, uint32_t grab, int per_sm) {
+    const int64_t per_block = (int64_t)(kWarpThreads / 32) * grab;
+    return (int)std::min<int64_t>((count + per_block - 1) / per_block, (int64_t)per_sm * ctx->num_sms);
+}
+
+// Blocks per SM of a block class, and whether the class has so few vertices
+// that each gets a block of 1024 threads (at most two waves of them): a short
+// list is bound by its largest vertex, not by the device.
+static int ego_blocks_per_sm(int c) { return c == kEgoA ? 8 : c == kEgoB ? 3 : 1; }
+static bool ego_wide(const pgd_ctx *ctx, const pgd_rank_graph &R, int c) {
+    return R.nlist[c] <= 2u * (uint32_t)ctx->num_sms;
+}
+static int ego_grid(const pgd_ctx *ctx, const pgd_rank_graph &R, int c) {
+    return (int)std::min<int64_t>(R.nlist[c], (int64_t)(ego_wide(ctx, R, c) ? 2 : ego_blocks_per_sm(c)) * ctx->num_sms);
+}
+
+// The ego classes' launches of one pass.
+template <int PASS>
+static void ego_pass(pgd_ctx *ctx, const pgd_rank_graph &R, EgoArgs A, unsigned long long *ctr, uint2 *hits,
+                     uint8_t *tables, int gblocks, int64_t table_bytes) {
+    auto args = [&](int c) {
+        EgoArgs B = A;
+        B.list = R.lists + (int64_t)c * R.n2;
+        B.count = R.nlist[c];
+        B.next = ctr + c;
+        return B;
+    };
+    if (R.nlist[kEgoGlobal]) {
+        EgoArgs B = args(kEgoGlobal);
+        B.hits = hits;
+        B.hits_stride = (int64_t)R.max_up * (R.max_up - 1) / 2;
+        B.tables = tables;
+        B.tables_stride = table_bytes;
+        PGD_LAUNCH(ctx, (k_ego_block<PASS, 1024, true>), gblocks, 1024, 0, B, R.max_up);
+    }
+    for (int c : {kEgoC, kEgoB, kEgoA}) {
+        if (!R.nlist[c]) continue;
+        EgoArgs B = args(c);
+        const int dmax = std::min(kEgoMax[c], (int)R.max_up);
+        B.hits = hits;
+        B.hits_stride = (int64_t)dmax * (dmax - 1) / 2;
+        const int blocks = ego_grid(ctx, R, c);
+        const size_t smem = (size_t)ego_table_bytes(dmax, PASS == 2);
+        if (c == kEgoC || ego_wide(ctx, R, c)) PGD_LAUNCH(ctx, (k_ego_block<PASS, 1024, false>), blocks, 1024, smem, B, dmax);
+        else if (c == kEgoB) PGD_LAUNCH(ctx, (k_ego_block<PASS, 512, false>), blocks, 512, smem, B, dmax);
+        else PGD_LAUNCH(ctx, (k_ego_block<PASS, 256, false>), blocks, 256, smem, B, dmax);
+    }
+    if (R.nlist[kEgoWarp]) {
+        EgoArgs B = args(kEgoWarp);
+        B.grab = grab_for(ctx, B.count);
+        PGD_LAUNCH(ctx, k_ego_warp<PASS>, warp_blocks(ctx, B.count, B.grab, 8), kWarpThreads, 0, B);
+    }
+}
+
+// Shared-memory limits of the kernels that use more than the default, set to
+// the same values by every caller.
+static cudaError_t rank_kernel_limits() {
+    cudaError_t e = cudaFuncSetAttribute(k_cycle_direct, cudaFuncAttributeMaxDynamicSharedMemorySize, kDirectWords * 4);
+    if (e == cudaSuccess) e = cudaFuncSetAttribute(k_cycle_hash, cudaFuncAttributeMaxDynamicSharedMemorySize, kHashSmem);
+    if (e == cudaSuccess) e = cudaFuncSetAttribute(k_cycle_warp, cudaFuncAttributeMaxDynamicSharedMemorySize, kWarpSmem);
+    const int b2 = (int)ego_table_bytes(kEgoMax[kEgoB], true), c1 = (int)ego_table_bytes(kEgoMax[kEgoC], false),
+              c2 = (int)ego_table_bytes(kEgoMax[kEgoC], true);
+    if (e == cudaSuccess) e = cudaFuncSetAttribute(k_ego_block<2, 512, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, b2);
+    if (e == cudaSuccess) e = cudaFuncSetAttribute(k_ego_block<1, 1024, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, c1);
+    if (e == cudaSuccess) e = cudaFuncSetAttribute(k_ego_block<2, 1024, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, c2);
+    return e;
+}
+
+// Runs the 4-cycle kernels on the context's second stream, beside the triangle
+// passes; the first stream waits for it before anything they used is freed.
+struct SideStream {
+    pgd_ctx *ctx;
+    cudaStream_t main;
+    bool forked = false;
+    explicit SideStream(pgd_ctx *c) : ctx(c), main(c->stream) {}
+    cudaError_t fork() {
+        cudaError_t e = cudaEventRecord(ctx->ev_fork, main);
+        if (e == cudaSuccess) e = cudaStreamWaitEvent(ctx->side, ctx->ev_fork, 0);
+        forked = e == cudaSuccess;
+        return e;
+    }
+    cudaError_t join() {
+        if (!forked) return cudaSuccess;
+        forked = false;
+        cudaError_t e = cudaEventRecord(ctx->ev_join, ctx->side);
+        if (e == cudaSuccess) e = cudaStreamWaitEvent(main, ctx->ev_join, 0);
+        return e;
+    }
+    ~SideStream() {
+        ctx->stream = main;
+        join();
+    }
+};
+
+static pgd_status cycle_pass(pgd_ctx *ctx, const pgd_rank_graph &R, CycArgs C, unsigned long long *ctr) {
+    const int nsm = ctx->num_sms;
+    PGD_CUDA(ctx, cudaEventRecord(ctx->evh0, ctx->stream));
+    if (R.nitems) {
+        CycArgs B = C;
+        B.items = R.items;
+        B.count = R.nitems;
+        B.next = ctr;
+        PGD_LAUNCH(ctx, k_cycle_direct, (int)std::min<int64_t>(R.nitems, nsm), kDirectThreads, kDirectWords * 4, B);
+    }
+    if (R.nlist[kCycHash]) {
+        CycArgs B = C;
+        B.list = R.lists + (int64_t)kCycHash * R.n2;
+        B.count = R.nlist[kCycHash];
+        B.next = ctr + 1;
+        PGD_LAUNCH(ctx, k_cycle_hash, (int)std::min<int64_t>(B.count, 4 * (int64_t)nsm), kHashThreads, kHashSmem, B);
+    }
+    if (R.nlist[kCycWarp]) {
+        CycArgs B = C;
+        B.list = R.lists + (int64_t)kCycWarp * R.n2;
+        B.count = R.nlist[kCycWarp];
+        B.grab = grab_for(ctx, B.count);
+        B.next = ctr + 2;
+        PGD_LAUNCH(ctx, k_cycle_warp, warp_blocks(ctx, B.count, B.grab, 4), kWarpThreads, kWarpSmem, B);
+    }
+    PGD_CUDA(ctx, cudaEventRecord(ctx->evh1, ctx->stream));
+    PGD_CUDA(ctx, cudaGetLastError());
+    return PGD_OK;
+}
+
+pgd_status pgd_rank_decompose(pgd_ctx *ctx, const pgd_rank_graph &R, const pgd_rank_out &out) {
+    cudaStream_t s = ctx->stream;
+    pgd_status st;
+    if (out.npos == 0 || R.nnz == 0) return PGD_OK;
+    const int nsm = ctx->num_sms;
+    PGD_CUDA(ctx, rank_kernel_limits());
+    // triangle lists (pass 2) and the tables of the largest neighbourhoods
+    int64_t hit_count = 0, table_bytes = 0;
+    int gblocks = 0;
+    for (int c : {kEgoA, kEgoB, kEgoC}) {
+        const int64_t dmax = std::min(kEgoMax[c], (int)R.max_up);
+        hit_count = std::max(hit_count, ego_grid(ctx, R, c) * (dmax * (dmax - 1) / 2));
+    }
+    if (R.nlist[kEgoGlobal]) {
+        const int64_t per = (int64_t)R.max_up * (R.max_up - 1) / 2;
+        table_bytes = ego_table_bytes(R.max_up, true);
+        // at most about 8 GB of tables and lists, at least one block's
+        gblocks = (int)std::max<int64_t>(1, std::min<int64_t>(std::min<int64_t>(nsm, R.nlist[kEgoGlobal]),
+                                                              (8ll << 30) / (per * 8 + table_bytes)));
+        hit_count = std::max(hit_count, per * gblocks);
+    }
+    // one block: counters, dk, t, cyc (zeroed), then the lists and tables
+    constexpr int kCounters = 16;   // [0..5) pass 1, [5..10) pass 2, [10..13) 4-cycles
+    const size_t zeroed = kCounters * 8 + (size_t)R.nnz * 16, zeroed_up = (zeroed + 127) & ~(size_t)127;
+    Tmp tg(ctx);
+    uint8_t *work = nullptr;
+    if ((st = tg.alloc(&work, zeroed_up + (size_t)hit_count * sizeof(uint2) + (size_t)gblocks * table_bytes + 128)))
+        return st;
+    unsigned long long *ctr = (unsigned long long *)work, *dk = ctr + kCounters;
+    uint32_t *t = (uint32_t *)(dk + R.nnz), *cyc = t + R.nnz;
+    uint2 *hits = (uint2 *)(work + zeroed_up);
+    uint8_t *tables = (uint8_t *)(((uintptr_t)(hits + hit_count) + 127) & ~(uintptr_t)127);
+    PGD_CUDA(ctx, cudaMemsetAsync(work, 0, zeroed, s));
+    SideStream side(ctx);   // joined before tg frees
+    PGD_CUDA(ctx, side.fork());
+    CycArgs C{};
+    C.roff = R.roff;
+    C.rup = R.rup;
+    C.radj = R.radj;
+    C.wcode = R.wcode;
+    C.tw = R.tw;
+    C.bend = R.bend;
+    C.bpos = R.bpos;
+    C.n2 = R.n2;
+    C.ranges = R.nranges;
+    C.M = (const RankMeta *)R.meta;
+    C.cyc = cyc;
+    ctx->stream = ctx->side;
+    st = cycle_pass(ctx, R, C, ctr + 10);
+    ctx->stream = s;
+    if (st) return st;
+    EgoArgs E{};
+    E.roff = R.roff;
+    E.rup = R.rup;
+    E.radj = R.radj;
+    E.t = t;
+    E.dk = dk;
+    PGD_CUDA(ctx, cudaEventRecord(ctx->evt0, s));
+    ego_pass<1>(ctx, R, E, ctr, hits, tables, gblocks, table_bytes);
+    ego_pass<2>(ctx, R, E, ctr + 5, hits, tables, gblocks, table_bytes);
+    PGD_CUDA(ctx, cudaEventRecord(ctx->evt1, s));
+    PGD_CUDA(ctx, side.join());
+    CloseArgs Z;
+    Z.o = out;
+    Z.eslot = R.eslot;
+    Z.tw = R.tw;
+    Z.t = t;
+    Z.dk = dk;
+    Z.cyc = cyc;
+    PGD_LAUNCH(ctx, k_rank_close, (int)std::min<int64_t>(grid_for(out.npos), 8 * (int64_t)nsm), kThreads, 0, Z);
+    PGD_CUDA(ctx, cudaGetLastError());
+    return PGD_OK;
+}
