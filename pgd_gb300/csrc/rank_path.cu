@@ -76,6 +76,7 @@ constexpr int kEgoMax[] = {32, 256, 512, 1024};
 constexpr int kCycWarpMax = 512;
 constexpr int kCycHashMax = 4096;
 constexpr int kMaxRanges = 8192;
+constexpr int64_t kKeepBytes = 16ll << 30;     // largest bound of the triangle lists kept between the passes
 constexpr int64_t kBposBytes = 4ll << 30;      // largest table of range boundaries per row
 constexpr int kDirectThreads = 1024;
 constexpr uint32_t kDirectWords = 50 * 1024;   // counter words of one item: 200 KB of shared memory
@@ -88,6 +89,7 @@ struct RankMeta {
     uint32_t entries2;       // entries of the rows of vertices of degree >= 2
     uint32_t nlist[kClasses];
     unsigned long long direct_wedges;   // wedges of the vertices beyond the lists
+    unsigned long long pairs;           // sum of |N+(a)| (|N+(a)| - 1) / 2
     uint32_t bound[kMaxRanges + 1];   // range boundaries (ranks)
 };
 
@@ -213,6 +215,7 @@ __global__ void k_rank_tiers(const uint32_t *rdeg, const uint32_t *roff, int64_t
     M->max_up = 0;
     M->entries2 = roff[prev];
     M->direct_wedges = 0;
+    M->pairs = 0;
     for (int i = 0; i < kClasses; i++) M->nlist[i] = 0;
 }
 
@@ -321,8 +324,10 @@ __device__ __forceinline__ void list_append(bool in, int32_t v, int32_t *list, u
     if (in) list[at + __popc(m & ((1u << lane) - 1))] = v;
 }
 
-// Every vertex into the lists of its classes.
-__global__ void k_rank_lists(const int32_t *rup, const uint32_t *wd, int n2, int32_t *lists, RankMeta *M) {
+// Every vertex into the lists of its classes, and a place for its triangles:
+// hbase[a], with room for every pair of N+(a).
+__global__ void k_rank_lists(const int32_t *rup, const uint32_t *wd, int n2, int32_t *lists, unsigned long long *hbase,
+                             RankMeta *M) {
     const int lane = threadIdx.x & 31;
     const int64_t stride = (int64_t)gridDim.x * blockDim.x;
     unsigned long long direct = 0;
@@ -337,6 +342,17 @@ __global__ void k_rank_lists(const int32_t *rup, const uint32_t *wd, int n2, int
         list_append(w > kCycWarpMax && w <= kCycHashMax, (int32_t)x, lists + (int64_t)kCycHash * n2, &M->nlist[kCycHash],
                     lane);
         if (w > kCycHashMax) direct += w;
+        const unsigned long long pairs = (unsigned long long)up * (unsigned)(up - (up > 0)) / 2;
+        unsigned long long incl = pairs;
+#pragma unroll
+        for (int o = 1; o < 32; o <<= 1) {
+            const unsigned long long y = __shfl_up_sync(kFull, incl, o);
+            if (lane >= o) incl += y;
+        }
+        unsigned long long at = 0;
+        if (lane == 31 && incl) at = atomicAdd(&M->pairs, incl);
+        at = __shfl_sync(kFull, at, 31);
+        if (x < n2) hbase[x] = at + incl - pairs;
     }
     direct = pgd_warp_sum(direct);
     if (lane == 0 && direct) atomicAdd(&M->direct_wedges, direct);
@@ -416,13 +432,12 @@ __device__ __forceinline__ int walk_search(const int *pre, int i) {   // first t
     return lo;
 }
 
-// Applies fn(code, position) to every wedge end w of u in the ranges [k0, k1):
-// the rows of NT middle vertices v at a time are concatenated and every warp
+// Applies fn(code, position) to every wedge end w of u: the rows of NT middle vertices v at a time are concatenated and every warp
 // takes an equal contiguous share, so short and long rows keep all lanes busy.
 // fn's results are added per v and, in the second walk (ACC), written to the
 // slot u -> v.  All threads of the block call; returns behind a barrier.
 template <int NT, bool ACC, typename Fn>
-__device__ __forceinline__ void walk_wedges(const CycArgs &A, Walk<NT> &W, uint32_t u, int k0, int k1, Fn fn) {
+__device__ __forceinline__ void walk_wedges(const CycArgs &A, Walk<NT> &W, uint32_t u, Fn fn) {
     const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
     const uint32_t j0 = A.roff[u] + (uint32_t)A.rup[u];
     const uint32_t j1 = A.bend[u];
@@ -433,15 +448,7 @@ __device__ __forceinline__ void walk_wedges(const CycArgs &A, Walk<NT> &W, uint3
         if (j < j1) {
             const int32_t v = __ldg(A.radj + j);
             s0 = (uint32_t)__ldg(A.tw + j) + 1;
-            uint32_t e0 = __ldg(A.bend + v);
-            if (A.bpos) {
-                if (k1 < A.ranges) e0 = __ldg(A.bpos + (int64_t)(k1 - 1) * A.n2 + v);
-                if (k0 > 0) s0 = max(s0, __ldg(A.bpos + (int64_t)(k0 - 1) * A.n2 + v));
-            } else {
-                if (k1 < A.ranges) e0 = lower_bound_u(A.radj, s0, max(s0, e0), (int32_t)A.M->bound[k1]);
-                if (k0 > 0) s0 = lower_bound_u(A.radj, s0, max(s0, e0), (int32_t)A.M->bound[k0]);
-            }
-            len = e0 > s0 ? (int)(e0 - s0) : 0;
+            len = (int)(__ldg(A.bend + v) - s0);
         }
         const int incl = pgd_warp_incl_scan(len);
         if (lane == 31) W.wtot[wid] = incl;
@@ -517,36 +524,197 @@ __device__ __forceinline__ void walk_wedges(const CycArgs &A, Walk<NT> &W, uint3
     }
 }
 
+// Rows of vertices of degree >= kCoopRow are dealt to all warps of
+// k_cycle_direct in pieces of 128 entries; of the others a warp takes about
+// kGrabEntries entries at a time.
+constexpr int kCoopRow = 4096;
+constexpr int kGrabEntries = 4096;
+
+// fn(code, position) over the entries p0 + lane, p0 + 32 + lane, ... below n of
+// the 128 starting at s + p0, with their loads in flight together.
+template <typename Fn>
+__device__ __forceinline__ uint32_t take_128(const uint32_t *wcode, uint32_t s, int n, int p0, int lane, Fn fn) {
+    const uint32_t q = s + (uint32_t)(p0 + lane);
+    const uint32_t *w = wcode + q;
+    const int left = n - p0 - lane;
+    uint32_t a = 0;
+    if (n - p0 >= 128) {
+        const uint32_t w0 = __ldg(w), w1 = __ldg(w + 32), w2 = __ldg(w + 64), w3 = __ldg(w + 96);
+        a = fn(w0, q) + fn(w1, q + 32) + fn(w2, q + 64) + fn(w3, q + 96);
+    } else {
+        uint32_t w0 = 0, w1 = 0, w2 = 0, w3 = 0;
+        if (left > 0) w0 = __ldg(w);
+        if (left > 32) w1 = __ldg(w + 32);
+        if (left > 64) w2 = __ldg(w + 64);
+        if (left > 96) w3 = __ldg(w + 96);
+        if (left > 0) a += fn(w0, q);
+        if (left > 32) a += fn(w1, q + 32);
+        if (left > 64) a += fn(w2, q + 64);
+        if (left > 96) a += fn(w3, q + 96);
+    }
+    return a;
+}
+
+// Applies fn(code, position) to every wedge end w of u in the ranges [k0, k1)
+// and, in the second walk (ACC), adds its results per v to the slot u -> v.
+// The rows of the middle vertices v come longest first.  The warps share the
+// pieces of the longest rows in turn; then they take 1 to 32 rows at a time from
+// a counter, rows of 64 or more entries one after the other, the rest flattened
+// over the lanes.  No barrier inside: warps only meet between the two walks.
+// (Sharing rows from 1,024 entries costs more turns than it balances: R-MAT 20
+// 30.0 against 25.3 ms; one block-wide prefix sum per 1,024 rows with equal
+// shares for the warps spent a third of its time at its barriers.)
+template <bool ACC, typename Fn>
+__device__ __forceinline__ void walk_rows(const CycArgs &A, uint32_t u, int k0, int k1, uint32_t *next, uint32_t *acc,
+                                          Fn fn) {
+    const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
+    const uint32_t j0 = A.roff[u] + (uint32_t)A.rup[u];
+    const uint32_t j1 = A.bend[u];
+    // the part of row radj[j] that ends wedges of u in the ranges: start and length
+    auto row_of = [&](uint32_t j, uint32_t &s0) {
+        const int32_t v = __ldg(A.radj + j);
+        s0 = (uint32_t)__ldg(A.tw + j) + 1;
+        uint32_t e0 = __ldg(A.bend + v);
+        if (A.bpos) {
+            if (k1 < A.ranges) e0 = __ldg(A.bpos + (int64_t)(k1 - 1) * A.n2 + v);
+            if (k0 > 0) s0 = max(s0, __ldg(A.bpos + (int64_t)(k0 - 1) * A.n2 + v));
+        } else {
+            if (k1 < A.ranges) e0 = lower_bound_u(A.radj, s0, max(s0, e0), (int32_t)A.M->bound[k1]);
+            if (k0 > 0) s0 = lower_bound_u(A.radj, s0, max(s0, e0), (int32_t)A.M->bound[k0]);
+        }
+        return e0 > s0 ? (int)(e0 - s0) : 0;
+    };
+    int turn = wid;   // pieces of 128 until this warp's next one
+    uint32_t jb = j0;
+    for (; jb < j1; jb += 32) {
+        const int32_t v0 = __ldg(A.radj + jb);   // the longest row left
+        if (__ldg(A.roff + v0 + 1) - __ldg(A.roff + v0) < (uint32_t)kCoopRow) break;
+        uint32_t s0 = 0;
+        const int len = jb + lane < j1 ? row_of(jb + lane, s0) : 0;
+        unsigned m = __ballot_sync(kFull, len > 0);
+        while (m) {
+            const int src = __ffs(m) - 1;
+            m &= m - 1;
+            const uint32_t s = __shfl_sync(kFull, s0, src);
+            const int n = __shfl_sync(kFull, len, src);
+            const int pieces = (n + 127) >> 7;
+            uint32_t a = 0;
+            const bool any = turn < pieces;
+            for (; turn < pieces; turn += kDirectThreads / 32) a += take_128(A.wcode, s, n, turn << 7, lane, fn);
+            turn -= pieces;
+            if (ACC && any) {
+                __syncwarp();
+                a = __reduce_add_sync(kFull, a);
+                if (lane == 0 && a) atomicAdd(A.cyc + jb + src, a);
+            }
+        }
+    }
+    uint32_t grab = 1;
+    while (true) {
+        uint32_t c0 = 0;
+        if (lane == 0) c0 = atomicAdd(next, grab);
+        c0 = __shfl_sync(kFull, c0, 0);
+        if (jb >= j1 || c0 >= j1 - jb) break;
+        c0 += jb;
+        uint32_t s0 = 0;
+        int len = (uint32_t)lane < grab && c0 + lane < j1 ? row_of(c0 + lane, s0) : 0;
+        const uint32_t taken = grab;
+        const int longest = __reduce_max_sync(kFull, len);   // the next rows are hardly longer
+        grab = longest <= kGrabEntries / 32 ? 32 : max(1u, (uint32_t)(kGrabEntries / longest));
+        uint32_t mine = 0;
+        if (ACC) acc[lane] = 0;
+        unsigned m = __ballot_sync(kFull, len >= 64);
+        while (m) {
+            const int src = __ffs(m) - 1;
+            m &= m - 1;
+            const uint32_t s = __shfl_sync(kFull, s0, src);
+            const int n = __shfl_sync(kFull, len, src);
+            uint32_t a = 0;
+            for (int p = 0; p < n; p += 128) a += take_128(A.wcode, s, n, p, lane, fn);
+            if (ACC) {
+                __syncwarp();
+                a = __reduce_add_sync(kFull, a);
+                if (lane == src) mine = a;
+            }
+        }
+        if (len >= 64) len = 0;
+        const int incl = pgd_warp_incl_scan(len);
+        const int total = __shfl_sync(kFull, incl, 31);
+        const uint32_t off0 = s0 - (uint32_t)(incl - len);   // slot = off0 + flattened index
+        for (int b = 0; b < total; b += 64) {
+            const int iA = b + lane, iB = b + 32 + lane;
+            const int ownA = owner_of(incl, iA) & 31, ownB = owner_of(incl, iB) & 31;
+            const uint32_t qA = __shfl_sync(kFull, off0, ownA) + (uint32_t)iA;
+            const uint32_t qB = __shfl_sync(kFull, off0, ownB) + (uint32_t)iB;
+            uint32_t wA = 0, wB = 0;
+            if (iA < total) wA = __ldg(A.wcode + qA);
+            if (iB < total) wB = __ldg(A.wcode + qB);
+            if (iA < total) {
+                const uint32_t a = fn(wA, qA);
+                if (ACC && a) atomicAdd(acc + ownA, a);
+            }
+            if (iB < total) {
+                const uint32_t a = fn(wB, qB);
+                if (ACC && a) atomicAdd(acc + ownB, a);
+            }
+            __syncwarp();
+        }
+        if (ACC) {
+            __syncwarp();
+            mine += acc[lane];
+            if ((uint32_t)lane < taken && c0 + lane < j1 && mine) atomicAdd(A.cyc + c0 + lane, mine);
+            __syncwarp();
+        }
+    }
+}
+
 // Many wedges: one block per (u, ranges of w), a counter per w in shared
 // memory at its bit address.
 __global__ void __launch_bounds__(kDirectThreads, 1) k_cycle_direct(CycArgs A) {
     extern __shared__ __align__(16) uint32_t s_dyn[];
-    __shared__ Walk<kDirectThreads> W;
-    __shared__ uint32_t s_item;
+    __shared__ uint32_t s_acc[kDirectThreads / 32][32];
+    __shared__ uint32_t s_item, s_next[2];
     const RankMeta *M = A.M;
+    uint32_t *acc = s_acc[threadIdx.x >> 5];
     while (true) {
-        if (threadIdx.x == 0) s_item = (uint32_t)atomicAdd(A.next, 1ull);
+        if (threadIdx.x == 0) {
+            s_item = (uint32_t)atomicAdd(A.next, 1ull);
+            s_next[0] = s_next[1] = 0;
+        }
         __syncthreads();
         const uint32_t item = s_item;
         if (item >= A.count) break;
         const int2 it = A.items[item];
         const uint32_t u = (uint32_t)it.x;
         const int k0 = it.y & 0xffff, k1 = it.y >> 16;
-        const uint32_t c0 = code_of(M, max(M->bound[k0], u + 1)) & ~31u;
-        const uint32_t words = (code_of(M, M->bound[k1]) - c0 + 31) / 32;
+        const uint32_t first = code_of(M, max(M->bound[k0], u + 1)), end = code_of(M, M->bound[k1]);
+        const uint32_t c0 = first & ~31u, words = (end - c0 + 31) / 32;
         for (uint32_t i = threadIdx.x; i < words; i += kDirectThreads) s_dyn[i] = 0;
+        // the item's counter widths: mostly two, below and from thr
+        int tier = 0;
+        while (tier < 4 && M->tcode[tier] <= first) tier++;
+        const uint32_t thr = M->tcode[tier];
+        const bool two = end <= thr || tier >= 3 || end <= M->tcode[tier + 1];
+        const uint32_t mlo = mask_of(M, first), mhi = mask_of(M, thr);
         __syncthreads();
-        walk_wedges<kDirectThreads, false>(A, W, u, k0, k1, [&](uint32_t c, uint32_t) {
+        walk_rows<false>(A, u, k0, k1, &s_next[0], acc, [&](uint32_t c, uint32_t) {
             atomicAdd(s_dyn + ((c - c0) >> 5), 1u << (c & 31));
             return 0u;
         });
-        const uint32_t t0 = M->tcode[0], t1 = M->tcode[1], t2 = M->tcode[2], t3 = M->tcode[3];
-        walk_wedges<kDirectThreads, true>(A, W, u, k0, k1, [&](uint32_t c, uint32_t q) {
-            const uint32_t mask = c >= t2 ? (c < t3 ? 0xfu : 0x3u) : (c >= t1 ? 0xffu : (c >= t0 ? 0xffffu : kFull));
-            const uint32_t k = ((s_dyn[(c - c0) >> 5] >> (c & 31)) & mask) - 1;
-            if (k) atomicAdd(A.cyc + q, k);
-            return k;
-        });
+        __syncthreads();
+        if (two) {
+            walk_rows<true>(A, u, k0, k1, &s_next[1], acc, [&](uint32_t c, uint32_t q) {
+                const uint32_t k = ((s_dyn[(c - c0) >> 5] >> (c & 31)) & (c < thr ? mlo : mhi)) - 1;
+                if (k) atomicAdd(A.cyc + q, k);
+                return k;
+            });
+        } else {
+            walk_rows<true>(A, u, k0, k1, &s_next[1], acc, [&](uint32_t c, uint32_t q) {
+                const uint32_t k = ((s_dyn[(c - c0) >> 5] >> (c & 31)) & mask_of(M, c)) - 1;
+                if (k) atomicAdd(A.cyc + q, k);
+                return k;
+            });
+        }
         __syncthreads();
     }
 }
@@ -596,12 +764,12 @@ __global__ void __launch_bounds__(kHashThreads, 4) k_cycle_hash(CycArgs A) {
         __syncthreads();
         constexpr int shift = 32 - 13;
         static_assert(kSlots == 1 << 13, "hash width");
-        walk_wedges<kHashThreads, false>(A, W, u, 0, A.ranges, [&](uint32_t c, uint32_t) {
+        walk_wedges<kHashThreads, false>(A, W, u, [&](uint32_t c, uint32_t) {
             const uint32_t h = hash_find_add(s_key, c, kSlots - 1, shift);
             atomicAdd(s_cnt + (h >> 1), 1u << ((h & 1) << 4));
             return 0u;
         });
-        walk_wedges<kHashThreads, true>(A, W, u, 0, A.ranges, [&](uint32_t c, uint32_t q) {
+        walk_wedges<kHashThreads, true>(A, W, u, [&](uint32_t c, uint32_t q) {
             const uint32_t h = hash_find(s_key, c, kSlots - 1, shift);
             const uint32_t k = ((s_cnt[h >> 1] >> ((h & 1) << 4)) & 0xffffu) - 1;
             if (k) atomicAdd(A.cyc + q, k);
@@ -697,7 +865,9 @@ struct EgoArgs {
     unsigned long long *next;
     uint32_t *t;                // per slot of the lower end: triangles
     unsigned long long *dk;     // per slot of the lower end: D << 32 | k4
-    uint2 *hits;                // pass 2: triangle list of each block ({i << 16 | j, slot x -> y})
+    uint2 *hits;                // triangles ({i << 16 | j, slot x -> y}): at hbase[a], or a list per block
+    const unsigned long long *hbase;
+    uint32_t *hcount;           // triangles of a, where they are kept from pass 1 to pass 2 (else null)
     int64_t hits_stride;
     uint8_t *tables;            // kEgoGlobal: tables of each block
     int64_t tables_stride;
@@ -745,6 +915,7 @@ __global__ void __launch_bounds__(kWarpThreads) k_ego_warp(EgoArgs A) {
             __syncwarp();
             const int np = d * (d - 1) / 2;
             int nh = 0;
+            const unsigned long long hb = PASS == 1 && A.hcount ? A.hbase[a] : 0;
             for (int b = 0; b < np; b += 32) {
                 const bool act = b + lane < np;
                 const int pr = act ? s_pair[b + lane] : 0x0100;
@@ -759,11 +930,14 @@ __global__ void __launch_bounds__(kWarpThreads) k_ego_warp(EgoArgs A) {
                     hit = pos < r0 + (uint32_t)ui && __ldg(A.radj + pos) == y;
                 }
                 if (PASS == 1) {
+                    const unsigned m = A.hcount ? __ballot_sync(kFull, hit) : 0;
                     if (hit) {
                         atomicAdd(A.t + pos, 1u);
                         atomicAdd(ca + i, 1u);
                         atomicAdd(ca + j, 1u);
+                        if (m) A.hits[hb + nh + __popc(m & ((1u << lane) - 1))] = make_uint2((uint32_t)i << 16 | j, pos);
                     }
+                    nh += __popc(m);
                 } else {
                     const unsigned m = __ballot_sync(kFull, hit);
                     if (hit) {
@@ -779,6 +953,7 @@ __global__ void __launch_bounds__(kWarpThreads) k_ego_warp(EgoArgs A) {
             __syncwarp();
             if (PASS == 1) {
                 if (lane < d && ca[lane]) atomicAdd(A.t + ra + lane, ca[lane]);
+                if (A.hcount && lane == 0) A.hcount[a] = (uint32_t)nh;
             } else {
                 for (int h = lane; h < nh; h += 32) {
                     const uint32_t pos = s_slot[wid][h];
@@ -806,16 +981,91 @@ __host__ __device__ __forceinline__ int ego_hash_bits(int dmax) {   // a table a
     while ((1 << b) < 4 * dmax) b++;
     return b;
 }
-__host__ __device__ __forceinline__ int ego_row_words(int dmax) { return ((dmax + 63) / 64) | 1; }   // odd: rows spread over banks
-inline int64_t ego_table_bytes(int dmax, bool pass2) {
-    int64_t b = ((int64_t)6 << ego_hash_bits(dmax)) + (int64_t)dmax * 4 * 4;
-    if (pass2) b += (int64_t)dmax * 4 * 2 + (int64_t)dmax * 8 * ego_row_words(dmax);
-    return (b + 127) & ~(int64_t)127;
+// 64-bit words of a row of F: odd, so that rows spread over the banks
+__host__ __device__ __forceinline__ int ego_row_words(int dmax) { return ((dmax + 63) / 64) | 1; }
+
+// Ranks below this have their index in N(+)(a) in a direct table, most entries
+// of the lists being of high rank; the others are looked up in the hash table.
+constexpr int kTopRanks = 8192;
+
+// One block's tables: [F] hash keys, N+(a)'s rows (start, length), list,
+// counts, [sums of t, t of (a, x)], hash indices, direct table
+struct EgoTables {
+    unsigned long long *F;
+    uint32_t *hkey, *rs;
+    int32_t *ru, *ls;
+    uint32_t *ck, *cd, *ta;
+    uint16_t *hidx, *top;
+};
+__host__ __device__ __forceinline__ int64_t ego_layout(uint8_t *base, int dmax, bool lookup, bool counts2,
+                                                       EgoTables *T) {
+    uint8_t *p = base;
+    auto take = [&](int64_t bytes) {
+        uint8_t *q = p;
+        p += bytes;
+        return q;
+    };
+    const int hb = ego_hash_bits(dmax);
+    T->F = (unsigned long long *)take(counts2 ? (int64_t)dmax * 8 * ego_row_words(dmax) : 0);
+    T->ck = (uint32_t *)take((int64_t)dmax * 4);
+    T->cd = (uint32_t *)take(counts2 ? (int64_t)dmax * 4 : 0);
+    T->ta = (uint32_t *)take(counts2 ? (int64_t)dmax * 4 : 0);
+    T->hkey = (uint32_t *)take(lookup ? (int64_t)4 << hb : 0);
+    T->rs = (uint32_t *)take(lookup ? (int64_t)dmax * 4 : 0);
+    T->ru = (int32_t *)take(lookup ? (int64_t)dmax * 4 : 0);
+    T->ls = (int32_t *)take(lookup ? (int64_t)dmax * 4 : 0);
+    T->hidx = (uint16_t *)take(lookup ? (int64_t)2 << hb : 0);
+    T->top = (uint16_t *)take(lookup ? (int64_t)2 * kTopRanks : 0);
+    return ((p - base) + 127) & ~(int64_t)127;
+}
+inline int64_t ego_table_bytes(int dmax, bool lookup, bool counts2) {
+    EgoTables T;
+    return ego_layout(nullptr, dmax, lookup, counts2, &T);
 }
 
-// |N+(a)| = d in a block's range: a block per vertex.  N+(a) goes into a hash
-// table rank -> index; each warp takes vertices x of N+(a) and looks the
-// entries of N+(x) up.
+// The second half of pass 2: each triangle {a, x, y} (indices i, j; slot x -> y)
+// with c = |F_i & F_j| 4-cliques.  All threads of the block call.
+template <int NT>
+__device__ __forceinline__ void clique_hits(const EgoArgs &A, const uint2 *hits, uint32_t nh, const EgoTables &T, int W,
+                                            int WS) {
+    const int lane = threadIdx.x & 31;
+    for (uint32_t h0 = threadIdx.x - lane; h0 < nh; h0 += NT) {
+        const uint32_t h = h0 + lane;
+        uint32_t c = 0, di = 0;
+        int i = -1;
+        if (h < nh) {
+            const uint2 e = hits[h];
+            const uint32_t tij = A.t[e.y];
+            i = (int)(e.x >> 16);
+            const int j = (int)(e.x & 0xffff);
+            const unsigned long long *fi = T.F + (int64_t)i * WS, *fj = T.F + (int64_t)j * WS;
+            for (int w = 0; w < W; w++) c += (uint32_t)__popcll(fi[w] & fj[w]);
+            const uint32_t ti = T.ta[i], tj = T.ta[j];
+            atomicAdd(A.dk + e.y, ((unsigned long long)(ti + tj) << 32) + c);
+            if (c) atomicAdd(T.ck + j, c);
+            atomicAdd(T.cd + j, ti + tij);
+            di = tj + tij;
+        }
+        // most warps hold one x: reduce its sums first
+        const int i0 = __shfl_sync(kFull, i, 0);
+        if (__all_sync(kFull, i == i0 || i < 0)) {
+            c = __reduce_add_sync(kFull, c);
+            di = __reduce_add_sync(kFull, di);
+            if (lane == 0) {
+                if (c) atomicAdd(T.ck + i0, c);
+                atomicAdd(T.cd + i0, di);
+            }
+        } else if (i >= 0) {
+            if (c) atomicAdd(T.ck + i, c);
+            atomicAdd(T.cd + i, di);
+        }
+    }
+}
+
+// |N+(a)| = d in a block's range: a block per vertex.  The indices of N+(a) go
+// into the lookup tables; each warp takes vertices x of N+(a) and looks the
+// entries of N+(x) up.  PASS 1 counts the triangles and, where there is room,
+// keeps them for k_clique_block; PASS 2 (else) lists them again, with F.
 template <int PASS, int NT, bool GLOBAL>
 __global__ void __launch_bounds__(NT) k_ego_block(EgoArgs A, int dmax) {
     extern __shared__ __align__(16) uint32_t s_dyn[];
@@ -825,19 +1075,11 @@ __global__ void __launch_bounds__(NT) k_ego_block(EgoArgs A, int dmax) {
     const int lane = threadIdx.x & 31;
     const int hb = ego_hash_bits(dmax), shift = 32 - hb;
     const uint32_t hmask = (1u << hb) - 1;
-    uint8_t *base = GLOBAL ? A.tables + (int64_t)blockIdx.x * A.tables_stride : (uint8_t *)s_dyn;
-    // [F rows (64-bit)] keys, positions of N+(a)'s rows, their lengths, list, counts, (sums of t, t), indices (16-bit)
+    EgoTables T;
+    ego_layout(GLOBAL ? A.tables + (int64_t)blockIdx.x * A.tables_stride : (uint8_t *)s_dyn, dmax, true, PASS == 2, &T);
     const int WS = ego_row_words(dmax);
-    unsigned long long *F = (unsigned long long *)base;
-    uint32_t *hkey = (uint32_t *)(base + (PASS == 2 ? (int64_t)dmax * 8 * WS : 0));
-    uint32_t *rs = hkey + (1 << hb);
-    int32_t *ru = (int32_t *)(rs + dmax);
-    int32_t *ls = ru + dmax;
-    uint32_t *ck = (uint32_t *)(ls + dmax);
-    uint32_t *cd = ck + dmax;                          // pass 2
-    uint32_t *ta = cd + (PASS == 2 ? dmax : 0);        // pass 2
-    uint16_t *hidx = (uint16_t *)(PASS == 2 ? ta + dmax : cd);
-    uint2 *hits = PASS == 2 ? A.hits + (int64_t)blockIdx.x * A.hits_stride : nullptr;
+    uint32_t *F32 = (uint32_t *)T.F;
+    for (int i = threadIdx.x; i < kTopRanks / 2; i += NT) ((uint32_t *)T.top)[i] = 0;
     while (true) {
         if (threadIdx.x == 0) {
             s_item = (uint32_t)atomicAdd(A.next, 1ull);
@@ -850,24 +1092,31 @@ __global__ void __launch_bounds__(NT) k_ego_block(EgoArgs A, int dmax) {
         const int d = A.rup[a];
         const uint32_t ra = A.roff[a];
         const int W = (d + 63) >> 6;
+        uint2 *hits = nullptr;
+        if (PASS == 2) hits = A.hits + (int64_t)blockIdx.x * A.hits_stride;
+        else if (A.hcount) hits = A.hits + A.hbase[a];
         if (threadIdx.x == 0) s_row = d - 1;
-        for (int i = threadIdx.x; i <= (int)hmask; i += NT) hkey[i] = kFull;
+        for (int i = threadIdx.x; i <= (int)hmask; i += NT) T.hkey[i] = kFull;
         if (PASS == 2)
-            for (int i = threadIdx.x; i < d * WS; i += NT) F[i] = 0;
+            for (int i = threadIdx.x; i < d * WS; i += NT) T.F[i] = 0;
         __syncthreads();
         for (int i = threadIdx.x; i < d; i += NT) {
             const int32_t x = __ldg(A.radj + ra + i);
-            ls[i] = x;
-            rs[i] = __ldg(A.roff + x);
-            ru[i] = __ldg(A.rup + x);
-            ck[i] = 0;
+            T.ls[i] = x;
+            T.rs[i] = __ldg(A.roff + x);
+            T.ru[i] = __ldg(A.rup + x);
+            T.ck[i] = 0;
             if (PASS == 2) {
-                cd[i] = 0;
-                ta[i] = A.t[ra + i];
+                T.cd[i] = 0;
+                T.ta[i] = A.t[ra + i];
             }
-            uint32_t h = hash_of((uint32_t)x, shift);
-            while (atomicCAS(hkey + h, kFull, (uint32_t)x) != kFull) h = (h + 1) & hmask;
-            hidx[h] = (uint16_t)i;
+            if (x < kTopRanks) {
+                T.top[x] = (uint16_t)(i + 1);
+            } else {
+                uint32_t h = hash_of((uint32_t)x, shift);
+                while (atomicCAS(T.hkey + h, kFull, (uint32_t)x) != kFull) h = (h + 1) & hmask;
+                T.hidx[h] = (uint16_t)i;
+            }
         }
         __syncthreads();
         while (true) {
@@ -875,90 +1124,152 @@ __global__ void __launch_bounds__(NT) k_ego_block(EgoArgs A, int dmax) {
             if (lane == 0) i = atomicSub(&s_row, 1);
             i = __shfl_sync(kFull, i, 0);
             if (i < 1) break;   // the first neighbour has none of the others above it
-            const uint32_t r0 = rs[i];
-            const int len = ru[i];
-            const int32_t last = ls[i - 1];
+            const uint32_t r0 = T.rs[i];
+            const int len = T.ru[i];
+            const int32_t last = T.ls[i - 1];
             uint32_t found = 0;
             for (int b = 0; b < len; b += 32) {
                 const int32_t y = b + lane < len ? __ldg(A.radj + r0 + b + lane) : 0x7fffffff;
-                bool hit = false;
-                int jx = 0;
-                if (y <= last) {
+                int jx = -1;
+                if (y < kTopRanks) {
+                    jx = (int)T.top[y] - 1;
+                } else if (y <= last) {
                     uint32_t h = hash_of((uint32_t)y, shift);
                     uint32_t k;
-                    while ((k = hkey[h]) != (uint32_t)y && k != kFull) h = (h + 1) & hmask;
-                    if (k == (uint32_t)y) {
-                        hit = true;
-                        jx = hidx[h];
-                    }
+                    while ((k = T.hkey[h]) != (uint32_t)y && k != kFull) h = (h + 1) & hmask;
+                    if (k == (uint32_t)y) jx = T.hidx[h];
                 }
+                const bool hit = jx >= 0;
                 const unsigned m = __ballot_sync(kFull, hit);
                 if (m) {
-                    if (PASS == 1) {
-                        if (hit) {
-                            atomicAdd(A.t + r0 + b + lane, 1u);
-                            atomicAdd(ck + jx, 1u);
-                        }
-                        found += __popc(m);
-                    } else {
+                    if (hits) {
                         uint32_t at = 0;
                         if (lane == 0) at = atomicAdd(&s_nhit, (uint32_t)__popc(m));
                         at = __shfl_sync(kFull, at, 0);
-                        if (hit) {
+                        if (hit)
                             hits[at + __popc(m & ((1u << lane) - 1))] =
                                 make_uint2((uint32_t)i << 16 | (uint32_t)jx, r0 + (uint32_t)(b + lane));
-                            atomicOr(F + (int64_t)i * WS + (jx >> 6), 1ull << (jx & 63));
-                            atomicOr(F + (int64_t)jx * WS + (i >> 6), 1ull << (i & 63));
+                    }
+                    if (PASS == 1) {
+                        if (hit) {
+                            atomicAdd(A.t + r0 + b + lane, 1u);
+                            atomicAdd(T.ck + jx, 1u);
                         }
+                        found += __popc(m);
+                    } else if (hit) {
+                        atomicOr(F32 + (int64_t)i * 2 * WS + (jx >> 5), 1u << (jx & 31));
+                        atomicOr(F32 + (int64_t)jx * 2 * WS + (i >> 5), 1u << (i & 31));
                     }
                 }
                 if (__shfl_sync(kFull, y, 31) > last) break;   // ascending: nothing more at or below last
             }
-            if (PASS == 1 && lane == 0 && found) atomicAdd(ck + i, found);
+            if (PASS == 1 && lane == 0 && found) atomicAdd(T.ck + i, found);
         }
         __syncthreads();
         if (PASS == 2) {
-            const uint32_t nh = s_nhit;
-            for (uint32_t h0 = threadIdx.x - lane; h0 < nh; h0 += NT) {
-                const uint32_t h = h0 + lane;
-                uint32_t c = 0, di = 0;
-                int i = -1;
-                if (h < nh) {
-                    const uint2 e = hits[h];
-                    i = (int)(e.x >> 16);
-                    const int jx = (int)(e.x & 0xffff);
-                    const unsigned long long *fi = F + (int64_t)i * WS, *fj = F + (int64_t)jx * WS;
-                    for (int w = 0; w < W; w++) c += (uint32_t)__popcll(fi[w] & fj[w]);
-                    const uint32_t tij = A.t[e.y], ti = ta[i], tj = ta[jx];
-                    atomicAdd(A.dk + e.y, ((unsigned long long)(ti + tj) << 32) + c);
-                    if (c) atomicAdd(ck + jx, c);
-                    atomicAdd(cd + jx, ti + tij);
-                    di = tj + tij;
-                }
-                // most warps hold one x: reduce its sums first
-                const int i0 = __shfl_sync(kFull, i, 0);
-                if (__all_sync(kFull, i == i0 || i < 0)) {
-                    c = __reduce_add_sync(kFull, c);
-                    di = __reduce_add_sync(kFull, di);
-                    if (lane == 0) {
-                        if (c) atomicAdd(ck + i0, c);
-                        atomicAdd(cd + i0, di);
-                    }
-                } else if (i >= 0) {
-                    if (c) atomicAdd(ck + i, c);
-                    atomicAdd(cd + i, di);
-                }
-            }
+            clique_hits<NT>(A, hits, s_nhit, T, W, WS);
             __syncthreads();
+        } else if (A.hcount && threadIdx.x == 0) {
+            A.hcount[a] = s_nhit;
         }
         for (int i = threadIdx.x; i < d; i += NT) {
             if (PASS == 1) {
-                if (ck[i]) atomicAdd(A.t + ra + i, ck[i]);
-            } else if (ck[i] | cd[i]) {
-                atomicAdd(A.dk + ra + i, ((unsigned long long)cd[i] << 32) + (ck[i] >> 1));
+                if (T.ck[i]) atomicAdd(A.t + ra + i, T.ck[i]);
+            } else if (T.ck[i] | T.cd[i]) {
+                atomicAdd(A.dk + ra + i, ((unsigned long long)T.cd[i] << 32) + (T.ck[i] >> 1));
             }
+            if (T.ls[i] < kTopRanks) T.top[T.ls[i]] = 0;
         }
         __syncthreads();
+    }
+}
+
+// Pass 2 from the triangles that pass 1 kept: F from the list, then the list again.
+template <int NT, bool GLOBAL>
+__global__ void __launch_bounds__(NT) k_clique_block(EgoArgs A, int dmax) {
+    extern __shared__ __align__(16) uint32_t s_dyn[];
+    __shared__ uint32_t s_item;
+    EgoTables T;
+    ego_layout(GLOBAL ? A.tables + (int64_t)blockIdx.x * A.tables_stride : (uint8_t *)s_dyn, dmax, false, true, &T);
+    const int WS = ego_row_words(dmax);
+    uint32_t *F32 = (uint32_t *)T.F;
+    while (true) {
+        if (threadIdx.x == 0) s_item = (uint32_t)atomicAdd(A.next, 1ull);
+        __syncthreads();
+        const uint32_t item = s_item;
+        if (item >= A.count) break;
+        const uint32_t a = (uint32_t)A.list[item];
+        const int d = A.rup[a];
+        const uint32_t ra = A.roff[a], nh = A.hcount[a];
+        const int W = (d + 63) >> 6;
+        const uint2 *hits = A.hits + A.hbase[a];
+        for (int i = threadIdx.x; i < d * WS; i += NT) T.F[i] = 0;
+        for (int i = threadIdx.x; i < d; i += NT) {
+            T.ck[i] = 0;
+            T.cd[i] = 0;
+            T.ta[i] = A.t[ra + i];
+        }
+        __syncthreads();
+        for (uint32_t h = threadIdx.x; h < nh; h += NT) {
+            const uint32_t e = hits[h].x;
+            const int i = (int)(e >> 16), j = (int)(e & 0xffff);
+            atomicOr(F32 + (int64_t)i * 2 * WS + (j >> 5), 1u << (j & 31));
+            atomicOr(F32 + (int64_t)j * 2 * WS + (i >> 5), 1u << (i & 31));
+        }
+        __syncthreads();
+        clique_hits<NT>(A, hits, nh, T, W, WS);
+        __syncthreads();
+        for (int i = threadIdx.x; i < d; i += NT)
+            if (T.ck[i] | T.cd[i])
+                atomicAdd(A.dk + ra + i, ((unsigned long long)T.cd[i] << 32) + (T.ck[i] >> 1));
+        __syncthreads();
+    }
+}
+
+// |N+(a)| <= 32: a warp per vertex, F one 32-bit word per row.
+__global__ void __launch_bounds__(kWarpThreads) k_clique_warp(EgoArgs A) {
+    constexpr int kW = kWarpThreads / 32;
+    __shared__ uint32_t s_a[kW][32], s_b[kW][32], s_f[kW][32], s_t[kW][32];
+    const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
+    uint32_t *ca = s_a[wid], *cb = s_b[wid], *f = s_f[wid], *ta = s_t[wid];
+    while (true) {
+        uint32_t i0 = 0;
+        if (lane == 0) i0 = (uint32_t)atomicAdd(A.next, (unsigned long long)A.grab);
+        i0 = __shfl_sync(kFull, i0, 0);
+        if (i0 >= A.count) break;
+        const uint32_t i1 = min(i0 + A.grab, A.count);
+        for (uint32_t ii = i0; ii < i1; ii++) {
+            const uint32_t a = (uint32_t)A.list[ii];
+            const uint32_t nh = A.hcount[a];
+            if (!nh) continue;
+            const int d = A.rup[a];
+            const uint32_t ra = A.roff[a];
+            const uint2 *hits = A.hits + A.hbase[a];
+            ca[lane] = cb[lane] = f[lane] = 0;
+            ta[lane] = lane < d ? A.t[ra + lane] : 0;
+            __syncwarp();
+            for (uint32_t h = lane; h < nh; h += 32) {
+                const uint32_t e = hits[h].x;
+                atomicOr(f + (e >> 16), 1u << (e & 31));
+                atomicOr(f + (e & 31), 1u << (e >> 16));
+            }
+            __syncwarp();
+            for (uint32_t h = lane; h < nh; h += 32) {
+                const uint2 e = hits[h];
+                const int i = (int)(e.x >> 16), j = (int)(e.x & 0xffff);
+                const uint32_t c = (uint32_t)__popc(f[i] & f[j]);
+                const uint32_t tij = A.t[e.y], ti = ta[i], tj = ta[j];
+                atomicAdd(A.dk + e.y, ((unsigned long long)(ti + tj) << 32) + c);
+                atomicAdd(ca + i, c);
+                atomicAdd(ca + j, c);
+                atomicAdd(cb + i, tj + tij);
+                atomicAdd(cb + j, ti + tij);
+            }
+            __syncwarp();
+            if (lane < d && (ca[lane] | cb[lane]))
+                atomicAdd(A.dk + ra + lane, ((unsigned long long)cb[lane] << 32) + (ca[lane] >> 1));
+            __syncwarp();
+        }
     }
 }
 
@@ -1194,14 +1505,16 @@ pgd_status pgd_rank_build(pgd_graph *g, int64_t nnz, const int32_t *vgraph, cons
     RB_TRY(tg.alloc(&wd, n2 * sizeof(uint32_t)));
     RB_TRY(keep(&R->bend, n2 * sizeof(uint32_t)));
     RB_TRY(keep(&R->lists, (size_t)kClasses * n2 * sizeof(int32_t)));
+    RB_TRY(keep(&R->hbase, n2 * sizeof(unsigned long long)));
     RB_CUDA(cudaMemsetAsync(wd, 0, n2 * sizeof(uint32_t), s));
     PGD_LAUNCH(ctx, k_rank_bend, grid_for(n2), kThreads, 0, R->roff, R->radj, n2, R->bend);
     PGD_LAUNCH(ctx, k_rank_wedges, grid_for(h.entries2), kThreads, 0, R->roff, R->radj, R->tw, R->bend, n, n2,
                (int64_t)h.entries2, wd);
-    PGD_LAUNCH(ctx, k_rank_lists, grid_for(n2), kThreads, 0, R->rup, wd, n2, R->lists, M);
+    PGD_LAUNCH(ctx, k_rank_lists, grid_for(n2), kThreads, 0, R->rup, wd, n2, R->lists, R->hbase, M);
     RB_CUDA(cudaMemcpyAsync(&h, M, kHead, cudaMemcpyDeviceToHost, s));
     RB_CUDA(cudaStreamSynchronize(s));
     for (int i = 0; i < kClasses; i++) R->nlist[i] = h.nlist[i];
+    R->pairs = (int64_t)h.pairs;
     if (h.direct_wedges == 0) return PGD_OK;
     // items of the vertices with many wedges, by ranges of the wedges' ends:
     // fine enough to balance the items, and at most half an item's counters each
@@ -1250,41 +1563,50 @@ static int ego_grid(const pgd_ctx *ctx, const pgd_rank_graph &R, int c) {
     return (int)std::min<int64_t>(R.nlist[c], (int64_t)(ego_wide(ctx, R, c) ? 2 : ego_blocks_per_sm(c)) * ctx->num_sms);
 }
 
-// The ego classes' launches of one pass.
-template <int PASS>
-static void ego_pass(pgd_ctx *ctx, const pgd_rank_graph &R, EgoArgs A, unsigned long long *ctr, uint2 *hits,
+// The ego classes' launches: pass 1, pass 2 that lists the triangles again, or
+// (kept) pass 2 from the triangles of pass 1.
+static void ego_pass(pgd_ctx *ctx, const pgd_rank_graph &R, EgoArgs A, int pass, unsigned long long *ctr,
                      uint8_t *tables, int gblocks, int64_t table_bytes) {
+    const bool kept = pass == 2 && A.hcount;
     auto args = [&](int c) {
         EgoArgs B = A;
         B.list = R.lists + (int64_t)c * R.n2;
         B.count = R.nlist[c];
         B.next = ctr + c;
+        B.grab = grab_for(ctx, B.count);
         return B;
     };
+#define EGO_BLOCK(NT, G, grid, smem, B, dmax)                                                    \
+    do {                                                                                         \
+        if (pass == 1) PGD_LAUNCH(ctx, (k_ego_block<1, NT, G>), grid, NT, smem, B, dmax);        \
+        else if (kept) PGD_LAUNCH(ctx, (k_clique_block<NT, G>), grid, NT, smem, B, dmax);        \
+        else PGD_LAUNCH(ctx, (k_ego_block<2, NT, G>), grid, NT, smem, B, dmax);                  \
+    } while (0)
     if (R.nlist[kEgoGlobal]) {
         EgoArgs B = args(kEgoGlobal);
-        B.hits = hits;
         B.hits_stride = (int64_t)R.max_up * (R.max_up - 1) / 2;
         B.tables = tables;
         B.tables_stride = table_bytes;
-        PGD_LAUNCH(ctx, (k_ego_block<PASS, 1024, true>), gblocks, 1024, 0, B, R.max_up);
+        EGO_BLOCK(1024, true, gblocks, 0, B, R.max_up);
     }
     for (int c : {kEgoC, kEgoB, kEgoA}) {
         if (!R.nlist[c]) continue;
         EgoArgs B = args(c);
         const int dmax = std::min(kEgoMax[c], (int)R.max_up);
-        B.hits = hits;
         B.hits_stride = (int64_t)dmax * (dmax - 1) / 2;
         const int blocks = ego_grid(ctx, R, c);
-        const size_t smem = (size_t)ego_table_bytes(dmax, PASS == 2);
-        if (c == kEgoC || ego_wide(ctx, R, c)) PGD_LAUNCH(ctx, (k_ego_block<PASS, 1024, false>), blocks, 1024, smem, B, dmax);
-        else if (c == kEgoB) PGD_LAUNCH(ctx, (k_ego_block<PASS, 512, false>), blocks, 512, smem, B, dmax);
-        else PGD_LAUNCH(ctx, (k_ego_block<PASS, 256, false>), blocks, 256, smem, B, dmax);
+        const size_t smem = (size_t)ego_table_bytes(dmax, !kept, pass == 2);
+        if (c == kEgoC || ego_wide(ctx, R, c)) EGO_BLOCK(1024, false, blocks, smem, B, dmax);
+        else if (c == kEgoB) EGO_BLOCK(512, false, blocks, smem, B, dmax);
+        else EGO_BLOCK(256, false, blocks, smem, B, dmax);
     }
+#undef EGO_BLOCK
     if (R.nlist[kEgoWarp]) {
         EgoArgs B = args(kEgoWarp);
-        B.grab = grab_for(ctx, B.count);
-        PGD_LAUNCH(ctx, k_ego_warp<PASS>, warp_blocks(ctx, B.count, B.grab, 8), kWarpThreads, 0, B);
+        const int blocks = warp_blocks(ctx, B.count, B.grab, 8);
+        if (pass == 1) PGD_LAUNCH(ctx, k_ego_warp<1>, blocks, kWarpThreads, 0, B);
+        else if (kept) PGD_LAUNCH(ctx, k_clique_warp, blocks, kWarpThreads, 0, B);
+        else PGD_LAUNCH(ctx, k_ego_warp<2>, blocks, kWarpThreads, 0, B);
     }
 }
 
@@ -1294,11 +1616,14 @@ static cudaError_t rank_kernel_limits() {
     cudaError_t e = cudaFuncSetAttribute(k_cycle_direct, cudaFuncAttributeMaxDynamicSharedMemorySize, kDirectWords * 4);
     if (e == cudaSuccess) e = cudaFuncSetAttribute(k_cycle_hash, cudaFuncAttributeMaxDynamicSharedMemorySize, kHashSmem);
     if (e == cudaSuccess) e = cudaFuncSetAttribute(k_cycle_warp, cudaFuncAttributeMaxDynamicSharedMemorySize, kWarpSmem);
-    const int b2 = (int)ego_table_bytes(kEgoMax[kEgoB], true), c1 = (int)ego_table_bytes(kEgoMax[kEgoC], false),
-              c2 = (int)ego_table_bytes(kEgoMax[kEgoC], true);
-    if (e == cudaSuccess) e = cudaFuncSetAttribute(k_ego_block<2, 512, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, b2);
-    if (e == cudaSuccess) e = cudaFuncSetAttribute(k_ego_block<1, 1024, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, c1);
-    if (e == cudaSuccess) e = cudaFuncSetAttribute(k_ego_block<2, 1024, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, c2);
+    const int cmax = kEgoMax[kEgoC];
+    const int c1 = (int)ego_table_bytes(cmax, true, false), c2 = (int)ego_table_bytes(cmax, true, true),
+              b2 = (int)ego_table_bytes(kEgoMax[kEgoB], true, true), k2 = (int)ego_table_bytes(cmax, false, true);
+    constexpr cudaFuncAttribute kDyn = cudaFuncAttributeMaxDynamicSharedMemorySize;
+    if (e == cudaSuccess) e = cudaFuncSetAttribute(k_ego_block<1, 1024, false>, kDyn, c1);
+    if (e == cudaSuccess) e = cudaFuncSetAttribute(k_ego_block<2, 1024, false>, kDyn, c2);
+    if (e == cudaSuccess) e = cudaFuncSetAttribute(k_ego_block<2, 512, false>, kDyn, b2);
+    if (e == cudaSuccess) e = cudaFuncSetAttribute(k_clique_block<1024, false>, kDyn, k2);
     return e;
 }
 
@@ -1373,23 +1698,27 @@ pgd_status pgd_rank_decompose(pgd_ctx *ctx, const pgd_rank_graph &R, const pgd_r
     }
     if (R.nlist[kEgoGlobal]) {
         const int64_t per = (int64_t)R.max_up * (R.max_up - 1) / 2;
-        table_bytes = ego_table_bytes(R.max_up, true);
+        table_bytes = ego_table_bytes(R.max_up, true, true);
         // at most about 8 GB of tables and lists, at least one block's
         gblocks = (int)std::max<int64_t>(1, std::min<int64_t>(std::min<int64_t>(nsm, R.nlist[kEgoGlobal]),
                                                               (8ll << 30) / (per * 8 + table_bytes)));
         hit_count = std::max(hit_count, per * gblocks);
     }
-    // one block: counters, dk, t, cyc (zeroed), then the lists and tables
+    // Every triangle of pass 1 is kept for pass 2 where the lists' bound (every
+    // pair of every N+) is at most kKeepBytes; else pass 2 lists them again.
+    const bool keep = R.pairs * (int64_t)sizeof(uint2) <= kKeepBytes;
+    if (keep) hit_count = R.pairs;
+    // one allocation: counters, dk, t, cyc (zeroed), then the lists and tables
     constexpr int kCounters = 16;   // [0..5) pass 1, [5..10) pass 2, [10..13) 4-cycles
-    const size_t zeroed = kCounters * 8 + (size_t)R.nnz * 16, zeroed_up = (zeroed + 127) & ~(size_t)127;
+    auto up128 = [](int64_t x) { return (x + 127) & ~(int64_t)127; };
+    const int64_t zeroed = kCounters * 8 + R.nnz * 16;
+    const int64_t at_count = up128(zeroed), at_hits = at_count + up128(keep ? (int64_t)R.n2 * 4 : 0),
+                  at_tables = at_hits + up128(hit_count * (int64_t)sizeof(uint2));
     Tmp tg(ctx);
     uint8_t *work = nullptr;
-    if ((st = tg.alloc(&work, zeroed_up + (size_t)hit_count * sizeof(uint2) + (size_t)gblocks * table_bytes + 128)))
-        return st;
+    if ((st = tg.alloc(&work, (size_t)(at_tables + gblocks * table_bytes)))) return st;
     unsigned long long *ctr = (unsigned long long *)work, *dk = ctr + kCounters;
     uint32_t *t = (uint32_t *)(dk + R.nnz), *cyc = t + R.nnz;
-    uint2 *hits = (uint2 *)(work + zeroed_up);
-    uint8_t *tables = (uint8_t *)(((uintptr_t)(hits + hit_count) + 127) & ~(uintptr_t)127);
     PGD_CUDA(ctx, cudaMemsetAsync(work, 0, zeroed, s));
     SideStream side(ctx);   // joined before tg frees
     PGD_CUDA(ctx, side.fork());
@@ -1415,9 +1744,12 @@ pgd_status pgd_rank_decompose(pgd_ctx *ctx, const pgd_rank_graph &R, const pgd_r
     E.radj = R.radj;
     E.t = t;
     E.dk = dk;
+    E.hits = (uint2 *)(work + at_hits);
+    E.hbase = R.hbase;
+    E.hcount = keep ? (uint32_t *)(work + at_count) : nullptr;
     PGD_CUDA(ctx, cudaEventRecord(ctx->evt0, s));
-    ego_pass<1>(ctx, R, E, ctr, hits, tables, gblocks, table_bytes);
-    ego_pass<2>(ctx, R, E, ctr + 5, hits, tables, gblocks, table_bytes);
+    ego_pass(ctx, R, E, 1, ctr, work + at_tables, gblocks, table_bytes);
+    ego_pass(ctx, R, E, 2, ctr + 5, work + at_tables, gblocks, table_bytes);
     PGD_CUDA(ctx, cudaEventRecord(ctx->evt1, s));
     PGD_CUDA(ctx, side.join());
     CloseArgs Z;

@@ -21,6 +21,8 @@ struct pgd_rank_graph {
     uint32_t *bpos = nullptr;    // (nranges - 1) x n2: first entry of the row at or beyond an inner range
                                  // boundary (null: searched when needed)
     int32_t *lists = nullptr;    // work lists by class, n2 entries each
+    unsigned long long *hbase = nullptr;   // n2: place of the vertex's triangles among all pairs of all N+
+    int64_t pairs = 0;           // those pairs
     int2 *items = nullptr;       // {u, first range | one past the last range << 16}
     void *meta = nullptr;        // device-side sizes (RankMeta)
     int32_t n2 = 0;              // vertices of degree >= 2
