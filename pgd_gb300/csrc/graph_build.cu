@@ -258,39 +258,56 @@ __global__ void k_assort_partial(const int32_t *ev, const int32_t *eu, const int
 // int (Vertex, graphlet_vertex.h:42); order is key then id, id always
 // descending (decr_bound / incr_bound, graphlet_vertex.h:57-75).
 
-// Keys of the edges to order: every edge (ids == null, count == m) or the
-// sampled edge ids ids[0..count) (sort_edges with E_s, graphlet_core.cpp:
-// 836-851), whose natural key is the position in the sample.
+// The key of edge e (position i of the natural order), as the reference's int.
+__device__ __forceinline__ int32_t edge_key(const int32_t *ev, const int32_t *eu, const int32_t *deg,
+                                            const int32_t *core, const uint64_t *vsum, int64_t e, int64_t i, int kind) {
+    const int32_t v = ev[e], u = eu[e];
+    long long val = i;
+    // core[] exists only for the k-core keys
+    const bool kc = kind == PGD_ORD_KCORE || kind == PGD_ORD_KCORE_DEG;
+    const int kv = (kc && v >= 1) ? core[v - 1] : 0, ku = (kc && u >= 1) ? core[u - 1] : 0;
+    switch (kind) {
+    case PGD_ORD_DEG: val = deg[u] + deg[v]; break;
+    case PGD_ORD_KCORE: val = ku + kv; break;
+    case PGD_ORD_KCORE_DEG: val = (int)((unsigned)(deg[u] + deg[v]) * (unsigned)(ku + kv)); break;
+    case PGD_ORD_DEG_VOL:
+    case PGD_ORD_KCORE_VOL:
+    case PGD_ORD_KCORE_DEG_VOL: val = (long long)(vsum[u] + vsum[v]); break;
+    case PGD_ORD_DEG_U: val = deg[u]; break;
+    default: break;
+    }
+    return (int32_t)val;
+}
+
+// Every edge, last id first, with its key: a stable sort by the key alone then
+// leaves ties in descending id order.  The sign bit is flipped where keys may
+// be negative (32-bit keys), so that they sort as unsigned.
 __global__ void k_edge_keys(const int32_t *ev, const int32_t *eu, const int32_t *deg, const int32_t *core,
-                            const uint64_t *vsum, const int32_t *ids, int64_t count, int kind, int s2l,
-                            uint64_t *keys) {
-    for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < count; i += (int64_t)gridDim.x * blockDim.x) {
-        const int64_t e = ids ? ids[i] : i;
-        int32_t v = ev[e], u = eu[e];
-        long long val = i;
-        // core[] exists only for the k-core keys
-        const bool kc = kind == PGD_ORD_KCORE || kind == PGD_ORD_KCORE_DEG;
-        int kv = (kc && v >= 1) ? core[v - 1] : 0, ku = (kc && u >= 1) ? core[u - 1] : 0;
-        switch (kind) {
-        case PGD_ORD_DEG: val = deg[u] + deg[v]; break;
-        case PGD_ORD_KCORE: val = ku + kv; break;
-        case PGD_ORD_KCORE_DEG: val = (int)((unsigned)(deg[u] + deg[v]) * (unsigned)(ku + kv)); break;
-        case PGD_ORD_DEG_VOL:
-        case PGD_ORD_KCORE_VOL:
-        case PGD_ORD_KCORE_DEG_VOL: val = (long long)(vsum[u] + vsum[v]); break;
-        case PGD_ORD_DEG_U: val = deg[u]; break;
-        default: break;
-        }
-        uint32_t k32 = (uint32_t)(int32_t)val ^ 0x80000000u;
-        uint32_t id = (uint32_t)e;
-        keys[i] = ((uint64_t)k32 << 32) | (s2l ? (0xffffffffu - id) : id);
+                            const uint64_t *vsum, int64_t m, int kind, uint32_t flip, uint32_t *keys, int32_t *ids) {
+    for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < m; i += (int64_t)gridDim.x * blockDim.x) {
+        const int64_t e = m - 1 - i;
+        keys[i] = (uint32_t)edge_key(ev, eu, deg, core, vsum, e, e, kind) ^ flip;
+        ids[i] = (int32_t)e;
     }
 }
 
-__global__ void k_keys_to_ids(const uint64_t *keys, int64_t m, int s2l, int32_t *order) {
+// The sampled edge ids ids[0..count) (sort_edges with E_s, graphlet_core.cpp:
+// 836-851; the natural key is the position in the sample): key above idb bits
+// of the id, so that one sort orders by both.
+__global__ void k_sample_keys(const int32_t *ev, const int32_t *eu, const int32_t *deg, const int32_t *core,
+                              const uint64_t *vsum, const int32_t *ids, int64_t count, int kind, int s2l, uint32_t flip,
+                              int idb, uint64_t *keys) {
+    for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < count; i += (int64_t)gridDim.x * blockDim.x) {
+        const uint64_t e = (uint64_t)ids[i];
+        const uint32_t k = (uint32_t)edge_key(ev, eu, deg, core, vsum, (int64_t)e, i, kind) ^ flip;
+        keys[i] = ((uint64_t)k << idb) | (s2l ? ((1ull << idb) - 1 - e) : e);
+    }
+}
+
+__global__ void k_keys_to_ids(const uint64_t *keys, int64_t m, int s2l, int idb, int32_t *order) {
     for (int64_t e = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; e < m; e += (int64_t)gridDim.x * blockDim.x) {
-        uint32_t lo = (uint32_t)(keys[e] & 0xffffffffu);
-        order[e] = (int32_t)(s2l ? (0xffffffffu - lo) : lo);
+        const uint64_t lo = keys[e] & ((1ull << idb) - 1);
+        order[e] = (int32_t)(s2l ? ((1ull << idb) - 1 - lo) : lo);
     }
 }
 
@@ -830,22 +847,59 @@ static pgd_status sort_edges_impl(pgd_graph *g, int kind, int s2l, const int32_t
         PGD_LAUNCH(ctx, k_neigh_sum, grid_for(g->n * 32), kThreads, 0, g->off, g->adj, g->deg, g->core, g->n,
                                                               kind == PGD_ORD_KCORE_VOL ? 1 : 2, vsum);
     }
-    uint64_t *keys = nullptr, *keys2 = nullptr;
-    if ((st = pgd_tmp_alloc(ctx, (void **)&keys, count * sizeof(uint64_t)))) return st;
-    if ((st = pgd_tmp_alloc(ctx, (void **)&keys2, count * sizeof(uint64_t)))) return st;
-    PGD_LAUNCH(ctx, k_edge_keys, grid_for(count), kThreads, 0, g->ev, g->eu, g->deg, g->core, vsum, d_ids, count, kind,
-               s2l, keys);
+    // bits of the keys: all 32 where they may be negative (volumes and products
+    // wrap as the reference's ints do)
+    const uint64_t d2 = 2 * (uint64_t)g->max_degree, c2 = 2 * (uint64_t)g->max_core;
+    uint64_t top = UINT64_MAX;   // largest key, where it is known
+    switch (kind) {
+    case PGD_ORD_DEG: top = d2; break;
+    case PGD_ORD_KCORE: top = c2; break;
+    case PGD_ORD_KCORE_DEG: top = d2 * c2; break;
+    case PGD_ORD_DEG_U: top = d2 / 2; break;
+    case PGD_ORD_DEG_VOL:
+    case PGD_ORD_KCORE_VOL:
+    case PGD_ORD_KCORE_DEG_VOL: break;
+    default: top = (uint64_t)count; break;
+    }
+    const bool small = top < 0x80000000ull;
+    const int kb = small ? std::max(1, bit_length(top)) : 32;
+    const uint32_t flip = small ? 0u : 0x80000000u;
     size_t tb = 0;
     void *tmp = nullptr;
-    if (s2l) cub::DeviceRadixSort::SortKeys(nullptr, tb, keys, keys2, count, 0, 64, s);
-    else cub::DeviceRadixSort::SortKeysDescending(nullptr, tb, keys, keys2, count, 0, 64, s);
-    if ((st = pgd_tmp_alloc(ctx, &tmp, tb))) return st;
-    if (s2l) cub::DeviceRadixSort::SortKeys(tmp, tb, keys, keys2, count, 0, 64, s);
-    else cub::DeviceRadixSort::SortKeysDescending(tmp, tb, keys, keys2, count, 0, 64, s);
-    pgd_tmp_free(ctx, tmp);
-    PGD_LAUNCH(ctx, k_keys_to_ids, grid_for(count), kThreads, 0, keys2, count, s2l, g->order);
-    pgd_tmp_free(ctx, keys);
-    pgd_tmp_free(ctx, keys2);
+    if (!d_ids) {
+        uint32_t *keys = nullptr, *keys2 = nullptr;
+        int32_t *ids = nullptr;
+        if ((st = pgd_tmp_alloc(ctx, (void **)&keys, count * sizeof(uint32_t)))) return st;
+        if ((st = pgd_tmp_alloc(ctx, (void **)&keys2, count * sizeof(uint32_t)))) return st;
+        if ((st = pgd_tmp_alloc(ctx, (void **)&ids, count * sizeof(int32_t)))) return st;
+        PGD_LAUNCH(ctx, k_edge_keys, grid_for(count), kThreads, 0, g->ev, g->eu, g->deg, g->core, vsum, count, kind,
+                   flip, keys, ids);
+        if (s2l) cub::DeviceRadixSort::SortPairs(nullptr, tb, keys, keys2, ids, g->order, count, 0, kb, s);
+        else cub::DeviceRadixSort::SortPairsDescending(nullptr, tb, keys, keys2, ids, g->order, count, 0, kb, s);
+        if ((st = pgd_tmp_alloc(ctx, &tmp, tb))) return st;
+        if (s2l) cub::DeviceRadixSort::SortPairs(tmp, tb, keys, keys2, ids, g->order, count, 0, kb, s);
+        else cub::DeviceRadixSort::SortPairsDescending(tmp, tb, keys, keys2, ids, g->order, count, 0, kb, s);
+        pgd_tmp_free(ctx, tmp);
+        pgd_tmp_free(ctx, keys);
+        pgd_tmp_free(ctx, keys2);
+        pgd_tmp_free(ctx, ids);
+    } else {
+        uint64_t *keys = nullptr, *keys2 = nullptr;
+        if ((st = pgd_tmp_alloc(ctx, (void **)&keys, count * sizeof(uint64_t)))) return st;
+        if ((st = pgd_tmp_alloc(ctx, (void **)&keys2, count * sizeof(uint64_t)))) return st;
+        const int idb = std::max(1, bit_length((uint64_t)m));
+        PGD_LAUNCH(ctx, k_sample_keys, grid_for(count), kThreads, 0, g->ev, g->eu, g->deg, g->core, vsum, d_ids, count,
+                   kind, s2l, flip, idb, keys);
+        if (s2l) cub::DeviceRadixSort::SortKeys(nullptr, tb, keys, keys2, count, 0, kb + idb, s);
+        else cub::DeviceRadixSort::SortKeysDescending(nullptr, tb, keys, keys2, count, 0, kb + idb, s);
+        if ((st = pgd_tmp_alloc(ctx, &tmp, tb))) return st;
+        if (s2l) cub::DeviceRadixSort::SortKeys(tmp, tb, keys, keys2, count, 0, kb + idb, s);
+        else cub::DeviceRadixSort::SortKeysDescending(tmp, tb, keys, keys2, count, 0, kb + idb, s);
+        pgd_tmp_free(ctx, tmp);
+        PGD_LAUNCH(ctx, k_keys_to_ids, grid_for(count), kThreads, 0, keys2, count, s2l, idb, g->order);
+        pgd_tmp_free(ctx, keys);
+        pgd_tmp_free(ctx, keys2);
+    }
     if (vsum && vsum != g->vol2) pgd_tmp_free(ctx, vsum);
     PGD_CUDA(ctx, cudaGetLastError());
     g->sorted = true;

@@ -78,7 +78,6 @@ constexpr int kCycHashMax = 4096;
 constexpr int kMaxRanges = 8192;
 constexpr int64_t kKeepBytes = 16ll << 30;     // largest bound of the triangle lists kept between the passes
 constexpr int64_t kBposBytes = 4ll << 30;      // largest table of range boundaries per row
-constexpr int kDirectThreads = 1024;
 constexpr uint32_t kDirectWords = 50 * 1024;   // counter words of one item: 200 KB of shared memory
 
 // Sizes found on the device while the graph is built.
@@ -564,7 +563,7 @@ __device__ __forceinline__ uint32_t take_128(const uint32_t *wcode, uint32_t s, 
 // (Sharing rows from 1,024 entries costs more turns than it balances: R-MAT 20
 // 30.0 against 25.3 ms; one block-wide prefix sum per 1,024 rows with equal
 // shares for the warps spent a third of its time at its barriers.)
-template <bool ACC, typename Fn>
+template <int NT, bool ACC, typename Fn>
 __device__ __forceinline__ void walk_rows(const CycArgs &A, uint32_t u, int k0, int k1, uint32_t *next, uint32_t *acc,
                                           Fn fn) {
     const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
@@ -600,7 +599,7 @@ __device__ __forceinline__ void walk_rows(const CycArgs &A, uint32_t u, int k0, 
             const int pieces = (n + 127) >> 7;
             uint32_t a = 0;
             const bool any = turn < pieces;
-            for (; turn < pieces; turn += kDirectThreads / 32) a += take_128(A.wcode, s, n, turn << 7, lane, fn);
+            for (; turn < pieces; turn += NT / 32) a += take_128(A.wcode, s, n, turn << 7, lane, fn);
             turn -= pieces;
             if (ACC && any) {
                 __syncwarp();
@@ -669,10 +668,12 @@ __device__ __forceinline__ void walk_rows(const CycArgs &A, uint32_t u, int k0, 
 }
 
 // Many wedges: one block per (u, ranges of w), a counter per w in shared
-// memory at its bit address.
-__global__ void __launch_bounds__(kDirectThreads, 1) k_cycle_direct(CycArgs A) {
+// memory at its bit address.  Graphs whose counters all fit in 100 or 50 KB run
+// it with 2 or 4 smaller blocks per SM, which hide each other's barriers.
+template <int NT>
+__global__ void __launch_bounds__(NT, 1024 / NT) k_cycle_direct(CycArgs A) {
     extern __shared__ __align__(16) uint32_t s_dyn[];
-    __shared__ uint32_t s_acc[kDirectThreads / 32][32];
+    __shared__ uint32_t s_acc[NT / 32][32];
     __shared__ uint32_t s_item, s_next[2];
     const RankMeta *M = A.M;
     uint32_t *acc = s_acc[threadIdx.x >> 5];
@@ -689,7 +690,7 @@ __global__ void __launch_bounds__(kDirectThreads, 1) k_cycle_direct(CycArgs A) {
         const int k0 = it.y & 0xffff, k1 = it.y >> 16;
         const uint32_t first = code_of(M, max(M->bound[k0], u + 1)), end = code_of(M, M->bound[k1]);
         const uint32_t c0 = first & ~31u, words = (end - c0 + 31) / 32;
-        for (uint32_t i = threadIdx.x; i < words; i += kDirectThreads) s_dyn[i] = 0;
+        for (uint32_t i = threadIdx.x; i < words; i += NT) s_dyn[i] = 0;
         // the item's counter widths: mostly two, below and from thr
         int tier = 0;
         while (tier < 4 && M->tcode[tier] <= first) tier++;
@@ -697,19 +698,19 @@ __global__ void __launch_bounds__(kDirectThreads, 1) k_cycle_direct(CycArgs A) {
         const bool two = end <= thr || tier >= 3 || end <= M->tcode[tier + 1];
         const uint32_t mlo = mask_of(M, first), mhi = mask_of(M, thr);
         __syncthreads();
-        walk_rows<false>(A, u, k0, k1, &s_next[0], acc, [&](uint32_t c, uint32_t) {
+        walk_rows<NT, false>(A, u, k0, k1, &s_next[0], acc, [&](uint32_t c, uint32_t) {
             atomicAdd(s_dyn + ((c - c0) >> 5), 1u << (c & 31));
             return 0u;
         });
         __syncthreads();
         if (two) {
-            walk_rows<true>(A, u, k0, k1, &s_next[1], acc, [&](uint32_t c, uint32_t q) {
+            walk_rows<NT, true>(A, u, k0, k1, &s_next[1], acc, [&](uint32_t c, uint32_t q) {
                 const uint32_t k = ((s_dyn[(c - c0) >> 5] >> (c & 31)) & (c < thr ? mlo : mhi)) - 1;
                 if (k) atomicAdd(A.cyc + q, k);
                 return k;
             });
         } else {
-            walk_rows<true>(A, u, k0, k1, &s_next[1], acc, [&](uint32_t c, uint32_t q) {
+            walk_rows<NT, true>(A, u, k0, k1, &s_next[1], acc, [&](uint32_t c, uint32_t q) {
                 const uint32_t k = ((s_dyn[(c - c0) >> 5] >> (c & 31)) & mask_of(M, c)) - 1;
                 if (k) atomicAdd(A.cyc + q, k);
                 return k;
@@ -1064,7 +1065,9 @@ __device__ __forceinline__ void clique_hits(const EgoArgs &A, const uint2 *hits,
 
 // |N+(a)| = d in a block's range: a block per vertex.  The indices of N+(a) go
 // into the lookup tables; each warp takes vertices x of N+(a) and looks the
-// entries of N+(x) up.  PASS 1 counts the triangles and, where there is room,
+// entries of N+(x) up (searching N+(a)'s entries in N+(x) where that takes fewer
+// instructions is bound by the searches' latency: 5.0 against 5.4 ms for the
+// smaller class on R-MAT 20, 2.9 against 2.1 ms for the next).  PASS 1 counts the triangles and, where there is room,
 // keeps them for k_clique_block; PASS 2 (else) lists them again, with F.
 template <int PASS, int NT, bool GLOBAL>
 __global__ void __launch_bounds__(NT) k_ego_block(EgoArgs A, int dmax) {
@@ -1126,8 +1129,30 @@ __global__ void __launch_bounds__(NT) k_ego_block(EgoArgs A, int dmax) {
             if (i < 1) break;   // the first neighbour has none of the others above it
             const uint32_t r0 = T.rs[i];
             const int len = T.ru[i];
-            const int32_t last = T.ls[i - 1];
             uint32_t found = 0;
+            // a triangle for each lane with j >= 0: index j of y in N+(a), slot pos
+            auto take = [&](int j, uint32_t pos) {
+                const unsigned m = __ballot_sync(kFull, j >= 0);
+                if (!m) return;
+                if (hits) {
+                    uint32_t at = 0;
+                    if (lane == 0) at = atomicAdd(&s_nhit, (uint32_t)__popc(m));
+                    at = __shfl_sync(kFull, at, 0);
+                    if (j >= 0)
+                        hits[at + __popc(m & ((1u << lane) - 1))] = make_uint2((uint32_t)i << 16 | (uint32_t)j, pos);
+                }
+                if (PASS == 1) {
+                    if (j >= 0) {
+                        atomicAdd(A.t + pos, 1u);
+                        atomicAdd(T.ck + j, 1u);
+                    }
+                    found += __popc(m);
+                } else if (j >= 0) {
+                    atomicOr(F32 + (int64_t)i * 2 * WS + (j >> 5), 1u << (j & 31));
+                    atomicOr(F32 + (int64_t)j * 2 * WS + (i >> 5), 1u << (i & 31));
+                }
+            };
+            const int32_t last = T.ls[i - 1];
             for (int b = 0; b < len; b += 32) {
                 const int32_t y = b + lane < len ? __ldg(A.radj + r0 + b + lane) : 0x7fffffff;
                 int jx = -1;
@@ -1139,28 +1164,7 @@ __global__ void __launch_bounds__(NT) k_ego_block(EgoArgs A, int dmax) {
                     while ((k = T.hkey[h]) != (uint32_t)y && k != kFull) h = (h + 1) & hmask;
                     if (k == (uint32_t)y) jx = T.hidx[h];
                 }
-                const bool hit = jx >= 0;
-                const unsigned m = __ballot_sync(kFull, hit);
-                if (m) {
-                    if (hits) {
-                        uint32_t at = 0;
-                        if (lane == 0) at = atomicAdd(&s_nhit, (uint32_t)__popc(m));
-                        at = __shfl_sync(kFull, at, 0);
-                        if (hit)
-                            hits[at + __popc(m & ((1u << lane) - 1))] =
-                                make_uint2((uint32_t)i << 16 | (uint32_t)jx, r0 + (uint32_t)(b + lane));
-                    }
-                    if (PASS == 1) {
-                        if (hit) {
-                            atomicAdd(A.t + r0 + b + lane, 1u);
-                            atomicAdd(T.ck + jx, 1u);
-                        }
-                        found += __popc(m);
-                    } else if (hit) {
-                        atomicOr(F32 + (int64_t)i * 2 * WS + (jx >> 5), 1u << (jx & 31));
-                        atomicOr(F32 + (int64_t)jx * 2 * WS + (i >> 5), 1u << (i & 31));
-                    }
-                }
+                take(jx, r0 + (uint32_t)(b + lane));
                 if (__shfl_sync(kFull, y, 31) > last) break;   // ascending: nothing more at or below last
             }
             if (PASS == 1 && lane == 0 && found) atomicAdd(T.ck + i, found);
@@ -1434,6 +1438,9 @@ void pgd_rank_drop(pgd_graph *g) {
         }                                                 \
     } while (0)
 
+// Blocks of k_cycle_direct per SM: as many as all counters fit in.
+static int direct_factor(int64_t words) { return words < kDirectWords / 4 ? 4 : words < kDirectWords / 2 ? 2 : 1; }
+
 pgd_status pgd_rank_build(pgd_graph *g, int64_t nnz, const int32_t *vgraph, const uint8_t *vmask, pgd_rank_graph *R) {
     pgd_ctx *ctx = g->ctx;
     cudaStream_t s = ctx->stream;
@@ -1518,7 +1525,7 @@ pgd_status pgd_rank_build(pgd_graph *g, int64_t nnz, const int32_t *vgraph, cons
     if (h.direct_wedges == 0) return PGD_OK;
     // items of the vertices with many wedges, by ranges of the wedges' ends:
     // fine enough to balance the items, and at most half an item's counters each
-    const int64_t words = ((int64_t)h.tcode[4] + 31) / 32;
+    const int64_t words = R->words = ((int64_t)h.tcode[4] + 31) / 32;
     R->nranges = (int32_t)std::min<int64_t>(kMaxRanges, std::max<int64_t>(16, 2 * (2 * words / kDirectWords + 1)));
     PGD_LAUNCH(ctx, k_rank_bounds, 1, 128, 0, R->roff, R->nranges, M);
     const int64_t bpos_bytes = (int64_t)(R->nranges - 1) * n2 * (int64_t)sizeof(uint32_t);
@@ -1530,7 +1537,7 @@ pgd_status pgd_rank_build(pgd_graph *g, int64_t nnz, const int32_t *vgraph, cons
     uint32_t *count = nullptr, *pos = nullptr;
     RB_TRY(tg.alloc(&count, ((size_t)n2 + 1) * sizeof(uint32_t)));
     RB_TRY(tg.alloc(&pos, ((size_t)n2 + 1) * sizeof(uint32_t)));
-    const int parts = ctx->num_sms * 8;
+    const int parts = ctx->num_sms * 4 * (1 + direct_factor(words));
     PGD_LAUNCH(ctx, k_rank_items, grid_for(n2 + 1), kThreads, 0, wd, n2, R->nranges, M, parts, count,
                (const uint32_t *)nullptr, (int2 *)nullptr);
     RB_CUDA(cub::DeviceScan::ExclusiveSum(tmp, tb, count, pos, (int64_t)n2 + 1, s));
@@ -1613,13 +1620,15 @@ static void ego_pass(pgd_ctx *ctx, const pgd_rank_graph &R, EgoArgs A, int pass,
 // Shared-memory limits of the kernels that use more than the default, set to
 // the same values by every caller.
 static cudaError_t rank_kernel_limits() {
-    cudaError_t e = cudaFuncSetAttribute(k_cycle_direct, cudaFuncAttributeMaxDynamicSharedMemorySize, kDirectWords * 4);
-    if (e == cudaSuccess) e = cudaFuncSetAttribute(k_cycle_hash, cudaFuncAttributeMaxDynamicSharedMemorySize, kHashSmem);
-    if (e == cudaSuccess) e = cudaFuncSetAttribute(k_cycle_warp, cudaFuncAttributeMaxDynamicSharedMemorySize, kWarpSmem);
+    constexpr cudaFuncAttribute kDyn = cudaFuncAttributeMaxDynamicSharedMemorySize;
+    cudaError_t e = cudaFuncSetAttribute(k_cycle_direct<1024>, kDyn, kDirectWords * 4);
+    if (e == cudaSuccess) e = cudaFuncSetAttribute(k_cycle_direct<512>, kDyn, kDirectWords * 2);
+    if (e == cudaSuccess) e = cudaFuncSetAttribute(k_cycle_direct<256>, kDyn, kDirectWords);
+    if (e == cudaSuccess) e = cudaFuncSetAttribute(k_cycle_hash, kDyn, kHashSmem);
+    if (e == cudaSuccess) e = cudaFuncSetAttribute(k_cycle_warp, kDyn, kWarpSmem);
     const int cmax = kEgoMax[kEgoC];
     const int c1 = (int)ego_table_bytes(cmax, true, false), c2 = (int)ego_table_bytes(cmax, true, true),
               b2 = (int)ego_table_bytes(kEgoMax[kEgoB], true, true), k2 = (int)ego_table_bytes(cmax, false, true);
-    constexpr cudaFuncAttribute kDyn = cudaFuncAttributeMaxDynamicSharedMemorySize;
     if (e == cudaSuccess) e = cudaFuncSetAttribute(k_ego_block<1, 1024, false>, kDyn, c1);
     if (e == cudaSuccess) e = cudaFuncSetAttribute(k_ego_block<2, 1024, false>, kDyn, c2);
     if (e == cudaSuccess) e = cudaFuncSetAttribute(k_ego_block<2, 512, false>, kDyn, b2);
@@ -1661,7 +1670,12 @@ static pgd_status cycle_pass(pgd_ctx *ctx, const pgd_rank_graph &R, CycArgs C, u
         B.items = R.items;
         B.count = R.nitems;
         B.next = ctr;
-        PGD_LAUNCH(ctx, k_cycle_direct, (int)std::min<int64_t>(R.nitems, nsm), kDirectThreads, kDirectWords * 4, B);
+        const int f = direct_factor(R.words);
+        const int blocks = (int)std::min<int64_t>(R.nitems, (int64_t)f * nsm);
+        const size_t smem = std::min<size_t>(kDirectWords * 4 / f, (size_t)(R.words + 1) * 4);
+        if (f == 1) PGD_LAUNCH(ctx, k_cycle_direct<1024>, blocks, 1024, smem, B);
+        else if (f == 2) PGD_LAUNCH(ctx, k_cycle_direct<512>, blocks, 512, smem, B);
+        else PGD_LAUNCH(ctx, k_cycle_direct<256>, blocks, 256, smem, B);
     }
     if (R.nlist[kCycHash]) {
         CycArgs B = C;

@@ -29,6 +29,7 @@ struct pgd_rank_graph {
     int32_t nranges = 0;
     int32_t max_up = 0;          // largest rup
     uint32_t nitems = 0;
+    int64_t words = 0;           // 32-bit words of all counters
     uint32_t nlist[8] = {0};
     void *held[12] = {nullptr};  // the allocations above
     size_t held_bytes[12] = {0};
