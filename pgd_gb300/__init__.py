@@ -69,6 +69,9 @@ class pgd_counts(ctypes.Structure):
                 ("hub_ms", ctypes.c_float), ("tri_ms", ctypes.c_float), ("reserved", ctypes.c_float)]
 
 
+_WORDS = ctypes.sizeof(pgd_counts) // 8
+
+
 class pgd_server_opts(ctypes.Structure):
     _fields_ = [("device", ctypes.c_int), ("workers", ctypes.c_int), ("max_batch", ctypes.c_int),
                 ("max_wait_ms", ctypes.c_int), ("hbm_budget", ctypes.c_uint64)]
@@ -184,16 +187,49 @@ def close_counts(sums, n, m):
 
 
 class Counts:
-    """Result of one decomposition."""
+    """Result of one decomposition: views of the 36 words of a pgd_counts."""
+
+    __slots__ = ("_w",)
 
     def __init__(self, c):
-        self.totals = np.array(list(c.totals), dtype=np.uint64)
-        self.sums = np.array(list(c.sums), dtype=np.uint64)
-        self.n, self.m, self.kernel_ms = c.n, c.m, c.kernel_ms
-        self.hub_ms, self.tri_ms = c.hub_ms, c.tri_ms
+        self._w = np.frombuffer(c, np.uint64, _WORDS) if isinstance(c, pgd_counts) else c
+
+    @property
+    def totals(self):
+        return self._w[:NTOTALS]
+
+    @property
+    def sums(self):
+        return self._w[NTOTALS:NTOTALS + NSUMS]
+
+    @property
+    def n(self):
+        return int(self._w[NTOTALS + NSUMS])
+
+    @property
+    def m(self):
+        return int(self._w[NTOTALS + NSUMS + 1])
+
+    @property
+    def kernel_ms(self):
+        return float(self._w[-2:].view(np.float32)[0])
+
+    @property
+    def hub_ms(self):
+        return float(self._w[-2:].view(np.float32)[1])
+
+    @property
+    def tri_ms(self):
+        return float(self._w[-2:].view(np.float32)[2])
 
     def as_dict(self):
         return {k: int(v) for k, v in zip(TOTAL_NAMES, self.totals)}
+
+
+def _counts_list(out):
+    """The results of a ctypes array of pgd_counts, each a view of its words
+    (no copy and no per-field conversion: a batch has thousands of them)."""
+    return [Counts(w) for w in np.frombuffer(out, np.uint64).reshape(-1, _WORDS)]
 
 
 class Context:
@@ -300,14 +336,14 @@ class Context:
         out = (pgd_counts * k)()
         self._check(lib().pgd_decompose_pairs_batch(self.h, k, off, src, dst, _ptr(nm), out),
                     "pgd_decompose_pairs_batch")
-        return [Counts(c) for c in out]
+        return _counts_list(out)
 
     def decompose_batch(self, graphs, micro=False):
         arr = (ctypes.c_void_p * len(graphs))(*[g.h.value for g in graphs])
         out = (pgd_counts * len(graphs))()
         self._check(lib().pgd_decompose_batch(self.h, arr, len(graphs), MICRO if micro else 0, out),
                     "pgd_decompose_batch")
-        return [Counts(c) for c in out]
+        return _counts_list(out)
 
 
 class Graph:
