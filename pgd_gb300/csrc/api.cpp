@@ -112,6 +112,8 @@ extern "C" pgd_status pgd_context_create(const pgd_opts *opts, pgd_ctx **out) {
         cudaEventCreate(&ctx->ev0) != cudaSuccess || cudaEventCreate(&ctx->ev1) != cudaSuccess ||
         cudaEventCreate(&ctx->evt0) != cudaSuccess || cudaEventCreate(&ctx->evt1) != cudaSuccess ||
         cudaEventCreate(&ctx->evh0) != cudaSuccess || cudaEventCreate(&ctx->evh1) != cudaSuccess ||
+        cudaHostAlloc((void **)&ctx->pin, kPinBytes, cudaHostAllocDefault) != cudaSuccess ||
+        pgd_decompose_limits() != cudaSuccess || pgd_rank_limits() != cudaSuccess ||
         cudaStreamCreateWithFlags(&ctx->side, cudaStreamNonBlocking) != cudaSuccess ||
         cudaEventCreateWithFlags(&ctx->ev_fork, cudaEventDisableTiming) != cudaSuccess ||
         cudaEventCreateWithFlags(&ctx->ev_join, cudaEventDisableTiming) != cudaSuccess) {
@@ -129,6 +131,7 @@ extern "C" pgd_status pgd_context_destroy(pgd_ctx *ctx) {
     if (ctx->stream) cudaStreamSynchronize(ctx->stream);
     if (ctx->d_sums) cudaFree(ctx->d_sums);
     if (ctx->d_ctr) cudaFree(ctx->d_ctr);
+    if (ctx->pin) cudaFreeHost(ctx->pin);
     if (ctx->ev0) cudaEventDestroy(ctx->ev0);
     if (ctx->ev1) cudaEventDestroy(ctx->ev1);
     for (cudaEvent_t e : {ctx->evt0, ctx->evt1, ctx->evh0, ctx->evh1, ctx->ev_fork, ctx->ev_join})

@@ -119,10 +119,6 @@ __device__ __forceinline__ int batch_find(const int64_t *base, int k, int64_t x)
     return lo;
 }
 
-__device__ __forceinline__ bool dense_edge(const DevGraph &G, int64_t e) {
-    return G.gdense && G.gdense[G.egraph[e]];
-}
-
 __device__ __forceinline__ bool ranks_above(int32_t a, int32_t b, const int32_t *deg) {
     int da = deg[a], db = deg[b];
     return da > db || (da == db && a > b);
@@ -278,9 +274,6 @@ __global__ void k_tslot(DevGraph G, int4 *slot, const int32_t *pos, int64_t coun
     const int64_t total = pos ? count : G.m;
     for (int64_t i = (blockIdx.x * (int64_t)blockDim.x + threadIdx.x) >> 5; i < total; i += nw) {
         const int64_t id = pos ? G.order[pos[i]] : i;
-        // in a batch each graph's edge ids and E_ordered positions cover the
-        // same range, so egraph[id] is the edge's graph
-        if (dense_edge(G, id)) continue;
         const int32_t a = G.ev[id], b = G.eu[id];
         const int da = G.deg[a], db = G.deg[b];
         const int32_t s = da <= db ? a : b, l = da <= db ? b : a;
@@ -302,29 +295,22 @@ __global__ void k_tslot(DevGraph G, int4 *slot, const int32_t *pos, int64_t coun
 // them by anchor, highest-degree anchors first (the largest work items are
 // handed out first).  (Heaviest-edge-first within an anchor shortens the
 // items' tails but was measured slower: all warps then gather hub lists at
-// once.)  Dense-graph edges (batches only) get class n, the rest n + 1, so
-// the sorted order is [hub-anchored, by anchor][dense][light].  eb bits hold
-// a position; the sort needs eb + bits(n + 2) key bits.
+// once.)  The other edges get class n, so the sorted order is [hub-anchored, by
+// anchor][light].  eb bits hold a position; the sort needs eb + bits(n + 1) key
+// bits.
 __global__ void k_plan_keys(DevGraph G, uint64_t *keys, int32_t *vals, unsigned long long *counts, int eb) {
-    unsigned long long hubs = 0, dense = 0;
+    unsigned long long hubs = 0;
     for (int64_t e = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; e < G.npos; e += (int64_t)gridDim.x * blockDim.x) {
         const int32_t id = G.order[e];
         const int32_t v = G.ev[id], u = G.eu[id];
         const int32_t p = ranks_above(v, u, G.deg) ? v : u;
-        const bool d = dense_edge(G, e);
-        const bool hub = !d && G.deg[p] >= G.anchor_hub;
-        const uint64_t cls = d ? (uint64_t)G.n : (hub ? (uint64_t)G.vrank[p] : (uint64_t)G.n + 1);
-        keys[e] = (cls << eb) | (uint64_t)e;
+        const bool hub = G.deg[p] >= G.anchor_hub;
+        keys[e] = ((hub ? (uint64_t)G.vrank[p] : (uint64_t)G.n) << eb) | (uint64_t)e;
         vals[e] = (int32_t)e;
         hubs += hub;
-        dense += d;
     }
     hubs = pgd_warp_sum(hubs);
-    dense = pgd_warp_sum(dense);
-    if ((threadIdx.x & 31) == 0) {
-        if (hubs) atomicAdd(counts, hubs);
-        if (dense) atomicAdd(counts + 3, dense);
-    }
+    if ((threadIdx.x & 31) == 0 && hubs) atomicAdd(counts, hubs);
 }
 
 // item i starts a chunk: the first edge of an anchor's run of L edges, or
@@ -1147,23 +1133,8 @@ __global__ void __launch_bounds__(kLightWarps * 32) k_light(LightArgs A) {
 }
 
 // ---------------------------------------------------------------------------
-// Small graphs (batches): one warp per edge with whole adjacency rows as
-// bitsets.  A row of up to 2048 vertices is 32 words of 64 bits, one per
-// lane, so with A_x the row of x, T = A_p & A_q,
-// S_p = A_p & ~A_q & ~{q}, S_q = A_q & ~A_p & ~{p}:
-//   t = popc(T),  c4 = sum_{w in S_q} popc(A_w & S_p),
-//   k4 = 1/2 sum_{x in T} popc(A_x & T),
-// each row read once, coalesced, from L2.
-
-struct DenseArgs {
-    DevGraph G;
-    const uint64_t *bits;     // rows of every dense graph, concatenated
-    const int64_t *wbase;     // per graph: first word of its rows
-    const int64_t *vbase;     // per graph: first union vertex id
-    const int32_t *dpos;      // E_ordered positions of dense-graph edges
-    int64_t ndense;
-    unsigned long long *next;
-};
+// Dense graphs (batches): adjacency rows as bitsets.  A row of up to 2048
+// vertices is 32 words of 64 bits, one per lane of a warp.
 
 __global__ void k_dense_bits(const int64_t *off, const int32_t *adj, const int32_t *vgraph, const uint8_t *gdense,
                              const int64_t *wbase, const int64_t *vbase, const long long *gnm, int64_t N,
@@ -1189,119 +1160,21 @@ __device__ __forceinline__ int32_t dense_q(const DevGraph &G, int64_t e) {
     return G.deg[v] <= G.deg[u] ? v : u;
 }
 
-// Sort keys grouping the dense-graph edges by q (then by position), so that
-// k_dense can serve several edges with one pass over A_q's rows:
-// (plain << (qb + eb)) | (q << eb) | position, q below 2^qb and positions
-// below 2^eb.  Edges of graphs with a common-neighbour matrix (cbase[g] >= 0,
-// plain = 0) sort first.
-__global__ void k_dense_keys(DevGraph G, const int32_t *dpos, int64_t nd, const int64_t *cbase, uint64_t *keys,
-                             int32_t *vals, unsigned long long *ncn, int qb, int eb) {
-    unsigned long long cnt = 0;
-    for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < nd; i += (int64_t)gridDim.x * blockDim.x) {
-        const int32_t e = dpos[i];
-        const uint64_t plain = (cbase && cbase[G.egraph[e]] >= 0) ? 0ull : 1ull;
-        keys[i] = (plain << (qb + eb)) | ((uint64_t)(uint32_t)dense_q(G, e) << eb) | (uint32_t)e;
-        vals[i] = e;
-        cnt += 1ull - plain;
+// Sort keys grouping the dense-graph edges by q (then by position), so that one
+// pass over the rows of q's neighbours serves several: (q << eb) | position, q
+// below 2^qb and positions below 2^eb.  A graph's edges are consecutive
+// positions; before[g] of the edges before them belong to sparse graphs.
+__global__ void k_dense_keys(DevGraph G, const int64_t *before, uint64_t *keys, int32_t *vals, int eb) {
+    for (int64_t e = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; e < G.npos; e += (int64_t)gridDim.x * blockDim.x) {
+        const int g = G.egraph[e];
+        if (!G.gdense[g]) continue;
+        const int64_t i = e - before[g];
+        keys[i] = ((uint64_t)(uint32_t)dense_q(G, e) << eb) | (uint64_t)e;
+        vals[i] = (int32_t)e;
     }
-    cnt = pgd_warp_sum(cnt);
-    if ((threadIdx.x & 31) == 0 && cnt) atomicAdd(ncn, cnt);
 }
 
 constexpr int kDenseGroup = 6;   // edges sharing q decomposed together
-
-// Up to kDenseGroup edges (p_j, q) with the same q: one pass over the rows of
-// A_q's neighbours w serves all of them -- row w is ANDed with S_p_j when
-// w is in S_q_j and with T_j when w is in T_j.
-__global__ void __launch_bounds__(256, 3) k_dense(DenseArgs A) {
-    __shared__ unsigned long long s_red[8][PGD_NSUMS];
-    const DevGraph &G = A.G;
-    const int lane = threadIdx.x & 31;
-    int cur_g = -1;
-    unsigned long long acc[PGD_NSUMS];
-#pragma unroll
-    for (int i = 0; i < PGD_NSUMS; i++) acc[i] = 0;
-    while (true) {
-        unsigned long long idx = 0;
-        if (lane == 0) idx = atomicAdd(A.next, (unsigned long long)kDenseGroup);
-        idx = __shfl_sync(0xffffffffu, idx, 0);
-        if (idx >= (unsigned long long)A.ndense) break;
-        const int64_t iend = min(idx + (unsigned long long)kDenseGroup, (unsigned long long)A.ndense);
-        int64_t i0 = (int64_t)idx;
-        while (i0 < iend) {
-            // the run of edges with the same q (dpos is grouped by q)
-            const int32_t qg = dense_q(G, A.dpos[i0]);
-            int64_t i1 = i0 + 1;
-            while (i1 < iend && dense_q(G, A.dpos[i1]) == qg) i1++;
-            const int R = (int)(i1 - i0);
-            const int g = G.egraph[A.dpos[i0]];
-            const int64_t vb = A.vbase[g];
-            const int W = (int)((G.gnm[2 * g] + 63) >> 6);
-            const uint64_t *rows = A.bits + A.wbase[g];
-            const int64_t q = qg - vb;
-            const uint64_t Aq = lane < W ? __ldg(rows + q * W + lane) : 0ull;
-            const uint64_t bq = (lane == (int)(q >> 6)) ? (1ull << (q & 63)) : 0ull;
-            uint64_t T[kDenseGroup], Sp[kDenseGroup], Sq[kDenseGroup];
-            unsigned c4[kDenseGroup], k4x2[kDenseGroup];
-#pragma unroll
-            for (int j = 0; j < kDenseGroup; j++) {
-                T[j] = Sp[j] = Sq[j] = 0;
-                c4[j] = k4x2[j] = 0;
-                if (j < R) {
-                    const int32_t id = G.order[A.dpos[i0 + j]];
-                    const int32_t v = G.ev[id], u = G.eu[id];
-                    const int64_t p = (v == qg ? u : v) - vb;
-                    const uint64_t Ap = lane < W ? __ldg(rows + p * W + lane) : 0ull;
-                    const uint64_t bp = (lane == (int)(p >> 6)) ? (1ull << (p & 63)) : 0ull;
-                    T[j] = Ap & Aq;
-                    Sp[j] = Ap & ~Aq & ~bq;
-                    Sq[j] = Aq & ~Ap & ~bp;
-                }
-            }
-            for (int L = 0; L < W; L++) {
-                uint64_t wq = __shfl_sync(0xffffffffu, Aq, L);
-                uint64_t ws[kDenseGroup], wt[kDenseGroup];
-#pragma unroll
-                for (int j = 0; j < kDenseGroup; j++) {
-                    ws[j] = __shfl_sync(0xffffffffu, Sq[j], L);
-                    wt[j] = __shfl_sync(0xffffffffu, T[j], L);
-                }
-                while (wq) {
-                    const int b0 = __ffsll(wq) - 1;
-                    wq &= wq - 1;
-                    int b1 = -1;
-                    if (wq) {
-                        b1 = __ffsll(wq) - 1;
-                        wq &= wq - 1;
-                    }
-                    const uint64_t r0 = lane < W ? __ldg(rows + ((int64_t)L * 64 + b0) * W + lane) : 0ull;
-                    const uint64_t r1 = (b1 >= 0 && lane < W) ? __ldg(rows + ((int64_t)L * 64 + b1) * W + lane) : 0ull;
-#pragma unroll
-                    for (int j = 0; j < kDenseGroup; j++) {
-                        if ((ws[j] >> b0) & 1ull) c4[j] += __popcll(r0 & Sp[j]);
-                        else if ((wt[j] >> b0) & 1ull) k4x2[j] += __popcll(r0 & T[j]);
-                        if (b1 >= 0) {
-                            if ((ws[j] >> b1) & 1ull) c4[j] += __popcll(r1 & Sp[j]);
-                            else if ((wt[j] >> b1) & 1ull) k4x2[j] += __popcll(r1 & T[j]);
-                        }
-                    }
-                }
-            }
-#pragma unroll
-            for (int j = 0; j < kDenseGroup; j++) {
-                if (j >= R) break;
-                const unsigned long long t = pgd_warp_sum(__popcll(T[j]));
-                const unsigned long long c = pgd_warp_sum(c4[j]);
-                const unsigned long long k2 = pgd_warp_sum(k4x2[j]);
-                const int64_t e = A.dpos[i0 + j];
-                const int32_t id = G.order[e];
-                edge_epilogue(G, acc, cur_g, e, G.ev[id], G.eu[id], t, k2 >> 1, c, lane);
-            }
-            i0 = i1;
-        }
-    }
-    block_flush(G, acc, cur_g, s_red, 8);
-}
 
 // ---------------------------------------------------------------------------
 // Dense graphs with a common-neighbour matrix.  For a graph of n vertices
@@ -1365,15 +1238,13 @@ struct DenseCnArgs {
     const uint16_t *cn;       // CN matrices of the graphs that have one
     const int64_t *cbase;     // per graph: first entry of its CN matrix
     const int32_t *dpos;      // E_ordered positions of those graphs' edges, grouped by q
-    const uint32_t *k4pre;    // per position of dpos: 0xffffffff where k_dense_tc did not take the run (or null)
     int64_t ndense;
     unsigned long long *next;
 };
 
-// Up to kDenseGroup edges (p_j, q) with the same q, as in k_dense; per row
-// word L of A_q the warp reads 64 entries of CN[q] and of each CN[p_j] (two
-// per lane) for the two sums, and the rows of the word's members of T_j.
-// Groups of the runs k_dense_tc took are left to k_dense_close.
+// Up to kDenseGroup edges (p_j, q) with the same q; per row word L of A_q the
+// warp reads 64 entries of CN[q] and of each CN[p_j] (two per lane) for the two
+// sums, and the rows of the word's members of T_j.
 __global__ void __launch_bounds__(256, 3) k_dense_cn(DenseCnArgs A) {
     __shared__ unsigned long long s_red[8][PGD_NSUMS];
     const DevGraph &G = A.G;
@@ -1400,12 +1271,6 @@ __global__ void __launch_bounds__(256, 3) k_dense_cn(DenseCnArgs A) {
             const int64_t stride = (int64_t)W * 64;
             const uint64_t *rows = A.bits + A.wbase[g];
             const uint16_t *cnb = A.cn + A.cbase[g];
-            // a run taken by the tensor cores (all edges of a group share q, so
-            // all or none of them are) is closed by k_dense_close
-            if (A.k4pre && A.k4pre[i0] != 0xffffffffu) {
-                i0 = i1;
-                continue;
-            }
             const int64_t q = qg - vb;
             const uint16_t *cq = cnb + q * stride;
             const uint64_t Aq = lane < W ? __ldg(rows + q * W + lane) : 0ull;
@@ -2272,6 +2137,14 @@ struct TmpGuard {
     ~TmpGuard() {
         for (void *p : held) pgd_tmp_free(ctx, p);
     }
+    // frees one of the held allocations early
+    void release(void *p) {
+        for (void *&q : held)
+            if (q == p) {
+                pgd_tmp_free(ctx, q);
+                q = nullptr;
+            }
+    }
     template <typename T>
     pgd_status alloc(T **out, size_t bytes) {
         void *p = nullptr;
@@ -2283,6 +2156,15 @@ struct TmpGuard {
         return st;
     }
 };
+
+cudaError_t pgd_decompose_limits() {
+    constexpr cudaFuncAttribute kDyn = cudaFuncAttributeMaxDynamicSharedMemorySize;
+    cudaError_t e = cudaFuncSetAttribute(k_hub, kDyn, kMaxDynSmem);
+    if (e == cudaSuccess) e = cudaFuncSetAttribute(k_tslot_hub, kDyn, kMaxTslotSmem);
+    if (e == cudaSuccess) e = cudaFuncSetAttribute(k_dense_tc, kDyn, kTcSmem);
+    if (e == cudaSuccess) e = cudaFuncSetAttribute(k_dense_gram, kDyn, kGramSmem);
+    return e;
+}
 
 static pgd_status build_aux(pgd_graph *g) {
     pgd_ctx *ctx = g->ctx;
@@ -2430,15 +2312,17 @@ static DevGraph dev_view(pgd_graph *g, bool micro) {
     return G;
 }
 
-// Triangle pass, work plan and both decomposition kernels for the graph view
-// G (one graph, or the union of a batch); *ms gets their device time.
+// The dense graphs of a batch: their edges are decomposed from adjacency bit
+// rows and common-neighbour matrices.
 struct DenseView {
     const uint64_t *bits;
     const int64_t *wbase;
     const int64_t *vbase;
-    const uint16_t *cn;       // common-neighbour matrices (null: none)
+    const uint16_t *cn;       // common-neighbour matrices
     const int64_t *cbase;     // per graph: first CN entry, or -1
+    const int64_t *before;    // per graph: edges of sparse graphs before it
     int ngraphs;
+    int64_t nedges;           // edges of the dense graphs
 };
 
 // The tensor-core part of the CN-graph edges: k4 of the runs whose q has
@@ -2481,7 +2365,6 @@ static pgd_status dense_tc(pgd_ctx *ctx, const DevGraph &G, TmpGuard &tg, const 
     pgd_tmp_free(ctx, tmp);
     PGD_LAUNCH(ctx, k_tc_run_fill, grid_for(ncn), kThreads, 0, keys, flag, pos, ncn, runs, ctr + 9, eb);
     PGD_CUDA(ctx, cudaMemsetAsync(k4, 0xff, ncn * sizeof(uint32_t), s));
-    PGD_CUDA(ctx, cudaFuncSetAttribute(k_dense_tc, cudaFuncAttributeMaxDynamicSharedMemorySize, kTcSmem));
     DenseTcArgs T;
     T.G = G;
     T.bits = dense->bits;
@@ -2507,7 +2390,6 @@ static pgd_status dense_tc(pgd_ctx *ctx, const DevGraph &G, TmpGuard &tg, const 
     if ((st = pgd_tmp_alloc(ctx, &tmp, tb))) return st;
     cub::DeviceScan::ExclusiveSum(tmp, tb, tiles, etile, k + 1, s);
     pgd_tmp_free(ctx, tmp);
-    PGD_CUDA(ctx, cudaFuncSetAttribute(k_dense_gram, cudaFuncAttributeMaxDynamicSharedMemorySize, kGramSmem));
     GramArgs E;
     E.bits = dense->bits;
     E.wbase = dense->wbase;
@@ -2579,10 +2461,10 @@ struct StageMs {
 
 // The work plan of the positions G.order[0..G.npos): hub-anchored positions
 // grouped by anchor into work items (with their {position, q} records), then
-// dense-graph positions, then light ones (posv).
+// light ones (posv).
 struct Plan {
     int32_t *posv = nullptr;
-    unsigned long long nh = 0, nd = 0;
+    unsigned long long nh = 0;
     int64_t nlight = 0, nitems = 0;
     int64_t *items = nullptr;
     int2 *hrec = nullptr;
@@ -2595,8 +2477,7 @@ static int bits_for(int64_t x) {
     return b;
 }
 
-static pgd_status build_plan(pgd_ctx *ctx, const DevGraph &G, TmpGuard &tg, Plan *P, uint64_t **keys_out = nullptr,
-                             int32_t **vals_out = nullptr, uint64_t **keys2_out = nullptr) {
+static pgd_status build_plan(pgd_ctx *ctx, const DevGraph &G, TmpGuard &tg, Plan *P) {
     cudaStream_t s = ctx->stream;
     pgd_status st;
     const int64_t m = G.npos;
@@ -2607,29 +2488,21 @@ static pgd_status build_plan(pgd_ctx *ctx, const DevGraph &G, TmpGuard &tg, Plan
     if ((st = tg.alloc(&keys2, m * sizeof(uint64_t)))) return st;
     if ((st = tg.alloc(&P->posv, m * sizeof(int32_t)))) return st;
     if ((st = tg.alloc(&vals, m * sizeof(int32_t)))) return st;
-    // [0] hub edges, [1] hub item counter, [2] light counter, [3] dense edges, [4] dense counter,
-    // [5] triangle-pass item counter
+    // [0] hub edges, [1] hub item counter, [2] light counter, [5] triangle-pass item counter
     unsigned long long *ctr = ctx->d_ctr;
     PGD_CUDA(ctx, cudaMemsetAsync(ctr, 0, 8 * sizeof(unsigned long long), s));
-    const int eb = bits_for(m), end_bit = eb + bits_for(G.n + 2);
+    const int eb = bits_for(m), end_bit = eb + bits_for(G.n + 1);
     PGD_LAUNCH(ctx, k_plan_keys, grid_for(m), kThreads, 0, G, keys, vals, ctr, eb);
-    unsigned long long cnt[4] = {0, 0, 0, 0};
-    PGD_CUDA(ctx, cudaMemcpyAsync(cnt, ctr, sizeof(cnt), cudaMemcpyDeviceToHost, s));
+    PGD_CUDA(ctx, pgd_fetch(ctx, 0, ctr, sizeof(P->nh)));
     PGD_CUDA(ctx, cudaStreamSynchronize(s));
-    P->nh = cnt[0];
-    P->nd = cnt[3];
-    P->nlight = m - (int64_t)P->nh - (int64_t)P->nd;
+    P->nh = pgd_pinned<unsigned long long>(ctx, 0);
+    P->nlight = m - (int64_t)P->nh;
     size_t tb = 0;
     void *tmp = nullptr;
-    if (P->nd == (unsigned long long)m) {
-        // every position is a dense-graph edge: the sorted order is the identity
-        PGD_CUDA(ctx, cudaMemcpyAsync(P->posv, vals, m * sizeof(int32_t), cudaMemcpyDeviceToDevice, s));
-    } else {
-        cub::DeviceRadixSort::SortPairs(nullptr, tb, keys, keys2, vals, P->posv, m, 0, end_bit, s);
-        if ((st = pgd_tmp_alloc(ctx, &tmp, tb))) return st;
-        cub::DeviceRadixSort::SortPairs(tmp, tb, keys, keys2, vals, P->posv, m, 0, end_bit, s);
-        pgd_tmp_free(ctx, tmp);
-    }
+    cub::DeviceRadixSort::SortPairs(nullptr, tb, keys, keys2, vals, P->posv, m, 0, end_bit, s);
+    if ((st = pgd_tmp_alloc(ctx, &tmp, tb))) return st;
+    cub::DeviceRadixSort::SortPairs(tmp, tb, keys, keys2, vals, P->posv, m, 0, end_bit, s);
+    pgd_tmp_free(ctx, tmp);
     const unsigned long long nh = P->nh;
     if (nh > 0) {
         if ((st = tg.alloc(&flag, (nh + 1) * sizeof(uint32_t)))) return st;
@@ -2650,9 +2523,6 @@ static pgd_status build_plan(pgd_ctx *ctx, const DevGraph &G, TmpGuard &tg, Plan
         if ((st = tg.alloc(&P->hrec, (nh + 1) * sizeof(int2)))) return st;
         PGD_LAUNCH(ctx, k_hub_recs, grid_for(nh), kThreads, 0, G, P->posv, (int64_t)nh, P->hrec);
     }
-    if (keys_out) *keys_out = keys;
-    if (vals_out) *vals_out = vals;
-    if (keys2_out) *keys2_out = keys2;
     return PGD_OK;
 }
 
@@ -2673,11 +2543,10 @@ static pgd_status triangle_pass(pgd_ctx *ctx, const DevGraph &G, int4 *slot, con
         // the whole dynamic shared memory holds bitmap ranks (no histogram here)
         const int64_t tw = std::min<int64_t>(H.nwords, kMaxTslotSmem / 4);
         T.split = (int32_t)std::min<int64_t>(tw * 32, 0x7fffffe0);
-        PGD_CUDA(ctx, cudaFuncSetAttribute(k_tslot_hub, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)(tw * 4)));
         PGD_LAUNCH(ctx, k_tslot_hub, nsm, kHubWarps * 32, (size_t)(tw * 4), T);
     }
     if (P.nlight > 0)
-        PGD_LAUNCH(ctx, k_tslot, grid_for(32 * P.nlight), kThreads, 0, G, slot, P.posv + P.nh + P.nd, P.nlight);
+        PGD_LAUNCH(ctx, k_tslot, grid_for(32 * P.nlight), kThreads, 0, G, slot, P.posv + P.nh, P.nlight);
     return PGD_OK;
 }
 
@@ -2686,9 +2555,9 @@ __global__ void k_iota(int32_t *a, int64_t n) {
         a[i] = (int32_t)i;
 }
 
+// The edge-by-edge decomposition of G's positions.
 static pgd_status run_decompose(pgd_ctx *ctx, const DevGraph &G, int4 *slot, int32_t nhubs, int32_t nwide,
-                                int32_t max_degree,
-                                StageMs *ms, const DenseView *dense = nullptr) {
+                                int32_t max_degree, StageMs *ms) {
     cudaStream_t s = ctx->stream;
     pgd_status st;
     const int64_t m = G.npos;   // positions to decompose (E_ordered length)
@@ -2701,7 +2570,6 @@ static pgd_status run_decompose(pgd_ctx *ctx, const DevGraph &G, int4 *slot, int
     int32_t *thigh = nullptr;
     TmpGuard tg(ctx);
     const int nsm = ctx->num_sms;
-    bool tc_ran = false;
     HubArgs H;
     const size_t smem = hub_layout(G.n, nhubs, nwide, max_degree, &H);
     if ((int64_t)H.split < G.n) {
@@ -2727,11 +2595,9 @@ static pgd_status run_decompose(pgd_ctx *ctx, const DevGraph &G, int4 *slot, int
         PGD_CUDA(ctx, cudaEventRecord(ctx->evt1, s));
     }
     Plan P;
-    uint64_t *keys = nullptr, *keys2 = nullptr;
-    int32_t *vals = nullptr;
-    if ((st = build_plan(ctx, G, tg, &P, &keys, &vals, &keys2))) return st;
+    if ((st = build_plan(ctx, G, tg, &P))) return st;
     int32_t *posv = P.posv;
-    const unsigned long long nh = P.nh, nd = P.nd;
+    const unsigned long long nh = P.nh;
     const int64_t nlight = P.nlight, nitems = P.nitems;
     int64_t *items = P.items;
     int2 *hrec = P.hrec;
@@ -2754,7 +2620,6 @@ static pgd_status run_decompose(pgd_ctx *ctx, const DevGraph &G, int4 *slot, int
             if ((st = tg.alloc(&H.twin, bytes))) return st;
             PGD_CUDA(ctx, cudaMemsetAsync(H.twin, 0, bytes, s));
         }
-        PGD_CUDA(ctx, cudaFuncSetAttribute(k_hub, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
         H.G = G;
         H.hpos = posv;
         H.hrec = hrec;
@@ -2768,79 +2633,10 @@ static pgd_status run_decompose(pgd_ctx *ctx, const DevGraph &G, int4 *slot, int
         PGD_LAUNCH(ctx, k_hub, nsm, kHubWarps * 32, smem, H);
         PGD_CUDA(ctx, cudaEventRecord(ctx->evh1, s));
     }
-    if (nd > 0 && dense) {
-        // dense edges grouped by q, so that k_dense serves several per row pass
-        // (edges of graphs with a CN matrix first, counted in ctr[7])
-        const int qb = bits_for(G.n), ebd = bits_for(G.npos);
-        PGD_LAUNCH(ctx, k_dense_keys, grid_for(nd), kThreads, 0, G, posv + nh, (int64_t)nd,
-                   dense->cn ? dense->cbase : nullptr, keys, vals, ctr + 7, qb, ebd);
-        size_t tbd = 0;
-        void *tmpd = nullptr;
-        cub::DeviceRadixSort::SortPairs(nullptr, tbd, keys, keys2, vals, posv + nh, (int64_t)nd, 0, 1 + qb + ebd, s);
-        if ((st = pgd_tmp_alloc(ctx, &tmpd, tbd))) return st;
-        cub::DeviceRadixSort::SortPairs(tmpd, tbd, keys, keys2, vals, posv + nh, (int64_t)nd, 0, 1 + qb + ebd, s);
-        pgd_tmp_free(ctx, tmpd);
-        int64_t ncn = 0;
-        if (dense->cn) {
-            unsigned long long h = 0;
-            PGD_CUDA(ctx, cudaMemcpyAsync(&h, ctr + 7, sizeof(h), cudaMemcpyDeviceToHost, s));
-            PGD_CUDA(ctx, cudaStreamSynchronize(s));
-            ncn = (int64_t)h;
-        }
-        TcOut tc;
-        if (ncn > 0 && ctx->tc_min_deg > 0) {
-            if ((st = dense_tc(ctx, G, tg, dense, posv + nh, keys2, ncn, ebd, &tc))) return st;
-            tc_ran = true;
-        }
-        if (ncn > 0 && (!tc.k4 || tc.nrest > 0)) {
-            DenseCnArgs C;
-            C.G = G;
-            C.bits = dense->bits;
-            C.wbase = dense->wbase;
-            C.vbase = dense->vbase;
-            C.cn = dense->cn;
-            C.cbase = dense->cbase;
-            // with the tensor-core path, only the positions outside its runs
-            C.dpos = tc.k4 ? tc.rest : posv + nh;
-            C.k4pre = nullptr;
-            C.ndense = tc.k4 ? tc.nrest : ncn;
-            C.next = ctr + 6;
-            PGD_LAUNCH(ctx, k_dense_cn, nsm * 8, 256, 0, C);
-        }
-        if (ncn > 0) {
-            if (tc.k4) {
-                DenseCloseArgs Z;
-                Z.G = G;
-                Z.bits = dense->bits;
-                Z.wbase = dense->wbase;
-                Z.vbase = dense->vbase;
-                Z.cn = dense->cn;
-                Z.cbase = dense->cbase;
-                Z.dpos = posv + nh;
-                Z.runs = tc.runs;
-                Z.nruns = tc.nruns;
-                Z.k4 = tc.k4;
-                Z.eslot = tc.eslot;
-                Z.next = ctr + 11;
-                PGD_LAUNCH(ctx, k_dense_close, nsm * 8, 256, 0, Z);
-            }
-        }
-        if ((int64_t)nd > ncn) {
-            DenseArgs D;
-            D.G = G;
-            D.bits = dense->bits;
-            D.wbase = dense->wbase;
-            D.vbase = dense->vbase;
-            D.dpos = posv + nh + ncn;
-            D.ndense = (int64_t)nd - ncn;
-            D.next = ctr + 4;
-            PGD_LAUNCH(ctx, k_dense, nsm * 8, 256, 0, D);
-        }
-    }
     if (nlight > 0) {
         LightArgs L;
         L.G = G;
-        L.lpos = posv + nh + nd;
+        L.lpos = posv + nh;
         L.nlight = nlight;
         L.next = ctr + 2;
         PGD_LAUNCH(ctx, k_light, nsm * 8, kLightWarps * 32, 0, L);
@@ -2851,11 +2647,70 @@ static pgd_status run_decompose(pgd_ctx *ctx, const DevGraph &G, int4 *slot, int
     PGD_CUDA(ctx, cudaEventElapsedTime(&ms->total, ctx->ev0, ctx->ev1));
     PGD_CUDA(ctx, cudaEventElapsedTime(&ms->tri, ctx->evt0, ctx->evt1));
     if (nitems > 0) PGD_CUDA(ctx, cudaEventElapsedTime(&ms->hub, ctx->evh0, ctx->evh1));
-    if (tc_ran) {
+    return PGD_OK;
+}
+
+// The edges of a batch's dense graphs, grouped by q: k4 and the c4 sums on the
+// tensor cores for the runs whose degree allows it (closed by k_dense_close), the
+// rest with k_dense_cn.
+static pgd_status dense_decompose(pgd_ctx *ctx, const DevGraph &G, const DenseView &dense) {
+    cudaStream_t s = ctx->stream;
+    pgd_status st;
+    const int nsm = ctx->num_sms;
+    const int64_t nd = dense.nedges;
+    TmpGuard tg(ctx);
+    uint64_t *keys = nullptr, *keys2 = nullptr;
+    int32_t *vals = nullptr, *dpos = nullptr;
+    if ((st = tg.alloc(&keys, nd * sizeof(uint64_t)))) return st;
+    if ((st = tg.alloc(&keys2, nd * sizeof(uint64_t)))) return st;
+    if ((st = tg.alloc(&vals, nd * sizeof(int32_t)))) return st;
+    if ((st = tg.alloc(&dpos, nd * sizeof(int32_t)))) return st;
+    unsigned long long *ctr = ctx->d_ctr;
+    PGD_CUDA(ctx, cudaMemsetAsync(ctr, 0, 8 * sizeof(unsigned long long), s));
+    const int qb = bits_for(G.n), eb = bits_for(G.npos);
+    PGD_LAUNCH(ctx, k_dense_keys, grid_for(G.npos), kThreads, 0, G, dense.before, keys, vals, eb);
+    size_t tb = 0;
+    void *tmp = nullptr;
+    cub::DeviceRadixSort::SortPairs(nullptr, tb, keys, keys2, vals, dpos, nd, 0, qb + eb, s);
+    if ((st = tg.alloc(&tmp, tb))) return st;
+    PGD_CUDA(ctx, cub::DeviceRadixSort::SortPairs(tmp, tb, keys, keys2, vals, dpos, nd, 0, qb + eb, s));
+    TcOut tc;
+    if (ctx->tc_min_deg > 0 && (st = dense_tc(ctx, G, tg, &dense, dpos, keys2, nd, eb, &tc))) return st;
+    if (!tc.k4 || tc.nrest > 0) {
+        DenseCnArgs C;
+        C.G = G;
+        C.bits = dense.bits;
+        C.wbase = dense.wbase;
+        C.vbase = dense.vbase;
+        C.cn = dense.cn;
+        C.cbase = dense.cbase;
+        // with the tensor-core path, only the positions outside its runs
+        C.dpos = tc.k4 ? tc.rest : dpos;
+        C.ndense = tc.k4 ? tc.nrest : nd;
+        C.next = ctr + 6;
+        PGD_LAUNCH(ctx, k_dense_cn, nsm * 8, 256, 0, C);
+    }
+    if (tc.k4) {
+        DenseCloseArgs Z;
+        Z.G = G;
+        Z.bits = dense.bits;
+        Z.wbase = dense.wbase;
+        Z.vbase = dense.vbase;
+        Z.cn = dense.cn;
+        Z.cbase = dense.cbase;
+        Z.dpos = dpos;
+        Z.runs = tc.runs;
+        Z.nruns = tc.nruns;
+        Z.k4 = tc.k4;
+        Z.eslot = tc.eslot;
+        Z.next = ctr + 11;
+        PGD_LAUNCH(ctx, k_dense_close, nsm * 8, 256, 0, Z);
         unsigned long long failed = 0;
-        PGD_CUDA(ctx, cudaMemcpy(&failed, ctr + 10, sizeof(failed), cudaMemcpyDeviceToHost));
+        PGD_CUDA(ctx, cudaMemcpyAsync(&failed, ctr + 10, sizeof(failed), cudaMemcpyDeviceToHost, s));
+        PGD_CUDA(ctx, cudaStreamSynchronize(s));
         if (failed) return pgd_fail(ctx, PGD_ETIMEOUT, "a tensor-core wait in k_dense_tc or k_dense_gram ran out");
     }
+    PGD_CUDA(ctx, cudaGetLastError());
     return PGD_OK;
 }
 
@@ -2885,7 +2740,8 @@ static pgd_status rank_decompose(pgd_graph *g, bool micro, StageMs *ms) {
     PGD_CUDA(ctx, cudaEventRecord(ctx->ev0, s));
     if ((st = pgd_rank_decompose(ctx, *g->ranked, o))) return st;
     PGD_CUDA(ctx, cudaEventRecord(ctx->ev1, s));
-    PGD_CUDA(ctx, cudaEventSynchronize(ctx->ev1));
+    PGD_CUDA(ctx, pgd_fetch(ctx, 0, ctx->d_sums, PGD_NSUMS * sizeof(unsigned long long)));
+    PGD_CUDA(ctx, cudaStreamSynchronize(s));
     PGD_CUDA(ctx, cudaEventElapsedTime(&ms->total, ctx->ev0, ctx->ev1));
     if (g->norder > 0 && g->m > 0) {
         PGD_CUDA(ctx, cudaEventElapsedTime(&ms->tri, ctx->evt0, ctx->evt1));
@@ -2909,11 +2765,10 @@ pgd_status pgd_dev_decompose(pgd_graph *g, bool micro, pgd_counts *out) {
         if ((!g->has_aux || g->aux_cache_hub != ctx->cache_hub) && (st = build_aux(g))) return st;
         if ((st = run_decompose(ctx, dev_view(g, micro), (int4 *)g->slot, g->nhubs, g->nhubs_wide, g->max_degree, &ms)))
             return st;
+        PGD_CUDA(ctx, pgd_fetch(ctx, 0, ctx->d_sums, PGD_NSUMS * sizeof(unsigned long long)));
+        PGD_CUDA(ctx, cudaStreamSynchronize(s));
     }
-    unsigned long long h[PGD_NSUMS];
-    PGD_CUDA(ctx, cudaMemcpyAsync(h, ctx->d_sums, sizeof(h), cudaMemcpyDeviceToHost, s));
-    PGD_CUDA(ctx, cudaStreamSynchronize(s));
-    for (int i = 0; i < PGD_NSUMS; i++) out->sums[i] = h[i];
+    memcpy(out->sums, ctx->pin, PGD_NSUMS * sizeof(uint64_t));
     out->n = g->n;
     out->m = g->m;
     out->kernel_ms = ms.total;
@@ -2970,30 +2825,143 @@ __global__ void k_union_edges(const BatchDesc *D, const int64_t *ebase, int k, i
     }
 }
 
-// Graphs of a batch that also get a common-neighbour matrix (k_dense_cn):
-// graphs on the row-bitset path whose average degree is at least n/16
-// (32·m >= n²), as long as the matrices stay within kCnMaxEntries.  Fills
-// cbase (first entry per graph, -1 for none) and ctile (first 32-row tile
-// per graph; k + 1 entries) and returns the number of 16-bit entries.
+// How a batch splits into dense graphs (bit rows and common-neighbour matrices)
+// and sparse ones (rank_path.cu): dense are those of at most dense_max vertices
+// whose average degree is at least n/16 (32·m >= n²), as long as the matrices
+// stay within kCnMaxEntries.
 constexpr int64_t kCnMaxEntries = 4ll << 30;   // 8 GiB
 
-static int64_t plan_common(int k, const std::vector<long long> &gnm, const std::vector<uint8_t> &gdense,
-                           std::vector<int64_t> &cbase, std::vector<int64_t> &ctile) {
-    cbase.assign((size_t)k, -1);
-    ctile.assign((size_t)k + 1, 0);
-    int64_t entries = 0, tiles = 0;
+struct BatchSplit {
+    std::vector<uint8_t> dense;      // per graph
+    std::vector<int64_t> tables;     // wbase, cbase and before (k each), ctile (k + 1)
+    int64_t words = 0, entries = 0, tiles = 0, dense_edges = 0, sparse_edges = 0;
+    int ndense = 0;
+};
+
+static BatchSplit split_batch(int k, const std::vector<long long> &gnm, int dense_max) {
+    BatchSplit B;
+    B.dense.assign((size_t)k, 0);
+    B.tables.assign((size_t)4 * k + 1, 0);
+    int64_t *wbase = B.tables.data(), *cbase = wbase + k, *before = cbase + k, *ctile = before + k;
     for (int g = 0; g < k; g++) {
-        ctile[(size_t)g] = tiles;
         const int64_t n = gnm[(size_t)2 * g], m = gnm[(size_t)2 * g + 1];
-        if (!gdense[(size_t)g] || 32 * m < n * n) continue;
+        wbase[g] = B.words;
+        cbase[g] = -1;
+        before[g] = B.sparse_edges;
+        ctile[g] = B.tiles;
         const int64_t e = n * (((n + 63) / 64) * 64);   // a multiple of 64: every matrix is 128-byte aligned
-        if (entries + e > kCnMaxEntries) continue;
-        cbase[(size_t)g] = entries;
-        entries += e;
-        tiles += (n + kCnRows - 1) / kCnRows;
+        if (m == 0 || n > dense_max || 32 * m < n * n || B.entries + e > kCnMaxEntries) {
+            B.sparse_edges += m;
+            continue;
+        }
+        B.dense[(size_t)g] = 1;
+        B.ndense++;
+        B.dense_edges += m;
+        cbase[g] = B.entries;
+        B.entries += e;
+        B.words += n * ((n + 63) / 64);
+        B.tiles += (n + kCnRows - 1) / kCnRows;
     }
-    ctile[(size_t)k] = tiles;
-    return entries;
+    ctile[k] = B.tiles;
+    return B;
+}
+
+// Decomposes the union U of k graphs (off, adj, deg, ev, eu, order of U set;
+// egraph and vgraph: graph of each edge position and vertex; d_gnm: n and m per
+// graph; d_vbase: first vertex per graph) into gsums and, if given, umicro.
+static pgd_status decompose_union(pgd_graph *U, int k, const std::vector<long long> &gnm, const long long *d_gnm,
+                                  const int64_t *d_vbase, const int32_t *vgraph, const int32_t *egraph,
+                                  unsigned long long *gsums, uint64_t *umicro, StageMs *ms) {
+    pgd_ctx *ctx = U->ctx;
+    cudaStream_t s = ctx->stream;
+    pgd_status st;
+    const BatchSplit B = split_batch(k, gnm, ctx->dense_max);
+    TmpGuard tg(ctx);
+    uint8_t *d_dense = nullptr;
+    *ms = StageMs();
+    if (B.ndense) {
+        if ((st = tg.alloc(&d_dense, (size_t)k))) return st;
+        PGD_CUDA(ctx, cudaMemcpyAsync(d_dense, B.dense.data(), (size_t)k, cudaMemcpyHostToDevice, s));
+    }
+    // a batch of sparse graphs only needs no mask
+    pgd_rank_graph R;
+    if (B.sparse_edges && (st = pgd_rank_build(U, 2 * B.sparse_edges, vgraph, d_dense, &R))) return st;
+    struct Release {
+        pgd_graph *U;
+        pgd_rank_graph *R;
+        ~Release() { pgd_rank_free(U, R); }
+    } release{U, &R};
+    DevGraph G{};
+    DenseView dv{};
+    if (B.ndense) {
+        int64_t *tables = nullptr;
+        unsigned long long *bits = nullptr;
+        uint16_t *cn = nullptr;
+        if ((st = tg.alloc(&tables, B.tables.size() * sizeof(int64_t)))) return st;
+        if ((st = tg.alloc(&bits, (size_t)B.words * sizeof(unsigned long long)))) return st;
+        if ((st = tg.alloc(&cn, (size_t)B.entries * sizeof(uint16_t)))) return st;
+        PGD_CUDA(ctx, cudaMemcpyAsync(tables, B.tables.data(), B.tables.size() * sizeof(int64_t), cudaMemcpyHostToDevice, s));
+        PGD_CUDA(ctx, cudaMemsetAsync(bits, 0, (size_t)B.words * sizeof(unsigned long long), s));
+        dv = DenseView{(const uint64_t *)bits, tables, d_vbase, cn, tables + k, tables + 2 * k, k, B.dense_edges};
+        PGD_LAUNCH(ctx, k_dense_bits, grid_for(32 * U->n), kThreads, 0, U->off, U->adj, vgraph, d_dense, dv.wbase,
+                   d_vbase, d_gnm, U->n, bits);
+        PGD_LAUNCH(ctx, k_dense_common, (int)std::min<int64_t>(B.tiles, (int64_t)ctx->num_sms * 8), 256, 0, dv.bits,
+                   dv.wbase, d_gnm, dv.cbase, tables + 3 * k, k, B.tiles, cn);
+        G.off = U->off;
+        G.adj = U->adj;
+        G.deg = U->deg;
+        G.ev = U->ev;
+        G.eu = U->eu;
+        G.order = U->order;
+        G.n = U->n;
+        G.m = U->m;
+        G.npos = U->m;
+        G.micro = umicro;
+        G.sums = gsums;
+        G.egraph = egraph;
+        G.gnm = d_gnm;
+        G.gdense = d_dense;
+    }
+    PGD_CUDA(ctx, cudaEventRecord(ctx->ev0, s));
+    if (B.sparse_edges) {
+        pgd_rank_out o{};
+        o.ev = U->ev;
+        o.eu = U->eu;
+        o.deg = U->deg;
+        o.order = U->order;
+        o.npos = U->m;
+        o.micro = umicro;
+        o.sums = gsums;
+        o.egraph = egraph;
+        o.gnm = d_gnm;
+        o.gdense = d_dense;
+        if ((st = pgd_rank_decompose(ctx, R, o))) return st;
+    }
+    if (B.ndense && (st = dense_decompose(ctx, G, dv))) return st;
+    PGD_CUDA(ctx, cudaEventRecord(ctx->ev1, s));
+    PGD_CUDA(ctx, cudaEventSynchronize(ctx->ev1));
+    PGD_CUDA(ctx, cudaEventElapsedTime(&ms->total, ctx->ev0, ctx->ev1));
+    if (B.sparse_edges) {
+        PGD_CUDA(ctx, cudaEventElapsedTime(&ms->tri, ctx->evt0, ctx->evt1));
+        PGD_CUDA(ctx, cudaEventElapsedTime(&ms->hub, ctx->evh0, ctx->evh1));
+    }
+    return PGD_OK;
+}
+
+// Results of a batch from the graphs' sums.
+static void close_batch(int k, const std::vector<unsigned long long> &h, const std::vector<long long> &gnm,
+                        const StageMs &ms, pgd_counts *out) {
+    for (int i = 0; i < k; i++) {
+        pgd_counts &o = out[i];
+        memset(&o, 0, sizeof(o));
+        for (int j = 0; j < PGD_NSUMS; j++) o.sums[j] = h[(size_t)i * PGD_NSUMS + j];
+        o.n = gnm[(size_t)2 * i];
+        o.m = gnm[(size_t)2 * i + 1];
+        o.kernel_ms = ms.total;
+        o.hub_ms = ms.hub;
+        o.tri_ms = ms.tri;
+        pgd_close_counts(o.sums, o.n, o.m, o.totals);
+    }
 }
 
 pgd_status pgd_dev_decompose_batch(pgd_ctx *ctx, pgd_graph *const *graphs, int k, bool micro, pgd_counts *out) {
@@ -3036,160 +3004,59 @@ pgd_status pgd_dev_decompose_batch(pgd_ctx *ctx, pgd_graph *const *graphs, int k
     }
     if (N > 0x7ffffffe || S > 0x7fffffff)
         return pgd_fail(ctx, PGD_EINVAL, "batch too large for 32-bit vertex and slot ids");
-    // the union, as a transient graph of this context
-    pgd_graph U;
-    U.ctx = ctx;
-    U.n = N;
-    U.m = M;
-    U.norder = M;
-    U.max_degree = max_degree;
+    // the union, as a transient graph of this context (destroyed on every return)
+    struct Union {
+        pgd_graph *g = new pgd_graph();
+        ~Union() { pgd_graph_destroy(g); }
+    } holder;
+    pgd_graph *U = holder.g;
+    U->ctx = ctx;
+    U->n = N;
+    U->m = M;
+    U->norder = M;
+    U->max_degree = max_degree;
+    TmpGuard tg(ctx);
     BatchDesc *d_desc = nullptr;
     int64_t *d_bases = nullptr;
     long long *d_gnm = nullptr;
     int32_t *egraph = nullptr, *vgraph = nullptr;
-    unsigned long long *gsums = nullptr, *bits = nullptr;
+    unsigned long long *gsums = nullptr;
     uint64_t *umicro = nullptr;
-    uint8_t *d_gdense = nullptr;
-    int64_t *d_wbase = nullptr, *d_cbase = nullptr, *d_ctile = nullptr;
-    uint16_t *cn = nullptr;
-    // graphs of at most dense_max vertices use the row-bitset kernel
-    std::vector<uint8_t> gdense((size_t)k, 0);
-    std::vector<int64_t> wbase((size_t)k, 0);
-    int64_t words = 0;
-    int ndense_graphs = 0;
-    for (int i = 0; i < k; i++) {
-        const int64_t n = graphs[i]->n;
-        if (n > 0 && n <= ctx->dense_max && graphs[i]->m > 0) {
-            gdense[(size_t)i] = 1;
-            wbase[(size_t)i] = words;
-            words += n * ((n + 63) / 64);
-            ndense_graphs++;
-        }
-    }
-    std::vector<int64_t> cbase, ctile;
-    const int64_t cn_entries = plan_common(k, gnm, gdense, cbase, ctile);
-    auto cleanup = [&]() {
-        pgd_tmp_free(ctx, cn);
-        pgd_tmp_free(ctx, d_cbase);
-        pgd_tmp_free(ctx, d_ctile);
-        pgd_tmp_free(ctx, vgraph);
-        pgd_tmp_free(ctx, bits);
-        pgd_tmp_free(ctx, d_gdense);
-        pgd_tmp_free(ctx, d_wbase);
-        pgd_tmp_free(ctx, d_desc);
-        pgd_tmp_free(ctx, d_bases);
-        pgd_tmp_free(ctx, d_gnm);
-        pgd_tmp_free(ctx, egraph);
-        pgd_tmp_free(ctx, gsums);
-        pgd_tmp_free(ctx, umicro);
-        pgd_graph_free(&U, U.off, (N + 1) * sizeof(int64_t));
-        pgd_graph_free(&U, U.adj, (S + 1) * sizeof(int32_t));
-        pgd_graph_free(&U, U.deg, (N + 1) * sizeof(int32_t));
-        pgd_graph_free(&U, U.ev, (M + 1) * sizeof(int32_t));
-        pgd_graph_free(&U, U.eu, (M + 1) * sizeof(int32_t));
-        pgd_graph_free(&U, U.order, (M + 1) * sizeof(int32_t));
-        pgd_graph_free(&U, U.offp, (N + 1) * sizeof(int64_t));
-        pgd_graph_free(&U, U.adjp, (M + 1) * sizeof(int32_t));
-        pgd_graph_free(&U, U.hubid, (N + 1) * sizeof(int32_t));
-        pgd_graph_free(&U, U.vrank, (N + 1) * sizeof(int32_t));
-        pgd_graph_free(&U, U.adjp_rank, (M + 1) * sizeof(int32_t));
-        pgd_graph_free(&U, U.slot, (S + 1) * sizeof(int4));
-        pgd_graph_free(&U, U.offh, (N + 1) * sizeof(int64_t));
-        pgd_graph_free(&U, U.adjh, (U.nadjh + 1) * sizeof(int32_t));
-        pgd_graph_free(&U, U.toprows, (U.top_words + 1) * sizeof(uint32_t));
-        pgd_graph_free(&U, U.vrec, (N + 1) * 32);
-        pgd_graph_free(&U, U.adj_rank, (S + 1) * sizeof(int32_t));
-    };
-#define BATCH_TRY(expr)                      \
-    do {                                     \
-        if ((st = (expr)) != PGD_OK) {       \
-            cleanup();                       \
-            return st;                       \
-        }                                    \
-    } while (0)
-    BATCH_TRY(pgd_tmp_alloc(ctx, (void **)&d_desc, (size_t)k * sizeof(BatchDesc)));
-    BATCH_TRY(pgd_tmp_alloc(ctx, (void **)&d_bases, bases.size() * sizeof(int64_t)));
-    BATCH_TRY(pgd_tmp_alloc(ctx, (void **)&d_gnm, gnm.size() * sizeof(long long)));
-    BATCH_TRY(pgd_tmp_alloc(ctx, (void **)&egraph, (M + 1) * sizeof(int32_t)));
-    BATCH_TRY(pgd_tmp_alloc(ctx, (void **)&vgraph, (N + 1) * sizeof(int32_t)));
-    BATCH_TRY(pgd_tmp_alloc(ctx, (void **)&d_gdense, (size_t)k));
-    BATCH_TRY(pgd_tmp_alloc(ctx, (void **)&d_wbase, (size_t)k * sizeof(int64_t)));
-    if (words > 0) BATCH_TRY(pgd_tmp_alloc(ctx, (void **)&bits, (size_t)words * sizeof(unsigned long long)));
-    if (cn_entries > 0) {
-        BATCH_TRY(pgd_tmp_alloc(ctx, (void **)&cn, (size_t)cn_entries * sizeof(uint16_t)));
-        BATCH_TRY(pgd_tmp_alloc(ctx, (void **)&d_cbase, (size_t)k * sizeof(int64_t)));
-        BATCH_TRY(pgd_tmp_alloc(ctx, (void **)&d_ctile, ((size_t)k + 1) * sizeof(int64_t)));
-    }
-    BATCH_TRY(pgd_tmp_alloc(ctx, (void **)&gsums, (size_t)k * PGD_NSUMS * sizeof(unsigned long long)));
-    if (micro) BATCH_TRY(pgd_tmp_alloc(ctx, (void **)&umicro, (M + 1) * PGD_NMICRO * sizeof(uint64_t)));
-    BATCH_TRY(pgd_graph_alloc(&U, (void **)&U.off, (N + 1) * sizeof(int64_t)));
-    BATCH_TRY(pgd_graph_alloc(&U, (void **)&U.adj, (S + 1) * sizeof(int32_t)));
-    BATCH_TRY(pgd_graph_alloc(&U, (void **)&U.deg, (N + 1) * sizeof(int32_t)));
-    BATCH_TRY(pgd_graph_alloc(&U, (void **)&U.ev, (M + 1) * sizeof(int32_t)));
-    BATCH_TRY(pgd_graph_alloc(&U, (void **)&U.eu, (M + 1) * sizeof(int32_t)));
-    BATCH_TRY(pgd_graph_alloc(&U, (void **)&U.order, (M + 1) * sizeof(int32_t)));
-    if (cudaMemcpyAsync(d_desc, desc.data(), (size_t)k * sizeof(BatchDesc), cudaMemcpyHostToDevice, s) ||
-        cudaMemcpyAsync(d_bases, bases.data(), bases.size() * sizeof(int64_t), cudaMemcpyHostToDevice, s) ||
-        cudaMemcpyAsync(d_gnm, gnm.data(), gnm.size() * sizeof(long long), cudaMemcpyHostToDevice, s) ||
-        cudaMemsetAsync(gsums, 0, (size_t)k * PGD_NSUMS * sizeof(unsigned long long), s) ||
-        cudaMemcpyAsync(d_gdense, gdense.data(), (size_t)k, cudaMemcpyHostToDevice, s) ||
-        cudaMemcpyAsync(d_wbase, wbase.data(), (size_t)k * sizeof(int64_t), cudaMemcpyHostToDevice, s) ||
-        (words > 0 && cudaMemsetAsync(bits, 0, (size_t)words * sizeof(unsigned long long), s)) ||
-        (cn_entries > 0 &&
-         (cudaMemcpyAsync(d_cbase, cbase.data(), (size_t)k * sizeof(int64_t), cudaMemcpyHostToDevice, s) ||
-          cudaMemcpyAsync(d_ctile, ctile.data(), ((size_t)k + 1) * sizeof(int64_t), cudaMemcpyHostToDevice, s)))) {
-        cleanup();
-        return pgd_fail(ctx, PGD_ECUDA, "batch set-up copy failed");
-    }
-    PGD_LAUNCH(ctx, k_union_vertices, grid_for(N), kThreads, 0, d_desc, d_bases, k, N, U.off, U.deg, vgraph);
-    PGD_CUDA(ctx, cudaMemcpyAsync(U.off + N, &S, sizeof(int64_t), cudaMemcpyHostToDevice, s));
-    PGD_LAUNCH(ctx, k_union_slots, grid_for(S), kThreads, 0, d_desc, d_bases + 2 * k + 2, k, S, U.adj);
-    PGD_LAUNCH(ctx, k_union_edges, grid_for(M), kThreads, 0, d_desc, d_bases + k + 1, k, M, U.ev, U.eu, U.order,
+    if ((st = tg.alloc(&d_desc, (size_t)k * sizeof(BatchDesc)))) return st;
+    if ((st = tg.alloc(&d_bases, bases.size() * sizeof(int64_t)))) return st;
+    if ((st = tg.alloc(&d_gnm, gnm.size() * sizeof(long long)))) return st;
+    if ((st = tg.alloc(&egraph, (M + 1) * sizeof(int32_t)))) return st;
+    if ((st = tg.alloc(&vgraph, (N + 1) * sizeof(int32_t)))) return st;
+    if ((st = tg.alloc(&gsums, (size_t)k * PGD_NSUMS * sizeof(unsigned long long)))) return st;
+    if (micro && (st = tg.alloc(&umicro, (M + 1) * PGD_NMICRO * sizeof(uint64_t)))) return st;
+    if ((st = pgd_graph_alloc(U, (void **)&U->off, (N + 1) * sizeof(int64_t)))) return st;
+    if ((st = pgd_graph_alloc(U, (void **)&U->adj, (S + 1) * sizeof(int32_t)))) return st;
+    if ((st = pgd_graph_alloc(U, (void **)&U->deg, (N + 1) * sizeof(int32_t)))) return st;
+    if ((st = pgd_graph_alloc(U, (void **)&U->ev, (M + 1) * sizeof(int32_t)))) return st;
+    if ((st = pgd_graph_alloc(U, (void **)&U->eu, (M + 1) * sizeof(int32_t)))) return st;
+    if ((st = pgd_graph_alloc(U, (void **)&U->order, (M + 1) * sizeof(int32_t)))) return st;
+    PGD_CUDA(ctx, cudaMemcpyAsync(d_desc, desc.data(), (size_t)k * sizeof(BatchDesc), cudaMemcpyHostToDevice, s));
+    PGD_CUDA(ctx, cudaMemcpyAsync(d_bases, bases.data(), bases.size() * sizeof(int64_t), cudaMemcpyHostToDevice, s));
+    PGD_CUDA(ctx, cudaMemcpyAsync(d_gnm, gnm.data(), gnm.size() * sizeof(long long), cudaMemcpyHostToDevice, s));
+    PGD_CUDA(ctx, cudaMemsetAsync(gsums, 0, (size_t)k * PGD_NSUMS * sizeof(unsigned long long), s));
+    PGD_LAUNCH(ctx, k_union_vertices, grid_for(N), kThreads, 0, d_desc, d_bases, k, N, U->off, U->deg, vgraph);
+    PGD_CUDA(ctx, cudaMemcpyAsync(U->off + N, &S, sizeof(int64_t), cudaMemcpyHostToDevice, s));
+    PGD_LAUNCH(ctx, k_union_slots, grid_for(S), kThreads, 0, d_desc, d_bases + 2 * k + 2, k, S, U->adj);
+    PGD_LAUNCH(ctx, k_union_edges, grid_for(M), kThreads, 0, d_desc, d_bases + k + 1, k, M, U->ev, U->eu, U->order,
                egraph);
-    BATCH_TRY(build_aux(&U));
-    if (words > 0)
-        PGD_LAUNCH(ctx, k_dense_bits, grid_for(32 * N), kThreads, 0, U.off, U.adj, vgraph, d_gdense, d_wbase, d_bases,
-                   d_gnm, N, bits);
-    if (cn_entries > 0)
-        PGD_LAUNCH(ctx, k_dense_common, (int)std::min<int64_t>(ctile[(size_t)k], (int64_t)ctx->num_sms * 8), 256, 0,
-                   (const uint64_t *)bits, d_wbase, d_gnm, d_cbase, d_ctile, k, ctile[(size_t)k], cn);
-    DevGraph G = dev_view(&U, micro);
-    G.micro = micro ? umicro : nullptr;
-    G.sums = gsums;
-    G.egraph = egraph;
-    G.gnm = d_gnm;
-    G.gdense = ndense_graphs ? d_gdense : nullptr;
-    DenseView dv{(const uint64_t *)bits, d_wbase, d_bases, cn, d_cbase, k};
     StageMs ms;
-    BATCH_TRY(run_decompose(ctx, G, (int4 *)U.slot, U.nhubs, U.nhubs_wide, U.max_degree, &ms, ndense_graphs ? &dv : nullptr));
+    if ((st = decompose_union(U, k, gnm, d_gnm, d_bases, vgraph, egraph, gsums, umicro, &ms))) return st;
     std::vector<unsigned long long> h((size_t)k * PGD_NSUMS);
-    if (cudaMemcpyAsync(h.data(), gsums, h.size() * sizeof(unsigned long long), cudaMemcpyDeviceToHost, s)) {
-        cleanup();
-        return pgd_fail(ctx, PGD_ECUDA, "batch result copy failed");
-    }
+    PGD_CUDA(ctx, cudaMemcpyAsync(h.data(), gsums, h.size() * sizeof(unsigned long long), cudaMemcpyDeviceToHost, s));
     for (int i = 0; micro && i < k; i++) {
         pgd_graph *g = graphs[i];
-        if (g->m && cudaMemcpyAsync(g->micro, umicro + desc[(size_t)i].ebase * PGD_NMICRO,
-                                    g->m * PGD_NMICRO * sizeof(uint64_t), cudaMemcpyDeviceToDevice, s)) {
-            cleanup();
-            return pgd_fail(ctx, PGD_ECUDA, "batch micro copy failed");
-        }
+        if (g->m)
+            PGD_CUDA(ctx, cudaMemcpyAsync(g->micro, umicro + desc[(size_t)i].ebase * PGD_NMICRO,
+                                          g->m * PGD_NMICRO * sizeof(uint64_t), cudaMemcpyDeviceToDevice, s));
     }
     PGD_CUDA(ctx, cudaStreamSynchronize(s));
-    for (int i = 0; i < k; i++) {
-        pgd_counts &o = out[i];
-        memset(&o, 0, sizeof(o));
-        for (int j = 0; j < PGD_NSUMS; j++) o.sums[j] = h[(size_t)i * PGD_NSUMS + j];
-        o.n = gnm[(size_t)2 * i];
-        o.m = gnm[(size_t)2 * i + 1];
-        o.kernel_ms = ms.total;
-        o.hub_ms = ms.hub;
-        o.tri_ms = ms.tri;
-        pgd_close_counts(o.sums, o.n, o.m, o.totals);
-        graphs[i]->has_micro = micro;
-    }
-    cleanup();
-#undef BATCH_TRY
+    close_batch(k, h, gnm, ms, out);
+    for (int i = 0; i < k; i++) graphs[i]->has_micro = micro;
     return PGD_OK;
 }
 
@@ -3514,7 +3381,7 @@ extern "C" pgd_status pgd_decompose_csr_noalloc(const int64_t *d_off, const int3
             return PGD_ECUDA;
         }
         if ((int64_t)H.split < n) NA_CUDA(cudaMemsetAsync(gbm, 0, (size_t)nsm * nwords * 4, s));
-        NA_CUDA(cudaFuncSetAttribute(k_hub, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+        NA_CUDA(cudaFuncSetAttribute(k_hub, cudaFuncAttributeMaxDynamicSharedMemorySize, kMaxDynSmem));
         H.G = G;
         H.hpos = posv;
         H.hrec = hrec;
@@ -3592,9 +3459,25 @@ __global__ void k_vertex_graph(const int64_t *vbase, int k, int64_t N, int32_t *
         vgraph[x] = batch_find(vbase, k, x);
 }
 
-__global__ void k_edge_graph(const int32_t *ev, const int32_t *vgraph, int64_t M, int32_t *egraph) {
-    for (int64_t e = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; e < M; e += (int64_t)gridDim.x * blockDim.x)
-        egraph[e] = vgraph[ev[e]];
+// The edges of a batch in row order (their order does not change a global
+// count): edge base[r] + i is row r's i-th entry above the diagonal.
+__global__ void k_upper_edges(const int64_t *off, const int32_t *adj, const uint32_t *first, const uint32_t *base,
+                              const int32_t *vgraph, int64_t N, int64_t nnz, int32_t *ev, int32_t *eu, int32_t *order,
+                              int32_t *egraph) {
+    const int lane = threadIdx.x & 31;
+    const int64_t stride = (int64_t)gridDim.x * blockDim.x;
+    for (int64_t p0 = blockIdx.x * (int64_t)blockDim.x + threadIdx.x - lane; p0 < nnz; p0 += stride) {
+        const int64_t p = min(p0 + lane, nnz - 1);
+        const int64_t lo = pgd_slot_row(off, N, p0, min(p0 + 31, nnz - 1), p, lane);
+        const uint32_t f = first[lo];
+        if (p0 + lane < nnz && (uint32_t)p >= f) {
+            const uint32_t id = base[lo] + ((uint32_t)p - f);
+            ev[id] = (int32_t)lo;
+            eu[id] = adj[p];
+            order[id] = (int32_t)id;
+            egraph[id] = vgraph[lo];
+        }
+    }
 }
 
 __global__ void k_gather_offsets(const int64_t *off, const int64_t *vbase, int k, int64_t *out) {
@@ -3613,182 +3496,97 @@ pgd_status pgd_dev_decompose_pairs_batch(pgd_ctx *ctx, int k, const int64_t *pai
     for (int g = 0; g < k; g++)
         if (pair_off[g + 1] < pair_off[g]) return pgd_fail(ctx, PGD_EINVAL, "pair offsets must not decrease");
     const int64_t P1 = P > 0 ? P : 1;
-    int32_t *d_src = nullptr, *d_dst = nullptr, *vgraph = nullptr, *egraph = nullptr, *row = nullptr;
-    int64_t *d_poff = nullptr, *d_vbase = nullptr, *d_goff = nullptr, *d_wbase = nullptr;
-    int64_t *d_cbase = nullptr, *d_ctile = nullptr;
-    uint16_t *cn = nullptr;
-    int *gmax = nullptr;
-    uint32_t *flag = nullptr, *pos = nullptr;
-    unsigned long long *gsums = nullptr, *bits = nullptr;
-    long long *d_gnm = nullptr;
-    uint8_t *d_gdense = nullptr;
-    pgd_graph *U = new pgd_graph();
+    std::vector<long long> gnm((size_t)2 * k);
+    std::vector<unsigned long long> h((size_t)k * PGD_NSUMS);
+    StageMs ms;
+    struct Union {
+        pgd_graph *g = new pgd_graph();
+        ~Union() { pgd_graph_destroy(g); }
+    } holder;
+    pgd_graph *U = holder.g;
     U->ctx = ctx;
-    auto cleanup = [&]() {
-        for (void *p : {(void *)d_src, (void *)d_dst, (void *)vgraph, (void *)egraph, (void *)row, (void *)d_poff,
-                        (void *)d_vbase, (void *)d_goff, (void *)d_wbase, (void *)gmax, (void *)flag, (void *)pos,
-                        (void *)gsums, (void *)bits, (void *)d_gnm, (void *)d_gdense, (void *)cn, (void *)d_cbase,
-                        (void *)d_ctile})
-            pgd_tmp_free(ctx, p);
-        pgd_graph_destroy(U);
-    };
-#define PB_TRY(expr)                   \
-    do {                               \
-        if ((st = (expr)) != PGD_OK) { \
-            cleanup();                 \
-            return st;                 \
-        }                              \
-    } while (0)
-#define PB_CUDA(call)                                                  \
-    do {                                                               \
-        cudaError_t e__ = (call);                                      \
-        if (e__ != cudaSuccess) {                                      \
-            st = pgd_cuda_fail(ctx, e__, #call);                       \
-            cleanup();                                                 \
-            return st;                                                 \
-        }                                                              \
-    } while (0)
-    PB_TRY(pgd_tmp_alloc(ctx, (void **)&d_src, P1 * sizeof(int32_t)));
-    PB_TRY(pgd_tmp_alloc(ctx, (void **)&d_dst, P1 * sizeof(int32_t)));
-    PB_TRY(pgd_tmp_alloc(ctx, (void **)&d_poff, (k + 1) * sizeof(int64_t)));
-    PB_TRY(pgd_tmp_alloc(ctx, (void **)&d_vbase, (k + 1) * sizeof(int64_t)));
-    PB_TRY(pgd_tmp_alloc(ctx, (void **)&d_goff, (k + 1) * sizeof(int64_t)));
-    PB_TRY(pgd_tmp_alloc(ctx, (void **)&gmax, (size_t)k * sizeof(int)));
+    TmpGuard tg(ctx);
+    int32_t *d_src = nullptr, *vgraph = nullptr, *egraph = nullptr;
+    int64_t *d_poff = nullptr;
+    uint32_t *first = nullptr;
+    unsigned long long *gsums = nullptr;
+    const int64_t P2 = (P1 + 63) & ~(int64_t)63;   // both halves 256-byte aligned
+    if ((st = tg.alloc(&d_src, 2 * P2 * sizeof(int32_t)))) return st;
+    int32_t *d_dst = d_src + P2;
+    // pair offsets, vertex and entry offsets, n and m, largest id per graph
+    if ((st = tg.alloc(&d_poff, ((size_t)6 * k + 3) * sizeof(int64_t)))) return st;
+    int64_t *d_vbase = d_poff + k + 1, *d_goff = d_vbase + k + 1;
+    long long *d_gnm = (long long *)(d_goff + k + 1);
+    int *gmax = (int *)(d_gnm + 2 * k);
     if (P > 0) {
-        PB_CUDA(pgd_h2d(ctx, d_src, src, P * sizeof(int32_t)));
-        PB_CUDA(pgd_h2d(ctx, d_dst, dst, P * sizeof(int32_t)));
+        PGD_CUDA(ctx, pgd_h2d(ctx, d_src, src, P * sizeof(int32_t)));
+        PGD_CUDA(ctx, pgd_h2d(ctx, d_dst, dst, P * sizeof(int32_t)));
     }
-    PB_CUDA(cudaMemcpyAsync(d_poff, pair_off, (k + 1) * sizeof(int64_t), cudaMemcpyHostToDevice, s));
-    PB_CUDA(cudaMemsetAsync(gmax, 0xff, (size_t)k * sizeof(int), s));
+    PGD_CUDA(ctx, cudaMemcpyAsync(d_poff, pair_off, (k + 1) * sizeof(int64_t), cudaMemcpyHostToDevice, s));
+    PGD_CUDA(ctx, cudaMemsetAsync(gmax, 0xff, (size_t)k * sizeof(int), s));
     unsigned long long *bad = ctx->d_ctr + 7;
-    PB_CUDA(cudaMemsetAsync(bad, 0, sizeof(unsigned long long), s));
-    if (P > 0) PGD_LAUNCH(ctx, k_pairs_graph_max, grid_for(P), kThreads, 0, d_poff, k, d_src, d_dst, P, gmax, bad);
+    PGD_CUDA(ctx, cudaMemsetAsync(bad, 0, sizeof(unsigned long long), s));
+    if (P > 0)
+        PGD_LAUNCH(ctx, k_pairs_graph_max, (int)std::min<int64_t>(grid_for(P), 8 * (int64_t)ctx->num_sms), kThreads, 0,
+                   d_poff, k, d_src, d_dst, P, gmax, bad);
     std::vector<int> hmax((size_t)k);
     unsigned long long hbad = 0;
-    PB_CUDA(cudaMemcpyAsync(hmax.data(), gmax, (size_t)k * sizeof(int), cudaMemcpyDeviceToHost, s));
-    PB_CUDA(cudaMemcpyAsync(&hbad, bad, sizeof(hbad), cudaMemcpyDeviceToHost, s));
-    PB_CUDA(cudaStreamSynchronize(s));
-    if (hbad) {
-        cleanup();
-        return pgd_fail(ctx, PGD_EINVAL, "negative vertex id in a batched edge list");
-    }
+    PGD_CUDA(ctx, cudaMemcpyAsync(hmax.data(), gmax, (size_t)k * sizeof(int), cudaMemcpyDeviceToHost, s));
+    PGD_CUDA(ctx, cudaMemcpyAsync(&hbad, bad, sizeof(hbad), cudaMemcpyDeviceToHost, s));
+    PGD_CUDA(ctx, cudaStreamSynchronize(s));
+    if (hbad) return pgd_fail(ctx, PGD_EINVAL, "negative vertex id in a batched edge list");
     std::vector<int64_t> vbase((size_t)k + 1, 0);
     for (int g = 0; g < k; g++) {
         int64_t ng = std::max<int64_t>(n_min ? n_min[g] : 0, (int64_t)hmax[(size_t)g] + 1);
         vbase[(size_t)g + 1] = vbase[(size_t)g] + ng;
     }
     const int64_t N = vbase[(size_t)k];
-    if (N > 0x7ffffffe) {
-        cleanup();
-        return pgd_fail(ctx, PGD_EINVAL, "batch too large for 32-bit vertex ids");
-    }
-    PB_CUDA(cudaMemcpyAsync(d_vbase, vbase.data(), (k + 1) * sizeof(int64_t), cudaMemcpyHostToDevice, s));
+    if (N > 0x7ffffffe) return pgd_fail(ctx, PGD_EINVAL, "batch too large for 32-bit vertex ids");
+    PGD_CUDA(ctx, cudaMemcpyAsync(d_vbase, vbase.data(), (k + 1) * sizeof(int64_t), cudaMemcpyHostToDevice, s));
     if (P > 0) PGD_LAUNCH(ctx, k_pairs_shift, grid_for(P), kThreads, 0, d_poff, k, d_vbase, P, d_src, d_dst);
     // one CSR for the whole batch: symmetrised, deduplicated, self loops dropped
-    PB_TRY(pgd_build_from_device_pairs(U, d_src, d_dst, P, N, true));
-    pgd_tmp_free(ctx, d_src);
-    pgd_tmp_free(ctx, d_dst);
-    d_src = d_dst = nullptr;
+    if ((st = pgd_build_from_device_pairs(U, d_src, d_dst, P, N, true, false))) return st;
+    tg.release(d_src);
     const int64_t M = U->m, nnz = 2 * M;
     // per-graph edge counts from the offsets at the range boundaries
     std::vector<int64_t> goff((size_t)k + 1);
     PGD_LAUNCH(ctx, k_gather_offsets, grid_for(k + 1), kThreads, 0, U->off, d_vbase, k, d_goff);
-    PB_CUDA(cudaMemcpyAsync(goff.data(), d_goff, (k + 1) * sizeof(int64_t), cudaMemcpyDeviceToHost, s));
-    // edge arrays (edge id = position: the order does not change a global count)
-    PB_TRY(pgd_graph_alloc(U, (void **)&U->ev, (M + 1) * sizeof(int32_t)));
-    PB_TRY(pgd_graph_alloc(U, (void **)&U->eu, (M + 1) * sizeof(int32_t)));
-    PB_TRY(pgd_graph_alloc(U, (void **)&U->order, (M + 1) * sizeof(int32_t)));
-    U->norder = M;
-    PB_TRY(pgd_tmp_alloc(ctx, (void **)&row, (nnz + 1) * sizeof(int32_t)));
-    PB_TRY(pgd_tmp_alloc(ctx, (void **)&flag, (nnz + 1) * sizeof(uint32_t)));
-    PB_TRY(pgd_tmp_alloc(ctx, (void **)&pos, (nnz + 1) * sizeof(uint32_t)));
-    PB_TRY(pgd_tmp_alloc(ctx, (void **)&vgraph, (N + 1) * sizeof(int32_t)));
-    PB_TRY(pgd_tmp_alloc(ctx, (void **)&egraph, (M + 1) * sizeof(int32_t)));
-    if (nnz > 0) {
-        PGD_LAUNCH(ctx, k_rows, grid_for(nnz), kThreads, 0, U->off, N, nnz, row);
-        PGD_LAUNCH(ctx, k_na_edge_flags, grid_for(nnz), kThreads, 0, row, U->adj, nnz, flag);
-        PB_CUDA(cudaMemsetAsync(flag + nnz, 0, sizeof(uint32_t), s));
-        size_t tb = 0;
-        void *tmp = nullptr;
-        cub::DeviceScan::ExclusiveSum(nullptr, tb, flag, pos, nnz + 1, s);
-        PB_TRY(pgd_tmp_alloc(ctx, &tmp, tb));
-        cub::DeviceScan::ExclusiveSum(tmp, tb, flag, pos, nnz + 1, s);
-        pgd_tmp_free(ctx, tmp);
-        PGD_LAUNCH(ctx, k_na_edges, grid_for(nnz), kThreads, 0, row, U->adj, flag, pos, nnz, U->ev, U->eu, U->order);
-    }
-    if (N > 0) PGD_LAUNCH(ctx, k_vertex_graph, grid_for(N), kThreads, 0, d_vbase, k, N, vgraph);
-    if (M > 0) PGD_LAUNCH(ctx, k_edge_graph, grid_for(M), kThreads, 0, U->ev, vgraph, M, egraph);
-    PB_CUDA(cudaStreamSynchronize(s));
-    // per-graph n, m, dense flags
-    std::vector<long long> gnm((size_t)2 * k);
-    std::vector<uint8_t> gdense((size_t)k, 0);
-    std::vector<int64_t> wbase((size_t)k, 0);
-    int64_t words = 0;
-    int ndense_graphs = 0;
-    for (int g = 0; g < k; g++) {
-        const int64_t ng = vbase[(size_t)g + 1] - vbase[(size_t)g];
-        const int64_t mg = (goff[(size_t)g + 1] - goff[(size_t)g]) / 2;
-        gnm[(size_t)2 * g] = ng;
-        gnm[(size_t)2 * g + 1] = mg;
-        if (ng > 0 && ng <= ctx->dense_max && mg > 0) {
-            gdense[(size_t)g] = 1;
-            wbase[(size_t)g] = words;
-            words += ng * ((ng + 63) / 64);
-            ndense_graphs++;
-        }
-    }
-    std::vector<int64_t> cbase, ctile;
-    const int64_t cn_entries = plan_common(k, gnm, gdense, cbase, ctile);
-    if (cn_entries > 0) {
-        PB_TRY(pgd_tmp_alloc(ctx, (void **)&cn, (size_t)cn_entries * sizeof(uint16_t)));
-        PB_TRY(pgd_tmp_alloc(ctx, (void **)&d_cbase, (size_t)k * sizeof(int64_t)));
-        PB_TRY(pgd_tmp_alloc(ctx, (void **)&d_ctile, ((size_t)k + 1) * sizeof(int64_t)));
-        PB_CUDA(cudaMemcpyAsync(d_cbase, cbase.data(), (size_t)k * sizeof(int64_t), cudaMemcpyHostToDevice, s));
-        PB_CUDA(cudaMemcpyAsync(d_ctile, ctile.data(), ((size_t)k + 1) * sizeof(int64_t), cudaMemcpyHostToDevice, s));
-    }
-    PB_TRY(pgd_tmp_alloc(ctx, (void **)&gsums, (size_t)k * PGD_NSUMS * sizeof(unsigned long long)));
-    PB_TRY(pgd_tmp_alloc(ctx, (void **)&d_gnm, gnm.size() * sizeof(long long)));
-    PB_TRY(pgd_tmp_alloc(ctx, (void **)&d_gdense, (size_t)k));
-    PB_TRY(pgd_tmp_alloc(ctx, (void **)&d_wbase, (size_t)k * sizeof(int64_t)));
-    if (words > 0) PB_TRY(pgd_tmp_alloc(ctx, (void **)&bits, (size_t)words * sizeof(unsigned long long)));
-    PB_CUDA(cudaMemsetAsync(gsums, 0, (size_t)k * PGD_NSUMS * sizeof(unsigned long long), s));
-    PB_CUDA(cudaMemcpyAsync(d_gnm, gnm.data(), gnm.size() * sizeof(long long), cudaMemcpyHostToDevice, s));
-    PB_CUDA(cudaMemcpyAsync(d_gdense, gdense.data(), (size_t)k, cudaMemcpyHostToDevice, s));
-    PB_CUDA(cudaMemcpyAsync(d_wbase, wbase.data(), (size_t)k * sizeof(int64_t), cudaMemcpyHostToDevice, s));
-    if (words > 0) PB_CUDA(cudaMemsetAsync(bits, 0, (size_t)words * sizeof(unsigned long long), s));
-    StageMs ms;
+    PGD_CUDA(ctx, cudaMemcpyAsync(goff.data(), d_goff, (k + 1) * sizeof(int64_t), cudaMemcpyDeviceToHost, s));
     if (M > 0) {
-        PB_TRY(build_aux(U));
-        if (words > 0)
-            PGD_LAUNCH(ctx, k_dense_bits, grid_for(32 * N), kThreads, 0, U->off, U->adj, vgraph, d_gdense, d_wbase,
-                       d_vbase, d_gnm, N, bits);
-        if (cn_entries > 0)
-            PGD_LAUNCH(ctx, k_dense_common, (int)std::min<int64_t>(ctile[(size_t)k], (int64_t)ctx->num_sms * 8), 256,
-                       0, (const uint64_t *)bits, d_wbase, d_gnm, d_cbase, d_ctile, k, ctile[(size_t)k], cn);
-        DevGraph G = dev_view(U, false);
-        G.sums = gsums;
-        G.egraph = egraph;
-        G.gnm = d_gnm;
-        G.gdense = ndense_graphs ? d_gdense : nullptr;
-        DenseView dv{(const uint64_t *)bits, d_wbase, d_vbase, cn, d_cbase, k};
-        PB_TRY(run_decompose(ctx, G, (int4 *)U->slot, U->nhubs, U->nhubs_wide, U->max_degree, &ms, ndense_graphs ? &dv : nullptr));
+        if ((st = pgd_graph_alloc(U, (void **)&U->ev, (M + 1) * sizeof(int32_t)))) return st;
+        if ((st = pgd_graph_alloc(U, (void **)&U->eu, (M + 1) * sizeof(int32_t)))) return st;
+        if ((st = pgd_graph_alloc(U, (void **)&U->order, (M + 1) * sizeof(int32_t)))) return st;
+        U->norder = M;
+        size_t tb = 0;
+        cub::DeviceScan::ExclusiveSum(nullptr, tb, first, first, N + 1, s);
+        const size_t nb = (N + 1) * sizeof(uint32_t);
+        pgd_pieces W;
+        W.add(nb); W.add(nb); W.add(nb); W.add(nb); W.add((M + 1) * sizeof(int32_t)); W.add(tb);
+        if ((st = tg.alloc(&W.base, W.bytes))) return st;
+        vgraph = W.take<int32_t>(nb);
+        first = W.take<uint32_t>(nb);
+        uint32_t *count = W.take<uint32_t>(nb), *base = W.take<uint32_t>(nb);
+        egraph = W.take<int32_t>((M + 1) * sizeof(int32_t));
+        void *tmp = W.take<void>(tb);
+        PGD_LAUNCH(ctx, k_vertex_graph, grid_for(N), kThreads, 0, d_vbase, k, N, vgraph);
+        PGD_LAUNCH(ctx, pgd_upper_rows, grid_for(N + 1), kThreads, 0, U->off, U->adj, N, first, count);
+        PGD_CUDA(ctx, cub::DeviceScan::ExclusiveSum(tmp, tb, count, base, N + 1, s));
+        PGD_LAUNCH(ctx, k_upper_edges, grid_for(nnz), kThreads, 0, U->off, U->adj, first, base, vgraph, N, nnz, U->ev,
+                   U->eu, U->order, egraph);
     }
-    std::vector<unsigned long long> h((size_t)k * PGD_NSUMS);
-    PB_CUDA(cudaMemcpyAsync(h.data(), gsums, h.size() * sizeof(unsigned long long), cudaMemcpyDeviceToHost, s));
-    PB_CUDA(cudaStreamSynchronize(s));
+    PGD_CUDA(ctx, cudaStreamSynchronize(s));
     for (int g = 0; g < k; g++) {
-        pgd_counts &o = out[g];
-        memset(&o, 0, sizeof(o));
-        for (int j = 0; j < PGD_NSUMS; j++) o.sums[j] = h[(size_t)g * PGD_NSUMS + j];
-        o.n = gnm[(size_t)2 * g];
-        o.m = gnm[(size_t)2 * g + 1];
-        o.kernel_ms = ms.total;
-        o.hub_ms = ms.hub;
-        o.tri_ms = ms.tri;
-        pgd_close_counts(o.sums, o.n, o.m, o.totals);
+        gnm[(size_t)2 * g] = vbase[(size_t)g + 1] - vbase[(size_t)g];
+        gnm[(size_t)2 * g + 1] = (goff[(size_t)g + 1] - goff[(size_t)g]) / 2;
     }
-    cleanup();
-#undef PB_TRY
-#undef PB_CUDA
+    if (M > 0) {
+        if ((st = tg.alloc(&gsums, (size_t)k * PGD_NSUMS * sizeof(unsigned long long)))) return st;
+        PGD_CUDA(ctx, cudaMemsetAsync(gsums, 0, (size_t)k * PGD_NSUMS * sizeof(unsigned long long), s));
+        PGD_CUDA(ctx, cudaMemcpyAsync(d_gnm, gnm.data(), gnm.size() * sizeof(long long), cudaMemcpyHostToDevice, s));
+        if ((st = decompose_union(U, k, gnm, d_gnm, d_vbase, vgraph, egraph, gsums, nullptr, &ms))) return st;
+        PGD_CUDA(ctx, cudaMemcpyAsync(h.data(), gsums, h.size() * sizeof(unsigned long long), cudaMemcpyDeviceToHost, s));
+        PGD_CUDA(ctx, cudaStreamSynchronize(s));
+    }
+    close_batch(k, h, gnm, ms, out);
     return PGD_OK;
 }

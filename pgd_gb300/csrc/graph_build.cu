@@ -16,7 +16,9 @@
 #include <cub/cub.cuh>
 #include <vector>
 
+#include "cluster_ptx.cuh"
 #include "pgd_internal.h"
+#include "pgd_kernels.cuh"
 
 namespace {
 
@@ -54,26 +56,25 @@ __global__ void k_pair_stats(const int32_t *src, const int32_t *dst, int64_t k, 
     }
 }
 
-// Pair i -> directed entries 2i (a->b) and 2i+1 (b->a), both carrying i as
-// their insertion rank.  Self loops get a key that sorts after every edge.
-__global__ void k_make_entries(const int32_t *src, const int32_t *dst, int64_t k, uint64_t sentinel,
+// Pair i -> directed entries 2i (a->b) and 2i+1 (b->a) as row << cb | col, both
+// carrying i as their insertion rank (vals may be null).  Self loops get a key
+// that sorts after every edge.
+__global__ void k_make_entries(const int32_t *src, const int32_t *dst, int64_t k, uint64_t sentinel, int cb,
                                uint64_t *keys, uint32_t *vals) {
     for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < k; i += (int64_t)gridDim.x * blockDim.x) {
         uint32_t a = (uint32_t)src[i], b = (uint32_t)dst[i];
         uint64_t k0 = sentinel, k1 = sentinel;
         if (a != b) {
-            k0 = ((uint64_t)a << 32) | b;
-            k1 = ((uint64_t)b << 32) | a;
+            k0 = ((uint64_t)a << cb) | b;
+            k1 = ((uint64_t)b << cb) | a;
         }
-        keys[2 * i] = k0;
-        keys[2 * i + 1] = k1;
-        vals[2 * i] = (uint32_t)i;
-        vals[2 * i + 1] = (uint32_t)i;
+        *(ulonglong2 *)(keys + 2 * i) = ulonglong2{k0, k1};
+        if (vals) *(uint2 *)(vals + 2 * i) = make_uint2((uint32_t)i, (uint32_t)i);
     }
 }
 
-// CSR input -> entries (row<<32 | col), rank = position in the input.
-__global__ void k_csr_entries(const int64_t *off, const int32_t *adj, int64_t n, int64_t nnz, uint64_t *keys,
+// CSR input -> entries (row << cb | col), rank = position in the input.
+__global__ void k_csr_entries(const int64_t *off, const int32_t *adj, int64_t n, int64_t nnz, int cb, uint64_t *keys,
                               uint32_t *vals, unsigned long long *bad) {
     for (int64_t j = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; j < nnz; j += (int64_t)gridDim.x * blockDim.x) {
         // row of position j: last r with off[r] <= j
@@ -84,25 +85,26 @@ __global__ void k_csr_entries(const int64_t *off, const int32_t *adj, int64_t n,
         }
         int32_t c = adj[j];
         if (c < 0 || c >= n || c == lo) atomicAdd(bad, 1ull);
-        keys[j] = ((uint64_t)(uint32_t)lo << 32) | (uint32_t)c;
+        keys[j] = ((uint64_t)(uint32_t)lo << cb) | (uint32_t)c;
         vals[j] = (uint32_t)j;
     }
 }
 
-// first-of-run flags over the sorted valid prefix
+// first-of-run flags over the sorted valid prefix (and a 0 behind it)
 __global__ void k_unique_flags(const uint64_t *keys, int64_t valid, uint32_t *flags) {
-    for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < valid; i += (int64_t)gridDim.x * blockDim.x)
-        flags[i] = (i == 0 || keys[i] != keys[i - 1]) ? 1u : 0u;
+    for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i <= valid; i += (int64_t)gridDim.x * blockDim.x)
+        flags[i] = i < valid && (i == 0 || keys[i] != keys[i - 1]) ? 1u : 0u;
 }
 
 __global__ void k_scatter_unique(const uint64_t *keys, const uint32_t *vals, const uint32_t *flags,
-                                 const uint32_t *pos, int64_t valid, int32_t *adj, int64_t *rank, int32_t *row) {
+                                 const uint32_t *pos, int64_t valid, int cb, int32_t *adj, int64_t *rank,
+                                 int32_t *row) {
     for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < valid; i += (int64_t)gridDim.x * blockDim.x) {
         if (!flags[i]) continue;
         uint32_t p = pos[i];
-        adj[p] = (int32_t)(uint32_t)(keys[i] & 0xffffffffu);
-        row[p] = (int32_t)(keys[i] >> 32);
-        rank[p] = vals[i];
+        adj[p] = (int32_t)(keys[i] & ((1ull << cb) - 1));
+        row[p] = (int32_t)(keys[i] >> cb);
+        if (rank) rank[p] = vals[i];
     }
 }
 
@@ -115,9 +117,16 @@ __global__ void k_offsets(const int32_t *row, int64_t nnz, int64_t n, int64_t *o
     }
 }
 
-__global__ void k_degrees(const int64_t *off, int64_t n, int32_t *deg) {
-    for (int64_t v = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; v < n; v += (int64_t)gridDim.x * blockDim.x)
-        deg[v] = (int32_t)(off[v + 1] - off[v]);
+// Degrees and their maximum (*max_deg starts at 0).
+__global__ void k_degrees(const int64_t *off, int64_t n, int32_t *deg, int *max_deg) {
+    int top = 0;
+    for (int64_t v = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; v < n; v += (int64_t)gridDim.x * blockDim.x) {
+        const int d = (int)(off[v + 1] - off[v]);
+        deg[v] = d;
+        top = max(top, d);
+    }
+    top = __reduce_max_sync(0xffffffffu, top);
+    if ((threadIdx.x & 31) == 0 && top > 0) atomicMax(max_deg, top);
 }
 
 // Per-vertex sum over neighbours of f(x), one warp per vertex.
@@ -167,6 +176,46 @@ __global__ void k_rows_of(const int64_t *off, int64_t n, int64_t nnz, int32_t *r
 
 // ---------------------------------------------------------------------------
 // Neighbour order and edge ids.
+
+// The entries above the diagonal in CSR order, each as one word that sorts into
+// the order in which edges get their ids: by row, then by neighbour key, then by
+// insertion rank, key and rank descending unless s2l (see k_neigh_keys).  vals
+// gets the other endpoint.
+template <typename K>
+__global__ void k_neigh_words(const int64_t *off, const int32_t *adj, const int64_t *rank, const int32_t *deg,
+                              const int32_t *core, const uint32_t *first, const uint32_t *base, int64_t n, int64_t nnz,
+                              int kind, int descending, int db, int kb, K *keys, int32_t *vals) {
+    const int lane = threadIdx.x & 31;
+    const int64_t stride = (int64_t)gridDim.x * blockDim.x;
+    for (int64_t p0 = blockIdx.x * (int64_t)blockDim.x + threadIdx.x - lane; p0 < nnz; p0 += stride) {
+        const int64_t p = min(p0 + lane, nnz - 1);
+        const int64_t r = pgd_slot_row(off, n, p0, min(p0 + 31, nnz - 1), p, lane);
+        const uint32_t f = first[r];
+        if (p0 + lane >= nnz || (uint32_t)p < f) continue;
+        const uint32_t i = base[r] + ((uint32_t)p - f);
+        const int32_t c = adj[p];
+        uint64_t key = 0;
+        if (kind == PGD_NEIGH_DEG) key = (uint32_t)deg[c];
+        else if (kind == PGD_NEIGH_KCORE) key = (uint32_t)(c >= 1 ? core[c - 1] : 0);
+        uint64_t lo = (key << kb) | (uint64_t)rank[p];
+        if (descending) lo = ((1ull << (db + kb)) - 1) - lo;
+        keys[i] = (K)(((uint64_t)r << (db + kb)) | lo);
+        vals[i] = c;
+    }
+}
+
+// create_edge_list_arrays (graphlet_core.cpp:929-949) on the sorted words: e_v is
+// the endpoint with the smaller degree, ties go to the larger id.
+template <typename K>
+__global__ void k_edge_assign(const K *keys, const int32_t *vals, const int32_t *deg, int64_t m, int shift, int32_t *ev,
+                              int32_t *eu) {
+    for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < m; i += (int64_t)gridDim.x * blockDim.x) {
+        const int32_t r = (int32_t)((uint64_t)keys[i] >> shift), c = vals[i];
+        const bool low = deg[r] < deg[c];
+        ev[i] = low ? r : c;
+        eu[i] = low ? c : r;
+    }
+}
 
 // Composite within-row sort key: (neighbour key, insertion rank).  The
 // reference's stable counting sort followed by a reversal
@@ -321,76 +370,66 @@ int bit_length(uint64_t x) {
 
 // ---------------------------------------------------------------------------
 
-static pgd_status finish_csr(pgd_graph *g, uint64_t *keys, uint32_t *vals, int64_t valid, bool dedup,
-                             bool csr_input) {
+// The CSR of the sorted entries (row << cb | col), of which the first `valid` are
+// edges.  vals (insertion ranks, below rank_limit) may be null: the graph then
+// keeps none.
+static pgd_status finish_csr(pgd_graph *g, uint64_t *keys, uint32_t *vals, int64_t valid, int cb, int64_t rank_limit,
+                             bool dedup, bool csr_input) {
     pgd_ctx *ctx = g->ctx;
     cudaStream_t s = ctx->stream;
     uint32_t *flags = nullptr, *pos = nullptr;
     int32_t *row = nullptr;
     pgd_status st;
-    if ((st = pgd_tmp_alloc(ctx, (void **)&flags, (valid + 1) * sizeof(uint32_t)))) return st;
-    if ((st = pgd_tmp_alloc(ctx, (void **)&pos, (valid + 1) * sizeof(uint32_t)))) return st;
-    PGD_LAUNCH(ctx, k_unique_flags, grid_for(valid), kThreads, 0, keys, valid, flags);
     size_t tb = 0;
-    void *tmp = nullptr;
     cub::DeviceScan::ExclusiveSum(nullptr, tb, flags, pos, (int64_t)valid + 1, s);
-    if ((st = pgd_tmp_alloc(ctx, &tmp, tb))) return st;
-    // flags[valid] is scratch: clear it so pos[valid] = number of unique
-    PGD_CUDA(ctx, cudaMemsetAsync(flags + valid, 0, sizeof(uint32_t), s));
-    cub::DeviceScan::ExclusiveSum(tmp, tb, flags, pos, (int64_t)valid + 1, s);
-    pgd_tmp_free(ctx, tmp);
-    uint32_t nnz32 = 0;
-    PGD_CUDA(ctx, cudaMemcpyAsync(&nnz32, pos + valid, sizeof(uint32_t), cudaMemcpyDeviceToHost, s));
+    const size_t vb = (valid + 1) * sizeof(uint32_t);
+    pgd_pieces P;
+    P.add(vb); P.add(vb); P.add(vb); P.add(tb);
+    void *work = nullptr;
+    if ((st = pgd_tmp_alloc(ctx, &work, P.bytes))) return st;
+    struct Free {
+        pgd_ctx *ctx;
+        void *p;
+        ~Free() { pgd_tmp_free(ctx, p); }
+    } guard{ctx, work};
+    P.base = (uint8_t *)work;
+    flags = P.take<uint32_t>(vb);
+    pos = P.take<uint32_t>(vb);
+    row = P.take<int32_t>(vb);
+    void *tmp = P.take<void>(tb);
+    PGD_LAUNCH(ctx, k_unique_flags, grid_for(valid + 1), kThreads, 0, keys, valid, flags);
+    PGD_CUDA(ctx, cub::DeviceScan::ExclusiveSum(tmp, tb, flags, pos, (int64_t)valid + 1, s));
+    PGD_CUDA(ctx, pgd_fetch(ctx, 0, pos + valid, sizeof(uint32_t)));
     PGD_CUDA(ctx, cudaStreamSynchronize(s));
-    int64_t nnz = nnz32;
+    const int64_t nnz = pgd_pinned<uint32_t>(ctx, 0);
     if (nnz != valid) {
         if (!dedup) {
-            pgd_tmp_free(ctx, flags); pgd_tmp_free(ctx, pos);
             return pgd_fail(ctx, PGD_EINVAL, csr_input ? "CSR row lists a neighbour twice"
                                                        : "repeated pair without PGD_EDGES_DEDUP (multigraph input)");
         }
         g->duplicates = (valid - nnz) / 2;
     }
     g->m = nnz / 2;
+    g->rank_limit = rank_limit;
     if ((st = pgd_graph_alloc(g, (void **)&g->adj, (nnz + 1) * sizeof(int32_t)))) return st;
-    if ((st = pgd_graph_alloc(g, (void **)&g->rank, (nnz + 1) * sizeof(int64_t)))) return st;
+    if (vals && (st = pgd_graph_alloc(g, (void **)&g->rank, (nnz + 1) * sizeof(int64_t)))) return st;
     if ((st = pgd_graph_alloc(g, (void **)&g->off, (g->n + 1) * sizeof(int64_t)))) return st;
     if ((st = pgd_graph_alloc(g, (void **)&g->deg, (g->n + 1) * sizeof(int32_t)))) return st;
-    if ((st = pgd_graph_alloc(g, (void **)&g->vol2, (g->n + 1) * sizeof(uint64_t)))) return st;
-    if ((st = pgd_tmp_alloc(ctx, (void **)&row, (nnz + 1) * sizeof(int32_t)))) return st;
-    PGD_LAUNCH(ctx, k_scatter_unique, grid_for(valid), kThreads, 0, keys, vals, flags, pos, valid, g->adj, g->rank, row);
+    if (vals && (st = pgd_graph_alloc(g, (void **)&g->vol2, (g->n + 1) * sizeof(uint64_t)))) return st;
+    // [0] the maximum degree, [1] entries without their reverse
+    unsigned long long *ctr = ctx->d_ctr;
+    PGD_CUDA(ctx, cudaMemsetAsync(ctr, 0, 2 * sizeof(unsigned long long), s));
+    PGD_LAUNCH(ctx, k_scatter_unique, grid_for(valid), kThreads, 0, keys, vals, flags, pos, valid, cb, g->adj, g->rank,
+               row);
     PGD_LAUNCH(ctx, k_offsets, grid_for(nnz + 1), kThreads, 0, row, nnz, g->n, g->off);
-    PGD_LAUNCH(ctx, k_degrees, grid_for(g->n), kThreads, 0, g->off, g->n, g->deg);
-    if (csr_input && nnz > 0) {
-        unsigned long long *bad = ctx->d_ctr;
-        PGD_CUDA(ctx, cudaMemsetAsync(bad, 0, sizeof(unsigned long long), s));
-        PGD_LAUNCH(ctx, k_check_symmetric, grid_for(nnz), kThreads, 0, g->off, g->adj, row, nnz, bad);
-        unsigned long long h_bad = 0;
-        PGD_CUDA(ctx, cudaMemcpyAsync(&h_bad, bad, sizeof(h_bad), cudaMemcpyDeviceToHost, s));
-        PGD_CUDA(ctx, cudaStreamSynchronize(s));
-        if (h_bad) {
-            pgd_tmp_free(ctx, flags); pgd_tmp_free(ctx, pos); pgd_tmp_free(ctx, row);
-            return pgd_fail(ctx, PGD_EINVAL, "CSR is not symmetric (undirected graphs list each edge both ways)");
-        }
-    }
-    pgd_tmp_free(ctx, flags);
-    pgd_tmp_free(ctx, pos);
-    pgd_tmp_free(ctx, row);
-    // max degree and 2-hop volumes
-    int *d_max = (int *)ctx->d_ctr;
-    PGD_CUDA(ctx, cudaMemsetAsync(d_max, 0, sizeof(int), s));
-    if (g->n > 0) {
-        size_t tb2 = 0;
-        cub::DeviceReduce::Max(nullptr, tb2, g->deg, d_max, g->n, s);
-        if ((st = pgd_tmp_alloc(ctx, &tmp, tb2))) return st;
-        cub::DeviceReduce::Max(tmp, tb2, g->deg, d_max, g->n, s);
-        pgd_tmp_free(ctx, tmp);
-        PGD_LAUNCH(ctx, k_neigh_sum, grid_for(g->n * 32), kThreads, 0, g->off, g->adj, g->deg, nullptr, g->n, 0, g->vol2);
-    }
-    int h_max = 0;
-    PGD_CUDA(ctx, cudaMemcpyAsync(&h_max, d_max, sizeof(int), cudaMemcpyDeviceToHost, s));
+    PGD_LAUNCH(ctx, k_degrees, grid_for(g->n), kThreads, 0, g->off, g->n, g->deg, (int *)ctr);
+    if (csr_input && nnz > 0)
+        PGD_LAUNCH(ctx, k_check_symmetric, grid_for(nnz), kThreads, 0, g->off, g->adj, row, nnz, ctr + 1);
+    PGD_CUDA(ctx, pgd_fetch(ctx, 0, ctr, 2 * sizeof(unsigned long long)));
     PGD_CUDA(ctx, cudaStreamSynchronize(s));
-    g->max_degree = h_max;
+    if (pgd_pinned<unsigned long long>(ctx, 8))
+        return pgd_fail(ctx, PGD_EINVAL, "CSR is not symmetric (undirected graphs list each edge both ways)");
+    g->max_degree = pgd_pinned<int32_t>(ctx, 0);
     PGD_CUDA(ctx, cudaGetLastError());
     return PGD_OK;
 }
@@ -422,13 +461,10 @@ pgd_status pgd_build_from_pairs(pgd_graph *g, const int32_t *h_src, const int32_
     pgd_ctx *ctx = g->ctx;
     if (k < 0 || k > (int64_t)0x7fffffff) return pgd_fail(ctx, PGD_EINVAL, "pair count out of range (0..2^31-1)");
     pgd_status st;
-    int32_t *d_src = nullptr, *d_dst = nullptr;
-    const int64_t k1 = k > 0 ? k : 1;
-    if ((st = pgd_tmp_alloc(ctx, (void **)&d_src, k1 * sizeof(int32_t)))) return st;
-    if ((st = pgd_tmp_alloc(ctx, (void **)&d_dst, k1 * sizeof(int32_t)))) {
-        pgd_tmp_free(ctx, d_src);
-        return st;
-    }
+    int32_t *d_src = nullptr;
+    const int64_t k1 = ((k > 0 ? k : 1) + 63) & ~(int64_t)63;   // both halves 256-byte aligned
+    if ((st = pgd_tmp_alloc(ctx, (void **)&d_src, 2 * k1 * sizeof(int32_t)))) return st;
+    int32_t *d_dst = d_src + k1;
     cudaError_t e = cudaSuccess;
     if (k > 0) {
         e = pgd_h2d(ctx, d_src, h_src, k * sizeof(int32_t));
@@ -437,54 +473,64 @@ pgd_status pgd_build_from_pairs(pgd_graph *g, const int32_t *h_src, const int32_
     st = e == cudaSuccess ? pgd_build_from_device_pairs(g, d_src, d_dst, k, n_min, dedup)
                           : pgd_cuda_fail(ctx, e, "upload of the pairs");
     pgd_tmp_free(ctx, d_src);
-    pgd_tmp_free(ctx, d_dst);
     return st;
 }
 
 pgd_status pgd_build_from_device_pairs(pgd_graph *g, const int32_t *d_src, const int32_t *d_dst, int64_t k,
-                                       int64_t n_min, bool dedup) {
+                                       int64_t n_min, bool dedup, bool ranks) {
     pgd_ctx *ctx = g->ctx;
     cudaStream_t s = ctx->stream;
     if (k < 0 || k > (int64_t)0x7fffffff) return pgd_fail(ctx, PGD_EINVAL, "pair count out of range (0..2^31-1)");
     pgd_status st;
-    uint64_t *keys = nullptr, *keys2 = nullptr;
-    uint32_t *vals = nullptr, *vals2 = nullptr;
-    const int64_t k1 = k > 0 ? k : 1;
     // stats: [0] max id (int), [1] self loops, [2] bad ids
     unsigned long long *stats = ctx->d_ctr;
-    PGD_CUDA(ctx, cudaMemsetAsync(stats, 0, 4 * sizeof(unsigned long long), s));
+    PGD_CUDA(ctx, cudaMemsetAsync(stats, 0, 3 * sizeof(unsigned long long), s));
     PGD_CUDA(ctx, cudaMemsetAsync(stats, 0xff, sizeof(int), s));  // max id = -1
     if (k > 0)
-        PGD_LAUNCH(ctx, k_pair_stats, grid_for(k), kThreads, 0, d_src, d_dst, k, (int *)stats, stats + 1, stats + 2);
-    unsigned long long h_stats[3];
-    PGD_CUDA(ctx, cudaMemcpyAsync(h_stats, stats, sizeof(h_stats), cudaMemcpyDeviceToHost, s));
+        PGD_LAUNCH(ctx, k_pair_stats, (int)std::min<int64_t>(grid_for(k), 8 * (int64_t)ctx->num_sms), kThreads, 0,
+                   d_src, d_dst, k, (int *)stats, stats + 1, stats + 2);
+    PGD_CUDA(ctx, pgd_fetch(ctx, 0, stats, 3 * sizeof(unsigned long long)));
     PGD_CUDA(ctx, cudaStreamSynchronize(s));
-    const int max_id = (int)(h_stats[0] & 0xffffffffu);
-    if (h_stats[2]) return pgd_fail(ctx, PGD_EINVAL, "negative vertex id in edge list");
-    g->self_loops = (int64_t)h_stats[1];
+    const int max_id = pgd_pinned<int>(ctx, 0);
+    if (pgd_pinned<unsigned long long>(ctx, 16)) return pgd_fail(ctx, PGD_EINVAL, "negative vertex id in edge list");
+    g->self_loops = pgd_pinned<int64_t>(ctx, 8);
     g->n = std::max<int64_t>(n_min, (int64_t)max_id + 1);
-    const int64_t valid = 2 * (k - g->self_loops);
-    const int64_t ne = 2 * k1;
-    if ((st = pgd_tmp_alloc(ctx, (void **)&keys, ne * sizeof(uint64_t)))) return st;
-    if ((st = pgd_tmp_alloc(ctx, (void **)&keys2, ne * sizeof(uint64_t)))) return st;
-    if ((st = pgd_tmp_alloc(ctx, (void **)&vals, ne * sizeof(uint32_t)))) return st;
-    if ((st = pgd_tmp_alloc(ctx, (void **)&vals2, ne * sizeof(uint32_t)))) return st;
-    const uint64_t sentinel = (uint64_t)(uint32_t)(max_id + 1) << 32;
-    if (k > 0) PGD_LAUNCH(ctx, k_make_entries, grid_for(k), kThreads, 0, d_src, d_dst, k, sentinel, keys, vals);
-    const int end_bit = 32 + bit_length((uint64_t)(max_id + 1));
-    if (k > 0) {
-        size_t tb = 0;
-        void *tmp = nullptr;
-        cub::DeviceRadixSort::SortPairs(nullptr, tb, keys, keys2, vals, vals2, (int64_t)(2 * k), 0, end_bit, s);
-        if ((st = pgd_tmp_alloc(ctx, &tmp, tb))) return st;
-        cub::DeviceRadixSort::SortPairs(tmp, tb, keys, keys2, vals, vals2, (int64_t)(2 * k), 0, end_bit, s);
-        pgd_tmp_free(ctx, tmp);
+    const int64_t valid = 2 * (k - g->self_loops), ne = 2 * k;
+    // a word holds row and column on the bits that ids up to max_id + 1 need
+    const int cb = std::max(1, bit_length((uint64_t)(max_id + 1)));
+    const uint64_t sentinel = (uint64_t)(uint32_t)(max_id + 1) << cb;
+    uint64_t *keys = nullptr, *keys2 = nullptr;
+    uint32_t *vals = nullptr, *vals2 = nullptr;
+    size_t tb = 0;
+    if (ranks) cub::DeviceRadixSort::SortPairs(nullptr, tb, keys, keys2, vals, vals2, ne, 0, 2 * cb, s);
+    else cub::DeviceRadixSort::SortKeys(nullptr, tb, keys, keys2, ne, 0, 2 * cb, s);
+    const size_t kbytes = ne * sizeof(uint64_t), vbytes = ranks ? ne * sizeof(uint32_t) : 0;
+    pgd_pieces P1, P2;   // the inputs of the sort are freed after it, its outputs after the CSR is built
+    P1.add(kbytes); P1.add(vbytes); P1.add(tb);
+    P2.add(kbytes); P2.add(vbytes);
+    void *w1 = nullptr, *w2 = nullptr;
+    if ((st = pgd_tmp_alloc(ctx, &w1, P1.bytes))) return st;
+    if ((st = pgd_tmp_alloc(ctx, &w2, P2.bytes))) {
+        pgd_tmp_free(ctx, w1);
+        return st;
     }
-    pgd_tmp_free(ctx, keys);
-    pgd_tmp_free(ctx, vals);
-    st = finish_csr(g, keys2, vals2, valid, dedup, false);
-    pgd_tmp_free(ctx, keys2);
-    pgd_tmp_free(ctx, vals2);
+    P1.base = (uint8_t *)w1;
+    P2.base = (uint8_t *)w2;
+    keys = P1.take<uint64_t>(kbytes);
+    keys2 = P2.take<uint64_t>(kbytes);
+    if (ranks) {
+        vals = P1.take<uint32_t>(vbytes);
+        vals2 = P2.take<uint32_t>(vbytes);
+    }
+    void *tmp = P1.take<void>(tb);
+    if (k > 0) {
+        PGD_LAUNCH(ctx, k_make_entries, grid_for(k), kThreads, 0, d_src, d_dst, k, sentinel, cb, keys, vals);
+        if (ranks) cub::DeviceRadixSort::SortPairs(tmp, tb, keys, keys2, vals, vals2, ne, 0, 2 * cb, s);
+        else cub::DeviceRadixSort::SortKeys(tmp, tb, keys, keys2, ne, 0, 2 * cb, s);
+    }
+    pgd_tmp_free(ctx, w1);
+    st = finish_csr(g, keys2, vals2, valid, cb, k, dedup, false);
+    pgd_tmp_free(ctx, w2);
     return st;
 }
 
@@ -514,7 +560,8 @@ pgd_status pgd_build_from_csr(pgd_graph *g, const int64_t *h_off, const int32_t 
     if ((st = pgd_tmp_alloc(ctx, (void **)&vals2, nz1 * sizeof(uint32_t)))) return st;
     unsigned long long *bad = ctx->d_ctr;
     PGD_CUDA(ctx, cudaMemsetAsync(bad, 0, sizeof(unsigned long long), s));
-    if (nnz) PGD_LAUNCH(ctx, k_csr_entries, grid_for(nnz), kThreads, 0, d_off, d_adj, n, nnz, keys, vals, bad);
+    const int cb = std::max(1, bit_length((uint64_t)n));
+    if (nnz) PGD_LAUNCH(ctx, k_csr_entries, grid_for(nnz), kThreads, 0, d_off, d_adj, n, nnz, cb, keys, vals, bad);
     unsigned long long h_bad = 0;
     PGD_CUDA(ctx, cudaMemcpyAsync(&h_bad, bad, sizeof(h_bad), cudaMemcpyDeviceToHost, s));
     PGD_CUDA(ctx, cudaStreamSynchronize(s));
@@ -525,7 +572,7 @@ pgd_status pgd_build_from_csr(pgd_graph *g, const int64_t *h_off, const int32_t 
         return pgd_fail(ctx, PGD_EINVAL, "CSR neighbour id out of range or a self loop");
     }
     if (nnz) {
-        int end_bit = 32 + bit_length((uint64_t)n);
+        const int end_bit = 2 * cb;
         size_t tb = 0;
         void *tmp = nullptr;
         cub::DeviceRadixSort::SortPairs(nullptr, tb, keys, keys2, vals, vals2, nnz, 0, end_bit, s);
@@ -535,10 +582,46 @@ pgd_status pgd_build_from_csr(pgd_graph *g, const int64_t *h_off, const int32_t 
     }
     pgd_tmp_free(ctx, keys);
     pgd_tmp_free(ctx, vals);
-    st = finish_csr(g, keys2, vals2, nnz, false, true);
+    st = finish_csr(g, keys2, vals2, nnz, cb, nnz, false, true);
     pgd_tmp_free(ctx, keys2);
     pgd_tmp_free(ctx, vals2);
     return st;
+}
+
+// Edge ids by one sort of words of type K (rb bits of row, db of key, kb of rank).
+template <typename K>
+static pgd_status order_by_words(pgd_graph *g, int kind, bool descending, int rb, int db, int kb) {
+    pgd_ctx *ctx = g->ctx;
+    cudaStream_t s = ctx->stream;
+    pgd_status st;
+    const int64_t n = g->n, m = g->m;
+    uint32_t *first = nullptr, *count = nullptr, *base = nullptr;
+    K *keys = nullptr;
+    int32_t *vals = nullptr;
+    size_t tb1 = 0, tb2 = 0;
+    cub::DeviceScan::ExclusiveSum(nullptr, tb1, first, first, n + 1, s);
+    cub::DeviceRadixSort::SortPairs(nullptr, tb2, keys, keys, vals, vals, m, 0, rb + db + kb, s);
+    const size_t nb = (n + 1) * sizeof(uint32_t), tb = std::max(tb1, tb2);
+    pgd_pieces P;
+    P.add(nb); P.add(nb); P.add(nb); P.add(2 * m * sizeof(K)); P.add(2 * m * sizeof(int32_t)); P.add(tb);
+    void *work = nullptr;
+    if ((st = pgd_tmp_alloc(ctx, &work, P.bytes))) return st;
+    P.base = (uint8_t *)work;
+    first = P.take<uint32_t>(nb);
+    count = P.take<uint32_t>(nb);
+    base = P.take<uint32_t>(nb);
+    keys = P.take<K>(2 * m * sizeof(K));
+    vals = P.take<int32_t>(2 * m * sizeof(int32_t));
+    void *tmp = P.take<void>(tb);
+    PGD_LAUNCH(ctx, pgd_upper_rows, grid_for(n + 1), kThreads, 0, g->off, g->adj, n, first, count);
+    cub::DeviceScan::ExclusiveSum(tmp, tb1, count, base, n + 1, s);
+    PGD_LAUNCH(ctx, k_neigh_words<K>, grid_for(2 * m), kThreads, 0, g->off, g->adj, g->rank, g->deg, g->core, first,
+               base, n, 2 * m, kind, (int)descending, db, kb, keys, vals);
+    cub::DeviceRadixSort::SortPairs(tmp, tb2, keys, keys + m, vals, vals + m, m, 0, rb + db + kb, s);
+    PGD_LAUNCH(ctx, k_edge_assign<K>, grid_for(m), kThreads, 0, keys + m, vals + m, g->deg, m, db + kb, g->ev, g->eu);
+    pgd_tmp_free(ctx, work);
+    PGD_CUDA(ctx, cudaGetLastError());
+    return PGD_OK;
 }
 
 pgd_status pgd_dev_preprocess(pgd_graph *g, int neigh_kind, int s2l) {
@@ -551,6 +634,22 @@ pgd_status pgd_dev_preprocess(pgd_graph *g, int neigh_kind, int s2l) {
         if ((st = pgd_graph_alloc(g, (void **)&g->eu, (g->m + 1) * sizeof(int32_t)))) return st;
     }
     if (nnz == 0) { g->preprocessed = true; return PGD_OK; }
+    // One sort of the m entries above the diagonal by (row, key, rank) where a
+    // 64-bit word holds them (32-bit where that does); else the rows' segments of
+    // all 2m entries are sorted.
+    const bool descend = (neigh_kind != PGD_NEIGH_ASREAD) && !s2l;
+    const int rb = std::max(1, bit_length((uint64_t)g->n)), kb = std::max(1, bit_length((uint64_t)g->rank_limit));
+    const int db = neigh_kind == PGD_NEIGH_ASREAD ? 0
+                   : std::max(1, bit_length((uint64_t)(neigh_kind == PGD_NEIGH_DEG ? g->max_degree : g->max_core)));
+    if (rb + db + kb <= 64) {
+        st = rb + db + kb <= 32 ? order_by_words<uint32_t>(g, neigh_kind, descend, rb, db, kb)
+                                : order_by_words<uint64_t>(g, neigh_kind, descend, rb, db, kb);
+        if (st) return st;
+        g->preprocessed = true;
+        g->sorted = false;
+        g->has_micro = false;
+        return PGD_OK;
+    }
     int32_t *row = nullptr;
     uint64_t *keys = nullptr, *keys2 = nullptr;
     uint32_t *idx = nullptr, *perm = nullptr, *flags = nullptr, *ids = nullptr;
@@ -599,6 +698,186 @@ pgd_status pgd_dev_preprocess(pgd_graph *g, int neigh_kind, int s2l) {
     return PGD_OK;
 }
 
+// k-core of graphs of up to kCoreClusterEntries adjacency entries: one cluster of
+// eight blocks peels the whole graph in one launch.  What bounds it is the chain
+// of steps (832 on R-MAT 20, 448 on R-MAT 16), each a few dependent L2 accesses
+// and a barrier: the cluster's hardware barrier replaces two graph nodes per step
+// (k_core_work and k_core_ctrl below, about 8 us together with their gaps), and
+// no graph is captured and instantiated for the call (180 us).
+namespace {
+
+constexpr int kCoreBlocks = 8;              // a portable cluster
+constexpr int kCoreThreads = 1024;
+constexpr int64_t kCoreClusterEntries = 64ll << 20;
+constexpr int kCoreLong = 1024;             // rows at least this long are shared by all warps
+
+struct CoreSlot {
+    unsigned int front, lng, alive;         // entries appended in this step
+    int min_rest;                           // smallest count among the vertices left
+};
+struct CoreShared {
+    CoreSlot slot[3];                       // by step modulo 3: written, read after the barrier, cleared a step later
+    int max_core, failed;
+};
+
+__device__ __forceinline__ void core_append(bool in, int32_t v, int32_t *list, unsigned int *count, int lane) {
+    const unsigned m = __ballot_sync(0xffffffffu, in);
+    if (!m) return;
+    unsigned at = 0;
+    if (lane == 0) at = atomicAdd(count, (unsigned)__popc(m));
+    at = __shfl_sync(0xffffffffu, at, 0);
+    if (in) list[at + __popc(m & ((1u << lane) - 1))] = v;
+}
+
+// f and b: two buffers each (n entries) of the frontier's short and long rows;
+// a0, a1: vertices alive.  A level scan moves every alive vertex of count <=
+// level to the frontier and the others to the other alive list; a peel round
+// takes one off the count of the frontier's neighbours.
+__global__ void __cluster_dims__(kCoreBlocks, 1, 1) __launch_bounds__(kCoreThreads, 1)
+k_core_cluster(const int64_t *off, const int32_t *adj, const int32_t *deg, int n, int32_t *cur, int32_t *core,
+               int32_t *f0, int32_t *f1, int32_t *b0, int32_t *b1, int32_t *a0, int32_t *a1, CoreShared *S,
+               int max_degree) {
+    const int lane = threadIdx.x & 31;
+    const int rank = (int)pgd_cl::cluster_rank();
+    constexpr int kAll = kCoreBlocks * kCoreThreads;
+    const int t = rank * kCoreThreads + (int)threadIdx.x, w = t >> 5;
+    const int t0 = t - lane;
+    for (int v = t; v < n; v += kAll) {
+        cur[v] = deg[v];
+        core[v] = -1;
+        a0[v] = v;
+    }
+    if (t == 0) {
+        for (int i = 0; i < 3; i++) S->slot[i] = CoreSlot{0, 0, 0, INT_MAX};
+        S->max_core = 0;
+        S->failed = 0;
+    }
+    pgd_cl::cluster_sync();
+    int level = 0, removed = 0;
+    unsigned na = (unsigned)n;
+    long long step = 0;
+    const long long max_steps = 2ll * n + max_degree + 8;   // every step removes a vertex or raises the level
+    int32_t *ain = a0, *aout = a1, *fin = f0, *fout = f1, *bin = b0, *bout = b1;
+    auto next_slot = [&]() -> CoreSlot * {   // this step's slot; the one after it is cleared
+        CoreSlot *s = &S->slot[step % 3];
+        if (t == 0) S->slot[(step + 1) % 3] = CoreSlot{0, 0, 0, INT_MAX};
+        step++;
+        return s;
+    };
+    while (removed < n && step < max_steps) {
+        CoreSlot *s = next_slot();
+        int low = INT_MAX;
+        for (unsigned i0 = (unsigned)t0; i0 < na; i0 += kAll) {
+            const unsigned i = i0 + lane;
+            bool leaves = false, stays = false;
+            int32_t v = 0;
+            int d = 0;
+            if (i < na) {
+                v = __ldcg(ain + i);
+                if (__ldcg(core + v) == -1) {
+                    const int c = __ldcg(cur + v);
+                    leaves = c <= level;
+                    stays = !leaves;
+                    if (leaves) {
+                        __stcg(core + v, level);
+                        d = deg[v];
+                    } else {
+                        low = min(low, c);
+                    }
+                }
+            }
+            core_append(leaves && d < kCoreLong, v, fin, &s->front, lane);
+            core_append(leaves && d >= kCoreLong, v, bin, &s->lng, lane);
+            core_append(stays, v, aout, &s->alive, lane);
+        }
+        low = __reduce_min_sync(0xffffffffu, low);
+        if (lane == 0 && low != INT_MAX) atomicMin(&s->min_rest, low);
+        pgd_cl::cluster_sync();
+        unsigned nf = __ldcg(&s->front), nb = __ldcg(&s->lng);
+        na = __ldcg(&s->alive);
+        int32_t *x = ain;
+        ain = aout;
+        aout = x;
+        if (nf + nb == 0) {
+            level = max(level + 1, __ldcg(&s->min_rest));   // nobody at this level: on to the smallest count
+            continue;
+        }
+        removed += (int)(nf + nb);
+        while (nf + nb > 0 && step < max_steps) {
+            s = next_slot();
+            // one off the count of neighbour x; it leaves when that drops to the level
+            auto visit = [&](bool act, int64_t j) {
+                bool leaves = false;
+                int32_t y = 0;
+                int d = 0;
+                if (act) {
+                    y = __ldg(adj + j);
+                    if (__ldcg(core + y) == -1 && atomicSub(cur + y, 1) == level + 1) {
+                        __stcg(core + y, level);
+                        leaves = true;
+                        d = deg[y];
+                    }
+                }
+                core_append(leaves && d < kCoreLong, y, fout, &s->front, lane);
+                core_append(leaves && d >= kCoreLong, y, bout, &s->lng, lane);
+            };
+            for (unsigned i = (unsigned)w; i < nf; i += kAll / 32) {   // a warp per short row
+                const int32_t v = __ldcg(fin + i);
+                const int64_t o = off[v], e = o + deg[v];
+                for (int64_t j = o; j < e; j += 32) visit(j + lane < e, j + lane);
+            }
+            for (unsigned i = 0; i < nb; i++) {                        // all warps share a long row
+                const int32_t v = __ldcg(bin + i);
+                const int64_t o = off[v], e = o + deg[v];
+                for (int64_t j = o + t0; j < e; j += kAll) visit(j + lane < e, j + lane);
+            }
+            pgd_cl::cluster_sync();
+            nf = __ldcg(&s->front);
+            nb = __ldcg(&s->lng);
+            removed += (int)(nf + nb);
+            x = fin;
+            fin = fout;
+            fout = x;
+            x = bin;
+            bin = bout;
+            bout = x;
+        }
+        level++;
+    }
+    // the value the reference prints leaves the last vertex out
+    int top = 0;
+    for (int v = t; v < n - 1; v += kAll) top = max(top, __ldcg(core + v));
+    top = __reduce_max_sync(0xffffffffu, top);
+    if (lane == 0 && top > 0) atomicMax(&S->max_core, top);
+    if (t == 0 && removed < n) S->failed = 1;
+}
+
+}  // namespace
+
+static pgd_status cores_by_cluster(pgd_graph *g) {
+    pgd_ctx *ctx = g->ctx;
+    cudaStream_t s = ctx->stream;
+    const int64_t n = g->n;
+    int32_t *work = nullptr;
+    pgd_status st;
+    const size_t lists = (7 * (size_t)n * sizeof(int32_t) + 15) & ~(size_t)15;
+    if ((st = pgd_tmp_alloc(ctx, (void **)&work, lists + sizeof(CoreShared)))) return st;
+    CoreShared *S = (CoreShared *)((uint8_t *)work + lists);
+    PGD_LAUNCH(ctx, k_core_cluster, kCoreBlocks, kCoreThreads, 0, g->off, g->adj, g->deg, (int)n, work, g->core,
+               work + n, work + 2 * n, work + 3 * n, work + 4 * n, work + 5 * n, work + 6 * n, S, g->max_degree);
+    cudaError_t e = cudaGetLastError();
+    if (e == cudaSuccess) e = pgd_fetch(ctx, 0, S, sizeof(CoreShared));
+    if (e == cudaSuccess) e = cudaStreamSynchronize(s);
+    pgd_tmp_free(ctx, work);
+    if (e != cudaSuccess) return pgd_cuda_fail(ctx, e, "k-core peeling");
+    const CoreShared h = pgd_pinned<CoreShared>(ctx, 0);
+    if (h.failed) return pgd_fail(ctx, PGD_EINVAL, "k-core peeling did not converge");
+    g->max_core = h.max_core;
+    g->has_cores = true;
+    return PGD_OK;
+}
+
+// Larger graphs, on the whole device.
 // Device-driven peeling: the state machine below replaces a host loop with
 // one round trip per level and per peel round.  Each step is a work kernel
 // (a level scan or a peel round, chosen from the state) and a one-thread
@@ -719,6 +998,7 @@ pgd_status pgd_dev_cores(pgd_graph *g) {
         if ((st = pgd_graph_alloc(g, (void **)&g->core, (n + 1) * sizeof(int32_t)))) return st;
     }
     if (n == 0) { g->has_cores = true; g->max_core = 0; return PGD_OK; }
+    if (2 * g->m <= kCoreClusterEntries) return cores_by_cluster(g);
     int32_t *cur = nullptr, *fa = nullptr, *fb = nullptr, *aa = nullptr, *ab = nullptr;
     CoreState *d_st = nullptr;
     if ((st = pgd_tmp_alloc(ctx, (void **)&cur, n * sizeof(int32_t)))) return st;
@@ -842,6 +1122,10 @@ static pgd_status sort_edges_impl(pgd_graph *g, int kind, int s2l, const int32_t
     uint64_t *vsum = nullptr;
     if (kind == PGD_ORD_DEG_VOL) {
         vsum = g->vol2;
+        if (!g->has_vol2) {
+            PGD_LAUNCH(ctx, k_neigh_sum, grid_for(g->n * 32), kThreads, 0, g->off, g->adj, g->deg, nullptr, g->n, 0, vsum);
+            g->has_vol2 = true;
+        }
     } else if (kind == PGD_ORD_KCORE_VOL || kind == PGD_ORD_KCORE_DEG_VOL) {
         if ((st = pgd_tmp_alloc(ctx, (void **)&vsum, g->n * sizeof(uint64_t)))) return st;
         PGD_LAUNCH(ctx, k_neigh_sum, grid_for(g->n * 32), kThreads, 0, g->off, g->adj, g->deg, g->core, g->n,
@@ -869,20 +1153,23 @@ static pgd_status sort_edges_impl(pgd_graph *g, int kind, int s2l, const int32_t
     if (!d_ids) {
         uint32_t *keys = nullptr, *keys2 = nullptr;
         int32_t *ids = nullptr;
-        if ((st = pgd_tmp_alloc(ctx, (void **)&keys, count * sizeof(uint32_t)))) return st;
-        if ((st = pgd_tmp_alloc(ctx, (void **)&keys2, count * sizeof(uint32_t)))) return st;
-        if ((st = pgd_tmp_alloc(ctx, (void **)&ids, count * sizeof(int32_t)))) return st;
-        PGD_LAUNCH(ctx, k_edge_keys, grid_for(count), kThreads, 0, g->ev, g->eu, g->deg, g->core, vsum, count, kind,
-                   flip, keys, ids);
         if (s2l) cub::DeviceRadixSort::SortPairs(nullptr, tb, keys, keys2, ids, g->order, count, 0, kb, s);
         else cub::DeviceRadixSort::SortPairsDescending(nullptr, tb, keys, keys2, ids, g->order, count, 0, kb, s);
-        if ((st = pgd_tmp_alloc(ctx, &tmp, tb))) return st;
+        const size_t cb = count * sizeof(uint32_t);
+        pgd_pieces P;
+        P.add(cb); P.add(cb); P.add(cb); P.add(tb);
+        void *work = nullptr;
+        if ((st = pgd_tmp_alloc(ctx, &work, P.bytes))) return st;
+        P.base = (uint8_t *)work;
+        keys = P.take<uint32_t>(cb);
+        keys2 = P.take<uint32_t>(cb);
+        ids = P.take<int32_t>(cb);
+        tmp = P.take<void>(tb);
+        PGD_LAUNCH(ctx, k_edge_keys, grid_for(count), kThreads, 0, g->ev, g->eu, g->deg, g->core, vsum, count, kind,
+                   flip, keys, ids);
         if (s2l) cub::DeviceRadixSort::SortPairs(tmp, tb, keys, keys2, ids, g->order, count, 0, kb, s);
         else cub::DeviceRadixSort::SortPairsDescending(tmp, tb, keys, keys2, ids, g->order, count, 0, kb, s);
-        pgd_tmp_free(ctx, tmp);
-        pgd_tmp_free(ctx, keys);
-        pgd_tmp_free(ctx, keys2);
-        pgd_tmp_free(ctx, ids);
+        pgd_tmp_free(ctx, work);
     } else {
         uint64_t *keys = nullptr, *keys2 = nullptr;
         if ((st = pgd_tmp_alloc(ctx, (void **)&keys, count * sizeof(uint64_t)))) return st;

@@ -3,6 +3,7 @@
 
 #include <cuda_runtime.h>
 #include <stdint.h>
+#include <string.h>
 
 #include <string>
 
@@ -21,6 +22,7 @@ struct pgd_ctx {
     // decomposition scratch: per-launch counters and sums
     unsigned long long *d_sums = nullptr;   // PGD_NSUMS
     unsigned long long *d_ctr = nullptr;    // work counters
+    uint8_t *pin = nullptr;                 // page-locked, for small results read back (kPinBytes)
     cudaEvent_t ev0 = nullptr, ev1 = nullptr;
     // stage events of a decomposition: triangle pass [evt0, evt1), k_hub [evh0, evh1)
     cudaEvent_t evt0 = nullptr, evt1 = nullptr, evh0 = nullptr, evh1 = nullptr;
@@ -45,7 +47,9 @@ struct pgd_graph {
     int32_t *adj = nullptr;           // 2m
     int32_t *deg = nullptr;           // n
     int64_t *rank = nullptr;          // 2m insertion rank of each entry
-    uint64_t *vol2 = nullptr;         // n: sum of neighbour degrees
+    int64_t rank_limit = 0;           // every rank is below this
+    uint64_t *vol2 = nullptr;         // n: sum of neighbour degrees, filled by the first order that uses it
+    bool has_vol2 = false;
 
     // preprocess: edge arrays by edge id (graphlet_core.cpp:929-949)
     bool preprocessed = false;
@@ -113,11 +117,46 @@ void pgd_rank_drop(pgd_graph *g);   // frees g's rank-ordered copy, if any
 pgd_status pgd_tmp_alloc(pgd_ctx *ctx, void **p, size_t bytes);
 void pgd_tmp_free(pgd_ctx *ctx, void *p);
 
+constexpr size_t kPinBytes = 4096;
+
+// Enqueues the copy of a small device result to page-locked memory; the value is
+// there (pgd_pinned) once the stream has been waited for.  The copy engine writes
+// page-locked memory without the staging and the wait of a pageable copy.
+inline cudaError_t pgd_fetch(pgd_ctx *ctx, size_t at, const void *src, size_t bytes) {
+    return cudaMemcpyAsync(ctx->pin + at, src, bytes, cudaMemcpyDeviceToHost, ctx->stream);
+}
+template <typename T>
+inline T pgd_pinned(const pgd_ctx *ctx, size_t at) {
+    T v;
+    memcpy(&v, ctx->pin + at, sizeof(T));
+    return v;
+}
+
+// Several arrays in one stream-ordered allocation, each 256-byte aligned: the
+// sizes are added up first, then the pieces are taken in the same order.
+struct pgd_pieces {
+    size_t bytes = 0;
+    uint8_t *base = nullptr;
+    static size_t up(size_t b) { return (b + 255) & ~(size_t)255; }
+    void add(size_t b) { bytes += up(b); }
+    template <typename T>
+    T *take(size_t b) {
+        T *p = (T *)base;
+        base += up(b);
+        return p;
+    }
+};
+
+// Limits of the kernels that use more shared memory than the default, set to
+// the same constants for every context of the device (decompose.cu, rank_path.cu).
+cudaError_t pgd_decompose_limits();
+cudaError_t pgd_rank_limits();
+
 // Device stages (graph_build.cu).
 pgd_status pgd_build_from_pairs(pgd_graph *g, const int32_t *h_src, const int32_t *h_dst, int64_t k,
                                 int64_t n_min, bool dedup);
 pgd_status pgd_build_from_device_pairs(pgd_graph *g, const int32_t *d_src, const int32_t *d_dst, int64_t k,
-                                       int64_t n_min, bool dedup);
+                                       int64_t n_min, bool dedup, bool ranks = true);
 pgd_status pgd_build_from_csr(pgd_graph *g, const int64_t *h_off, const int32_t *h_adj, int64_t n);
 // ingest.cu: a graph file parsed on the device with the reference reader's rules
 pgd_status pgd_build_from_file(pgd_graph *g, const char *path, bool *mtx);

@@ -37,6 +37,50 @@ __device__ __forceinline__ int pgd_warp_incl_scan(int x) {
     return x;
 }
 
+// Last row r in [lo, hi) with off[r] <= p, by the whole warp (the same for all lanes).
+__device__ __forceinline__ int64_t pgd_warp_row(const int64_t *off, int64_t lo, int64_t hi, int64_t p, int lane) {
+    while (hi - lo > 1) {
+        const int64_t step = (hi - lo + 31) / 32;
+        const int64_t at = min(lo + (lane + 1) * step, hi);
+        const int k = __popc(__ballot_sync(0xffffffffu, at < hi && __ldg(off + at) <= p));
+        const int64_t nlo = lo + k * step;
+        hi = min(nlo + step, hi);
+        lo = nlo;
+    }
+    return lo;
+}
+
+// Row of slot p, one of a warp's consecutive slots p0..p1: the rows of p0 and p1
+// are found by searches of the whole warp, p's by a short one between them.  All
+// lanes call.
+__device__ __forceinline__ int64_t pgd_slot_row(const int64_t *off, int64_t n, int64_t p0, int64_t p1, int64_t p,
+                                                int lane) {
+    int64_t lo = pgd_warp_row(off, 0, n, p0, lane), hi = lo + 1;
+    if (off[hi] <= p1) hi = pgd_warp_row(off, lo, n, p1, lane) + 1;
+    while (hi - lo > 1) {
+        const int64_t mid = (lo + hi) >> 1;
+        if (off[mid] <= p) lo = mid;
+        else hi = mid;
+    }
+    return lo;
+}
+
+// First entry of each row above the diagonal, and how many there are (0 for row N).
+static __global__ void pgd_upper_rows(const int64_t *off, const int32_t *adj, int64_t N, uint32_t *first,
+                                      uint32_t *count) {
+    for (int64_t v = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; v <= N; v += (int64_t)gridDim.x * blockDim.x) {
+        uint32_t c = 0;
+        if (v < N) {
+            const int64_t o = off[v];
+            const int d = (int)(off[v + 1] - o);
+            const int at = pgd_lower_bound(adj + o, d, (int32_t)v);
+            first[v] = (uint32_t)(o + at);
+            c = (uint32_t)(d - at);
+        }
+        count[v] = c;
+    }
+}
+
 // (unsigned long long)(x / 2.0) as the reference computes it: conversion to
 // double (round to nearest), scale, truncate.  Below 2^53 the conversion and
 // the halving are exact, so the result is x >> 1; only larger x take the

@@ -82,10 +82,9 @@ constexpr uint32_t kDirectWords = 50 * 1024;   // counter words of one item: 200
 
 // Sizes found on the device while the graph is built.
 struct RankMeta {
-    uint32_t tier[5];        // ranks below tier[i] have degree >= 65536, 256, 16, 4, 2
+    uint32_t tier[6];        // ranks below tier[i] have degree >= 65536, 256, 16, 4, 2, 1
     uint32_t tcode[5];       // bit address at which tier i + 1 ends (counter widths 32, 16, 8, 4, 2)
     uint32_t max_up;
-    uint32_t entries2;       // entries of the rows of vertices of degree >= 2
     uint32_t nlist[kClasses];
     unsigned long long direct_wedges;   // wedges of the vertices beyond the lists
     unsigned long long pairs;           // sum of |N+(a)| (|N+(a)| - 1) / 2
@@ -155,16 +154,27 @@ __device__ __forceinline__ int rows_of_warp(const uint32_t *roff, int64_t n, uin
 // ---------------------------------------------------------------------------
 // building
 
+// Sort keys of the ranks; also clears the sizes.
 __global__ void k_rank_keys2(const int32_t *deg, const int32_t *vgraph, const uint8_t *vmask, int64_t n,
-                             int32_t max_degree, int vb, uint64_t *keys) {
+                             int32_t max_degree, int vb, uint64_t *keys, RankMeta *M) {
+    if (blockIdx.x == 0 && threadIdx.x < 6) M->tier[threadIdx.x] = 0;
+    if (blockIdx.x == 0 && threadIdx.x < kClasses) M->nlist[threadIdx.x] = 0;
+    if (blockIdx.x == 0 && threadIdx.x == 0) {
+        M->max_up = 0;
+        M->direct_wedges = 0;
+        M->pairs = 0;
+    }
     for (int64_t v = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; v < n; v += (int64_t)gridDim.x * blockDim.x) {
         const int32_t d = vmask && vmask[vgraph[v]] ? 0 : deg[v];
         keys[v] = ((uint64_t)(uint32_t)(max_degree - d) << vb) | (uint64_t)(n - 1 - v);
     }
 }
 
+// Ranks from the sorted keys, the degree tiers (where the degree falls below a
+// tier's), and zeroes for what k_rank_slots and k_rank_wedges fill.
 __global__ void k_rank_scatter2(const uint64_t *sorted, int64_t n, int32_t max_degree, int vb, int32_t *vrank,
-                                int32_t *rv, uint32_t *rdeg) {
+                                int32_t *rv, uint32_t *rdeg, int32_t *rup, uint32_t *bend, uint32_t *wd, RankMeta *M) {
+    constexpr uint32_t lim[6] = {65536, 256, 16, 4, 2, 1};
     for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i <= n; i += (int64_t)gridDim.x * blockDim.x) {
         if (i == n) {
             rdeg[n] = 0;
@@ -172,9 +182,17 @@ __global__ void k_rank_scatter2(const uint64_t *sorted, int64_t n, int32_t max_d
         }
         const uint64_t k = sorted[i];
         const int32_t v = (int32_t)(n - 1 - (int64_t)(k & ((1ull << vb) - 1)));
+        const uint32_t d = (uint32_t)(max_degree - (int32_t)(k >> vb));
+        const uint32_t dn = i + 1 < n ? (uint32_t)(max_degree - (int32_t)(sorted[i + 1] >> vb)) : 0;
         vrank[v] = (int32_t)i;
         rv[i] = v;
-        rdeg[i] = (uint32_t)(max_degree - (int32_t)(k >> vb));
+        rdeg[i] = d;
+        rup[i] = 0;
+        bend[i] = 0;
+        wd[i] = 0;
+#pragma unroll
+        for (int t = 0; t < 6; t++)
+            if (d >= lim[t] && dn < lim[t]) M->tier[t] = (uint32_t)i + 1;
     }
 }
 
@@ -195,29 +213,6 @@ __global__ void k_rank_entries(const uint32_t *roff, const int32_t *rv, const in
     }
 }
 
-// Degree tiers and their counter addresses (one thread).
-__global__ void k_rank_tiers(const uint32_t *rdeg, const uint32_t *roff, int64_t n, RankMeta *M) {
-    const uint32_t lim[5] = {65536, 256, 16, 4, 2};
-    uint32_t c = 0, prev = 0;
-    for (int i = 0; i < 5; i++) {
-        int64_t lo = prev, hi = n;   // first rank of degree below lim[i]
-        while (lo < hi) {
-            const int64_t mid = (lo + hi) >> 1;
-            if (rdeg[mid] >= lim[i]) lo = mid + 1;
-            else hi = mid;
-        }
-        M->tier[i] = (uint32_t)lo;
-        c += ((uint32_t)lo - prev) << (5 - i);
-        M->tcode[i] = c;
-        prev = (uint32_t)lo;
-    }
-    M->max_up = 0;
-    M->entries2 = roff[prev];
-    M->direct_wedges = 0;
-    M->pairs = 0;
-    for (int i = 0; i < kClasses; i++) M->nlist[i] = 0;
-}
-
 // Range boundaries: `ranges` parts of about equal weight, a rank's weight being
 // half its share of the entries and half its share of the counter bits (so a
 // range holds at most 2 / ranges of the bits).
@@ -236,23 +231,42 @@ __global__ void k_rank_bounds(const uint32_t *roff, int ranges, RankMeta *M) {
     }
 }
 
-// Per slot: the entry's counter address; the row's count of entries above it;
-// and, from the side of the lower end, the slots of the two directions.
+// Per slot: the entry's counter address; the row's count of entries above it and
+// its first entry of degree 1 (those come last); and, from the side of the lower
+// end, the slots of the two directions.
 __global__ void k_rank_slots(const uint32_t *roff, const int32_t *radj, int64_t n, int64_t nnz, RankMeta *M,
-                             uint32_t *wcode, int32_t *tw, int32_t *rup) {
+                             uint32_t *wcode, int32_t *tw, int32_t *rup, uint32_t *bend) {
     const int lane = threadIdx.x & 31;
     const int64_t stride = (int64_t)gridDim.x * blockDim.x;
+    // where each tier's counters end, from the tiers (then kept for the others)
+    uint32_t lo[6], end[6];
+    lo[0] = end[0] = 0;
+#pragma unroll
+    for (int i = 0; i < 5; i++) {
+        lo[i + 1] = M->tier[i];
+        end[i + 1] = end[i] + ((lo[i + 1] - lo[i]) << (5 - i));
+    }
+    if (blockIdx.x == 0 && threadIdx.x == 0)
+#pragma unroll
+        for (int i = 0; i < 5; i++) M->tcode[i] = end[i + 1];
+    const int32_t n2 = (int32_t)lo[5];
     for (int64_t p0 = blockIdx.x * (int64_t)blockDim.x + threadIdx.x - lane; p0 < nnz; p0 += stride) {
         const int64_t p = min(p0 + lane, nnz - 1);
         const int r = rows_of_warp(roff, n, (uint32_t)p0, (uint32_t)p, lane);
         if (p0 + lane >= nnz) continue;
         const int32_t x = radj[p];
-        wcode[p] = code_of(M, (uint32_t)x);
+        uint32_t c = end[5];
+#pragma unroll
+        for (int i = 4; i >= 0; i--)
+            if ((uint32_t)x < lo[i + 1]) c = end[i] + (((uint32_t)x - lo[i]) << (5 - i));
+        wcode[p] = c;
+        const bool first = p == (int64_t)roff[r], last = p + 1 == (int64_t)roff[r + 1];
+        if (x >= n2 ? first || radj[p - 1] < n2 : last) bend[r] = (uint32_t)(x >= n2 ? p : p + 1);
         if (x < r) {
             const uint32_t s = lower_bound_u(radj, roff[x], roff[x + 1], r);
             tw[p] = (int32_t)s;
             tw[s] = (int32_t)p;
-            if (p + 1 == (int64_t)roff[r + 1] || radj[p + 1] > r) {
+            if (last || radj[p + 1] > r) {
                 const uint32_t up = (uint32_t)p + 1 - roff[r];
                 rup[r] = (int32_t)up;
                 if (up > 32) atomicMax(&M->max_up, up);
@@ -276,12 +290,6 @@ __global__ void k_rank_eslot(const int32_t *ev, const int32_t *eu, const int32_t
     }
 }
 
-// First entry of degree 1 of each row (the vertices of degree 1 come last).
-__global__ void k_rank_bend(const uint32_t *roff, const int32_t *radj, int n2, uint32_t *bend) {
-    for (int64_t v = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; v < n2; v += (int64_t)gridDim.x * blockDim.x)
-        bend[v] = lower_bound_u(radj, roff[v], roff[v + 1], n2);
-}
-
 // First entry of each row at or beyond each inner range boundary.
 __global__ void k_rank_bpos(const uint32_t *roff, const int32_t *radj, int n2, int ranges, const RankMeta *M,
                             uint32_t *bpos) {
@@ -295,8 +303,10 @@ __global__ void k_rank_bpos(const uint32_t *roff, const int32_t *radj, int n2, i
 // Wedges of every top vertex u (its lower neighbours' entries below u), with
 // one atomic per warp where its slots belong to one row.
 __global__ void k_rank_wedges(const uint32_t *roff, const int32_t *radj, const int32_t *tw, const uint32_t *bend,
-                              int64_t n, int n2, int64_t nnz2, uint32_t *wd) {
+                              int64_t n, const RankMeta *M, uint32_t *wd) {
     const int lane = threadIdx.x & 31;
+    const int32_t n2 = (int32_t)M->tier[4];
+    const int64_t nnz2 = roff[n2];
     const int64_t stride = (int64_t)gridDim.x * blockDim.x;
     for (int64_t p0 = blockIdx.x * (int64_t)blockDim.x + threadIdx.x - lane; p0 < nnz2; p0 += stride) {
         const int64_t p = min(p0 + lane, nnz2 - 1);
@@ -325,9 +335,10 @@ __device__ __forceinline__ void list_append(bool in, int32_t v, int32_t *list, u
 
 // Every vertex into the lists of its classes, and a place for its triangles:
 // hbase[a], with room for every pair of N+(a).
-__global__ void k_rank_lists(const int32_t *rup, const uint32_t *wd, int n2, int32_t *lists, unsigned long long *hbase,
-                             RankMeta *M) {
+__global__ void k_rank_lists(const int32_t *rup, const uint32_t *wd, int64_t n, int32_t *lists,
+                             unsigned long long *hbase, RankMeta *M) {
     const int lane = threadIdx.x & 31;
+    const int32_t n2 = (int32_t)M->tier[4];
     const int64_t stride = (int64_t)gridDim.x * blockDim.x;
     unsigned long long direct = 0;
     for (int64_t x0 = blockIdx.x * (int64_t)blockDim.x + threadIdx.x - lane; x0 < n2; x0 += stride) {
@@ -336,9 +347,9 @@ __global__ void k_rank_lists(const int32_t *rup, const uint32_t *wd, int n2, int
         const uint32_t w = x < n2 ? wd[x] : 0;
         const int ec = up < 2 ? -1 : up <= kEgoMax[0] ? 0 : up <= kEgoMax[1] ? 1 : up <= kEgoMax[2] ? 2 : up <= kEgoMax[3] ? 3 : 4;
 #pragma unroll
-        for (int c = 0; c < kCycWarp; c++) list_append(ec == c, (int32_t)x, lists + (int64_t)c * n2, &M->nlist[c], lane);
-        list_append(w >= 2 && w <= kCycWarpMax, (int32_t)x, lists + (int64_t)kCycWarp * n2, &M->nlist[kCycWarp], lane);
-        list_append(w > kCycWarpMax && w <= kCycHashMax, (int32_t)x, lists + (int64_t)kCycHash * n2, &M->nlist[kCycHash],
+        for (int c = 0; c < kCycWarp; c++) list_append(ec == c, (int32_t)x, lists + (int64_t)c * n, &M->nlist[c], lane);
+        list_append(w >= 2 && w <= kCycWarpMax, (int32_t)x, lists + (int64_t)kCycWarp * n, &M->nlist[kCycWarp], lane);
+        list_append(w > kCycWarpMax && w <= kCycHashMax, (int32_t)x, lists + (int64_t)kCycHash * n, &M->nlist[kCycHash],
                     lane);
         if (w > kCycHashMax) direct += w;
         const unsigned long long pairs = (unsigned long long)up * (unsigned)(up - (up > 0)) / 2;
@@ -1458,71 +1469,74 @@ pgd_status pgd_rank_build(pgd_graph *g, int64_t nnz, const int32_t *vgraph, cons
         }
         return e;
     };
-    RB_TRY(keep(&R->roff, (n + 1) * sizeof(uint32_t)));
-    RB_TRY(keep(&R->rup, n * sizeof(int32_t)));
-    RB_TRY(keep(&R->radj, nnz * sizeof(int32_t)));
-    RB_TRY(keep(&R->wcode, nnz * sizeof(uint32_t)));
-    RB_TRY(keep(&R->tw, nnz * sizeof(int32_t)));
-    RB_TRY(keep(&R->eslot, m * sizeof(int32_t)));
-    RB_TRY(keep(&R->meta, sizeof(RankMeta)));
-    RankMeta *M = (RankMeta *)R->meta;
+    // kept arrays in one allocation
+    pgd_pieces K;
+    const size_t nb = (n + 1) * sizeof(uint32_t), eb = nnz * sizeof(uint32_t), mb = m * sizeof(int32_t),
+                 lb = (size_t)kClasses * n * sizeof(int32_t), hb = n * sizeof(unsigned long long);
+    K.add(sizeof(RankMeta)); K.add(nb); K.add(nb); K.add(nb); K.add(eb); K.add(eb); K.add(eb); K.add(mb); K.add(lb); K.add(hb);
+    RB_TRY(keep(&K.base, K.bytes));
+    RankMeta *M = K.take<RankMeta>(sizeof(RankMeta));
+    R->meta = M;
+    R->roff = K.take<uint32_t>(nb);
+    R->rup = K.take<int32_t>(nb);
+    R->bend = K.take<uint32_t>(nb);
+    R->radj = K.take<int32_t>(eb);
+    R->wcode = K.take<uint32_t>(eb);
+    R->tw = K.take<int32_t>(eb);
+    R->eslot = K.take<int32_t>(mb);
+    R->lists = K.take<int32_t>(lb);
+    R->hbase = K.take<unsigned long long>(hb);
+    // and the temporaries in another
     Tmp tg(ctx);
     uint64_t *keys = nullptr, *keys2 = nullptr;
     int32_t *vrank = nullptr, *rv = nullptr, *val = nullptr;
-    uint32_t *rdeg = nullptr, *key = nullptr, *key2 = nullptr;
-    RB_TRY(tg.alloc(&keys, n * sizeof(uint64_t)));
-    RB_TRY(tg.alloc(&keys2, n * sizeof(uint64_t)));
-    RB_TRY(tg.alloc(&vrank, n * sizeof(int32_t)));
-    RB_TRY(tg.alloc(&rv, n * sizeof(int32_t)));
-    RB_TRY(tg.alloc(&rdeg, (n + 1) * sizeof(uint32_t)));
-    RB_TRY(tg.alloc(&key, nnz * sizeof(uint32_t)));
-    RB_TRY(tg.alloc(&key2, nnz * sizeof(uint32_t)));
-    RB_TRY(tg.alloc(&val, nnz * sizeof(int32_t)));
+    uint32_t *rdeg = nullptr, *key = nullptr, *key2 = nullptr, *wd = nullptr;
     const int vb = bits_for(n), db = bits_for((int64_t)g->max_degree + 1);
     size_t tb1 = 0, tb2 = 0, tb3 = 0;
     cub::DeviceRadixSort::SortKeys(nullptr, tb1, keys, keys2, n, 0, vb + db, s);
     cub::DeviceScan::ExclusiveSum(nullptr, tb2, rdeg, R->roff, n + 1, s);
     cub::DeviceRadixSort::SortPairs(nullptr, tb3, key, key2, val, R->radj, nnz, 0, vb, s);
     size_t tb = std::max(tb1, std::max(tb2, tb3));
-    void *tmp = nullptr;
-    RB_TRY(tg.alloc(&tmp, tb));
-    // ranks, row offsets and tiers
-    PGD_LAUNCH(ctx, k_rank_keys2, grid_for(n), kThreads, 0, g->deg, vgraph, vmask, n, g->max_degree, vb, keys);
+    pgd_pieces W;
+    W.add(2 * nb); W.add(2 * nb); W.add(nb); W.add(nb); W.add(nb); W.add(nb); W.add(eb); W.add(eb); W.add(eb); W.add(tb);
+    RB_TRY(tg.alloc(&W.base, W.bytes));
+    keys = W.take<uint64_t>(2 * nb);
+    keys2 = W.take<uint64_t>(2 * nb);
+    vrank = W.take<int32_t>(nb);
+    rv = W.take<int32_t>(nb);
+    rdeg = W.take<uint32_t>(nb);
+    wd = W.take<uint32_t>(nb);
+    key = W.take<uint32_t>(eb);
+    key2 = W.take<uint32_t>(eb);
+    val = W.take<int32_t>(eb);
+    void *tmp = W.take<void>(tb);
+    // ranks and row offsets
+    PGD_LAUNCH(ctx, k_rank_keys2, grid_for(n), kThreads, 0, g->deg, vgraph, vmask, n, g->max_degree, vb, keys, M);
     RB_CUDA(cub::DeviceRadixSort::SortKeys(tmp, tb, keys, keys2, n, 0, vb + db, s));
-    PGD_LAUNCH(ctx, k_rank_scatter2, grid_for(n + 1), kThreads, 0, keys2, n, g->max_degree, vb, vrank, rv, rdeg);
+    PGD_LAUNCH(ctx, k_rank_scatter2, grid_for(n + 1), kThreads, 0, keys2, n, g->max_degree, vb, vrank, rv, rdeg, R->rup,
+               R->bend, wd, M);
     RB_CUDA(cub::DeviceScan::ExclusiveSum(tmp, tb, rdeg, R->roff, n + 1, s));
-    PGD_LAUNCH(ctx, k_rank_tiers, 1, 1, 0, rdeg, R->roff, n, M);
     // rows in rank order
     PGD_LAUNCH(ctx, k_rank_entries, grid_for(nnz), kThreads, 0, R->roff, rv, g->off, g->adj, vrank, n, nnz, key, val);
     RB_CUDA(cub::DeviceRadixSort::SortPairs(tmp, tb, key, key2, val, R->radj, nnz, 0, vb, s));
-    RB_CUDA(cudaMemsetAsync(R->rup, 0, n * sizeof(int32_t), s));
-    PGD_LAUNCH(ctx, k_rank_slots, grid_for(nnz), kThreads, 0, R->roff, R->radj, n, nnz, M, R->wcode, R->tw, R->rup);
+    PGD_LAUNCH(ctx, k_rank_slots, grid_for(nnz), kThreads, 0, R->roff, R->radj, n, nnz, M, R->wcode, R->tw, R->rup,
+               R->bend);
     PGD_LAUNCH(ctx, k_rank_eslot, grid_for(m), kThreads, 0, g->ev, g->eu, vrank, R->roff, R->rup, R->radj, vgraph,
                vmask, m, R->eslot);
-    RankMeta h;
-    constexpr size_t kHead = offsetof(RankMeta, bound);
-    RB_CUDA(cudaMemcpyAsync(&h, M, kHead, cudaMemcpyDeviceToHost, s));
-    RB_CUDA(cudaStreamSynchronize(s));
-    R->n2 = (int32_t)h.tier[4];
-    R->max_up = (int32_t)std::max((uint32_t)kEgoMax[kEgoWarp], h.max_up);
-    if (R->n2 == 0) return PGD_OK;
     // wedges per vertex and the work lists
-    const int n2 = R->n2;
-    uint32_t *wd = nullptr;
-    RB_TRY(tg.alloc(&wd, n2 * sizeof(uint32_t)));
-    RB_TRY(keep(&R->bend, n2 * sizeof(uint32_t)));
-    RB_TRY(keep(&R->lists, (size_t)kClasses * n2 * sizeof(int32_t)));
-    RB_TRY(keep(&R->hbase, n2 * sizeof(unsigned long long)));
-    RB_CUDA(cudaMemsetAsync(wd, 0, n2 * sizeof(uint32_t), s));
-    PGD_LAUNCH(ctx, k_rank_bend, grid_for(n2), kThreads, 0, R->roff, R->radj, n2, R->bend);
-    PGD_LAUNCH(ctx, k_rank_wedges, grid_for(h.entries2), kThreads, 0, R->roff, R->radj, R->tw, R->bend, n, n2,
-               (int64_t)h.entries2, wd);
-    PGD_LAUNCH(ctx, k_rank_lists, grid_for(n2), kThreads, 0, R->rup, wd, n2, R->lists, R->hbase, M);
-    RB_CUDA(cudaMemcpyAsync(&h, M, kHead, cudaMemcpyDeviceToHost, s));
+    PGD_LAUNCH(ctx, k_rank_wedges, grid_for(nnz), kThreads, 0, R->roff, R->radj, R->tw, R->bend, n, M, wd);
+    PGD_LAUNCH(ctx, k_rank_lists, grid_for(n), kThreads, 0, R->rup, wd, n, R->lists, R->hbase, M);
+    constexpr size_t kHead = offsetof(RankMeta, bound);
+    static_assert(kHead <= kPinBytes, "the sizes fit the read-back buffer");
+    RB_CUDA(pgd_fetch(ctx, 0, M, kHead));
     RB_CUDA(cudaStreamSynchronize(s));
+    RankMeta h;
+    memcpy((void *)&h, ctx->pin, kHead);
+    const int n2 = R->n2 = (int32_t)h.tier[4];
+    R->max_up = (int32_t)std::max((uint32_t)kEgoMax[kEgoWarp], h.max_up);
     for (int i = 0; i < kClasses; i++) R->nlist[i] = h.nlist[i];
     R->pairs = (int64_t)h.pairs;
-    if (h.direct_wedges == 0) return PGD_OK;
+    if (n2 == 0 || h.direct_wedges == 0) return PGD_OK;
     // items of the vertices with many wedges, by ranges of the wedges' ends:
     // fine enough to balance the items, and at most half an item's counters each
     const int64_t words = R->words = ((int64_t)h.tcode[4] + 31) / 32;
@@ -1535,14 +1549,15 @@ pgd_status pgd_rank_build(pgd_graph *g, int64_t nnz, const int32_t *vgraph, cons
                    R->nranges, M, R->bpos);
     }
     uint32_t *count = nullptr, *pos = nullptr;
-    RB_TRY(tg.alloc(&count, ((size_t)n2 + 1) * sizeof(uint32_t)));
-    RB_TRY(tg.alloc(&pos, ((size_t)n2 + 1) * sizeof(uint32_t)));
+    RB_TRY(tg.alloc(&count, 2 * ((size_t)n2 + 1) * sizeof(uint32_t)));
+    pos = count + n2 + 1;
     const int parts = ctx->num_sms * 4 * (1 + direct_factor(words));
     PGD_LAUNCH(ctx, k_rank_items, grid_for(n2 + 1), kThreads, 0, wd, n2, R->nranges, M, parts, count,
                (const uint32_t *)nullptr, (int2 *)nullptr);
     RB_CUDA(cub::DeviceScan::ExclusiveSum(tmp, tb, count, pos, (int64_t)n2 + 1, s));
-    RB_CUDA(cudaMemcpyAsync(&R->nitems, pos + n2, sizeof(uint32_t), cudaMemcpyDeviceToHost, s));
+    RB_CUDA(pgd_fetch(ctx, 0, pos + n2, sizeof(uint32_t)));
     RB_CUDA(cudaStreamSynchronize(s));
+    R->nitems = pgd_pinned<uint32_t>(ctx, 0);
     RB_TRY(keep(&R->items, (size_t)R->nitems * sizeof(int2)));
     PGD_LAUNCH(ctx, k_rank_items, grid_for(n2 + 1), kThreads, 0, wd, n2, R->nranges, M, parts, (uint32_t *)nullptr,
                (const uint32_t *)pos, R->items);
@@ -1577,7 +1592,7 @@ static void ego_pass(pgd_ctx *ctx, const pgd_rank_graph &R, EgoArgs A, int pass,
     const bool kept = pass == 2 && A.hcount;
     auto args = [&](int c) {
         EgoArgs B = A;
-        B.list = R.lists + (int64_t)c * R.n2;
+        B.list = R.lists + (int64_t)c * R.n;
         B.count = R.nlist[c];
         B.next = ctr + c;
         B.grab = grab_for(ctx, B.count);
@@ -1617,9 +1632,7 @@ static void ego_pass(pgd_ctx *ctx, const pgd_rank_graph &R, EgoArgs A, int pass,
     }
 }
 
-// Shared-memory limits of the kernels that use more than the default, set to
-// the same values by every caller.
-static cudaError_t rank_kernel_limits() {
+cudaError_t pgd_rank_limits() {
     constexpr cudaFuncAttribute kDyn = cudaFuncAttributeMaxDynamicSharedMemorySize;
     cudaError_t e = cudaFuncSetAttribute(k_cycle_direct<1024>, kDyn, kDirectWords * 4);
     if (e == cudaSuccess) e = cudaFuncSetAttribute(k_cycle_direct<512>, kDyn, kDirectWords * 2);
@@ -1679,14 +1692,14 @@ static pgd_status cycle_pass(pgd_ctx *ctx, const pgd_rank_graph &R, CycArgs C, u
     }
     if (R.nlist[kCycHash]) {
         CycArgs B = C;
-        B.list = R.lists + (int64_t)kCycHash * R.n2;
+        B.list = R.lists + (int64_t)kCycHash * R.n;
         B.count = R.nlist[kCycHash];
         B.next = ctr + 1;
         PGD_LAUNCH(ctx, k_cycle_hash, (int)std::min<int64_t>(B.count, 4 * (int64_t)nsm), kHashThreads, kHashSmem, B);
     }
     if (R.nlist[kCycWarp]) {
         CycArgs B = C;
-        B.list = R.lists + (int64_t)kCycWarp * R.n2;
+        B.list = R.lists + (int64_t)kCycWarp * R.n;
         B.count = R.nlist[kCycWarp];
         B.grab = grab_for(ctx, B.count);
         B.next = ctr + 2;
@@ -1702,7 +1715,6 @@ pgd_status pgd_rank_decompose(pgd_ctx *ctx, const pgd_rank_graph &R, const pgd_r
     pgd_status st;
     if (out.npos == 0 || R.nnz == 0) return PGD_OK;
     const int nsm = ctx->num_sms;
-    PGD_CUDA(ctx, rank_kernel_limits());
     // triangle lists (pass 2) and the tables of the largest neighbourhoods
     int64_t hit_count = 0, table_bytes = 0;
     int gblocks = 0;

@@ -17,10 +17,10 @@ struct pgd_rank_graph {
     uint32_t *wcode = nullptr;   // nnz: bit address of the entry's counter
     int32_t *tw = nullptr;       // nnz: slot of the reversed edge
     int32_t *eslot = nullptr;    // per edge id: slot of the edge in the row of its lower-ranked end (or -1)
-    uint32_t *bend = nullptr;    // n2: first entry of the row whose vertex has degree 1
+    uint32_t *bend = nullptr;    // n: first entry of the row whose vertex has degree 1
     uint32_t *bpos = nullptr;    // (nranges - 1) x n2: first entry of the row at or beyond an inner range
                                  // boundary (null: searched when needed)
-    int32_t *lists = nullptr;    // work lists by class, n2 entries each
+    int32_t *lists = nullptr;    // work lists by class, n entries each
     unsigned long long *hbase = nullptr;   // n2: place of the vertex's triangles among all pairs of all N+
     int64_t pairs = 0;           // those pairs
     int2 *items = nullptr;       // {u, first range | one past the last range << 16}
