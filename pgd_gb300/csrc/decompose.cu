@@ -1160,16 +1160,16 @@ __device__ __forceinline__ int32_t dense_q(const DevGraph &G, int64_t e) {
     return G.deg[v] <= G.deg[u] ? v : u;
 }
 
-// Sort keys grouping the dense-graph edges by q (then by position), so that one
-// pass over the rows of q's neighbours serves several: (q << eb) | position, q
-// below 2^qb and positions below 2^eb.  A graph's edges are consecutive
-// positions; before[g] of the edges before them belong to sparse graphs.
-__global__ void k_dense_keys(DevGraph G, const int64_t *before, uint64_t *keys, int32_t *vals, int eb) {
+// The dense-graph edges by position, each with its q: stably sorted by q, one pass
+// over the rows of q's neighbours serves several.  A graph's edges are
+// consecutive positions; before[g] of the edges before them belong to sparse
+// graphs.
+__global__ void k_dense_keys(DevGraph G, const int64_t *before, uint32_t *keys, int32_t *vals) {
     for (int64_t e = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; e < G.npos; e += (int64_t)gridDim.x * blockDim.x) {
         const int g = G.egraph[e];
         if (!G.gdense[g]) continue;
         const int64_t i = e - before[g];
-        keys[i] = ((uint64_t)(uint32_t)dense_q(G, e) << eb) | (uint64_t)e;
+        keys[i] = (uint32_t)dense_q(G, e);
         vals[i] = (int32_t)e;
     }
 }
@@ -1191,8 +1191,11 @@ constexpr int kDenseGroup = 6;   // edges sharing q decomposed together
 constexpr int kCnRows = 32;   // rows a of CN computed by one block
 
 // One block per tile of 32 rows a of one graph: the tile's bit rows in shared
-// memory, one column b per thread, 32 counters in registers.  ctile[g] is
-// the first tile of graph g (k + 1 entries, non-decreasing).
+// memory, one column b per thread, 32 counters in registers.  CN is symmetric:
+// only the columns from the tile's first row on are counted, and those beyond
+// the tile are also written as 64 bytes of row b (half the popcounts: 2.0 -> 1.1
+// ms on 128 graphs of up to 2048 vertices).  ctile[g] is the first tile of graph
+// g (k + 1 entries, non-decreasing).
 __global__ void __launch_bounds__(256) k_dense_common(const uint64_t *bits, const int64_t *wbase,
                                                       const long long *gnm, const int64_t *cbase,
                                                       const int64_t *ctile, int k, int64_t ntiles, uint16_t *cn) {
@@ -1211,7 +1214,7 @@ __global__ void __launch_bounds__(256) k_dense_common(const uint64_t *bits, cons
         }
         __syncthreads();
         uint16_t *out = cn + cbase[g];
-        for (int64_t b = threadIdx.x; b < stride; b += blockDim.x) {
+        for (int64_t b = a0 + threadIdx.x; b < stride; b += blockDim.x) {
             uint32_t acc[kCnRows];
 #pragma unroll
             for (int i = 0; i < kCnRows; i++) acc[i] = 0;
@@ -1226,6 +1229,29 @@ __global__ void __launch_bounds__(256) k_dense_common(const uint64_t *bits, cons
 #pragma unroll
             for (int i = 0; i < kCnRows; i++)
                 if (a0 + i < n) out[(a0 + i) * stride + b] = (uint16_t)acc[i];
+            if (b >= a0 + kCnRows && b < n) {
+                // columns a0 .. a0 + 31 of row b (0 beyond n: no bits there)
+                uint4 *q = (uint4 *)(out + b * stride + a0);
+#pragma unroll
+                for (int i = 0; i < kCnRows; i += 8)
+                    q[i / 8] = make_uint4(acc[i] | acc[i + 1] << 16, acc[i + 2] | acc[i + 3] << 16,
+                                          acc[i + 4] | acc[i + 5] << 16, acc[i + 6] | acc[i + 7] << 16);
+            }
+        }
+    }
+}
+
+// Per word of a bit row, the bits in the words before it.
+__global__ void k_dense_prefix(const uint64_t *bits, const int64_t *wbase, const int64_t *vbase, const int32_t *vgraph,
+                               const uint8_t *gdense, const long long *gnm, int64_t N, uint16_t *pre) {
+    for (int64_t x = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; x < N; x += (int64_t)gridDim.x * blockDim.x) {
+        const int g = vgraph[x];
+        if (!gdense[g]) continue;
+        const int64_t W = (gnm[2 * g] + 63) >> 6, at = wbase[g] + (x - vbase[g]) * W;
+        int c = 0;
+        for (int64_t w = 0; w < W; w++) {
+            pre[at + w] = (uint16_t)c;
+            c += __popcll(bits[at + w]);
         }
     }
 }
@@ -1372,12 +1398,13 @@ __global__ void __launch_bounds__(256, 3) k_dense_cn(DenseCnArgs A) {
 // ---------------------------------------------------------------------------
 // k4 of dense graphs on the tensor cores.  For an edge (p, q) with
 // T = N(p) ∩ N(q),
-//   2·k4(p, q) = sum_{y in T} |N(y) ∩ T| = sum_{y in N(q)} A_py · D[p][y],
-//   D[p][y]    = sum_{x in N(q)} A_px · A_yx = |N(p) ∩ N(y) ∩ N(q)|,
+//   k4(p, q) = sum_{y in T} |{x in N(y) ∩ T, x < y}| = sum_{y in N(q)} A_py · D[p][y],
+//   D[p][y]  = sum_{x in N(q), x < y} A_px · A_yx,
 // so for all edges (p_i, q) of one run (same q) D is a product of rows of the
 // ego network of q, compacted to the columns N(q): the rows p_i (M side, one
-// TMEM lane each) times every row y of N(q) (N side, one TMEM column each),
-// over K = N(q).  0/1 entries are exact in e4m3 and every fp32 sum stays below
+// TMEM lane each) times every row y of N(q) below its diagonal (N side, one TMEM
+// column each), over K = N(q).  The columns past a row tile's last row are zero
+// and skipped (with full rows 2·k4 came out, for twice the products).  0/1 entries are exact in e4m3 and every fp32 sum stays below
 // 2^24 (d_q <= kTcMaxDeg), so the counts are exact.
 //
 // One CTA of 16 warps per SM takes runs from a counter.  Per run: the rows of
@@ -1422,13 +1449,12 @@ struct DenseTcArgs {
     unsigned long long *err;            // waits that ran out
 };
 
-// run starts of the CN-graph edges (sorted dense keys: q above the eb
-// position bits) whose q has degree in [min_deg, kTcMaxDeg]
-__global__ void k_tc_run_flags(const uint64_t *keys, int64_t ncn, const int32_t *deg, int min_deg, uint32_t *flag,
-                               int eb) {
+// run starts of the CN-graph edges (sorted by q) whose q has degree in [min_deg,
+// kTcMaxDeg]
+__global__ void k_tc_run_flags(const uint32_t *keys, int64_t ncn, const int32_t *deg, int min_deg, uint32_t *flag) {
     for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < ncn; i += (int64_t)gridDim.x * blockDim.x) {
-        const uint32_t q = (uint32_t)(keys[i] >> eb);
-        const bool start = i == 0 || (uint32_t)(keys[i - 1] >> eb) != q;
+        const uint32_t q = keys[i];
+        const bool start = i == 0 || keys[i - 1] != q;
         const int d = deg[q];
         flag[i] = (start && d >= min_deg && d <= kTcMaxDeg) ? 1u : 0u;
     }
@@ -1436,10 +1462,9 @@ __global__ void k_tc_run_flags(const uint64_t *keys, int64_t ncn, const int32_t 
 
 // positions of the CN-graph edges whose q's degree is outside [min_deg,
 // kTcMaxDeg]: the ones k_dense_cn decomposes, kept in their order
-__global__ void k_tc_rest_flags(const uint64_t *keys, int64_t ncn, const int32_t *deg, int min_deg, uint32_t *flag,
-                                int eb) {
+__global__ void k_tc_rest_flags(const uint32_t *keys, int64_t ncn, const int32_t *deg, int min_deg, uint32_t *flag) {
     for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < ncn; i += (int64_t)gridDim.x * blockDim.x) {
-        const int d = deg[(uint32_t)(keys[i] >> eb)];
+        const int d = deg[keys[i]];
         flag[i] = (d < min_deg || d > kTcMaxDeg) ? 1u : 0u;
     }
 }
@@ -1451,15 +1476,15 @@ __global__ void k_tc_rest_fill(const int32_t *dpos, const uint32_t *flag, const 
     if (blockIdx.x == 0 && threadIdx.x == 0) *nrest = pos[ncn];
 }
 
-__global__ void k_tc_run_fill(const uint64_t *keys, const uint32_t *flag, const uint32_t *pos, int64_t ncn,
-                              int64_t *runs, unsigned long long *nruns, int eb) {
+__global__ void k_tc_run_fill(const uint32_t *keys, const uint32_t *flag, const uint32_t *pos, int64_t ncn,
+                              int64_t *runs, unsigned long long *nruns) {
     for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < ncn; i += (int64_t)gridDim.x * blockDim.x) {
         if (!flag[i]) continue;
-        const uint32_t q = (uint32_t)(keys[i] >> eb);
+        const uint32_t q = keys[i];
         int64_t lo = i + 1, hi = ncn;   // one past the run's last position
         while (lo < hi) {
             const int64_t mid = (lo + hi) >> 1;
-            if ((uint32_t)(keys[mid] >> eb) == q) lo = mid + 1; else hi = mid;
+            if (keys[mid] == q) lo = mid + 1; else hi = mid;
         }
         runs[2 * pos[i]] = i;
         runs[2 * pos[i] + 1] = lo;
@@ -1672,6 +1697,7 @@ __global__ void __launch_bounds__(kTcThreads, 1) k_dense_tc(DenseTcArgs A) {
                 // item i of a tile lives at byte 16·i; a stage holds A of tile
                 // 0, A of tile 1, B.
                 const int nA = ntiles * kTcM * 4, nItems = nA + nt * 4;
+                const int KT = min(KW, (n0 + nt + 63) >> 6);   // chunks with columns below some row of the tile
                 constexpr int kPer = (2 * kTcM * 4 + kTcN * 4 + 32 * kTcBuilders - 1) / (32 * kTcBuilders);
                 if (warp < kTcBuilders) {
                     // per item: its 16 bits of chunk 0 as a halfword of C (chunk kc
@@ -1682,6 +1708,7 @@ __global__ void __launch_bounds__(kTcThreads, 1) k_dense_tc(DenseTcArgs A) {
                     // row's bits, which are zero past d_q).
                     const uint16_t *C16 = (const uint16_t *)C;
                     int src[kPer];
+                    int below[kPer];   // B: columns of the row below its diagonal, from this item's first one
                     uint32_t dst[kPer];
 #pragma unroll
                     for (int k = 0; k < kPer; k++) {
@@ -1692,11 +1719,12 @@ __global__ void __launch_bounds__(kTcThreads, 1) k_dense_tc(DenseTcArgs A) {
                         int cr = -1;
                         if (it < nItems) cr = isA ? s_jrow[it >> 9][row] : (n0 + row < d ? n0 + row : -1);
                         src[k] = 4 * cr * KS + ((i2 >> 3) & 3);
+                        below[k] = isA ? 0x7fffffff : n0 + row - 16 * ((i2 >> 3) & 3);
                         dst[k] = cr < 0 ? 0xffffffffu
                                  : isA ? (uint32_t)((it >> 9) * kTcM * kTcK + 16 * i2)
                                        : (uint32_t)(2 * kTcM * kTcK + 16 * i2);
                     }
-                    for (int kc = 0; kc < KW; kc++) {
+                    for (int kc = 0; kc < KT; kc++) {
                         const int c = chunk + kc, st = c & 1, u = c >> 1;
                         // the MMAs that read this stage last (chunk c - 2) are done
                         int ok = 1;
@@ -1707,6 +1735,13 @@ __global__ void __launch_bounds__(kTcThreads, 1) k_dense_tc(DenseTcArgs A) {
                         uint32_t b16[kPer];
 #pragma unroll
                         for (int k = 0; k < kPer; k++) b16[k] = dst[k] != 0xffffffffu ? C16[src[k] + 4 * kc] : 0u;
+                        if (64 * kc + 63 >= n0) {   // the tile's diagonal runs through this chunk
+#pragma unroll
+                            for (int k = 0; k < kPer; k++) {
+                                const int left = min(16, max(0, below[k] - 64 * kc));
+                                b16[k] &= (1u << left) - 1;
+                            }
+                        }
 #pragma unroll
                         for (int k = 0; k < kPer; k++) {
                             if (dst[k] != 0xffffffffu)
@@ -1719,7 +1754,7 @@ __global__ void __launch_bounds__(kTcThreads, 1) k_dense_tc(DenseTcArgs A) {
                         if (lane == 0) mbar_arrive(&s_full[st]);
                     }
                 } else if (issuer) {
-                    for (int kc = 0; kc < KW; kc++) {
+                    for (int kc = 0; kc < KT; kc++) {
                         const int c = chunk + kc, st = c & 1, u = c >> 1;
                         bad |= !mbar_wait_or_abort(&s_full[st], u & 1, kTcWaitCycles, &s_abort);
                         fence_after_sync();
@@ -1736,7 +1771,7 @@ __global__ void __launch_bounds__(kTcThreads, 1) k_dense_tc(DenseTcArgs A) {
                     // the accumulators are complete once the last commit lands
                     bad |= !mbar_wait_or_abort(&s_empty[last & 1], (last >> 1) & 1, kTcWaitCycles, &s_abort);
                 }
-                chunk += KW;
+                chunk += KT;
                 if (__syncthreads_or(bad)) {
                     bad = true;
                     break;
@@ -1770,9 +1805,8 @@ __global__ void __launch_bounds__(kTcThreads, 1) k_dense_tc(DenseTcArgs A) {
             __syncthreads();
             if (tid < ntiles * kTcM && m0 + tid < rr) {
                 const int t = tid >> 7, row = tid & (kTcM - 1);
-                // (sum of D·A_py) · 2^12 = 2·k4
-                const float k2 = (s_part[t][0][row] + s_part[t][1][row]) * 4096.f;
-                A.k4[i0 + m0 + tid] = (uint32_t)k2 >> 1;
+                // (sum of D·A_py) · 2^12 = k4
+                A.k4[i0 + m0 + tid] = (uint32_t)((s_part[t][0][row] + s_part[t][1][row]) * 4096.f);
             }
         }
         if (bad) break;
@@ -1797,15 +1831,17 @@ __global__ void __launch_bounds__(kTcThreads, 1) k_dense_tc(DenseTcArgs A) {
 //   E = A·(CN - TA) - TA·A.
 // One CTA per SM takes (graph, 128-row tile, 256-column tile) items; each
 // item runs the chain over K = n of A × (CN - TA), then of TA × A with the
-// product negated, in tf32 (entries below 2^11 are exact, |sums| < 2^23 stay
-// exact in fp32), 16 columns per stage from four stages.  The tile is read
-// back one row per thread and E[x][y] written for the edges only, at the
-// adjacency slot x -> y.
+// product negated, in f16 (entries below 2^11 are exact, |sums| < 2^23 stay
+// exact in fp32), 32 columns per stage from four stages: twice the columns per
+// barrier and twice the rate of tf32.  E is symmetric: only tiles with columns
+// above the diagonal are taken, read back one row per thread, and E[x][y] of an
+// edge x < y is written at both adjacency slots, y -> x (consecutive for a warp's
+// rows) and x -> y.  6.5 -> 2.4 ms on 128 graphs of up to 2048 vertices.
 
 constexpr int kGramThreads = 512;
 constexpr int kGramM = 128, kGramN = 256;
 constexpr int kGramStages = 4;
-constexpr int kGramStageBytes = (kGramM + kGramN) * 64;   // 16 tf32 columns per row
+constexpr int kGramStageBytes = (kGramM + kGramN) * 64;   // 32 f16 columns per row
 constexpr int kGramSmem = kGramStages * kGramStageBytes + 1024;
 static_assert(kGramStageBytes % 1024 == 0, "stage tiles stay 1024-byte aligned");
 
@@ -1815,6 +1851,7 @@ struct GramArgs {
     const int64_t *vbase;
     const uint16_t *cn;
     const int64_t *cbase;
+    const uint16_t *pre;       // per word of bits: bits of its row before it
     const long long *gnm;
     const int64_t *off;        // union adjacency offsets
     const int64_t *etile;      // first item of each graph (k + 1 entries)
@@ -1828,12 +1865,16 @@ __global__ void k_gram_tiles(const long long *gnm, const int64_t *cbase, int k, 
     for (int g = blockIdx.x * blockDim.x + threadIdx.x; g <= k; g += gridDim.x * blockDim.x) {
         int64_t t = 0;
         if (g < k && cbase[g] >= 0) {
-            const int64_t n = gnm[2 * g];
-            t = ((n + kGramM - 1) / kGramM) * ((n + kGramN - 1) / kGramN);
+            // row tile i takes the column tiles from i / 2 on
+            const int64_t n = gnm[2 * g], tc = (n + kGramN - 1) / kGramN, tr = (n + kGramM - 1) / kGramM;
+            for (int64_t i = 0; i < tr; i++) t += tc - i / 2;
         }
         tiles[g] = t;
     }
 }
+
+// 0xffff in each half whose bit is set in the low two bits of b
+__device__ __forceinline__ uint32_t pair_mask(uint32_t b) { return ((b & 1u) | (b & 2u) << 15) * 0xffffu; }
 
 __global__ void __launch_bounds__(kGramThreads, 1) k_dense_gram(GramArgs A) {
     extern __shared__ uint8_t gram_smem[];
@@ -1867,14 +1908,15 @@ __global__ void __launch_bounds__(kGramThreads, 1) k_dense_gram(GramArgs A) {
         const int W = (n + 63) >> 6;
         const int64_t stride = (int64_t)W * 64;
         const int tcols = (n + kGramN - 1) / kGramN;
-        const int local = (int)(item - A.etile[g]);
-        const int i0 = (local / tcols) * kGramM, j0 = (local % tcols) * kGramN;
+        int local = (int)(item - A.etile[g]), ti = 0;
+        while (local >= tcols - ti / 2) local -= tcols - ti++ / 2;
+        const int i0 = ti * kGramM, j0 = (ti / 2 + local) * kGramN;
         const int nt = min(kGramN, ((n - j0 + 15) >> 4) << 4);
         const uint64_t *rows = A.bits + A.wbase[g];
         const uint16_t *cng = A.cn + A.cbase[g];
-        const int nK = (n + 15) >> 4;
-        const uint32_t id_pos = idesc_tf32_f32(kGramM, nt, false), id_neg = idesc_tf32_f32(kGramM, nt, true);
-        // this thread's items (4 columns of one row each, 16 bytes): A tile
+        const int nK = (n + 31) >> 5;
+        const uint32_t id_pos = idesc_f16_f32(kGramM, nt, false), id_neg = idesc_f16_f32(kGramM, nt, true);
+        // this thread's items (8 columns of one row each, 16 bytes): A tile
         // items 0..511, B tile items after them; in the core-matrix layout
         // (LBO 128, SBO 512) item i of a tile lives at byte 16·i
         const int nItems = kGramM * 4 + nt * 4;
@@ -1893,50 +1935,53 @@ __global__ void __launch_bounds__(kGramThreads, 1) k_dense_gram(GramArgs A) {
             dst[k] = isA[k] ? (uint32_t)(16 * i2) : (uint32_t)(kGramM * 64 + 16 * i2);
         }
         // the global words of one chunk's items: the bit-row word and, where the
-        // item takes CN, its four entries; loaded one chunk ahead
-        auto fetch = [&](int ch, uint64_t *bw, uint64_t *cw) {
+        // item takes CN, its eight entries; loaded one chunk ahead
+        auto fetch = [&](int ch, uint64_t *bw, uint4 *cw) {
             const bool second = ch >= nK;
             const int kc = second ? ch - nK : ch;
 #pragma unroll
             for (int k = 0; k < 3; k++) {
-                bw[k] = cw[k] = 0ull;
+                bw[k] = 0ull;
+                cw[k] = make_uint4(0u, 0u, 0u, 0u);
                 if (tid + k * kGramThreads < nItems && grow[k] >= 0) {
-                    const int k0 = kc * 16 + gblk[k] * 4;   // first column, below 64·W
+                    const int k0 = kc * 32 + gblk[k] * 8;   // first column, below 64·W
                     bw[k] = rows[(int64_t)grow[k] * W + (k0 >> 6)];
-                    if (isA[k] == second) cw[k] = *(const uint64_t *)(cng + (int64_t)grow[k] * stride + k0);
+                    if (isA[k] == second) cw[k] = *(const uint4 *)(cng + (int64_t)grow[k] * stride + k0);
                 }
             }
         };
-        uint64_t pbw[3], pcw[3];
+        uint64_t pbw[3];
+        uint4 pcw[3];
         fetch(0, pbw, pcw);
         for (int ch = 0; ch < 2 * nK; ch++) {
             const bool second = ch >= nK;   // TA x A, negated
             const int kc = second ? ch - nK : ch;
             const int st = chunk % kGramStages;
             uint8_t *stg = base + st * kGramStageBytes;
-            uint64_t nbw[3] = {0ull, 0ull, 0ull}, ncw[3] = {0ull, 0ull, 0ull};
+            uint64_t nbw[3] = {0ull, 0ull, 0ull};
+            uint4 ncw[3] = {};
             if (ch + 1 < 2 * nK) fetch(ch + 1, nbw, ncw);
 #pragma unroll
             for (int k = 0; k < 3; k++) {
                 if (tid + k * kGramThreads >= nItems) continue;
                 uint4 v = make_uint4(0u, 0u, 0u, 0u);
                 if (grow[k] >= 0) {
-                    const int k0 = kc * 16 + gblk[k] * 4;
-                    const uint32_t b4 = (uint32_t)(pbw[k] >> (k0 & 63)) & 15u;
+                    const int k0 = kc * 32 + gblk[k] * 8;
+                    const uint32_t b8 = (uint32_t)(pbw[k] >> (k0 & 63)) & 0xffu;
                     // A x (CN - TA): A side bits, B side CN off the edges;
                     // TA x A: A side CN on the edges, B side bits
                     if (isA[k] == second) {
-                        const uint64_t c4 = pcw[k];
-                        const uint32_t keep = second ? b4 : ~b4;
-                        v.x = (keep & 1u) ? __float_as_uint((float)(uint32_t)(c4 & 0xffffu)) : 0u;
-                        v.y = (keep & 2u) ? __float_as_uint((float)(uint32_t)((c4 >> 16) & 0xffffu)) : 0u;
-                        v.z = (keep & 4u) ? __float_as_uint((float)(uint32_t)((c4 >> 32) & 0xffffu)) : 0u;
-                        v.w = (keep & 8u) ? __float_as_uint((float)(uint32_t)(c4 >> 48)) : 0u;
+                        const uint32_t keep = second ? b8 : ~b8;
+                        v.x = f16_pair(pcw[k].x & pair_mask(keep));
+                        v.y = f16_pair(pcw[k].y & pair_mask(keep >> 2));
+                        v.z = f16_pair(pcw[k].z & pair_mask(keep >> 4));
+                        v.w = f16_pair(pcw[k].w & pair_mask(keep >> 6));
                     } else {
-                        v.x = (b4 & 1u) ? 0x3f800000u : 0u;
-                        v.y = (b4 & 2u) ? 0x3f800000u : 0u;
-                        v.z = (b4 & 4u) ? 0x3f800000u : 0u;
-                        v.w = (b4 & 8u) ? 0x3f800000u : 0u;
+                        // 1.0 is 0x3c00
+                        v.x = pair_mask(b8) & 0x3c003c00u;
+                        v.y = pair_mask(b8 >> 2) & 0x3c003c00u;
+                        v.z = pair_mask(b8 >> 4) & 0x3c003c00u;
+                        v.w = pair_mask(b8 >> 6) & 0x3c003c00u;
                     }
                 }
                 *(uint4 *)(stg + dst[k]) = v;
@@ -1953,7 +1998,7 @@ __global__ void __launch_bounds__(kGramThreads, 1) k_dense_gram(GramArgs A) {
                 const uint32_t sa = smem_addr(stg), sb = sa + kGramM * 64;
 #pragma unroll
                 for (int ks = 0; ks < 2; ks++)
-                    mma_tf32(tmem, smem_desc(sa + 256 * ks, 128, 512), smem_desc(sb + 256 * ks, 128, 512),
+                    mma_f16(tmem, smem_desc(sa + 256 * ks, 128, 512), smem_desc(sb + 256 * ks, 128, 512),
                              second ? id_neg : id_pos, (ch | ks) != 0);
                 mma_commit(&s_bar[st]);
                 pend |= 1u << st;
@@ -1985,23 +2030,37 @@ __global__ void __launch_bounds__(kGramThreads, 1) k_dense_gram(GramArgs A) {
         }
         fence_after_sync();
         if (cq * 64 < nt) {
-            const int i = i0 + 32 * lg + lane;
-            const int jw = (j0 + cq * 64) >> 6;   // the columns' word of row i
+            const int ib = i0 + 32 * lg, i = ib + lane;   // the warp's 32 rows share the word ib >> 6 of a row j
+            const int jb = j0 + cq * 64, jw = jb >> 6;    // the columns' word of row i
             uint64_t word = 0;
             int64_t slot = 0;
+            const int64_t vb = A.vbase[g];
+            const uint16_t *pre = A.pre + A.wbase[g];
             if (i < n) {
-                const uint64_t *ri = rows + (int64_t)i * W;
-                word = ri[jw];
-                int before = 0;
-                for (int w = 0; w < jw; w++) before += __popcll(ri[w]);
-                slot = A.off[A.vbase[g] + i] + before;
+                word = rows[(int64_t)i * W + jw];
+                // the columns above the diagonal, and the slot of the first of them
+                const uint64_t low = i < jb ? 0ull : (i - jb >= 63 ? ~0ull : (2ull << (i - jb)) - 1);
+                slot = A.off[vb + i] + pre[(int64_t)i * W + jw] + __popcll(word & low);
+                word &= ~low;
             }
             for (int c0 = 0; c0 < 64 && cq * 64 + c0 < nt; c0 += 16) {
                 uint32_t v[16];
                 tmem_ld16(tmem + ((uint32_t)(32 * lg) << 16) + (uint32_t)(cq * 64 + c0), v);
+                const uint32_t w16 = (uint32_t)(word >> c0) & 0xffffu;
 #pragma unroll
-                for (int e = 0; e < 16; e++)
-                    if ((word >> (c0 + e)) & 1ull) A.eslot[slot++] = (int32_t)__uint_as_float(v[e]);
+                for (int e = 0; e < 16; e++) {
+                    if (__any_sync(0xffffffffu, (w16 >> e) & 1u)) {
+                        // row j holds bit i for every such lane: its slots for ib .. ib + 31 are consecutive
+                        const int64_t j = jb + c0 + e;
+                        const uint64_t wj = rows[j * W + (ib >> 6)];
+                        if ((w16 >> e) & 1u) {
+                            const int32_t val = (int32_t)__uint_as_float(v[e]);
+                            A.eslot[slot++] = val;
+                            A.eslot[A.off[vb + j] + pre[j * W + (ib >> 6)] + __popcll(wj & ((1ull << (i & 63)) - 1))] =
+                                val;
+                        }
+                    }
+                }
             }
         }
         fence_before_sync();
@@ -2320,6 +2379,7 @@ struct DenseView {
     const int64_t *vbase;
     const uint16_t *cn;       // common-neighbour matrices
     const int64_t *cbase;     // per graph: first CN entry, or -1
+    const uint16_t *pre;      // per word of bits: bits of its row before it
     const int64_t *before;    // per graph: edges of sparse graphs before it
     int ngraphs;
     int64_t nedges;           // edges of the dense graphs
@@ -2343,7 +2403,7 @@ struct TcOut {
 };
 
 static pgd_status dense_tc(pgd_ctx *ctx, const DevGraph &G, TmpGuard &tg, const DenseView *dense,
-                           const int32_t *dpos, const uint64_t *keys, int64_t ncn, int eb, TcOut *out) {
+                           const int32_t *dpos, const uint32_t *keys, int64_t ncn, TcOut *out) {
     cudaStream_t s = ctx->stream;
     pgd_status st;
     uint32_t *flag = nullptr, *pos = nullptr, *k4 = nullptr;
@@ -2355,7 +2415,7 @@ static pgd_status dense_tc(pgd_ctx *ctx, const DevGraph &G, TmpGuard &tg, const 
     if ((st = tg.alloc(&runs, (2 * maxruns + 2) * sizeof(int64_t)))) return st;
     unsigned long long *ctr = ctx->d_ctr;
     PGD_CUDA(ctx, cudaMemsetAsync(ctr + 8, 0, 6 * sizeof(unsigned long long), s));
-    PGD_LAUNCH(ctx, k_tc_run_flags, grid_for(ncn), kThreads, 0, keys, ncn, G.deg, ctx->tc_min_deg, flag, eb);
+    PGD_LAUNCH(ctx, k_tc_run_flags, grid_for(ncn), kThreads, 0, keys, ncn, G.deg, ctx->tc_min_deg, flag);
     PGD_CUDA(ctx, cudaMemsetAsync(flag + ncn, 0, sizeof(uint32_t), s));
     size_t tb = 0;
     void *tmp = nullptr;
@@ -2363,7 +2423,7 @@ static pgd_status dense_tc(pgd_ctx *ctx, const DevGraph &G, TmpGuard &tg, const 
     if ((st = pgd_tmp_alloc(ctx, &tmp, tb))) return st;
     cub::DeviceScan::ExclusiveSum(tmp, tb, flag, pos, ncn + 1, s);
     pgd_tmp_free(ctx, tmp);
-    PGD_LAUNCH(ctx, k_tc_run_fill, grid_for(ncn), kThreads, 0, keys, flag, pos, ncn, runs, ctr + 9, eb);
+    PGD_LAUNCH(ctx, k_tc_run_fill, grid_for(ncn), kThreads, 0, keys, flag, pos, ncn, runs, ctr + 9);
     PGD_CUDA(ctx, cudaMemsetAsync(k4, 0xff, ncn * sizeof(uint32_t), s));
     DenseTcArgs T;
     T.G = G;
@@ -2396,6 +2456,7 @@ static pgd_status dense_tc(pgd_ctx *ctx, const DevGraph &G, TmpGuard &tg, const 
     E.vbase = dense->vbase;
     E.cn = dense->cn;
     E.cbase = dense->cbase;
+    E.pre = dense->pre;
     E.gnm = G.gnm;
     E.off = G.off;
     E.etile = etile;
@@ -2407,7 +2468,7 @@ static pgd_status dense_tc(pgd_ctx *ctx, const DevGraph &G, TmpGuard &tg, const 
     // the positions left to k_dense_cn (flag and pos arrays reused)
     int32_t *rest = nullptr;
     if ((st = tg.alloc(&rest, (ncn + 1) * sizeof(int32_t)))) return st;
-    PGD_LAUNCH(ctx, k_tc_rest_flags, grid_for(ncn), kThreads, 0, keys, ncn, G.deg, ctx->tc_min_deg, flag, eb);
+    PGD_LAUNCH(ctx, k_tc_rest_flags, grid_for(ncn), kThreads, 0, keys, ncn, G.deg, ctx->tc_min_deg, flag);
     PGD_CUDA(ctx, cudaMemsetAsync(flag + ncn, 0, sizeof(uint32_t), s));
     tb = 0;
     cub::DeviceScan::ExclusiveSum(nullptr, tb, flag, pos, ncn + 1, s);
@@ -2659,23 +2720,23 @@ static pgd_status dense_decompose(pgd_ctx *ctx, const DevGraph &G, const DenseVi
     const int nsm = ctx->num_sms;
     const int64_t nd = dense.nedges;
     TmpGuard tg(ctx);
-    uint64_t *keys = nullptr, *keys2 = nullptr;
+    uint32_t *keys = nullptr, *keys2 = nullptr;
     int32_t *vals = nullptr, *dpos = nullptr;
-    if ((st = tg.alloc(&keys, nd * sizeof(uint64_t)))) return st;
-    if ((st = tg.alloc(&keys2, nd * sizeof(uint64_t)))) return st;
+    if ((st = tg.alloc(&keys, nd * sizeof(uint32_t)))) return st;
+    if ((st = tg.alloc(&keys2, nd * sizeof(uint32_t)))) return st;
     if ((st = tg.alloc(&vals, nd * sizeof(int32_t)))) return st;
     if ((st = tg.alloc(&dpos, nd * sizeof(int32_t)))) return st;
     unsigned long long *ctr = ctx->d_ctr;
     PGD_CUDA(ctx, cudaMemsetAsync(ctr, 0, 8 * sizeof(unsigned long long), s));
-    const int qb = bits_for(G.n), eb = bits_for(G.npos);
-    PGD_LAUNCH(ctx, k_dense_keys, grid_for(G.npos), kThreads, 0, G, dense.before, keys, vals, eb);
+    const int qb = bits_for(G.n);
+    PGD_LAUNCH(ctx, k_dense_keys, grid_for(G.npos), kThreads, 0, G, dense.before, keys, vals);
     size_t tb = 0;
     void *tmp = nullptr;
-    cub::DeviceRadixSort::SortPairs(nullptr, tb, keys, keys2, vals, dpos, nd, 0, qb + eb, s);
+    cub::DeviceRadixSort::SortPairs(nullptr, tb, keys, keys2, vals, dpos, nd, 0, qb, s);
     if ((st = tg.alloc(&tmp, tb))) return st;
-    PGD_CUDA(ctx, cub::DeviceRadixSort::SortPairs(tmp, tb, keys, keys2, vals, dpos, nd, 0, qb + eb, s));
+    PGD_CUDA(ctx, cub::DeviceRadixSort::SortPairs(tmp, tb, keys, keys2, vals, dpos, nd, 0, qb, s));
     TcOut tc;
-    if (ctx->tc_min_deg > 0 && (st = dense_tc(ctx, G, tg, &dense, dpos, keys2, nd, eb, &tc))) return st;
+    if (ctx->tc_min_deg > 0 && (st = dense_tc(ctx, G, tg, &dense, dpos, keys2, nd, &tc))) return st;
     if (!tc.k4 || tc.nrest > 0) {
         DenseCnArgs C;
         C.G = G;
@@ -2896,15 +2957,18 @@ static pgd_status decompose_union(pgd_graph *U, int k, const std::vector<long lo
     if (B.ndense) {
         int64_t *tables = nullptr;
         unsigned long long *bits = nullptr;
-        uint16_t *cn = nullptr;
+        uint16_t *cn = nullptr, *pre = nullptr;
         if ((st = tg.alloc(&tables, B.tables.size() * sizeof(int64_t)))) return st;
         if ((st = tg.alloc(&bits, (size_t)B.words * sizeof(unsigned long long)))) return st;
         if ((st = tg.alloc(&cn, (size_t)B.entries * sizeof(uint16_t)))) return st;
+        if ((st = tg.alloc(&pre, (size_t)B.words * sizeof(uint16_t)))) return st;
         PGD_CUDA(ctx, cudaMemcpyAsync(tables, B.tables.data(), B.tables.size() * sizeof(int64_t), cudaMemcpyHostToDevice, s));
         PGD_CUDA(ctx, cudaMemsetAsync(bits, 0, (size_t)B.words * sizeof(unsigned long long), s));
-        dv = DenseView{(const uint64_t *)bits, tables, d_vbase, cn, tables + k, tables + 2 * k, k, B.dense_edges};
+        dv = DenseView{(const uint64_t *)bits, tables, d_vbase, cn, tables + k, pre, tables + 2 * k, k, B.dense_edges};
         PGD_LAUNCH(ctx, k_dense_bits, grid_for(32 * U->n), kThreads, 0, U->off, U->adj, vgraph, d_dense, dv.wbase,
                    d_vbase, d_gnm, U->n, bits);
+        PGD_LAUNCH(ctx, k_dense_prefix, grid_for(U->n), kThreads, 0, dv.bits, dv.wbase, d_vbase, vgraph, d_dense, d_gnm,
+                   U->n, pre);
         PGD_LAUNCH(ctx, k_dense_common, (int)std::min<int64_t>(B.tiles, (int64_t)ctx->num_sms * 8), 256, 0, dv.bits,
                    dv.wbase, d_gnm, dv.cbase, tables + 3 * k, k, B.tiles, cn);
         G.off = U->off;

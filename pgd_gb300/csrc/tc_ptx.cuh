@@ -24,11 +24,20 @@ __device__ __forceinline__ uint32_t idesc_e4m3_f32(int m, int n) {
     return (1u << 4) | ((uint32_t)(n >> 3) << 17) | ((uint32_t)(m >> 4) << 24);
 }
 
-// instruction descriptor of kind::tf32 (format code 2 for A and B), fp32 D, both
+// instruction descriptor of kind::f16 with f16 A and B (format code 0), fp32 D, both
 // K-major; negate_a subtracts the product from the accumulator
-__device__ __forceinline__ uint32_t idesc_tf32_f32(int m, int n, bool negate_a) {
-    return (1u << 4) | (2u << 7) | (2u << 10) | ((uint32_t)negate_a << 13) | ((uint32_t)(n >> 3) << 17) |
-           ((uint32_t)(m >> 4) << 24);
+__device__ __forceinline__ uint32_t idesc_f16_f32(int m, int n, bool negate_a) {
+    return (1u << 4) | ((uint32_t)negate_a << 13) | ((uint32_t)(n >> 3) << 17) | ((uint32_t)(m >> 4) << 24);
+}
+
+// two 16-bit whole numbers (at most 2048: exact) as two f16
+__device__ __forceinline__ uint32_t f16_pair(uint32_t two) {
+    uint32_t r;
+    asm("{\n.reg .b16 a, b, x, y;\nmov.b32 {a, b}, %1;\ncvt.rn.f16.u16 x, a;\ncvt.rn.f16.u16 y, b;\n"
+        "mov.b32 %0, {x, y};\n}"
+        : "=r"(r)
+        : "r"(two));
+    return r;
 }
 
 __device__ __forceinline__ void tmem_alloc(uint32_t *dst_smem, uint32_t ncols) {   // one full warp
@@ -106,12 +115,12 @@ __device__ __forceinline__ void mma_e4m3(uint32_t d_tmem, uint64_t a_desc, uint6
         : "memory");
 }
 
-// D[tmem] (+)= A[smem] * B[smem]^T, tf32 operands (32-bit containers), fp32 accumulator
-__device__ __forceinline__ void mma_tf32(uint32_t d_tmem, uint64_t a_desc, uint64_t b_desc, uint32_t idesc,
-                                         bool accumulate) {
+// D[tmem] (+)= A[smem] * B[smem]^T, f16 operands, fp32 accumulator
+__device__ __forceinline__ void mma_f16(uint32_t d_tmem, uint64_t a_desc, uint64_t b_desc, uint32_t idesc,
+                                        bool accumulate) {
     asm volatile(
         "{\n.reg .pred p;\nsetp.ne.u32 p, %4, 0;\n"
-        "tcgen05.mma.cta_group::1.kind::tf32 [%0], %1, %2, %3, p;\n}" ::"r"(d_tmem),
+        "tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, p;\n}" ::"r"(d_tmem),
         "l"(a_desc), "l"(b_desc), "r"(idesc), "r"((uint32_t)accumulate)
         : "memory");
 }
