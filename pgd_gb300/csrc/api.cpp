@@ -113,7 +113,7 @@ extern "C" pgd_status pgd_context_create(const pgd_opts *opts, pgd_ctx **out) {
         cudaEventCreate(&ctx->evt0) != cudaSuccess || cudaEventCreate(&ctx->evt1) != cudaSuccess ||
         cudaEventCreate(&ctx->evh0) != cudaSuccess || cudaEventCreate(&ctx->evh1) != cudaSuccess ||
         cudaHostAlloc((void **)&ctx->pin, kPinBytes, cudaHostAllocDefault) != cudaSuccess ||
-        pgd_decompose_limits() != cudaSuccess || pgd_rank_limits() != cudaSuccess ||
+        pgd_build_limits() != cudaSuccess || pgd_decompose_limits() != cudaSuccess || pgd_rank_limits() != cudaSuccess ||
         cudaStreamCreateWithFlags(&ctx->side, cudaStreamNonBlocking) != cudaSuccess ||
         cudaEventCreateWithFlags(&ctx->ev_fork, cudaEventDisableTiming) != cudaSuccess ||
         cudaEventCreateWithFlags(&ctx->ev_join, cudaEventDisableTiming) != cudaSuccess) {

@@ -1836,7 +1836,7 @@ __global__ void __launch_bounds__(kTcThreads, 1) k_dense_tc(DenseTcArgs A) {
 // barrier and twice the rate of tf32.  E is symmetric: only tiles with columns
 // above the diagonal are taken, read back one row per thread, and E[x][y] of an
 // edge x < y is written at both adjacency slots, y -> x (consecutive for a warp's
-// rows) and x -> y.  6.5 -> 2.4 ms on 128 graphs of up to 2048 vertices.
+// rows) and x -> y.  6.5 -> 2.7 ms on 128 graphs of up to 2048 vertices.
 
 constexpr int kGramThreads = 512;
 constexpr int kGramM = 128, kGramN = 256;

@@ -729,6 +729,61 @@ __device__ __forceinline__ void core_append(bool in, int32_t v, int32_t *list, u
     if (in) list[at + __popc(m & ((1u << lane) - 1))] = v;
 }
 
+// visit(active, neighbour) over the rows of a frontier's entries 0..nf, by `warps`
+// warps of which this is the w-th: as many vertices per warp as fill them (at
+// most 32), whose offsets are then loaded together; rows of 64 or more entries
+// one after the other, shorter ones flattened over the lanes.
+template <typename Get, typename Visit>
+__device__ __forceinline__ void core_rows(const int64_t *off, const int32_t *adj, const int32_t *deg, unsigned nf, int w,
+                                          int warps, Get get, Visit visit) {
+    const int lane = threadIdx.x & 31;
+    const unsigned per = min(32u, max(1u, (nf + (unsigned)warps - 1) / (unsigned)warps));
+    for (unsigned i0 = (unsigned)w * per; i0 < nf; i0 += (unsigned)warps * per) {
+        int64_t o = 0;
+        int d = 0;
+        if ((unsigned)lane < per && i0 + lane < nf) {
+            const int32_t v = get(i0 + lane);
+            o = off[v];
+            d = deg[v];
+        }
+        unsigned lm = __ballot_sync(0xffffffffu, d >= 64);
+        while (lm) {
+            const int src = __ffs(lm) - 1;
+            lm &= lm - 1;
+            const int64_t os = __shfl_sync(0xffffffffu, o, src);
+            const int ds = __shfl_sync(0xffffffffu, d, src);
+            for (int j = 0; j < ds; j += 128) {
+                int32_t y[4];
+#pragma unroll
+                for (int k = 0; k < 4; k++) y[k] = j + 32 * k + lane < ds ? __ldg(adj + os + j + 32 * k + lane) : 0;
+#pragma unroll
+                for (int k = 0; k < 4; k++)
+                    if (j + 32 * k < ds) visit(j + 32 * k + lane < ds, y[k]);
+            }
+        }
+        if (d >= 64) d = 0;
+        const int incl = pgd_warp_incl_scan(d);
+        const int total = __shfl_sync(0xffffffffu, incl, 31);
+        const int64_t first = o - (incl - d);   // slot = first + flattened index
+        for (int b = 0; b < total; b += 64) {
+            int32_t y[2];
+#pragma unroll
+            for (int k = 0; k < 2; k++) {
+                const int it = b + 32 * k + lane;
+                int own = 0;
+#pragma unroll
+                for (int step = 16; step > 0; step >>= 1)
+                    if (__shfl_sync(0xffffffffu, incl, own + step - 1) <= it) own += step;
+                const int64_t f = __shfl_sync(0xffffffffu, first, own & 31);
+                y[k] = it < total ? __ldg(adj + f + it) : 0;
+            }
+#pragma unroll
+            for (int k = 0; k < 2; k++)
+                if (b + 32 * k < total) visit(b + 32 * k + lane < total, y[k]);
+        }
+    }
+}
+
 // f and b: two buffers each (n entries) of the frontier's short and long rows;
 // a0, a1: vertices alive.  A level scan moves every alive vertex of count <=
 // level to the frontier and the others to the other alive list; a peel round
@@ -805,31 +860,25 @@ k_core_cluster(const int64_t *off, const int32_t *adj, const int32_t *deg, int n
         removed += (int)(nf + nb);
         while (nf + nb > 0 && step < max_steps) {
             s = next_slot();
-            // one off the count of neighbour x; it leaves when that drops to the level
-            auto visit = [&](bool act, int64_t j) {
+            // one off the count of neighbour y; it leaves when that drops to the level
+            auto visit = [&](bool act, int32_t y) {
                 bool leaves = false;
-                int32_t y = 0;
                 int d = 0;
-                if (act) {
-                    y = __ldg(adj + j);
-                    if (__ldcg(core + y) == -1 && atomicSub(cur + y, 1) == level + 1) {
-                        __stcg(core + y, level);
-                        leaves = true;
-                        d = deg[y];
-                    }
+                if (act && __ldcg(core + y) == -1 && atomicSub(cur + y, 1) == level + 1) {
+                    __stcg(core + y, level);
+                    leaves = true;
+                    d = deg[y];
                 }
-                core_append(leaves && d < kCoreLong, y, fout, &s->front, lane);
-                core_append(leaves && d >= kCoreLong, y, bout, &s->lng, lane);
+                if (__any_sync(0xffffffffu, leaves)) {
+                    core_append(leaves && d < kCoreLong, y, fout, &s->front, lane);
+                    core_append(leaves && d >= kCoreLong, y, bout, &s->lng, lane);
+                }
             };
-            for (unsigned i = (unsigned)w; i < nf; i += kAll / 32) {   // a warp per short row
-                const int32_t v = __ldcg(fin + i);
-                const int64_t o = off[v], e = o + deg[v];
-                for (int64_t j = o; j < e; j += 32) visit(j + lane < e, j + lane);
-            }
-            for (unsigned i = 0; i < nb; i++) {                        // all warps share a long row
+            core_rows(off, adj, deg, nf, w, kAll / 32, [&](unsigned i) { return __ldcg(fin + i); }, visit);
+            for (unsigned i = 0; i < nb; i++) {   // all warps share a long row
                 const int32_t v = __ldcg(bin + i);
                 const int64_t o = off[v], e = o + deg[v];
-                for (int64_t j = o + t0; j < e; j += kAll) visit(j + lane < e, j + lane);
+                for (int64_t j = o + t0; j < e; j += kAll) visit(j + lane < e, j + lane < e ? __ldg(adj + j + lane) : 0);
             }
             pgd_cl::cluster_sync();
             nf = __ldcg(&s->front);
@@ -852,7 +901,139 @@ k_core_cluster(const int64_t *off, const int32_t *adj, const int32_t *deg, int n
     if (t == 0 && removed < n) S->failed = 1;
 }
 
+// Small graphs: one block with every count (16 bits) and a bit per vertex removed
+// in shared memory, so that a step is a shared-memory scan or one round over the
+// frontier's rows, and a block barrier.  R-MAT 14: 320 steps.
+constexpr int kCoreSmallBytes = 200 * 1024;
+constexpr int64_t kCoreSmallEntries = 1ll << 20;
+constexpr int kCoreQueue = 2048;            // frontier entries kept in shared memory (the rest in global)
+
+__host__ __device__ __forceinline__ size_t core_small_bytes(int64_t n) {
+    return (size_t)((n + 63) / 64) * 64 * 2 + (size_t)((n + 63) / 64) * 8;
+}
+
+__global__ void __launch_bounds__(kCoreThreads, 1)
+k_core_block(const int64_t *off, const int32_t *adj, const int32_t *deg, int n, int32_t *core, int32_t *g0, int32_t *g1,
+             int32_t *b0, int32_t *b1, CoreShared *S) {
+    extern __shared__ __align__(16) uint32_t s_dyn[];
+    __shared__ int32_t s_q[2][kCoreQueue];
+    __shared__ unsigned int s_nf[2], s_nb[2];
+    __shared__ int s_low[2], s_max;
+    const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
+    const int groups = (n + 63) / 64;       // 64 vertices: 32 words of counts, 2 of bits
+    uint32_t *cur = s_dyn, *gone = s_dyn + 32 * groups;
+    for (int i = threadIdx.x; i < 32 * groups; i += kCoreThreads) {
+        const uint32_t lo = 2 * i < n ? (uint32_t)deg[2 * i] : 0, hi = 2 * i + 1 < n ? (uint32_t)deg[2 * i + 1] : 0;
+        cur[i] = lo | hi << 16;
+    }
+    for (int i = threadIdx.x; i < 2 * groups; i += kCoreThreads)
+        gone[i] = 32 * i + 32 <= n ? 0u : (32 * i >= n ? 0xffffffffu : 0xffffffffu << (n - 32 * i));
+    if (threadIdx.x < 2) {
+        s_nf[threadIdx.x] = s_nb[threadIdx.x] = 0;
+        s_low[threadIdx.x] = INT_MAX;
+        s_max = 0;
+    }
+    __syncthreads();
+    int level = 0, removed = 0, sel = 0, scan = 0;
+    // v leaves at this level: into the frontier of buffer q
+    auto leave = [&](bool in, int32_t v, int q) {
+        const bool lng = in && deg[v] >= kCoreLong;
+        const unsigned m = __ballot_sync(0xffffffffu, in && !lng);
+        if (m) {
+            unsigned at = 0;
+            if (lane == 0) at = atomicAdd(&s_nf[q], (unsigned)__popc(m));
+            at = __shfl_sync(0xffffffffu, at, 0) + (unsigned)__popc(m & ((1u << lane) - 1));
+            if (in && !lng) {
+                if (at < kCoreQueue) s_q[q][at] = v;
+                else (q ? g1 : g0)[at - kCoreQueue] = v;
+            }
+        }
+        if (lng) (q ? b1 : b0)[atomicAdd(&s_nb[q], 1u)] = v;
+        if (in) core[v] = level;
+    };
+    while (removed < n) {
+        // every vertex left of count <= level leaves; the smallest count of the rest is the next level
+        int low = INT_MAX;
+        for (int g = wid; g < groups; g += kCoreThreads / 32) {
+            const uint32_t out = gone[2 * g + (lane >> 4)];
+            if (__all_sync(0xffffffffu, out == 0xffffffffu)) continue;
+            const uint32_t c2 = cur[32 * g + lane];
+            const int b = 2 * (lane & 15), ca = (int)(c2 & 0xffffu), cb = (int)(c2 >> 16);
+            const bool ha = !((out >> b) & 1u), hb = !((out >> b) & 2u);
+            const bool ia = ha && ca <= level, ib = hb && cb <= level;
+            if (ha && !ia) low = min(low, ca);
+            if (hb && !ib) low = min(low, cb);
+            if (__any_sync(0xffffffffu, ia || ib)) {
+                leave(ia, 64 * g + 2 * lane, sel);
+                leave(ib, 64 * g + 2 * lane + 1, sel);
+                if (ia || ib) atomicOr(gone + 2 * g + (lane >> 4), (ia ? 1u << b : 0u) | (ib ? 2u << b : 0u));
+            }
+        }
+        low = __reduce_min_sync(0xffffffffu, low);
+        if (lane == 0 && low != INT_MAX) atomicMin(&s_low[scan], low);
+        __syncthreads();
+        unsigned nf = s_nf[sel], nb = s_nb[sel];
+        low = s_low[scan];
+        scan ^= 1;
+        if (nf + nb == 0) {
+            level = max(level + 1, low);
+            __syncthreads();               // everyone has read before the next scan writes
+            if (threadIdx.x == 0) s_low[scan ^ 1] = INT_MAX;
+            __syncthreads();
+            continue;
+        }
+        removed += (int)(nf + nb);
+        while (nf + nb > 0) {
+            const int to = sel ^ 1;
+            __syncthreads();               // the counts are read
+            if (threadIdx.x == 0) {
+                s_nf[sel] = s_nb[sel] = 0;  // read again only when this buffer has been refilled
+                s_low[scan ^ 1] = INT_MAX;
+            }
+            auto visit = [&](bool act, int32_t y) {
+                bool in = false;
+                if (act && !((gone[y >> 5] >> (y & 31)) & 1u)) {
+                    const int sh = (y & 1) << 4;
+                    // at most deg(y) take one off: the half never borrows
+                    in = (int)((atomicSub(cur + (y >> 1), 1u << sh) >> sh) & 0xffffu) == level + 1;
+                    if (in) atomicOr(gone + (y >> 5), 1u << (y & 31));
+                }
+                if (__any_sync(0xffffffffu, in)) leave(in, y, to);
+            };
+            core_rows(off, adj, deg, nf, wid, kCoreThreads / 32,
+                      [&](unsigned i) { return i < kCoreQueue ? s_q[sel][i] : (sel ? g1 : g0)[i - kCoreQueue]; }, visit);
+            for (unsigned i = 0; i < nb; i++) {
+                const int32_t v = (sel ? b1 : b0)[i];
+                const int64_t o = off[v];
+                const int d = deg[v];
+                for (int j = 32 * wid; j < d; j += kCoreThreads)
+                    visit(j + lane < d, j + lane < d ? __ldg(adj + o + j + lane) : 0);
+            }
+            __syncthreads();
+            sel = to;
+            nf = s_nf[sel];
+            nb = s_nb[sel];
+            removed += (int)(nf + nb);
+        }
+        __syncthreads();
+        level++;
+    }
+    int top = 0;
+    for (int v = threadIdx.x; v < n - 1; v += kCoreThreads) top = max(top, core[v]);
+    top = __reduce_max_sync(0xffffffffu, top);
+    if (lane == 0 && top > 0) atomicMax(&s_max, top);
+    __syncthreads();
+    if (threadIdx.x == 0) {
+        S->max_core = s_max;
+        S->failed = 0;
+    }
+}
+
 }  // namespace
+
+cudaError_t pgd_build_limits() {
+    return cudaFuncSetAttribute(k_core_block, cudaFuncAttributeMaxDynamicSharedMemorySize, kCoreSmallBytes);
+}
 
 static pgd_status cores_by_cluster(pgd_graph *g) {
     pgd_ctx *ctx = g->ctx;
@@ -863,7 +1044,11 @@ static pgd_status cores_by_cluster(pgd_graph *g) {
     const size_t lists = (7 * (size_t)n * sizeof(int32_t) + 15) & ~(size_t)15;
     if ((st = pgd_tmp_alloc(ctx, (void **)&work, lists + sizeof(CoreShared)))) return st;
     CoreShared *S = (CoreShared *)((uint8_t *)work + lists);
-    PGD_LAUNCH(ctx, k_core_cluster, kCoreBlocks, kCoreThreads, 0, g->off, g->adj, g->deg, (int)n, work, g->core,
+    if (g->max_degree < 65536 && 2 * g->m <= kCoreSmallEntries && core_small_bytes(n) <= (size_t)kCoreSmallBytes)
+        PGD_LAUNCH(ctx, k_core_block, 1, kCoreThreads, core_small_bytes(n), g->off, g->adj, g->deg, (int)n, g->core, work,
+                   work + n, work + 2 * n, work + 3 * n, S);
+    else
+        PGD_LAUNCH(ctx, k_core_cluster, kCoreBlocks, kCoreThreads, 0, g->off, g->adj, g->deg, (int)n, work, g->core,
                work + n, work + 2 * n, work + 3 * n, work + 4 * n, work + 5 * n, work + 6 * n, S, g->max_degree);
     cudaError_t e = cudaGetLastError();
     if (e == cudaSuccess) e = pgd_fetch(ctx, 0, S, sizeof(CoreShared));

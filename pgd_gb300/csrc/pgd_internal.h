@@ -148,7 +148,9 @@ struct pgd_pieces {
 };
 
 // Limits of the kernels that use more shared memory than the default, set to
-// the same constants for every context of the device (decompose.cu, rank_path.cu).
+// the same constants for every context of the device (graph_build.cu,
+// decompose.cu, rank_path.cu).
+cudaError_t pgd_build_limits();
 cudaError_t pgd_decompose_limits();
 cudaError_t pgd_rank_limits();
 
