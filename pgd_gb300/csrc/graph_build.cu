@@ -434,6 +434,184 @@ static pgd_status finish_csr(pgd_graph *g, uint64_t *keys, uint32_t *vals, int64
     return PGD_OK;
 }
 
+// ---------------------------------------------------------------------------
+// Small graphs: each stage by one block.
+
+namespace {
+
+struct SmallResult {
+    int nnz, max_degree, loops;
+};
+
+// CSR of k <= kSmallPairs pairs (ids below n): words of row, column and pair index
+// (ib bits) sorted in shared memory, the first of each run kept.
+__global__ void __launch_bounds__(kSmallThreads) k_small_build(const int32_t *src, const int32_t *dst, int k, int n,
+                                                               int cb, int ib, int P, int64_t *off, int32_t *adj,
+                                                               int64_t *rank, int32_t *deg, SmallResult *out) {
+    extern __shared__ __align__(16) uint32_t s_dyn[];
+    uint64_t *w = (uint64_t *)s_dyn;
+    __shared__ int sh[33], s_loops, s_max;
+    if (threadIdx.x == 0) s_loops = s_max = 0;
+    __syncthreads();
+    for (int i = threadIdx.x; 2 * i < P; i += kSmallThreads) {
+        uint64_t x = ~0ull, y = ~0ull;
+        if (i < k) {
+            const uint64_t a = (uint32_t)src[i], b = (uint32_t)dst[i];
+            if (a != b) {
+                x = (a << (cb + ib)) | (b << ib) | (uint64_t)i;
+                y = (b << (cb + ib)) | (a << ib) | (uint64_t)i;
+            } else {
+                atomicAdd(&s_loops, 1);
+            }
+        }
+        w[2 * i] = x;
+        w[2 * i + 1] = y;
+    }
+    __syncthreads();
+    pgd_block_sort(w, P);
+    // each thread a contiguous part: its runs' first words, counted then written
+    const int per = (P + kSmallThreads - 1) / kSmallThreads, b0 = min(P, (int)threadIdx.x * per), b1 = min(P, b0 + per);
+    auto first = [&](int i) { return w[i] != ~0ull && (i == 0 || (w[i] >> ib) != (w[i - 1] >> ib)); };
+    int c = 0, total = 0;
+    for (int i = b0; i < b1; i++) c += first(i);
+    int at = pgd_block_excl_scan(c, sh, &total);
+    for (int i = b0; i < b1; i++) {
+        if (!first(i)) continue;
+        const int r = (int)(w[i] >> (cb + ib)), rp = i == 0 ? -1 : (int)(w[i - 1] >> (cb + ib));
+        adj[at] = (int32_t)((w[i] >> ib) & ((1ull << cb) - 1));
+        rank[at] = (int64_t)(w[i] & ((1ull << ib) - 1));
+        for (int x = rp + 1; x <= r; x++) off[x] = at;
+        at++;
+    }
+    // rows behind the last one with entries (the sentinels' row id is beyond n)
+    const int valid = 2 * (k - s_loops);
+    const int last = valid > 0 ? (int)(w[valid - 1] >> (cb + ib)) : -1;
+    for (int x = last + 1 + (int)threadIdx.x; x <= n; x += kSmallThreads) off[x] = total;
+    __syncthreads();
+    int top = 0;
+    for (int v = threadIdx.x; v < n; v += kSmallThreads) {
+        const int d = (int)(off[v + 1] - off[v]);
+        deg[v] = d;
+        top = max(top, d);
+    }
+    top = __reduce_max_sync(0xffffffffu, top);
+    if ((threadIdx.x & 31) == 0 && top > 0) atomicMax(&s_max, top);
+    __syncthreads();
+    if (threadIdx.x == 0) *out = SmallResult{total, s_max, s_loops};
+}
+
+// Edge arrays of a small graph: as k_neigh_words, one sort and k_edge_assign, with
+// the other endpoint (cb bits) in the word.
+__global__ void __launch_bounds__(kSmallThreads) k_small_edges(const int64_t *off, const int32_t *adj,
+                                                               const int64_t *rank, const int32_t *deg,
+                                                               const int32_t *core, int n, int nnz, int m, int kind,
+                                                               int descending, int db, int kb, int cb, int P,
+                                                               int32_t *ev, int32_t *eu) {
+    extern __shared__ __align__(16) uint32_t s_dyn[];
+    uint64_t *w = (uint64_t *)s_dyn;
+    __shared__ int s_count;
+    if (threadIdx.x == 0) s_count = 0;
+    for (int i = m + (int)threadIdx.x; i < P; i += kSmallThreads) w[i] = ~0ull;
+    __syncthreads();
+    for (int p = threadIdx.x; p < nnz; p += kSmallThreads) {
+        int lo = 0, hi = n;   // last row with off <= p
+        while (hi - lo > 1) {
+            const int mid = (lo + hi) >> 1;
+            if (off[mid] <= p) lo = mid;
+            else hi = mid;
+        }
+        const int32_t c = adj[p];
+        if (c <= lo) continue;
+        uint64_t key = 0;
+        if (kind == PGD_NEIGH_DEG) key = (uint32_t)deg[c];
+        else if (kind == PGD_NEIGH_KCORE) key = (uint32_t)(c >= 1 ? core[c - 1] : 0);
+        uint64_t x = (key << kb) | (uint64_t)rank[p];
+        if (descending) x = ((1ull << (db + kb)) - 1) - x;
+        w[atomicAdd(&s_count, 1)] = ((((uint64_t)lo << (db + kb)) | x) << cb) | (uint64_t)c;
+    }
+    __syncthreads();
+    pgd_block_sort(w, P);
+    for (int i = threadIdx.x; i < m; i += kSmallThreads) {
+        const int32_t r = (int32_t)(w[i] >> (db + kb + cb)), c = (int32_t)(w[i] & ((1ull << cb) - 1));
+        const bool low = deg[r] < deg[c];
+        ev[i] = low ? r : c;
+        eu[i] = low ? c : r;
+    }
+}
+
+// E_ordered of a small graph: (key, id) words, key descending unless s2l, ties by
+// descending id.
+__global__ void __launch_bounds__(kSmallThreads) k_small_order(const int32_t *ev, const int32_t *eu, const int32_t *deg,
+                                                               const int32_t *core, const uint64_t *vsum, int m,
+                                                               int kind, int s2l, int P, int32_t *order) {
+    extern __shared__ __align__(16) uint32_t s_dyn[];
+    uint64_t *w = (uint64_t *)s_dyn;
+    for (int e = threadIdx.x; e < P; e += kSmallThreads) {
+        uint64_t x = ~0ull;
+        if (e < m) {
+            uint32_t key = (uint32_t)edge_key(ev, eu, deg, core, vsum, e, e, kind) ^ 0x80000000u;
+            if (!s2l) key = ~key;
+            x = ((uint64_t)key << 16) | (uint64_t)(0xfffe - e);   // m < 65535; all ones stays last
+        }
+        w[e] = x;
+    }
+    __syncthreads();
+    pgd_block_sort(w, P);
+    for (int i = threadIdx.x; i < m; i += kSmallThreads) order[i] = 0xfffe - (int32_t)(w[i] & 0xffff);
+}
+
+}  // namespace
+
+// A graph of at most kSmallPairs host pairs with ids below n: the pairs go through
+// the context's page-locked buffer, which the kernel reads and answers in.
+static pgd_status build_small(pgd_graph *g, const int32_t *h_src, const int32_t *h_dst, int64_t k, int64_t n, bool dedup) {
+    pgd_ctx *ctx = g->ctx;
+    cudaStream_t s = ctx->stream;
+    pgd_status st;
+    // the buffer's last use was waited for (every fetch is); its second half holds the pairs
+    int32_t *p_src = (int32_t *)(ctx->pin + kPinBytes / 2), *p_dst = p_src + kSmallPairs;
+    memcpy(p_src, h_src, k * sizeof(int32_t));
+    memcpy(p_dst, h_dst, k * sizeof(int32_t));
+    g->n = n;
+    g->rank_limit = k;
+    if ((st = pgd_graph_alloc(g, (void **)&g->off, (n + 1) * sizeof(int64_t)))) return st;
+    if ((st = pgd_graph_alloc(g, (void **)&g->deg, (n + 1) * sizeof(int32_t)))) return st;
+    if ((st = pgd_graph_alloc(g, (void **)&g->vol2, (n + 1) * sizeof(uint64_t)))) return st;
+    // entries: room for every pair, counted against the budget by what is kept
+    int32_t *adj = nullptr;
+    int64_t *rank = nullptr;
+    if ((st = pgd_tmp_alloc(ctx, (void **)&adj, (2 * k + 1) * sizeof(int32_t)))) return st;
+    if ((st = pgd_tmp_alloc(ctx, (void **)&rank, (2 * k + 1) * sizeof(int64_t)))) {
+        pgd_tmp_free(ctx, adj);
+        return st;
+    }
+    g->adj = adj;
+    g->rank = rank;
+    const int cb = std::max(1, bit_length((uint64_t)n)), ib = std::max(1, bit_length((uint64_t)k));
+    const int P = pgd_small_words(2 * k);
+    PGD_LAUNCH(ctx, k_small_build, 1, kSmallThreads, P * sizeof(uint64_t), p_src, p_dst, (int)k, (int)n, cb, ib, P, g->off,
+               adj, rank, g->deg, (SmallResult *)ctx->pin);
+    cudaError_t e = cudaGetLastError();
+    if (e == cudaSuccess) e = cudaStreamSynchronize(s);
+    const SmallResult r = e == cudaSuccess ? pgd_pinned<SmallResult>(ctx, 0) : SmallResult{0, 0, 0};
+    const int64_t valid = 2 * (k - r.loops);
+    g->m = r.nnz / 2;
+    const uint64_t bytes = (2 * (uint64_t)g->m + 1) * (sizeof(int32_t) + sizeof(int64_t));
+    ctx->resident += bytes;
+    g->bytes += bytes;
+    if (e != cudaSuccess) return pgd_cuda_fail(ctx, e, "build of a small graph");
+    if (ctx->resident > ctx->budget)
+        return pgd_fail(ctx, PGD_ENOMEM, "HBM budget of the context exceeded (" + std::to_string(ctx->resident) + " > " +
+                                             std::to_string(ctx->budget) + " bytes)");
+    g->self_loops = r.loops;
+    g->max_degree = r.max_degree;
+    if (r.nnz != valid) {
+        if (!dedup) return pgd_fail(ctx, PGD_EINVAL, "repeated pair without PGD_EDGES_DEDUP (multigraph input)");
+        g->duplicates = (valid - r.nnz) / 2;
+    }
+    return PGD_OK;
+}
+
 // 16-byte words from a mapped host source, then the tail bytes
 __global__ void k_copy_mapped(const uint4 *src, uint4 *dst, int64_t n16, const uint8_t *src_tail, uint8_t *dst_tail,
                               int tail) {
@@ -461,6 +639,17 @@ pgd_status pgd_build_from_pairs(pgd_graph *g, const int32_t *h_src, const int32_
     pgd_ctx *ctx = g->ctx;
     if (k < 0 || k > (int64_t)0x7fffffff) return pgd_fail(ctx, PGD_EINVAL, "pair count out of range (0..2^31-1)");
     pgd_status st;
+    if (k > 0 && k <= kSmallPairs) {
+        int32_t top = -1;   // largest id of an edge
+        bool bad = false;
+        for (int64_t i = 0; i < k; i++) {
+            bad |= (h_src[i] | h_dst[i]) < 0;
+            if (h_src[i] != h_dst[i]) top = std::max(top, std::max(h_src[i], h_dst[i]));
+        }
+        if (bad) return pgd_fail(ctx, PGD_EINVAL, "negative vertex id in edge list");
+        const int64_t n = std::max<int64_t>(n_min, (int64_t)top + 1);
+        if (n > 0 && n <= kSmallVertices) return build_small(g, h_src, h_dst, k, n, dedup);
+    }
     int32_t *d_src = nullptr;
     const int64_t k1 = ((k > 0 ? k : 1) + 63) & ~(int64_t)63;   // both halves 256-byte aligned
     if ((st = pgd_tmp_alloc(ctx, (void **)&d_src, 2 * k1 * sizeof(int32_t)))) return st;
@@ -641,6 +830,16 @@ pgd_status pgd_dev_preprocess(pgd_graph *g, int neigh_kind, int s2l) {
     const int rb = std::max(1, bit_length((uint64_t)g->n)), kb = std::max(1, bit_length((uint64_t)g->rank_limit));
     const int db = neigh_kind == PGD_NEIGH_ASREAD ? 0
                    : std::max(1, bit_length((uint64_t)(neigh_kind == PGD_NEIGH_DEG ? g->max_degree : g->max_core)));
+    if (g->m <= kSmallPairs && g->n <= kSmallVertices && 2 * rb + db + kb <= 63) {
+        const int P = pgd_small_words(g->m);
+        PGD_LAUNCH(ctx, k_small_edges, 1, kSmallThreads, P * sizeof(uint64_t), g->off, g->adj, g->rank, g->deg, g->core,
+                   (int)g->n, (int)nnz, (int)g->m, neigh_kind, (int)descend, db, kb, rb, P, g->ev, g->eu);
+        PGD_CUDA(ctx, cudaGetLastError());
+        g->preprocessed = true;
+        g->sorted = false;
+        g->has_micro = false;
+        return PGD_OK;
+    }
     if (rb + db + kb <= 64) {
         st = rb + db + kb <= 32 ? order_by_words<uint32_t>(g, neigh_kind, descend, rb, db, kb)
                                 : order_by_words<uint64_t>(g, neigh_kind, descend, rb, db, kb);
@@ -1032,7 +1231,13 @@ k_core_block(const int64_t *off, const int32_t *adj, const int32_t *deg, int n, 
 }  // namespace
 
 cudaError_t pgd_build_limits() {
-    return cudaFuncSetAttribute(k_core_block, cudaFuncAttributeMaxDynamicSharedMemorySize, kCoreSmallBytes);
+    constexpr cudaFuncAttribute kDyn = cudaFuncAttributeMaxDynamicSharedMemorySize;
+    constexpr int kSort = 2 * (int)kSmallPairs * 8;
+    cudaError_t e = cudaFuncSetAttribute(k_core_block, kDyn, kCoreSmallBytes);
+    if (e == cudaSuccess) e = cudaFuncSetAttribute(k_small_build, kDyn, kSort);
+    if (e == cudaSuccess) e = cudaFuncSetAttribute(k_small_edges, kDyn, kSort);
+    if (e == cudaSuccess) e = cudaFuncSetAttribute(k_small_order, kDyn, kSort);
+    return e;
 }
 
 static pgd_status cores_by_cluster(pgd_graph *g) {
@@ -1335,7 +1540,11 @@ static pgd_status sort_edges_impl(pgd_graph *g, int kind, int s2l, const int32_t
     const uint32_t flip = small ? 0u : 0x80000000u;
     size_t tb = 0;
     void *tmp = nullptr;
-    if (!d_ids) {
+    if (!d_ids && count <= kSmallPairs) {
+        const int P = pgd_small_words(count);
+        PGD_LAUNCH(ctx, k_small_order, 1, kSmallThreads, P * sizeof(uint64_t), g->ev, g->eu, g->deg, g->core, vsum,
+                   (int)count, kind, s2l, P, g->order);
+    } else if (!d_ids) {
         uint32_t *keys = nullptr, *keys2 = nullptr;
         int32_t *ids = nullptr;
         if (s2l) cub::DeviceRadixSort::SortPairs(nullptr, tb, keys, keys2, ids, g->order, count, 0, kb, s);

@@ -117,7 +117,7 @@ void pgd_rank_drop(pgd_graph *g);   // frees g's rank-ordered copy, if any
 pgd_status pgd_tmp_alloc(pgd_ctx *ctx, void **p, size_t bytes);
 void pgd_tmp_free(pgd_ctx *ctx, void *p);
 
-constexpr size_t kPinBytes = 4096;
+constexpr size_t kPinBytes = 64 << 10;   // the first half for results, the second for a small graph's pairs
 
 // Enqueues the copy of a small device result to page-locked memory; the value is
 // there (pgd_pinned) once the stream has been waited for.  The copy engine writes

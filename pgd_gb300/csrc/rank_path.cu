@@ -72,7 +72,8 @@ enum {
     kCycHash,        // .. kCycHashMax wedges: a block per vertex, hashed counters
     kClasses         // more wedges: items of k_cycle_direct
 };
-constexpr int kEgoMax[] = {32, 256, 512, 1024};
+constexpr int kEgoWarpMax = 32, kEgoAMax = 256, kEgoBMax = 512, kEgoCMax = 1024;
+constexpr int kEgoMax[] = {kEgoWarpMax, kEgoAMax, kEgoBMax, kEgoCMax};
 constexpr int kCycWarpMax = 512;
 constexpr int kCycHashMax = 4096;
 constexpr int kMaxRanges = 8192;
@@ -366,6 +367,177 @@ __global__ void k_rank_lists(const int32_t *rup, const uint32_t *wd, int64_t n, 
     }
     direct = pgd_warp_sum(direct);
     if (lane == 0 && direct) atomicAdd(&M->direct_wedges, direct);
+}
+
+// The whole of the above for a graph of at most 2 kSmallPairs entries and
+// kSmallVertices vertices, by one block: twelve launches of a few microseconds
+// each become one.  Ids take 14 bits.
+constexpr int kSmallIdBits = 14;
+static_assert(kSmallVertices < 1 << kSmallIdBits, "ids of a small graph");
+
+struct RankSmallArgs {
+    const int64_t *off;
+    const int32_t *adj, *deg, *ev, *eu;
+    int n, nnz, m, max_degree;
+    int pv, pe;               // words of the two sorts
+    uint32_t *roff;
+    int32_t *rup;
+    uint32_t *bend;
+    int32_t *radj;
+    uint32_t *wcode;
+    int32_t *tw, *eslot, *lists;
+    unsigned long long *hbase;
+    uint32_t *wd;
+    RankMeta *M, *host;       // the sizes, on the device and in page-locked memory
+};
+inline size_t rank_small_bytes(int n, int pv, int pe) {
+    return (size_t)std::max(pv, pe) * 8 + ((size_t)n + 1) * 8 + (size_t)n * 2 + (size_t)pe * 2 + 16;
+}
+
+__global__ void __launch_bounds__(kSmallThreads) k_rank_small(RankSmallArgs A) {
+    extern __shared__ __align__(16) uint32_t s_dyn[];
+    __shared__ int sh[33];
+    __shared__ uint32_t s_tier[6], s_code[6], s_n[kClasses], s_up, s_pairs;
+    __shared__ unsigned int s_direct;
+    constexpr uint32_t idm = (1u << kSmallIdBits) - 1;
+    constexpr uint32_t lim[6] = {65536, 256, 16, 4, 2, 1};
+    const int n = A.n, nnz = A.nnz, tid = threadIdx.x;
+    uint64_t *w = (uint64_t *)s_dyn;
+    uint32_t *roff = (uint32_t *)(w + max(A.pv, A.pe)), *wd = roff + n + 1;
+    uint16_t *vr = (uint16_t *)(wd + n + 1), *rad = vr + n;
+    if (tid < 6) s_tier[tid] = 0;
+    if (tid < kClasses) s_n[tid] = 0;
+    if (tid == 0) {
+        s_up = s_pairs = 0;
+        s_direct = 0;
+        A.wd[n] = 0;
+    }
+    // ranks and degree tiers
+    for (int v = tid; v < A.pv; v += kSmallThreads)
+        w[v] = v < n ? ((uint64_t)(uint32_t)(A.max_degree - A.deg[v]) << kSmallIdBits) | (uint64_t)(n - 1 - v) : ~0ull;
+    __syncthreads();
+    pgd_block_sort(w, A.pv);
+    for (int i = tid; i < n; i += kSmallThreads) {
+        const uint32_t d = (uint32_t)(A.max_degree - (int)(w[i] >> kSmallIdBits));
+        const uint32_t dn = i + 1 < n ? (uint32_t)(A.max_degree - (int)(w[i + 1] >> kSmallIdBits)) : 0;
+        vr[n - 1 - (int)(w[i] & idm)] = (uint16_t)i;
+        roff[i] = d;
+        wd[i] = 0;
+        A.rup[i] = 0;
+        A.bend[i] = 0;
+        A.wd[i] = 0;
+#pragma unroll
+        for (int t = 0; t < 6; t++)
+            if (d >= lim[t] && dn < lim[t]) s_tier[t] = (uint32_t)i + 1;
+    }
+    __syncthreads();
+    {   // row offsets: each thread a contiguous part
+        const int per = (n + kSmallThreads - 1) / kSmallThreads, b0 = min(n, tid * per), b1 = min(n, b0 + per);
+        int c = 0, total = 0;
+        for (int i = b0; i < b1; i++) c += (int)roff[i];
+        int at = pgd_block_excl_scan(c, sh, &total);
+        for (int i = b0; i < b1; i++) {
+            const int d = (int)roff[i];
+            roff[i] = (uint32_t)at;
+            A.roff[i] = (uint32_t)at;
+            at += d;
+        }
+        if (tid == 0) {
+            roff[n] = (uint32_t)total;
+            A.roff[n] = (uint32_t)total;
+            uint32_t c0 = 0, lo = 0;
+            s_code[0] = 0;
+            for (int t = 0; t < 5; t++) {
+                c0 += (s_tier[t] - lo) << (5 - t);
+                lo = s_tier[t];
+                s_code[t + 1] = c0;
+            }
+        }
+    }
+    // rows in rank order
+    for (int p = tid; p < A.pe; p += kSmallThreads) {
+        uint64_t x = ~0ull;
+        if (p < nnz) {
+            int lo = 0, hi = n;   // last row with off <= p
+            while (hi - lo > 1) {
+                const int mid = (lo + hi) >> 1;
+                if (A.off[mid] <= p) lo = mid;
+                else hi = mid;
+            }
+            x = ((uint64_t)vr[lo] << kSmallIdBits) | vr[A.adj[p]];
+        }
+        w[p] = x;
+    }
+    __syncthreads();
+    pgd_block_sort(w, A.pe);
+    for (int p = tid; p < nnz; p += kSmallThreads) {
+        const uint32_t x = (uint32_t)(w[p] & idm);
+        rad[p] = (uint16_t)x;
+        A.radj[p] = (int32_t)x;
+    }
+    __syncthreads();
+    const uint32_t n2 = s_tier[4];
+    auto find = [&](uint32_t r, uint32_t x) {   // slot of x in row r
+        uint32_t lo = roff[r], hi = roff[r + 1];
+        while (lo < hi) {
+            const uint32_t mid = (lo + hi) >> 1;
+            if (rad[mid] < x) lo = mid + 1;
+            else hi = mid;
+        }
+        return lo;
+    };
+    for (int p = tid; p < nnz; p += kSmallThreads) {
+        const uint32_t r = (uint32_t)(w[p] >> kSmallIdBits), x = rad[p];
+        uint32_t c = s_code[5];
+#pragma unroll
+        for (int i = 4; i >= 0; i--)
+            if (x < s_tier[i]) c = s_code[i] + ((x - (i ? s_tier[i - 1] : 0)) << (5 - i));
+        A.wcode[p] = c;
+        const bool first = (uint32_t)p == roff[r], last = (uint32_t)p + 1 == roff[r + 1];
+        if (x >= n2 ? first || rad[p - 1] < n2 : last) A.bend[r] = (uint32_t)(x >= n2 ? p : p + 1);
+        if (x < r) {
+            const uint32_t s = find(x, r);
+            A.tw[p] = (int32_t)s;
+            A.tw[s] = p;
+            if (last || rad[p + 1] > r) {
+                const uint32_t up = (uint32_t)p + 1 - roff[r];
+                A.rup[r] = (int32_t)up;
+                atomicMax(&s_up, up);
+            }
+        }
+    }
+    for (int e = tid; e < A.m; e += kSmallThreads) {
+        const uint32_t a = vr[A.ev[e]], b = vr[A.eu[e]];
+        A.eslot[e] = (int32_t)find(max(a, b), min(a, b));
+    }
+    __syncthreads();
+    // wedges below each vertex, and the lists
+    for (int p = tid; p < nnz; p += kSmallThreads) {
+        const uint32_t u = (uint32_t)(w[p] >> kSmallIdBits), v = rad[p];
+        if (v > u && v < n2) atomicAdd(wd + u, A.bend[v] - (uint32_t)A.tw[p] - 1);
+    }
+    __syncthreads();
+    for (int x = tid; x < (int)n2; x += kSmallThreads) {
+        const int up = A.rup[x];
+        const uint32_t c = wd[x];
+        const int ec = up < 2 ? -1 : up <= kEgoWarpMax ? 0 : up <= kEgoAMax ? 1 : up <= kEgoBMax ? 2 : up <= kEgoCMax ? 3 : 4;
+        const int cc = c < 2 || c > kCycHashMax ? -1 : c <= kCycWarpMax ? (int)kCycWarp : (int)kCycHash;
+        if (ec >= 0) A.lists[(int64_t)ec * n + atomicAdd(&s_n[ec], 1u)] = x;
+        if (cc >= 0) A.lists[(int64_t)cc * n + atomicAdd(&s_n[cc], 1u)] = x;
+        if (c > kCycHashMax) atomicAdd(&s_direct, c);
+        A.hbase[x] = atomicAdd(&s_pairs, (uint32_t)up * (uint32_t)(up - (up > 0)) / 2);
+        A.wd[x] = c;
+    }
+    __syncthreads();
+    if (tid < 2) {
+        RankMeta *M = tid ? A.host : A.M;
+        for (int i = 0; i < 6; i++) M->tier[i] = s_tier[i];
+        for (int i = 0; i < 5; i++) M->tcode[i] = s_code[i + 1];
+        for (int i = 0; i < kClasses; i++) M->nlist[i] = s_n[i];
+        M->max_up = s_up;
+        M->direct_wedges = s_direct;
+        M->pairs = s_pairs;
+    }
 }
 
 // Ranges [k, end) of u's next item: as many as its counters and its share of
@@ -1449,6 +1621,60 @@ void pgd_rank_drop(pgd_graph *g) {
         }                                                 \
     } while (0)
 
+// Ranks, rows, slots, wedges and lists of a graph of any size; *wd_out, *tmp_out and
+// *tb_out get the wedge counts and CUB's temporary storage, held by tg.
+static pgd_status rank_build_large(pgd_graph *g, int64_t nnz, const int32_t *vgraph, const uint8_t *vmask,
+                                   pgd_rank_graph *R, RankMeta *M, Tmp &tg, uint32_t **wd_out, void **tmp_out,
+                                   size_t *tb_out) {
+    pgd_ctx *ctx = g->ctx;
+    cudaStream_t s = ctx->stream;
+    pgd_status st;
+    const int64_t n = g->n, m = g->m;
+    const size_t nb = (n + 1) * sizeof(uint32_t), eb = nnz * sizeof(uint32_t);
+    uint64_t *keys = nullptr, *keys2 = nullptr;
+    int32_t *vrank = nullptr, *rv = nullptr, *val = nullptr;
+    uint32_t *rdeg = nullptr, *key = nullptr, *key2 = nullptr;
+    const int vb = bits_for(n), db = bits_for((int64_t)g->max_degree + 1);
+    size_t tb1 = 0, tb2 = 0, tb3 = 0;
+    cub::DeviceRadixSort::SortKeys(nullptr, tb1, keys, keys2, n, 0, vb + db, s);
+    cub::DeviceScan::ExclusiveSum(nullptr, tb2, rdeg, R->roff, n + 1, s);
+    cub::DeviceRadixSort::SortPairs(nullptr, tb3, key, key2, val, R->radj, nnz, 0, vb, s);
+    const size_t tb = *tb_out = std::max(tb1, std::max(tb2, tb3));
+    pgd_pieces W;
+    W.add(2 * nb); W.add(2 * nb); W.add(nb); W.add(nb); W.add(nb); W.add(nb); W.add(eb); W.add(eb); W.add(eb); W.add(tb);
+    if ((st = tg.alloc(&W.base, W.bytes))) return st;
+    keys = W.take<uint64_t>(2 * nb);
+    keys2 = W.take<uint64_t>(2 * nb);
+    vrank = W.take<int32_t>(nb);
+    rv = W.take<int32_t>(nb);
+    rdeg = W.take<uint32_t>(nb);
+    uint32_t *wd = *wd_out = W.take<uint32_t>(nb);
+    key = W.take<uint32_t>(eb);
+    key2 = W.take<uint32_t>(eb);
+    val = W.take<int32_t>(eb);
+    void *tmp = *tmp_out = W.take<void>(tb);
+    // ranks and row offsets
+    PGD_LAUNCH(ctx, k_rank_keys2, grid_for(n), kThreads, 0, g->deg, vgraph, vmask, n, g->max_degree, vb, keys, M);
+    PGD_CUDA(ctx, cub::DeviceRadixSort::SortKeys(tmp, *tb_out, keys, keys2, n, 0, vb + db, s));
+    PGD_LAUNCH(ctx, k_rank_scatter2, grid_for(n + 1), kThreads, 0, keys2, n, g->max_degree, vb, vrank, rv, rdeg, R->rup,
+               R->bend, wd, M);
+    PGD_CUDA(ctx, cub::DeviceScan::ExclusiveSum(tmp, *tb_out, rdeg, R->roff, n + 1, s));
+    // rows in rank order
+    PGD_LAUNCH(ctx, k_rank_entries, grid_for(nnz), kThreads, 0, R->roff, rv, g->off, g->adj, vrank, n, nnz, key, val);
+    PGD_CUDA(ctx, cub::DeviceRadixSort::SortPairs(tmp, *tb_out, key, key2, val, R->radj, nnz, 0, vb, s));
+    PGD_LAUNCH(ctx, k_rank_slots, grid_for(nnz), kThreads, 0, R->roff, R->radj, n, nnz, M, R->wcode, R->tw, R->rup,
+               R->bend);
+    PGD_LAUNCH(ctx, k_rank_eslot, grid_for(m), kThreads, 0, g->ev, g->eu, vrank, R->roff, R->rup, R->radj, vgraph,
+               vmask, m, R->eslot);
+    // wedges per vertex and the work lists
+    PGD_LAUNCH(ctx, k_rank_wedges, grid_for(nnz), kThreads, 0, R->roff, R->radj, R->tw, R->bend, n, M, wd);
+    PGD_LAUNCH(ctx, k_rank_lists, grid_for(n), kThreads, 0, R->rup, wd, n, R->lists, R->hbase, M);
+    PGD_CUDA(ctx, cudaGetLastError());
+    PGD_CUDA(ctx, pgd_fetch(ctx, 0, M, offsetof(RankMeta, bound)));
+    PGD_CUDA(ctx, cudaStreamSynchronize(s));
+    return PGD_OK;
+}
+
 // Blocks of k_cycle_direct per SM: as many as all counters fit in.
 static int direct_factor(int64_t words) { return words < kDirectWords / 4 ? 4 : words < kDirectWords / 2 ? 2 : 1; }
 
@@ -1486,50 +1712,48 @@ pgd_status pgd_rank_build(pgd_graph *g, int64_t nnz, const int32_t *vgraph, cons
     R->eslot = K.take<int32_t>(mb);
     R->lists = K.take<int32_t>(lb);
     R->hbase = K.take<unsigned long long>(hb);
-    // and the temporaries in another
     Tmp tg(ctx);
-    uint64_t *keys = nullptr, *keys2 = nullptr;
-    int32_t *vrank = nullptr, *rv = nullptr, *val = nullptr;
-    uint32_t *rdeg = nullptr, *key = nullptr, *key2 = nullptr, *wd = nullptr;
-    const int vb = bits_for(n), db = bits_for((int64_t)g->max_degree + 1);
-    size_t tb1 = 0, tb2 = 0, tb3 = 0;
-    cub::DeviceRadixSort::SortKeys(nullptr, tb1, keys, keys2, n, 0, vb + db, s);
-    cub::DeviceScan::ExclusiveSum(nullptr, tb2, rdeg, R->roff, n + 1, s);
-    cub::DeviceRadixSort::SortPairs(nullptr, tb3, key, key2, val, R->radj, nnz, 0, vb, s);
-    size_t tb = std::max(tb1, std::max(tb2, tb3));
-    pgd_pieces W;
-    W.add(2 * nb); W.add(2 * nb); W.add(nb); W.add(nb); W.add(nb); W.add(nb); W.add(eb); W.add(eb); W.add(eb); W.add(tb);
-    RB_TRY(tg.alloc(&W.base, W.bytes));
-    keys = W.take<uint64_t>(2 * nb);
-    keys2 = W.take<uint64_t>(2 * nb);
-    vrank = W.take<int32_t>(nb);
-    rv = W.take<int32_t>(nb);
-    rdeg = W.take<uint32_t>(nb);
-    wd = W.take<uint32_t>(nb);
-    key = W.take<uint32_t>(eb);
-    key2 = W.take<uint32_t>(eb);
-    val = W.take<int32_t>(eb);
-    void *tmp = W.take<void>(tb);
-    // ranks and row offsets
-    PGD_LAUNCH(ctx, k_rank_keys2, grid_for(n), kThreads, 0, g->deg, vgraph, vmask, n, g->max_degree, vb, keys, M);
-    RB_CUDA(cub::DeviceRadixSort::SortKeys(tmp, tb, keys, keys2, n, 0, vb + db, s));
-    PGD_LAUNCH(ctx, k_rank_scatter2, grid_for(n + 1), kThreads, 0, keys2, n, g->max_degree, vb, vrank, rv, rdeg, R->rup,
-               R->bend, wd, M);
-    RB_CUDA(cub::DeviceScan::ExclusiveSum(tmp, tb, rdeg, R->roff, n + 1, s));
-    // rows in rank order
-    PGD_LAUNCH(ctx, k_rank_entries, grid_for(nnz), kThreads, 0, R->roff, rv, g->off, g->adj, vrank, n, nnz, key, val);
-    RB_CUDA(cub::DeviceRadixSort::SortPairs(tmp, tb, key, key2, val, R->radj, nnz, 0, vb, s));
-    PGD_LAUNCH(ctx, k_rank_slots, grid_for(nnz), kThreads, 0, R->roff, R->radj, n, nnz, M, R->wcode, R->tw, R->rup,
-               R->bend);
-    PGD_LAUNCH(ctx, k_rank_eslot, grid_for(m), kThreads, 0, g->ev, g->eu, vrank, R->roff, R->rup, R->radj, vgraph,
-               vmask, m, R->eslot);
-    // wedges per vertex and the work lists
-    PGD_LAUNCH(ctx, k_rank_wedges, grid_for(nnz), kThreads, 0, R->roff, R->radj, R->tw, R->bend, n, M, wd);
-    PGD_LAUNCH(ctx, k_rank_lists, grid_for(n), kThreads, 0, R->rup, wd, n, R->lists, R->hbase, M);
+    uint32_t *wd = nullptr;
+    void *tmp = nullptr;
+    size_t tb = 0;
+    if (!vgraph && nnz <= 2 * kSmallPairs && n <= kSmallVertices) {
+        RankSmallArgs A{};
+        A.off = g->off;
+        A.adj = g->adj;
+        A.deg = g->deg;
+        A.ev = g->ev;
+        A.eu = g->eu;
+        A.n = (int)n;
+        A.nnz = (int)nnz;
+        A.m = (int)m;
+        A.max_degree = g->max_degree;
+        A.pv = pgd_small_words(n);
+        A.pe = pgd_small_words(nnz);
+        A.roff = R->roff;
+        A.rup = R->rup;
+        A.bend = R->bend;
+        A.radj = R->radj;
+        A.wcode = R->wcode;
+        A.tw = R->tw;
+        A.eslot = R->eslot;
+        A.lists = R->lists;
+        A.hbase = R->hbase;
+        A.M = M;
+        A.host = (RankMeta *)ctx->pin;
+        cub::DeviceScan::ExclusiveSum(nullptr, tb, wd, wd, n + 1, s);
+        pgd_pieces W;
+        W.add(nb); W.add(tb);
+        RB_TRY(tg.alloc(&W.base, W.bytes));
+        A.wd = wd = W.take<uint32_t>(nb);
+        tmp = W.take<void>(tb);
+        PGD_LAUNCH(ctx, k_rank_small, 1, kSmallThreads, rank_small_bytes((int)n, A.pv, A.pe), A);
+        RB_CUDA(cudaGetLastError());
+        RB_CUDA(cudaStreamSynchronize(s));
+    } else {
+        RB_TRY(rank_build_large(g, nnz, vgraph, vmask, R, M, tg, &wd, &tmp, &tb));
+    }
     constexpr size_t kHead = offsetof(RankMeta, bound);
     static_assert(kHead <= kPinBytes, "the sizes fit the read-back buffer");
-    RB_CUDA(pgd_fetch(ctx, 0, M, kHead));
-    RB_CUDA(cudaStreamSynchronize(s));
     RankMeta h;
     memcpy((void *)&h, ctx->pin, kHead);
     const int n2 = R->n2 = (int32_t)h.tier[4];
@@ -1635,6 +1859,9 @@ static void ego_pass(pgd_ctx *ctx, const pgd_rank_graph &R, EgoArgs A, int pass,
 cudaError_t pgd_rank_limits() {
     constexpr cudaFuncAttribute kDyn = cudaFuncAttributeMaxDynamicSharedMemorySize;
     cudaError_t e = cudaFuncSetAttribute(k_cycle_direct<1024>, kDyn, kDirectWords * 4);
+    if (e == cudaSuccess)
+        e = cudaFuncSetAttribute(k_rank_small, kDyn,
+                                 (int)rank_small_bytes((int)kSmallVertices, (int)kSmallVertices, 2 * (int)kSmallPairs));
     if (e == cudaSuccess) e = cudaFuncSetAttribute(k_cycle_direct<512>, kDyn, kDirectWords * 2);
     if (e == cudaSuccess) e = cudaFuncSetAttribute(k_cycle_direct<256>, kDyn, kDirectWords);
     if (e == cudaSuccess) e = cudaFuncSetAttribute(k_cycle_hash, kDyn, kHashSmem);
