@@ -2512,8 +2512,13 @@ static size_t hub_layout(int64_t n, int32_t nhubs, int32_t nwide, int32_t max_de
 
 // A sample of fewer than one edge in kSampleShare is decomposed edge by edge
 // (run_decompose), everything else by the passes of rank_path.cu, whose cost
-// does not depend on the number of edges asked for.
-constexpr int64_t kSampleShare = 64;
+// does not depend on the number of edges asked for.  Microseconds for order and
+// counts of 1/2000, 1/500 and 1/66 of the edges, edge by edge against whole-graph:
+// RMAT-16 2151, 2298, 2609 / 699, 702, 771; RMAT-20 39110, 55900, 83642 / 32673,
+// 32721, 32978; 1M-vertex BA 3257, 3452, 3909 / 1315, 1334, 1422; rgg-20 4345,
+// 4368, 4714 / 3333, 3336, 3466; dense G(1000, 0.5) 636, 790, 1107 / 992, 926,
+// 968.  At 1/10000 RMAT-20 takes 27447 / 32621.
+constexpr int64_t kSampleShare = 2048;
 
 // Device times of one decomposition: all kernels, the triangle pass, k_hub.
 struct StageMs {

@@ -76,7 +76,7 @@ def test_random_graphs_match_the_oracle(ctx, kind, order):
     assert (x == ox).all() and (y == oy).all() and (cols == ocols).all()
 
 
-@pytest.mark.parametrize("share", [0.005, 0.014, 0.017, 0.5])
+@pytest.mark.parametrize("share", [0.0003, 0.0006, 0.005, 0.014, 0.017, 0.5])
 def test_sample_rows_equal_the_full_run(ctx, share):
     """Samples below and above the share of edges from which the passes over
     the whole graph are taken give the same rows."""
