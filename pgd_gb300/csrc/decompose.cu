@@ -1407,42 +1407,63 @@ __global__ void __launch_bounds__(256, 3) k_dense_cn(DenseCnArgs A) {
 // and skipped (with full rows 2·k4 came out, for twice the products).  0/1 entries are exact in e4m3 and every fp32 sum stays below
 // 2^24 (d_q <= kTcMaxDeg), so the counts are exact.
 //
-// One CTA of 16 warps per SM takes runs from a counter.  Per run: the rows of
-// N(q), compacted to N(q)'s columns (a software bit-compress per 64-bit word,
-// the "compress" of Hacker's Delight §7-4 with its masks computed once per word
-// of A_q), go to shared memory.  Then for each pair of 128-edge tiles and each
-// 256-row tile of N(q), every 64-column chunk is expanded to e4m3 tiles (one B
-// tile shared by both edge tiles) by 15 builder warps into one of two
-// alternating stages while the tensor cores run the previous chunk's MMAs,
-// which one thread of the last warp issues into two TMEM accumulators.  The
-// builders and the issuing thread meet at per-stage mbarriers only: "full"
-// (every builder warp arrived) and "empty" (tcgen05.commit of the MMAs that
-// read the stage); at the end of a row tile every warp reads back one
-// accumulator quarter (a row per thread) and dots it with the rows' own
-// compact bits.  A one is encoded as 2^-6 (0x08), so that a nibble spreads to
-// four bytes in two instructions; all sums are multiples of 2^-12 below 2^9,
-// exact in fp32.
+// One CTA of 17 warps per SM takes runs from a counter.  Per run: the rows of
+// N(q), compacted to N(q)'s columns, go to shared memory; A being symmetric, they
+// are 32 x 32 bit blocks of N(q)'s rows transposed, of which N(q)'s columns are
+// kept.  Then for each pair of 128-edge tiles and each 256-row tile of N(q), every
+// 64-column chunk is expanded to e4m3 tiles (one B tile shared by both edge tiles)
+// by 16 builder warps into one of two alternating stages while the tensor cores
+// run the previous chunk's MMAs, which one thread of the last warp issues into two
+// TMEM accumulators.  The builders and the issuing thread meet at per-stage
+// mbarriers only: "full" (every builder warp arrived) and "empty" (tcgen05.commit
+// of the MMAs that read the stage); at the end of a row tile every warp reads back
+// one accumulator quarter (a row per thread) and dots it with the rows' own
+// compact bits.  A one is encoded as 2 (0x40) and the columns of a 32-bit word are
+// taken in the order of its bytes' bits, so that four bytes are a shift and an AND;
+// all sums are multiples of 4 below 2^24, exact in fp32.
+//
+// Builders start on the next row tile's stages before they read back the last
+// one's accumulators.  Of the time on 131 graphs of up to 2048 vertices about two
+// thirds go to the stages, a quarter to the compaction and the rest to the
+// read-back; the bound is the integer work of building the operands (the tensor
+// cores are busy for about 0.4 of it), not a memory.  27.5 -> 24.6 ms with the
+// products below the diagonal only, -> 21.9 ms with transposes instead of bit
+// compression and word-wise spreading, the next run fetched in advance and records
+// of the runs, -> 18.5 ms with as many 64-column stages as fit and two builder
+// groups (32-column stages with four groups: 25 ms, the issuing thread's 470 cycles
+// per stage), -> 17.2 ms with the compaction's targets kept in registers and the
+// stages built ahead.
 
-constexpr int kTcThreads = 512;
-constexpr int kTcBuilders = 15;            // warps that expand operand tiles; the last warp issues the MMAs
+constexpr int kTcBuilders = 16;            // warps that expand operand tiles; one more issues the MMAs
+constexpr int kTcThreads = 32 * (kTcBuilders + 1);
 constexpr int kTcM = 128;                  // edges per tile (TMEM lanes); two tiles per pass
 constexpr int kTcN = 256;                  // ego rows per tile (TMEM columns per accumulator)
-constexpr int kTcK = 64;                   // ego columns per stage: one compact word
+constexpr int kTcK = 64;                   // ego columns per stage: one compact word, two MMAs per edge tile
 constexpr int kTcMaxDeg = 1088;            // largest d_q whose compacted ego network fits shared memory
 constexpr int kTcMaxWords = kTcMaxDeg / 64;
 constexpr int kTcStageBytes = (2 * kTcM + kTcN) * kTcK;   // A tiles of both edge tiles, then B
-constexpr int kTcSmem = 2 * kTcStageBytes + kTcMaxDeg * kTcMaxWords * 8 + 1024;
+constexpr int kTcMaxStages = 6;
+constexpr int kTcGroups = 2;               // of builder warps, which take the stages in turn
+constexpr int kTcGroup = 32 * kTcBuilders / kTcGroups;
+constexpr int kTcSmem = 218 * 1024;        // compact rows first, then 1024-byte aligned stages in what is left
 constexpr long long kTcWaitCycles = 1ll << 30;   // about half a second: a wait that long has failed
 static_assert(kTcStageBytes % 1024 == 0, "stage tiles stay 1024-byte aligned");
 static_assert(kTcMaxDeg % 64 == 0, "whole compact words");
+static_assert(kTcGroup == 2 * kTcM && kTcN == 2 * kTcM, "an A and a B row per builder thread");
+// a group waits for the MMAs of its stage's last use: with fewer stages than groups
+// it could be two uses behind, which a phase bit cannot tell
+static_assert(kTcMaxDeg * (kTcMaxWords | 1) * 8 + kTcGroups * kTcStageBytes + 2048 <= kTcSmem, "stages for every group");
+
+struct TcRun {
+    int64_t first, last;   // its edges: places among the CN-graph edges, one past the last
+    int64_t vbase, wbase;  // its graph's first vertex and first bit word
+    int32_t q, W;          // q within the graph, words per row
+};
 
 struct DenseTcArgs {
-    DevGraph G;
     const uint64_t *bits;
-    const int64_t *wbase;
-    const int64_t *vbase;
-    const int32_t *dpos;                // positions of the CN-graph edges, grouped by q
-    const int64_t *runs;                // per run taken: {first, one past last} position
+    const uint16_t *ends;               // per CN-graph edge (grouped by q): the other endpoint, within the graph
+    const TcRun *runs;
     const unsigned long long *nruns;
     uint32_t *k4;                       // per position: k4 (left at 0xffffffff outside the runs)
     unsigned long long *next;
@@ -1476,82 +1497,125 @@ __global__ void k_tc_rest_fill(const int32_t *dpos, const uint32_t *flag, const 
     if (blockIdx.x == 0 && threadIdx.x == 0) *nrest = pos[ncn];
 }
 
-__global__ void k_tc_run_fill(const uint32_t *keys, const uint32_t *flag, const uint32_t *pos, int64_t ncn,
-                              int64_t *runs, unsigned long long *nruns) {
+// the runs taken, and the other endpoint of every CN-graph edge
+__global__ void k_tc_run_fill(DevGraph G, const int32_t *dpos, const uint32_t *keys, const uint32_t *flag,
+                              const uint32_t *pos, const int64_t *vbase, const int64_t *wbase, int64_t ncn, TcRun *runs,
+                              uint16_t *ends, unsigned long long *nruns) {
     for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < ncn; i += (int64_t)gridDim.x * blockDim.x) {
-        if (!flag[i]) continue;
         const uint32_t q = keys[i];
+        const int32_t e = dpos[i], id = G.order[e], g = G.egraph[e];
+        const int32_t v = G.ev[id], u = G.eu[id];
+        const int64_t vb = vbase[g];
+        ends[i] = (uint16_t)((v == (int32_t)q ? u : v) - vb);
+        if (!flag[i]) continue;
         int64_t lo = i + 1, hi = ncn;   // one past the run's last position
         while (lo < hi) {
             const int64_t mid = (lo + hi) >> 1;
             if (keys[mid] == q) lo = mid + 1; else hi = mid;
         }
-        runs[2 * pos[i]] = i;
-        runs[2 * pos[i] + 1] = lo;
+        runs[pos[i]] = TcRun{i, lo, vb, wbase[g], (int32_t)((int64_t)q - vb), (int32_t)((G.gnm[2 * g] + 63) >> 6)};
     }
     if (blockIdx.x == 0 && threadIdx.x == 0) *nruns = pos[ncn];
 }
 
-// masks of the compress of Hacker's Delight §7-4 (bits of x at the set bits of
-// m, packed to the low end), for repeated use with one m
-__device__ __forceinline__ void tc_compress_masks(uint64_t m, uint64_t mv[6]) {
-    uint64_t mk = ~m << 1;
+// word (lane & 3) of rows i of the lane's quad in v[i] -> words k of row (lane & 3)
+// in x[2k], x[2k + 1]
+__device__ __forceinline__ void tc_quad_exchange(uint2 v[4], int lane, uint32_t x[8]) {
 #pragma unroll
-    for (int i = 0; i < 6; i++) {
-        uint64_t mp = mk ^ (mk << 1);
-        mp ^= mp << 2;
-        mp ^= mp << 4;
-        mp ^= mp << 8;
-        mp ^= mp << 16;
-        mp ^= mp << 32;
-        const uint64_t v = mp & m;
-        mv[i] = v;
-        m = (m ^ v) | (v >> (1 << i));
-        mk &= ~mp;
+    for (int b = 1; b <= 2; b <<= 1) {
+        const bool hi = lane & b;
+#pragma unroll
+        for (int i = 0; i < 4; i++) {
+            if (i & b) continue;
+            uint2 t = hi ? v[i] : v[i | b];
+            t.x = __shfl_xor_sync(0xffffffffu, t.x, b);
+            t.y = __shfl_xor_sync(0xffffffffu, t.y, b);
+            if (hi) v[i] = t;
+            else v[i | b] = t;
+        }
+    }
+#pragma unroll
+    for (int k = 0; k < 4; k++) {
+        x[2 * k] = v[k].x;
+        x[2 * k + 1] = v[k].y;
     }
 }
 
-__device__ __forceinline__ uint64_t tc_compress(uint64_t x, uint64_t m, const uint64_t mv[6]) {
-    x &= m;
+// eight blocks of 32 x 32 bits, each one row per lane -> one column per lane, in
+// five exchanges of 32/2^i-bit halves (the first two of whole bytes)
+__device__ __forceinline__ void tc_transpose32(uint32_t x[8], int lane) {
+    constexpr uint32_t low[3] = {0x0f0f0f0fu, 0x33333333u, 0x55555555u};
+    const uint32_t pick16 = lane & 16 ? 0x3276u : 0x5410u, pick8 = lane & 8 ? 0x3715u : 0x6240u;
 #pragma unroll
-    for (int i = 0; i < 6; i++) {
-        const uint64_t t = x & mv[i];
-        x = (x ^ t) | (t >> (1 << i));
+    for (int i = 0; i < 2; i++) {
+        uint32_t o[8];
+#pragma unroll
+        for (int k = 0; k < 8; k++) o[k] = __shfl_xor_sync(0xffffffffu, x[k], 16 >> i);
+#pragma unroll
+        for (int k = 0; k < 8; k++) x[k] = __byte_perm(x[k], o[k], i ? pick8 : pick16);
     }
-    return x;
+#pragma unroll
+    for (int i = 0; i < 3; i++) {
+        const int w = 4 >> i;
+        const bool hi = lane & w;
+        const uint32_t keep = hi ? ~low[i] : low[i];
+        uint32_t o[8];
+#pragma unroll
+        for (int k = 0; k < 8; k++) o[k] = __shfl_xor_sync(0xffffffffu, x[k], w);
+#pragma unroll
+        for (int k = 0; k < 8; k++) x[k] = (x[k] & keep) | (__funnelshift_l(o[k], o[k], hi ? 32 - w : w) & ~keep);
+    }
 }
 
-// four bits -> four e4m3 bytes, 2^-6 (0x08) where the bit is set: the
-// product places bit i of nib at bit 8i + 3, and no two shifted copies overlap
-__device__ __forceinline__ uint32_t tc_spread4(uint32_t nib) { return (nib * 0x01020408u) & 0x08080808u; }
+// bits i, i + 8, i + 16, i + 24 of x as four e4m3 bytes: 2 (0x40) where set
+__device__ __forceinline__ uint32_t tc_spread(uint32_t x, int i) {
+    return (i <= 6 ? x << (6 - i) : x >> 1) & 0x40404040u;
+}
 
 __global__ void __launch_bounds__(kTcThreads, 1) k_dense_tc(DenseTcArgs A) {
-    extern __shared__ uint8_t tc_smem[];
+    extern __shared__ __align__(16) uint8_t tc_smem[];
     __shared__ uint64_t s_m[32];          // A_q, per word
-    __shared__ uint64_t s_mv[32][6];      // compress masks per word of A_q
+    __shared__ uint64_t s_mnext[32];      // the same of the next run
     __shared__ int32_t s_o[33];           // compact offset of each word (prefix of popcounts)
-    __shared__ uint16_t s_col[kTcMaxDeg]; // N(q), ascending
+    __shared__ __align__(8) uint16_t s_col[kTcMaxDeg + 32];   // N(q), ascending
+    __shared__ uint16_t s_p[2][2 * kTcM];   // this and the next run: the other endpoints of the first pass's edges
     __shared__ int16_t s_jrow[2][kTcM];   // compact row of each edge's p in the pass, -1 past the run
     __shared__ float s_part[2][2][kTcM];  // per edge tile and column half
     __shared__ uint32_t s_taddr;
-    __shared__ __align__(8) uint64_t s_full[2];
-    __shared__ __align__(8) uint64_t s_empty[2];
-    __shared__ long long s_run;
+    __shared__ __align__(8) uint64_t s_full[kTcMaxStages];
+    __shared__ __align__(8) uint64_t s_empty[kTcMaxStages];
+    __shared__ __align__(8) uint64_t s_done, s_read;   // a tile's accumulators complete, read back
+    __shared__ TcRun s_next;              // the next run (first -1: none)
     __shared__ int s_abort;
     using namespace pgd_tc;
-    const DevGraph &G = A.G;
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
-    // 1024-aligned stages, then the compacted ego rows
-    uint8_t *base = tc_smem + ((1024u - (smem_addr(tc_smem) & 1023u)) & 1023u);
-    uint64_t *C = (uint64_t *)(base + 2 * kTcStageBytes);
+    uint64_t *C = (uint64_t *)tc_smem;
     if (warp == 0) tmem_alloc(&s_taddr, 2 * kTcN);
     if (tid == 0) {
-        for (int i = 0; i < 2; i++) {
-            mbar_init(&s_full[i], kTcBuilders);
+        for (int i = 0; i < kTcMaxStages; i++) {
+            mbar_init(&s_full[i], kTcBuilders / kTcGroups);
             mbar_init(&s_empty[i], 1);
         }
+        mbar_init(&s_done, 1);
+        mbar_init(&s_read, kTcBuilders);
         s_abort = 0;
     }
+    const int64_t nruns = (int64_t)*A.nruns;
+    // the last warp fetches the run that comes next, A_q of its q and its first
+    // edges while the others compact
+    auto fetch_run = [&](int buf) {
+        int64_t r = 0;
+        if (lane == 0) r = (int64_t)atomicAdd(A.next, 1ull);
+        r = __shfl_sync(0xffffffffu, r, 0);
+        TcRun R{-1, -1, 0, 0, 0, 0};
+        if (r < nruns) R = A.runs[r];
+        if (lane == 0) s_next = R;
+        s_mnext[lane] = lane < R.W ? __ldg(A.bits + R.wbase + (int64_t)R.q * R.W + lane) : 0ull;
+#pragma unroll
+        for (int k = 0; k < 2 * kTcM / 32; k++)
+            s_p[buf][32 * k + lane] = R.first + 32 * k + lane < R.last ? A.ends[R.first + 32 * k + lane] : (uint16_t)0;
+    };
+    if (warp == kTcBuilders) fetch_run(0);
     fence_before_sync();
     __syncthreads();
     fence_after_sync();
@@ -1560,35 +1624,17 @@ __global__ void __launch_bounds__(kTcThreads, 1) k_dense_tc(DenseTcArgs A) {
     const int et = warp >> 3, eh = (warp >> 2) & 1, erow = 32 * (warp & 3) + lane;
     const uint32_t etaddr = tmem + ((uint32_t)(32 * (warp & 3)) << 16) + (uint32_t)(et * kTcN);
     const bool issuer = warp == kTcBuilders && lane == 0;
-    int chunk = 0;      // chunks so far: chunk c uses stage c & 1 for the (c >> 1)-th time
-    int last = -1;      // issuer: the last chunk committed
+    uint32_t phase = 0;   // bit i: parity of stage i's next use (builders and issuer alike)
+    uint32_t tile = 0;    // row tiles so far (builders and issuer alike)
+    int last = -1;        // issuer: the stage committed last, if its commit is not yet waited for
     bool bad = false;
-    const int64_t nruns = (int64_t)*A.nruns;
-    while (true) {
-        if (tid == 0) s_run = (long long)atomicAdd(A.next, 1ull);
-        __syncthreads();
-        const int64_t r = s_run;
-        __syncthreads();
-        if (r >= nruns) break;
-        const int64_t i0 = A.runs[2 * r], i1 = A.runs[2 * r + 1];
-        const int32_t qg = dense_q(G, A.dpos[i0]);
-        const int g = G.egraph[A.dpos[i0]];
-        const int64_t vb = A.vbase[g];
-        const int W = (int)((G.gnm[2 * g] + 63) >> 6);
-        const uint64_t *rows = A.bits + A.wbase[g];
-        const int64_t q = qg - vb;
-        // the first pass's edges: their other endpoints p, loaded by the upper
-        // half of the CTA now, so that the latency of the chain hides under the
-        // set-up (warp 0) and the compaction
-        const int ptid = tid - (kTcThreads - 2 * kTcM);   // this thread's edge of the first pass, if >= 0
-        int pfirst = 0;
-        if (ptid >= 0 && ptid < (int)(i1 - i0)) {
-            const int32_t id = G.order[A.dpos[i0 + ptid]];
-            const int32_t v = G.ev[id], u = G.eu[id];
-            pfirst = (int)((v == qg ? u : v) - vb);
-        }
+    for (int run = 0;; run++) {
+        const int64_t i0 = s_next.first;
+        const int rr = (int)(s_next.last - i0), W = s_next.W;
+        const uint64_t *rows = A.bits + s_next.wbase;
+        if (i0 < 0) break;
         if (warp == 0) {
-            const uint64_t mq = lane < W ? __ldg(rows + q * W + lane) : 0ull;
+            const uint64_t mq = s_mnext[lane];
             const int c = __popcll(mq);
             int o = c;
 #pragma unroll
@@ -1600,18 +1646,22 @@ __global__ void __launch_bounds__(kTcThreads, 1) k_dense_tc(DenseTcArgs A) {
             s_m[lane] = mq;
             s_o[lane] = o;
             if (lane == 31) s_o[32] = o + c;
-            uint64_t mv[6];
-            tc_compress_masks(mq, mv);
-#pragma unroll
-            for (int i = 0; i < 6; i++) s_mv[lane][i] = mv[i];
         }
         __syncthreads();
+        if (warp == kTcBuilders) fetch_run((run + 1) & 1);
         const int d = s_o[32];   // = deg(q), which the run flags bound; a run beyond the
-        if (d > kTcMaxDeg) continue;   // shared-memory limit is left to k_dense_cn
+        if (d > kTcMaxDeg) {     // shared-memory limit is left to k_dense_cn
+            __syncthreads();
+            continue;
+        }
         // compact words per ego row, and the row stride: odd, so that the
         // rows a warp reads together fall in different banks
         const int KW = (d + 63) >> 6, KS = KW | 1;
-        // N(q) in ascending order (four bits of A_q per thread) and the compact rows cleared
+        // the stages behind the compact rows: few columns leave room for more of them
+        const uint32_t sbase = (smem_addr(C) + (uint32_t)(d * KS * 8) + 1023u) & ~1023u;
+        uint8_t *const stages = tc_smem + (sbase - smem_addr(tc_smem));
+        const int nst = min(kTcMaxStages, (int)(smem_addr(tc_smem) + kTcSmem - sbase) / kTcStageBytes);
+        // N(q) in ascending order (four bits of A_q per thread)
         for (int t = tid; t < 32 * 16; t += kTcThreads) {
             const int w = t >> 4, b0 = 4 * (t & 15);
             const uint64_t mw = s_m[w];
@@ -1622,199 +1672,185 @@ __global__ void __launch_bounds__(kTcThreads, 1) k_dense_tc(DenseTcArgs A) {
                 nib &= nib - 1;
             }
         }
-        for (int i = tid; i < d * KS; i += kTcThreads) C[i] = 0ull;
         __syncthreads();
-        {   // C[j] = compact(A_{col[j]}), lane = word of the uncompacted row; eight rows in
-            // flight.  Lane w's compressed bits start at bit ow of the compact row, in word
-            // w0; the lanes starting in one word form a contiguous segment, and only the
-            // segment's last lane can spill into the next word.  A segmented OR-scan over
-            // the lanes assembles each word in its segment's last lane: no atomics.
-            uint64_t mv[6];
+        const int W4 = (W + 3) >> 2, lines = kTcBuilders / W4;
+        if (warp < lines * W4) {
+            // C by symmetry: the column words of 32 rows of N(q), one row per lane,
+            // transposed; each column of N(q) is then 32 bits of its own compact row.
+            // A warp keeps to four 64-bit words, so that the rows its lanes write stay
+            // the same, and goes down the rows, eight transposes interleaved.  Four
+            // lanes read a sector of one row together, then exchange words.
+            uint32_t *C32 = (uint32_t *)C;
+            const int w0 = 4 * (warp % W4), wl = w0 + (lane & 3);
+            const uint32_t below = (1u << lane) - 1;
+            int to[8];   // the compact row of this lane's column, -1 if it is none of N(q)'s
 #pragma unroll
-            for (int i = 0; i < 6; i++) mv[i] = s_mv[lane][i];
-            const uint64_t mw = s_m[lane];
-            const int ow = s_o[lane], cw = __popcll(mw), sh = ow & 63, w0 = ow >> 6;
-            const bool spills = sh && sh + cw > 64;
-            const int w0prev = __shfl_up_sync(0xffffffffu, w0, 1), w0next = __shfl_down_sync(0xffffffffu, w0, 1);
-            const bool first = lane == 0 || w0prev != w0, lastl = lane == 31 || w0next != w0;
-            unsigned same = 0;   // bit i: lane - 2^i is in this lane's segment
-#pragma unroll
-            for (int i = 0; i < 5; i++) {
-                const int o2 = __shfl_up_sync(0xffffffffu, w0, 1 << i);
-                if (lane >= (1 << i) && o2 == w0) same |= 1u << i;
+            for (int k = 0; k < 4; k++) {
+                const uint64_t mw = s_m[w0 + k];   // zero from W on
+                const int o = s_o[w0 + k];
+                const uint32_t ml = (uint32_t)mw, mh = (uint32_t)(mw >> 32);
+                to[2 * k] = (ml >> lane) & 1u ? (o + __popc(ml & below)) * 2 * KS : -1;
+                to[2 * k + 1] = (mh >> lane) & 1u ? (o + __popc(ml) + __popc(mh & below)) * 2 * KS : -1;
             }
-            constexpr int kWarps = kTcThreads / 32, kFly = 8;
-            for (int jb = warp; jb < d; jb += kFly * kWarps) {
-                uint64_t w[kFly];
+            for (int yb = warp / W4; yb < 2 * KW; yb += lines) {
+                const int y0 = 32 * yb + (lane & ~3);
+                const uint64_t cols = *(const uint64_t *)(s_col + y0);
+                uint2 v[4];
 #pragma unroll
-                for (int k = 0; k < kFly; k++) {
-                    const int j = jb + k * kWarps;
-                    w[k] = (cw && j < d) ? __ldg(rows + (int64_t)s_col[j] * W + lane) : 0ull;
+                for (int i = 0; i < 4; i++) {
+                    const int c = (int)((cols >> (16 * i)) & 0xffff);
+                    v[i] = y0 + i < d && wl < W ? __ldg((const uint2 *)rows + c * W + wl) : make_uint2(0u, 0u);
                 }
+                uint32_t x[8];
+                tc_quad_exchange(v, lane, x);
+                tc_transpose32(x, lane);
 #pragma unroll
-                for (int k = 0; k < kFly; k++) {
-                    const int j = jb + k * kWarps;   // uniform over the warp
-                    if (j >= d) break;
-                    const uint64_t v = cw ? tc_compress(w[k], mw, mv) : 0ull;
-                    const uint64_t hi = spills ? v >> (64 - sh) : 0ull;
-                    const uint64_t hprev = __shfl_up_sync(0xffffffffu, hi, 1);
-                    uint64_t val = (v << sh) | (first && lane > 0 ? hprev : 0ull);
-#pragma unroll
-                    for (int i = 0; i < 5; i++) {
-                        const uint64_t t = __shfl_up_sync(0xffffffffu, val, 1 << i);
-                        if ((same >> i) & 1u) val |= t;
-                    }
-                    if (lastl && w0 < KW) C[j * KS + w0] = val;
-                    if (lane == 31 && hi) C[j * KS + w0 + 1] = hi;
-                }
+                for (int k = 0; k < 8; k++)
+                    if (to[k] >= 0) C32[to[k] + yb] = x[k];
             }
         }
-        const int rr = (int)(i1 - i0);
-        for (int m0 = 0; m0 < rr && !bad; m0 += 2 * kTcM) {
+        int st = 0;   // next stage: all are idle between runs
+        for (int m0 = 0; m0 < rr; m0 += 2 * kTcM) {
             const int ntiles = rr - m0 > kTcM ? 2 : 1;   // edge tiles of this pass
             __syncthreads();   // C complete; the previous pass's s_jrow and s_part read
-            if (ptid >= 0) {
+            if (tid < 2 * kTcM) {
                 int jr = -1;
-                if (m0 + ptid < rr) {
-                    int p = pfirst;
-                    if (m0 > 0) {
-                        const int32_t id = G.order[A.dpos[i0 + m0 + ptid]];
-                        const int32_t v = G.ev[id], u = G.eu[id];
-                        p = (int)((v == qg ? u : v) - vb);
-                    }
+                if (m0 + tid < rr) {
+                    const int p = m0 > 0 ? A.ends[i0 + m0 + tid] : s_p[run & 1][tid];
                     jr = s_o[p >> 6] + __popcll(s_m[p >> 6] & ((1ull << (p & 63)) - 1));
                 }
-                s_jrow[ptid >> 7][ptid & (kTcM - 1)] = (int16_t)jr;
+                s_jrow[tid >> 7][tid & (kTcM - 1)] = (int16_t)jr;
             }
             __syncthreads();
             float acc = 0.f;   // row erow of edge tile et, column half eh
-            for (int n0 = 0; n0 < d && !bad; n0 += kTcN) {
-                const int nt = min(kTcN, ((d - n0 + 15) >> 4) << 4);
-                const uint32_t idesc = idesc_e4m3_f32(kTcM, nt);
-                // this builder thread's items (16 columns of one row each) of
-                // every chunk of this tile: compact source word, shift,
-                // destination.  In the core-matrix layout (LBO 128, SBO 512)
-                // item i of a tile lives at byte 16·i; a stage holds A of tile
-                // 0, A of tile 1, B.
-                const int nA = ntiles * kTcM * 4, nItems = nA + nt * 4;
-                const int KT = min(KW, (n0 + nt + 63) >> 6);   // chunks with columns below some row of the tile
-                constexpr int kPer = (2 * kTcM * 4 + kTcN * 4 + 32 * kTcBuilders - 1) / (32 * kTcBuilders);
-                if (warp < kTcBuilders) {
-                    // per item: its 16 bits of chunk 0 as a halfword of C (chunk kc
-                    // is 4·kc halfwords further), and its destination.  Rows past
-                    // the run's edges and past d_q are not built: they only feed
-                    // accumulator rows and columns that are never read (stale
-                    // stage bytes there are harmless: the read-back selects by the
-                    // row's bits, which are zero past d_q).
-                    const uint16_t *C16 = (const uint16_t *)C;
-                    int src[kPer];
-                    int below[kPer];   // B: columns of the row below its diagonal, from this item's first one
-                    uint32_t dst[kPer];
+            // row tiles of N(q): columns (rows of N(q)) and chunks with columns below some row of the tile
+            auto tile_cols = [&](int n0) { return min(kTcN, ((d - n0 + 15) >> 4) << 4); };
+            auto tile_chunks = [&](int n0) { return min(KW, (n0 + tile_cols(n0) + 63) >> 6); };
+            if (warp < kTcBuilders) {
+                // this builder thread's rows of its group's stages: one of the A
+                // tiles, one of B.  In the core-matrix layout (LBO 128, SBO 512) 16
+                // columns of eight rows are 128 consecutive bytes.  Rows past the
+                // run's edges and past d_q are not built: they only feed
+                // accumulator rows and columns that are never read (stale stage
+                // bytes there are harmless: the read-back selects by the row's
+                // bits, which are zero past d_q).  Within 32 columns both
+                // operands take the order 0, 8, 16, 24, 1, 9, ...: a sum over K
+                // does not mind.
+                const int grp = warp / (kTcBuilders / kTcGroups), t = tid & (kTcGroup - 1);
+                const int ca = t < ntiles * kTcM ? s_jrow[t >> 7][t & (kTcM - 1)] : -1;
+                uint8_t *const dst = stages + (t >> 3) * 512 + (t & 7) * 16;
+                auto build = [&](int n0, int kc) {
+                    if ((kc & (kTcGroups - 1)) == grp) {
+                        const int cr[2] = {ca, n0 + t < d ? n0 + t : -1};
+                        uint64_t x[2];
 #pragma unroll
-                    for (int k = 0; k < kPer; k++) {
-                        const int it = tid + k * 32 * kTcBuilders;
-                        const bool isA = it < nA;
-                        const int i2 = isA ? (it & (kTcM * 4 - 1)) : it - nA;
-                        const int row = ((i2 >> 5) << 3) | (i2 & 7);
-                        int cr = -1;
-                        if (it < nItems) cr = isA ? s_jrow[it >> 9][row] : (n0 + row < d ? n0 + row : -1);
-                        src[k] = 4 * cr * KS + ((i2 >> 3) & 3);
-                        below[k] = isA ? 0x7fffffff : n0 + row - 16 * ((i2 >> 3) & 3);
-                        dst[k] = cr < 0 ? 0xffffffffu
-                                 : isA ? (uint32_t)((it >> 9) * kTcM * kTcK + 16 * i2)
-                                       : (uint32_t)(2 * kTcM * kTcK + 16 * i2);
-                    }
-                    for (int kc = 0; kc < KT; kc++) {
-                        const int c = chunk + kc, st = c & 1, u = c >> 1;
-                        // the MMAs that read this stage last (chunk c - 2) are done
-                        int ok = 1;
-                        if (lane == 0 && u > 0)
-                            ok = mbar_wait_or_abort(&s_empty[st], (u - 1) & 1, kTcWaitCycles, &s_abort);
-                        bad |= !__shfl_sync(0xffffffffu, ok, 0);
-                        uint8_t *stg = base + st * kTcStageBytes;
-                        uint32_t b16[kPer];
-#pragma unroll
-                        for (int k = 0; k < kPer; k++) b16[k] = dst[k] != 0xffffffffu ? C16[src[k] + 4 * kc] : 0u;
+                        for (int k = 0; k < 2; k++) x[k] = cr[k] >= 0 ? C[cr[k] * KS + kc] : 0ull;
                         if (64 * kc + 63 >= n0) {   // the tile's diagonal runs through this chunk
-#pragma unroll
-                            for (int k = 0; k < kPer; k++) {
-                                const int left = min(16, max(0, below[k] - 64 * kc));
-                                b16[k] &= (1u << left) - 1;
-                            }
+                            const int left = cr[1] - 64 * kc;
+                            x[1] &= left >= 64 ? ~0ull : (1ull << max(0, left)) - 1;
                         }
+                        // the MMAs that read this stage last are done
+                        if (!bad)
+                            bad = !mbar_wait_or_abort(&s_empty[st], ((phase >> st) & 1u) ^ 1u, kTcWaitCycles, &s_abort);
 #pragma unroll
-                        for (int k = 0; k < kPer; k++) {
-                            if (dst[k] != 0xffffffffu)
-                                *(uint4 *)(stg + dst[k]) =
-                                    make_uint4(tc_spread4(b16[k] & 15u), tc_spread4((b16[k] >> 4) & 15u),
-                                               tc_spread4((b16[k] >> 8) & 15u), tc_spread4(b16[k] >> 12));
+                        for (int k = 0; k < 2; k++) {
+                            if (cr[k] < 0) continue;
+                            uint4 *to = (uint4 *)(dst + st * kTcStageBytes + k * 2 * kTcM * kTcK);
+#pragma unroll
+                            for (int h = 0; h < 2; h++) {
+                                const uint32_t y = (uint32_t)(x[k] >> (32 * h));
+                                to[16 * h] = make_uint4(tc_spread(y, 0), tc_spread(y, 1), tc_spread(y, 2), tc_spread(y, 3));
+                                to[16 * h + 8] =
+                                    make_uint4(tc_spread(y, 4), tc_spread(y, 5), tc_spread(y, 6), tc_spread(y, 7));
+                            }
                         }
                         fence_async_smem();
                         __syncwarp();
                         if (lane == 0) mbar_arrive(&s_full[st]);
                     }
-                } else if (issuer) {
-                    for (int kc = 0; kc < KT; kc++) {
-                        const int c = chunk + kc, st = c & 1, u = c >> 1;
-                        bad |= !mbar_wait_or_abort(&s_full[st], u & 1, kTcWaitCycles, &s_abort);
+                    phase ^= 1u << st;
+                    st = st + 1 < nst ? st + 1 : 0;
+                };
+                int built = 0;   // chunks of this tile built before the last one was read back
+                for (int n0 = 0; n0 < d; n0 += kTcN, tile++) {
+                    const int KT = tile_chunks(n0);
+                    for (int kc = built; kc < KT; kc++) build(n0, kc);
+                    built = n0 + kTcN < d ? min(nst, tile_chunks(n0 + kTcN)) : 0;
+                    for (int kc = 0; kc < built; kc++) build(n0 + kTcN, kc);
+                    if (!bad) bad = !mbar_wait_or_abort(&s_done, tile & 1u, kTcWaitCycles, &s_abort);
+                    bad = __any_sync(0xffffffffu, bad);   // the read-back is the whole warp's
+                    fence_after_sync();
+                    if (et < ntiles && !bad) {
+                        const int nt = tile_cols(n0);
+                        const int jr = s_jrow[et][erow];
+                        const int cend = min(nt, eh * 128 + 128);
+                        // 32 columns per step: two loads in flight, one wait
+                        for (int c0 = eh * 128; c0 < cend; c0 += 32) {
+                            uint32_t v[32];
+                            const bool two = c0 + 16 < cend;   // nt is a multiple of 16
+                            tmem_ld16_async(etaddr + (uint32_t)c0, v);
+                            if (two) tmem_ld16_async(etaddr + (uint32_t)(c0 + 16), v + 16);
+                            const int y0 = n0 + c0;   // a multiple of 32, below d
+                            const uint32_t b32 = jr >= 0 ? ((const uint32_t *)C)[jr * 2 * KS + (y0 >> 5)] : 0u;
+                            tmem_wait_ld();
+#pragma unroll
+                            for (int i = 0; i < 16; i++) acc += ((b32 >> i) & 1u) ? __uint_as_float(v[i]) : 0.f;
+                            if (two) {
+#pragma unroll
+                                for (int i = 16; i < 32; i++) acc += ((b32 >> i) & 1u) ? __uint_as_float(v[i]) : 0.f;
+                            }
+                        }
+                    }
+                    fence_before_sync();
+                    __syncwarp();
+                    if (lane == 0) mbar_arrive(&s_read);
+                }
+            } else if (issuer) {
+                const uint64_t da0 = smem_desc(sbase, 128, 512), db0 = smem_desc(sbase + 2 * kTcM * kTcK, 128, 512);
+                for (int n0 = 0; n0 < d; n0 += kTcN, tile++) {
+                    const int KT = tile_chunks(n0);
+                    const uint32_t idesc = idesc_e4m3_f32(kTcM, tile_cols(n0));
+                    // the last tile's accumulators are read
+                    if (tile > 0) bad = !mbar_wait_or_abort(&s_read, (tile - 1) & 1u, kTcWaitCycles, &s_abort);
+                    for (int kc = 0; kc < KT && !bad; kc++) {
+                        bad = !mbar_wait_or_abort(&s_full[st], (phase >> st) & 1u, kTcWaitCycles, &s_abort);
+                        if (bad) break;   // last stays the stage of the last commit
                         fence_after_sync();
-                        const uint32_t sa = smem_addr(base + st * kTcStageBytes), sb = sa + 2 * kTcM * kTcK;
+                        const uint32_t at = (uint32_t)(st * (kTcStageBytes >> 4));   // in 16-byte units, as the descriptors
                         for (int t = 0; t < ntiles; t++)
 #pragma unroll
                             for (int ks = 0; ks < 2; ks++)
-                                mma_e4m3(tmem + (uint32_t)(t * kTcN),
-                                         smem_desc(sa + t * kTcM * kTcK + 256 * ks, 128, 512),
-                                         smem_desc(sb + 256 * ks, 128, 512), idesc, (kc | ks) != 0);
+                                mma_e4m3(tmem + (uint32_t)(t * kTcN), smem_desc_add(da0, at + t * (kTcM * kTcK >> 4) + 16 * ks),
+                                         smem_desc_add(db0, at + 16 * ks), idesc, (kc | ks) != 0);
                         mma_commit(&s_empty[st]);
-                        last = c;
+                        last = st;
+                        phase ^= 1u << st;
+                        st = st + 1 < nst ? st + 1 : 0;
                     }
-                    // the accumulators are complete once the last commit lands
-                    bad |= !mbar_wait_or_abort(&s_empty[last & 1], (last >> 1) & 1, kTcWaitCycles, &s_abort);
+                    if (bad) break;
+                    mma_commit(&s_done);   // the accumulators are complete once this lands
                 }
-                chunk += KT;
-                if (__syncthreads_or(bad)) {
-                    bad = true;
-                    break;
-                }
-                fence_after_sync();
-                if (et < ntiles) {
-                    const int jr = s_jrow[et][erow];
-                    const int cend = min(nt, eh * 128 + 128);
-                    // 32 columns per step: two loads in flight, one wait
-                    for (int c0 = eh * 128; c0 < cend; c0 += 32) {
-                        uint32_t v[32];
-                        const bool two = c0 + 16 < cend;   // nt is a multiple of 16
-                        tmem_ld16_async(etaddr + (uint32_t)c0, v);
-                        if (two) tmem_ld16_async(etaddr + (uint32_t)(c0 + 16), v + 16);
-                        const int y0 = n0 + c0;   // a multiple of 32, below d
-                        const uint32_t b32 = jr >= 0 ? (uint32_t)(C[jr * KS + (y0 >> 6)] >> (y0 & 63)) : 0u;
-                        tmem_wait_ld();
-#pragma unroll
-                        for (int i = 0; i < 16; i++) acc += ((b32 >> i) & 1u) ? __uint_as_float(v[i]) : 0.f;
-                        if (two) {
-#pragma unroll
-                            for (int i = 16; i < 32; i++) acc += ((b32 >> i) & 1u) ? __uint_as_float(v[i]) : 0.f;
-                        }
-                    }
-                }
-                fence_before_sync();
-                __syncthreads();   // accumulators read before the next tile's MMAs
             }
-            if (bad) break;
+            if (__syncthreads_or(bad)) {
+                bad = true;
+                break;
+            }
+            last = -1;   // every tile was waited for and read
             if (et < ntiles) s_part[et][eh][erow] = acc;
             __syncthreads();
             if (tid < ntiles * kTcM && m0 + tid < rr) {
                 const int t = tid >> 7, row = tid & (kTcM - 1);
-                // (sum of D·A_py) · 2^12 = k4
-                A.k4[i0 + m0 + tid] = (uint32_t)((s_part[t][0][row] + s_part[t][1][row]) * 4096.f);
+                // sum of D·A_py = 4·k4
+                A.k4[i0 + m0 + tid] = (uint32_t)((s_part[t][0][row] + s_part[t][1][row]) * 0.25f);
             }
         }
         if (bad) break;
+        __syncthreads();   // s_jrow, s_part, s_m and C read
     }
     if (bad && issuer) {
         atomicAdd(A.err, 1ull);
         // MMAs still in flight: one more bounded wait for the last commit
-        if (last >= 0) mbar_wait(&s_empty[last & 1], (last >> 1) & 1, kTcWaitCycles);
+        if (last >= 0) mbar_wait(&s_empty[last], ((phase >> last) & 1u) ^ 1u, kTcWaitCycles);
     }
     fence_before_sync();
     __syncthreads();
@@ -2088,7 +2124,8 @@ struct DenseCloseArgs {
     const uint16_t *cn;
     const int64_t *cbase;
     const int32_t *dpos;
-    const int64_t *runs;
+    const uint16_t *ends;
+    const TcRun *runs;
     const unsigned long long *nruns;
     const uint32_t *k4;
     const int32_t *eslot;
@@ -2118,20 +2155,18 @@ __global__ void __launch_bounds__(256) k_dense_close(DenseCloseArgs A) {
         if (lane == 0) r = atomicAdd(A.next, 1ull);
         r = __shfl_sync(0xffffffffu, r, 0);
         if (r >= nruns) break;
-        const int64_t i0 = A.runs[2 * r], i1 = A.runs[2 * r + 1];
-        const int32_t qg = dense_q(G, A.dpos[i0]);
+        const TcRun R = A.runs[r];
+        const int64_t i0 = R.first, i1 = R.last, vb = R.vbase, q = R.q, qg = vb + q;
         const int g = G.egraph[A.dpos[i0]];
         if (g != cur_g) {
             if (cur_g >= 0) warp_flush_graph(G, acc, cur_g, lane);
             cur_g = g;
         }
-        const int64_t vb = A.vbase[g];
         const long long n = G.gnm[2 * g], m = G.gnm[2 * g + 1];
-        const int W = (int)((n + 63) >> 6);
+        const int W = R.W;
         const int64_t stride = (int64_t)W * 64;
-        const uint64_t *rows = A.bits + A.wbase[g];
+        const uint64_t *rows = A.bits + R.wbase;
         const uint16_t *cnb = A.cn + A.cbase[g];
-        const int64_t q = qg - vb;
         const uint64_t Aq = lane < W ? __ldg(rows + q * W + lane) : 0ull;
         const int c = __popcll(Aq);
         int o = c;
@@ -2153,7 +2188,7 @@ __global__ void __launch_bounds__(256) k_dense_close(DenseCloseArgs A) {
                 const int32_t id = G.order[e];
                 v = G.ev[id];
                 u = G.eu[id];
-                pl = (int32_t)((v == qg ? u : v) - vb);
+                pl = A.ends[i];
             }
             const int pw = pl >> 6;
             const uint64_t aw = __shfl_sync(0xffffffffu, Aq, pw);
@@ -2396,7 +2431,8 @@ struct DenseView {
 struct TcOut {
     uint32_t *k4 = nullptr;
     int32_t *eslot = nullptr;
-    int64_t *runs = nullptr;
+    TcRun *runs = nullptr;
+    uint16_t *ends = nullptr;
     const unsigned long long *nruns = nullptr;
     int32_t *rest = nullptr;    // positions left to k_dense_cn, in dpos order
     int64_t nrest = 0;
@@ -2407,12 +2443,14 @@ static pgd_status dense_tc(pgd_ctx *ctx, const DevGraph &G, TmpGuard &tg, const 
     cudaStream_t s = ctx->stream;
     pgd_status st;
     uint32_t *flag = nullptr, *pos = nullptr, *k4 = nullptr;
-    int64_t *runs = nullptr;
+    TcRun *runs = nullptr;
+    uint16_t *ends = nullptr;
     const int64_t maxruns = std::min<int64_t>(ncn, G.n);
     if ((st = tg.alloc(&flag, (ncn + 1) * sizeof(uint32_t)))) return st;
     if ((st = tg.alloc(&pos, (ncn + 1) * sizeof(uint32_t)))) return st;
     if ((st = tg.alloc(&k4, ncn * sizeof(uint32_t)))) return st;
-    if ((st = tg.alloc(&runs, (2 * maxruns + 2) * sizeof(int64_t)))) return st;
+    if ((st = tg.alloc(&runs, (maxruns + 1) * sizeof(TcRun)))) return st;
+    if ((st = tg.alloc(&ends, (ncn + 1) * sizeof(uint16_t)))) return st;
     unsigned long long *ctr = ctx->d_ctr;
     PGD_CUDA(ctx, cudaMemsetAsync(ctr + 8, 0, 6 * sizeof(unsigned long long), s));
     PGD_LAUNCH(ctx, k_tc_run_flags, grid_for(ncn), kThreads, 0, keys, ncn, G.deg, ctx->tc_min_deg, flag);
@@ -2423,14 +2461,12 @@ static pgd_status dense_tc(pgd_ctx *ctx, const DevGraph &G, TmpGuard &tg, const 
     if ((st = pgd_tmp_alloc(ctx, &tmp, tb))) return st;
     cub::DeviceScan::ExclusiveSum(tmp, tb, flag, pos, ncn + 1, s);
     pgd_tmp_free(ctx, tmp);
-    PGD_LAUNCH(ctx, k_tc_run_fill, grid_for(ncn), kThreads, 0, keys, flag, pos, ncn, runs, ctr + 9);
+    PGD_LAUNCH(ctx, k_tc_run_fill, grid_for(ncn), kThreads, 0, G, dpos, keys, flag, pos, dense->vbase, dense->wbase, ncn, runs,
+               ends, ctr + 9);
     PGD_CUDA(ctx, cudaMemsetAsync(k4, 0xff, ncn * sizeof(uint32_t), s));
     DenseTcArgs T;
-    T.G = G;
     T.bits = dense->bits;
-    T.wbase = dense->wbase;
-    T.vbase = dense->vbase;
-    T.dpos = dpos;
+    T.ends = ends;
     T.runs = runs;
     T.nruns = ctr + 9;
     T.k4 = k4;
@@ -2482,6 +2518,7 @@ static pgd_status dense_tc(pgd_ctx *ctx, const DevGraph &G, TmpGuard &tg, const 
     out->k4 = k4;
     out->eslot = eslot;
     out->runs = runs;
+    out->ends = ends;
     out->nruns = ctr + 9;
     out->rest = rest;
     out->nrest = (int64_t)nrest;
@@ -2766,6 +2803,7 @@ static pgd_status dense_decompose(pgd_ctx *ctx, const DevGraph &G, const DenseVi
         Z.cbase = dense.cbase;
         Z.dpos = dpos;
         Z.runs = tc.runs;
+        Z.ends = tc.ends;
         Z.nruns = tc.nruns;
         Z.k4 = tc.k4;
         Z.eslot = tc.eslot;

@@ -19,6 +19,9 @@ __device__ __forceinline__ uint64_t smem_desc(uint32_t addr, uint32_t lbo, uint3
            ((uint64_t)((sbo >> 4) & 0x3FFF) << 32) | (1ull << 46);
 }
 
+// the descriptor of a tile that starts `units` 16-byte units further
+__device__ __forceinline__ uint64_t smem_desc_add(uint64_t desc, uint32_t units) { return desc + units; }
+
 // instruction descriptor of kind::f8f6f4 with e4m3 A and B, fp32 D, both K-major
 __device__ __forceinline__ uint32_t idesc_e4m3_f32(int m, int n) {
     return (1u << 4) | ((uint32_t)(n >> 3) << 17) | ((uint32_t)(m >> 4) << 24);
