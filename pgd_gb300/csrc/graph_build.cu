@@ -932,18 +932,17 @@ __device__ __forceinline__ void core_append(bool in, int32_t v, int32_t *list, u
 // warps of which this is the w-th: as many vertices per warp as fill them (at
 // most 32), whose offsets are then loaded together; rows of 64 or more entries
 // one after the other, shorter ones flattened over the lanes.
-template <typename Get, typename Visit>
-__device__ __forceinline__ void core_rows(const int64_t *off, const int32_t *adj, const int32_t *deg, unsigned nf, int w,
-                                          int warps, Get get, Visit visit) {
+// row(v, o, d) gives v's row.
+template <typename Get, typename Row, typename Visit>
+__device__ __forceinline__ void core_rows(const int32_t *adj, unsigned nf, int w, int warps, Get get, Row row,
+                                          Visit visit) {
     const int lane = threadIdx.x & 31;
     const unsigned per = min(32u, max(1u, (nf + (unsigned)warps - 1) / (unsigned)warps));
     for (unsigned i0 = (unsigned)w * per; i0 < nf; i0 += (unsigned)warps * per) {
         int64_t o = 0;
         int d = 0;
         if ((unsigned)lane < per && i0 + lane < nf) {
-            const int32_t v = get(i0 + lane);
-            o = off[v];
-            d = deg[v];
+            row(get(i0 + lane), o, d);
         }
         unsigned lm = __ballot_sync(0xffffffffu, d >= 64);
         while (lm) {
@@ -1073,7 +1072,12 @@ k_core_cluster(const int64_t *off, const int32_t *adj, const int32_t *deg, int n
                     core_append(leaves && d >= kCoreLong, y, bout, &s->lng, lane);
                 }
             };
-            core_rows(off, adj, deg, nf, w, kAll / 32, [&](unsigned i) { return __ldcg(fin + i); }, visit);
+            core_rows(adj, nf, w, kAll / 32, [&](unsigned i) { return __ldcg(fin + i); },
+                      [&](int32_t v, int64_t &o, int &d) {
+                          o = off[v];
+                          d = deg[v];
+                      },
+                      visit);
             for (unsigned i = 0; i < nb; i++) {   // all warps share a long row
                 const int32_t v = __ldcg(bin + i);
                 const int64_t o = off[v], e = o + deg[v];
@@ -1102,7 +1106,9 @@ k_core_cluster(const int64_t *off, const int32_t *adj, const int32_t *deg, int n
 
 // Small graphs: one block with every count (16 bits) and a bit per vertex removed
 // in shared memory, so that a step is a shared-memory scan or one round over the
-// frontier's rows, and a block barrier.  R-MAT 14: 320 steps.
+// frontier's rows, and a block barrier.  A step is a chain of latencies: where the
+// row offsets fit as well (about 32,000 vertices), only the entries come from L2.
+// R-MAT 14: 320 steps.
 constexpr int kCoreSmallBytes = 200 * 1024;
 constexpr int64_t kCoreSmallEntries = 1ll << 20;
 constexpr int kCoreQueue = 2048;            // frontier entries kept in shared memory (the rest in global)
@@ -1111,6 +1117,12 @@ __host__ __device__ __forceinline__ size_t core_small_bytes(int64_t n) {
     return (size_t)((n + 63) / 64) * 64 * 2 + (size_t)((n + 63) / 64) * 8;
 }
 
+// ... and with the row offsets
+__host__ __device__ __forceinline__ size_t core_small_bytes_off(int64_t n) {
+    return core_small_bytes(n) + ((size_t)n + 1) * 4;
+}
+
+template <bool OFF>
 __global__ void __launch_bounds__(kCoreThreads, 1)
 k_core_block(const int64_t *off, const int32_t *adj, const int32_t *deg, int n, int32_t *core, int32_t *g0, int32_t *g1,
              int32_t *b0, int32_t *b1, CoreShared *S) {
@@ -1120,7 +1132,19 @@ k_core_block(const int64_t *off, const int32_t *adj, const int32_t *deg, int n, 
     __shared__ int s_low[2], s_max;
     const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
     const int groups = (n + 63) / 64;       // 64 vertices: 32 words of counts, 2 of bits
-    uint32_t *cur = s_dyn, *gone = s_dyn + 32 * groups;
+    uint32_t *cur = s_dyn, *gone = s_dyn + 32 * groups, *s_off = gone + 2 * groups;
+    if (OFF)
+        for (int i = threadIdx.x; i <= n; i += kCoreThreads) s_off[i] = (uint32_t)off[i];
+    auto row = [&](int32_t v, int64_t &o, int &d) {
+        if (OFF) {
+            o = s_off[v];
+            d = (int)(s_off[v + 1] - s_off[v]);
+        } else {
+            o = off[v];
+            d = deg[v];
+        }
+    };
+    auto degree = [&](int32_t v) { return OFF ? (int)(s_off[v + 1] - s_off[v]) : deg[v]; };
     for (int i = threadIdx.x; i < 32 * groups; i += kCoreThreads) {
         const uint32_t lo = 2 * i < n ? (uint32_t)deg[2 * i] : 0, hi = 2 * i + 1 < n ? (uint32_t)deg[2 * i + 1] : 0;
         cur[i] = lo | hi << 16;
@@ -1136,7 +1160,7 @@ k_core_block(const int64_t *off, const int32_t *adj, const int32_t *deg, int n, 
     int level = 0, removed = 0, sel = 0, scan = 0;
     // v leaves at this level: into the frontier of buffer q
     auto leave = [&](bool in, int32_t v, int q) {
-        const bool lng = in && deg[v] >= kCoreLong;
+        const bool lng = in && degree(v) >= kCoreLong;
         const unsigned m = __ballot_sync(0xffffffffu, in && !lng);
         if (m) {
             unsigned at = 0;
@@ -1199,12 +1223,13 @@ k_core_block(const int64_t *off, const int32_t *adj, const int32_t *deg, int n, 
                 }
                 if (__any_sync(0xffffffffu, in)) leave(in, y, to);
             };
-            core_rows(off, adj, deg, nf, wid, kCoreThreads / 32,
-                      [&](unsigned i) { return i < kCoreQueue ? s_q[sel][i] : (sel ? g1 : g0)[i - kCoreQueue]; }, visit);
+            core_rows(adj, nf, wid, kCoreThreads / 32,
+                      [&](unsigned i) { return i < kCoreQueue ? s_q[sel][i] : (sel ? g1 : g0)[i - kCoreQueue]; }, row,
+                      visit);
             for (unsigned i = 0; i < nb; i++) {
-                const int32_t v = (sel ? b1 : b0)[i];
-                const int64_t o = off[v];
-                const int d = deg[v];
+                int64_t o;
+                int d;
+                row((sel ? b1 : b0)[i], o, d);
                 for (int j = 32 * wid; j < d; j += kCoreThreads)
                     visit(j + lane < d, j + lane < d ? __ldg(adj + o + j + lane) : 0);
             }
@@ -1233,7 +1258,8 @@ k_core_block(const int64_t *off, const int32_t *adj, const int32_t *deg, int n, 
 cudaError_t pgd_build_limits() {
     constexpr cudaFuncAttribute kDyn = cudaFuncAttributeMaxDynamicSharedMemorySize;
     constexpr int kSort = 2 * (int)kSmallPairs * 8;
-    cudaError_t e = cudaFuncSetAttribute(k_core_block, kDyn, kCoreSmallBytes);
+    cudaError_t e = cudaFuncSetAttribute(k_core_block<false>, kDyn, kCoreSmallBytes);
+    if (e == cudaSuccess) e = cudaFuncSetAttribute(k_core_block<true>, kDyn, kCoreSmallBytes);
     if (e == cudaSuccess) e = cudaFuncSetAttribute(k_small_build, kDyn, kSort);
     if (e == cudaSuccess) e = cudaFuncSetAttribute(k_small_edges, kDyn, kSort);
     if (e == cudaSuccess) e = cudaFuncSetAttribute(k_small_order, kDyn, kSort);
@@ -1249,8 +1275,12 @@ static pgd_status cores_by_cluster(pgd_graph *g) {
     const size_t lists = (7 * (size_t)n * sizeof(int32_t) + 15) & ~(size_t)15;
     if ((st = pgd_tmp_alloc(ctx, (void **)&work, lists + sizeof(CoreShared)))) return st;
     CoreShared *S = (CoreShared *)((uint8_t *)work + lists);
-    if (g->max_degree < 65536 && 2 * g->m <= kCoreSmallEntries && core_small_bytes(n) <= (size_t)kCoreSmallBytes)
-        PGD_LAUNCH(ctx, k_core_block, 1, kCoreThreads, core_small_bytes(n), g->off, g->adj, g->deg, (int)n, g->core, work,
+    const bool small = g->max_degree < 65536 && 2 * g->m <= kCoreSmallEntries;
+    if (small && core_small_bytes_off(n) <= (size_t)kCoreSmallBytes)
+        PGD_LAUNCH(ctx, k_core_block<true>, 1, kCoreThreads, core_small_bytes_off(n), g->off, g->adj, g->deg, (int)n,
+                   g->core, work, work + n, work + 2 * n, work + 3 * n, S);
+    else if (small && core_small_bytes(n) <= (size_t)kCoreSmallBytes)
+        PGD_LAUNCH(ctx, k_core_block<false>, 1, kCoreThreads, core_small_bytes(n), g->off, g->adj, g->deg, (int)n, g->core, work,
                    work + n, work + 2 * n, work + 3 * n, S);
     else
         PGD_LAUNCH(ctx, k_core_cluster, kCoreBlocks, kCoreThreads, 0, g->off, g->adj, g->deg, (int)n, work, g->core,
