@@ -898,16 +898,22 @@ pgd_status pgd_dev_preprocess(pgd_graph *g, int neigh_kind, int s2l) {
 }
 
 // k-core of graphs of up to kCoreClusterEntries adjacency entries: one cluster of
-// eight blocks peels the whole graph in one launch.  What bounds it is the chain
+// sixteen blocks peels the whole graph in one launch.  What bounds it is the chain
 // of steps (832 on R-MAT 20, 448 on R-MAT 16), each a few dependent L2 accesses
 // and a barrier: the cluster's hardware barrier replaces two graph nodes per step
 // (k_core_work and k_core_ctrl below, about 8 us together with their gaps), and
-// no graph is captured and instantiated for the call (180 us).
+// no graph is captured and instantiated for the call (180 us).  Sixteen blocks
+// rather than the portable eight for the graphs of few wide steps: milliseconds of
+// the call with 8 / 16 / the whole device, R-MAT 16 2.2 / 2.25 / 3.2, R-MAT 20 12.1 /
+// 8.0 / 12.2, BA of 400,000 2.8 / 2.0 / 2.4 and of 1M vertices 3.2 / 1.7 / 2.0,
+// geometric with 1M vertices 12.1 / 6.7 / 6.4, G(6000, 0.5) 1.8 / 1.0 / 2.0.
 namespace {
 
-constexpr int kCoreBlocks = 8;              // a portable cluster
+constexpr int kCoreBlocks = 16;             // the largest cluster (beyond the portable eight)
 constexpr int kCoreThreads = 1024;
 constexpr int64_t kCoreClusterEntries = 64ll << 20;
+constexpr int64_t kCoreEvenEntries = 16ll << 20;   // the same for graphs of small largest degree:
+constexpr int kCoreEvenDegree = 64;                // few levels, wide steps (the geometric graph above)
 constexpr int kCoreLong = 1024;             // rows at least this long are shared by all warps
 
 struct CoreSlot {
@@ -1078,10 +1084,15 @@ k_core_cluster(const int64_t *off, const int32_t *adj, const int32_t *deg, int n
                           d = deg[v];
                       },
                       visit);
-            for (unsigned i = 0; i < nb; i++) {   // all warps share a long row
+            // a long row is shared by all warps, by a block's where there is one for
+            // each block, or taken by one warp where there are plenty (the chains of
+            // loads then run side by side: G(3000, 0.5) 2.6 -> 0.57 ms with eight blocks)
+            const int share = nb >= (unsigned)(kAll / 32) ? 32 : nb >= (unsigned)kCoreBlocks ? kCoreThreads : kAll;
+            for (unsigned i = (unsigned)(t / share); i < nb; i += (unsigned)(kAll / share)) {
                 const int32_t v = __ldcg(bin + i);
                 const int64_t o = off[v], e = o + deg[v];
-                for (int64_t j = o + t0; j < e; j += kAll) visit(j + lane < e, j + lane < e ? __ldg(adj + j + lane) : 0);
+                for (int64_t j = o + t0 % share; j < e; j += share)
+                    visit(j + lane < e, j + lane < e ? __ldg(adj + j + lane) : 0);
             }
             pgd_cl::cluster_sync();
             nf = __ldcg(&s->front);
@@ -1104,143 +1115,200 @@ k_core_cluster(const int64_t *off, const int32_t *adj, const int32_t *deg, int n
     if (t == 0 && removed < n) S->failed = 1;
 }
 
-// Small graphs: one block with every count (16 bits) and a bit per vertex removed
-// in shared memory, so that a step is a shared-memory scan or one round over the
-// frontier's rows, and a block barrier.  A step is a chain of latencies: where the
-// row offsets fit as well (about 32,000 vertices), only the entries come from L2.
-// R-MAT 14: 320 steps.
-constexpr int kCoreSmallBytes = 200 * 1024;
+// Small graphs: one block with every count (16 bits), a bit per vertex removed and
+// the row offsets in shared memory.  The bound is the chain of removals, one L2
+// latency (the row) and some shared-memory operations per link, so the warps of a level never wait for each other: each takes its part
+// of the vertices of count <= level, then whatever a removal has pushed onto the
+// level's queue, until nothing is queued or in work.  A vertex belongs to the warp
+// that sets its bit.  What finds the queue full is left to another turn of the same
+// level.
+// Up to 2^20 entries and about 32,000 vertices, microseconds of the call against
+// the cluster's: R-MAT 12 261 / 695, R-MAT 14 656 / 1197 (1239 for eight blocks),
+// R-MAT 15 1148 / 1496, G(1000, 0.5) 176 / 313, a 20,000-vertex BA graph 349 / 350,
+// a path of 20,000 7.9 / 33 ms.  Without the offsets in shared memory (R-MAT 16 with
+// 5 edges per vertex 1357 / 1270, a geometric graph of 60,000 987 / 498) and for
+// more entries (G(1500, 0.9) 421 / 168) the cluster is the faster one.
+constexpr int kCoreSmallBytes = 196 * 1024;
 constexpr int64_t kCoreSmallEntries = 1ll << 20;
-constexpr int kCoreQueue = 2048;            // frontier entries kept in shared memory (the rest in global)
+constexpr int kCoreQueue = 4096;
+constexpr int kCoreQueueRoom = kCoreQueue - kCoreThreads;   // every warp may add 32 after it has seen room
+constexpr int kCoreSpins = 1 << 26;                         // turns without work after which a warp gives up
 
-__host__ __device__ __forceinline__ size_t core_small_bytes(int64_t n) {
-    return (size_t)((n + 63) / 64) * 64 * 2 + (size_t)((n + 63) / 64) * 8;
+static size_t core_small_bytes(int64_t n) {
+    return (size_t)((n + 63) / 64) * 64 * 2 + (size_t)((n + 63) / 64) * 8 + ((size_t)n + 1) * 4;
 }
 
-// ... and with the row offsets
-__host__ __device__ __forceinline__ size_t core_small_bytes_off(int64_t n) {
-    return core_small_bytes(n) + ((size_t)n + 1) * 4;
-}
-
-template <bool OFF>
 __global__ void __launch_bounds__(kCoreThreads, 1)
-k_core_block(const int64_t *off, const int32_t *adj, const int32_t *deg, int n, int32_t *core, int32_t *g0, int32_t *g1,
-             int32_t *b0, int32_t *b1, CoreShared *S) {
+k_core_block(const int64_t *off, const int32_t *adj, const int32_t *deg, int n, int32_t *core, CoreShared *S) {
     extern __shared__ __align__(16) uint32_t s_dyn[];
-    __shared__ int32_t s_q[2][kCoreQueue];
-    __shared__ unsigned int s_nf[2], s_nb[2];
-    __shared__ int s_low[2], s_max;
+    constexpr int kWarps = kCoreThreads / 32;
+    __shared__ int32_t s_queue[kCoreQueue];          // vertex + 1, 0 until written
+    __shared__ int32_t s_mine[kWarps][64];           // a warp's vertices of one group
+    __shared__ unsigned int s_head, s_tail, s_done;  // entries taken, reserved, worked off
+    __shared__ unsigned int s_scanned;               // warps through with their part
+    __shared__ int s_removed, s_low, s_again, s_fail, s_max;
     const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
     const int groups = (n + 63) / 64;       // 64 vertices: 32 words of counts, 2 of bits
     uint32_t *cur = s_dyn, *gone = s_dyn + 32 * groups, *s_off = gone + 2 * groups;
-    if (OFF)
-        for (int i = threadIdx.x; i <= n; i += kCoreThreads) s_off[i] = (uint32_t)off[i];
+    for (int i = threadIdx.x; i <= n; i += kCoreThreads) s_off[i] = (uint32_t)off[i];
     auto row = [&](int32_t v, int64_t &o, int &d) {
-        if (OFF) {
-            o = s_off[v];
-            d = (int)(s_off[v + 1] - s_off[v]);
-        } else {
-            o = off[v];
-            d = deg[v];
-        }
+        o = s_off[v];
+        d = (int)(s_off[v + 1] - s_off[v]);
     };
-    auto degree = [&](int32_t v) { return OFF ? (int)(s_off[v + 1] - s_off[v]) : deg[v]; };
     for (int i = threadIdx.x; i < 32 * groups; i += kCoreThreads) {
         const uint32_t lo = 2 * i < n ? (uint32_t)deg[2 * i] : 0, hi = 2 * i + 1 < n ? (uint32_t)deg[2 * i + 1] : 0;
         cur[i] = lo | hi << 16;
     }
     for (int i = threadIdx.x; i < 2 * groups; i += kCoreThreads)
         gone[i] = 32 * i + 32 <= n ? 0u : (32 * i >= n ? 0xffffffffu : 0xffffffffu << (n - 32 * i));
-    if (threadIdx.x < 2) {
-        s_nf[threadIdx.x] = s_nb[threadIdx.x] = 0;
-        s_low[threadIdx.x] = INT_MAX;
-        s_max = 0;
+    for (int i = threadIdx.x; i < kCoreQueue; i += kCoreThreads) s_queue[i] = 0;
+    if (threadIdx.x == 0) {
+        s_head = s_tail = s_done = s_scanned = 0;
+        s_removed = s_again = s_fail = s_max = 0;
+        s_low = INT_MAX;
     }
     __syncthreads();
-    int level = 0, removed = 0, sel = 0, scan = 0;
-    // v leaves at this level: into the frontier of buffer q
-    auto leave = [&](bool in, int32_t v, int q) {
-        const bool lng = in && degree(v) >= kCoreLong;
-        const unsigned m = __ballot_sync(0xffffffffu, in && !lng);
-        if (m) {
-            unsigned at = 0;
-            if (lane == 0) at = atomicAdd(&s_nf[q], (unsigned)__popc(m));
-            at = __shfl_sync(0xffffffffu, at, 0) + (unsigned)__popc(m & ((1u << lane) - 1));
-            if (in && !lng) {
-                if (at < kCoreQueue) s_q[q][at] = v;
-                else (q ? g1 : g0)[at - kCoreQueue] = v;
+    volatile unsigned int *head = &s_head, *tail = &s_tail, *done = &s_done, *scanned = &s_scanned;
+    volatile int *fail = &s_fail;
+    volatile int32_t *queue = s_queue;
+    int level = 0, before = 0;
+    while (true) {
+        int taken = 0;                      // vertices this warp has removed in this turn
+        auto visit = [&](bool act, int32_t y) {
+            bool in = false;
+            if (act && !((gone[y >> 5] >> (y & 31)) & 1u)) {
+                const int sh = (y & 1) << 4;
+                // at most deg(y) take one off: the half never borrows
+                in = (int)((atomicSub(cur + (y >> 1), 1u << sh) >> sh) & 0xffffu) == level + 1;
             }
-        }
-        if (lng) (q ? b1 : b0)[atomicAdd(&s_nb[q], 1u)] = v;
-        if (in) core[v] = level;
-    };
-    while (removed < n) {
-        // every vertex left of count <= level leaves; the smallest count of the rest is the next level
+            if (!__any_sync(0xffffffffu, in)) return;
+            const bool room = __shfl_sync(0xffffffffu, (int)(*tail <= (unsigned)kCoreQueueRoom), 0);
+            if (!room) {
+                if (lane == 0) s_again = 1;
+                return;
+            }
+            // a part of this level still ahead may have taken it already
+            if (in) in = !((atomicOr(gone + (y >> 5), 1u << (y & 31)) >> (y & 31)) & 1u);
+            const unsigned m = __ballot_sync(0xffffffffu, in);
+            if (!m) return;
+            unsigned at = 0;
+            if (lane == 0) at = atomicAdd(&s_tail, (unsigned)__popc(m));
+            at = __shfl_sync(0xffffffffu, at, 0) + (unsigned)__popc(m & ((1u << lane) - 1));
+            if (in) {
+                queue[at] = y + 1;
+                core[y] = level;
+            }
+            taken += __popc(m);
+        };
+        auto one_row = [&](int32_t v) {     // the same v in all lanes
+            int64_t o;
+            int d;
+            row(v, o, d);
+            for (int j = 0; j < d; j += 128) {
+                int32_t y[4];
+#pragma unroll
+                for (int k = 0; k < 4; k++) y[k] = j + 32 * k + lane < d ? __ldg(adj + o + j + 32 * k + lane) : 0;
+#pragma unroll
+                for (int k = 0; k < 4; k++)
+                    if (j + 32 * k < d) visit(j + 32 * k + lane < d, y[k]);
+            }
+        };
+        // this warp's part: every vertex left of count <= level
         int low = INT_MAX;
-        for (int g = wid; g < groups; g += kCoreThreads / 32) {
+        for (int g = wid; g < groups; g += kWarps) {
             const uint32_t out = gone[2 * g + (lane >> 4)];
             if (__all_sync(0xffffffffu, out == 0xffffffffu)) continue;
             const uint32_t c2 = cur[32 * g + lane];
             const int b = 2 * (lane & 15), ca = (int)(c2 & 0xffffu), cb = (int)(c2 >> 16);
             const bool ha = !((out >> b) & 1u), hb = !((out >> b) & 2u);
-            const bool ia = ha && ca <= level, ib = hb && cb <= level;
+            bool ia = ha && ca <= level, ib = hb && cb <= level;
             if (ha && !ia) low = min(low, ca);
             if (hb && !ib) low = min(low, cb);
-            if (__any_sync(0xffffffffu, ia || ib)) {
-                leave(ia, 64 * g + 2 * lane, sel);
-                leave(ib, 64 * g + 2 * lane + 1, sel);
-                if (ia || ib) atomicOr(gone + 2 * g + (lane >> 4), (ia ? 1u << b : 0u) | (ib ? 2u << b : 0u));
+            if (!__any_sync(0xffffffffu, ia || ib)) continue;
+            if (ia || ib) {
+                const uint32_t had = atomicOr(gone + 2 * g + (lane >> 4), (ia ? 1u << b : 0u) | (ib ? 2u << b : 0u));
+                ia = ia && !((had >> b) & 1u);
+                ib = ib && !((had >> b) & 2u);
             }
+            const unsigned ma = __ballot_sync(0xffffffffu, ia), mb = __ballot_sync(0xffffffffu, ib);
+            const unsigned below = (1u << lane) - 1;
+            const int32_t v = 64 * g + 2 * lane;
+            if (ia) {
+                s_mine[wid][__popc(ma & below)] = v;
+                core[v] = level;
+            }
+            if (ib) {
+                s_mine[wid][__popc(ma) + __popc(mb & below)] = v + 1;
+                core[v + 1] = level;
+            }
+            __syncwarp();
+            const unsigned nf = (unsigned)(__popc(ma) + __popc(mb));
+            taken += (int)nf;
+            if (nf == 1) one_row(s_mine[wid][0]);
+            else core_rows(adj, nf, 0, 1, [&](unsigned i) { return s_mine[wid][i]; }, row, visit);
+            __syncwarp();
         }
         low = __reduce_min_sync(0xffffffffu, low);
-        if (lane == 0 && low != INT_MAX) atomicMin(&s_low[scan], low);
-        __syncthreads();
-        unsigned nf = s_nf[sel], nb = s_nb[sel];
-        low = s_low[scan];
-        scan ^= 1;
-        if (nf + nb == 0) {
-            level = max(level + 1, low);
-            __syncthreads();               // everyone has read before the next scan writes
-            if (threadIdx.x == 0) s_low[scan ^ 1] = INT_MAX;
-            __syncthreads();
-            continue;
+        if (lane == 0) {
+            if (low != INT_MAX) atomicMin(&s_low, low);
+            __threadfence_block();
+            atomicAdd(&s_scanned, 1u);
         }
-        removed += (int)(nf + nb);
-        while (nf + nb > 0) {
-            const int to = sel ^ 1;
-            __syncthreads();               // the counts are read
-            if (threadIdx.x == 0) {
-                s_nf[sel] = s_nb[sel] = 0;  // read again only when this buffer has been refilled
-                s_low[scan ^ 1] = INT_MAX;
-            }
-            auto visit = [&](bool act, int32_t y) {
-                bool in = false;
-                if (act && !((gone[y >> 5] >> (y & 31)) & 1u)) {
-                    const int sh = (y & 1) << 4;
-                    // at most deg(y) take one off: the half never borrows
-                    in = (int)((atomicSub(cur + (y >> 1), 1u << sh) >> sh) & 0xffffu) == level + 1;
-                    if (in) atomicOr(gone + (y >> 5), 1u << (y & 31));
+        // then what is queued
+        int spins = 0;
+        while (true) {
+            unsigned h = 0;
+            int take = 0;                   // -1: nothing queued or in work
+            if (lane == 0) {
+                const bool all = *scanned == (unsigned)kWarps;
+                const unsigned over = *done;   // before the tail: equal means that nothing was left
+                h = *head;
+                const unsigned t = *tail;
+                if (h < t) {
+                    const int want = (int)min(32u, max(1u, (t - h) / kWarps));
+                    if (atomicCAS(&s_head, h, h + (unsigned)want) == h) take = want;
+                } else if (all && over == t) {
+                    take = -1;
+                } else {
+                    if (++spins > kCoreSpins) s_fail = 1;
+                    if (*fail) take = -1;
+                    __nanosleep(20);
                 }
-                if (__any_sync(0xffffffffu, in)) leave(in, y, to);
-            };
-            core_rows(adj, nf, wid, kCoreThreads / 32,
-                      [&](unsigned i) { return i < kCoreQueue ? s_q[sel][i] : (sel ? g1 : g0)[i - kCoreQueue]; }, row,
-                      visit);
-            for (unsigned i = 0; i < nb; i++) {
-                int64_t o;
-                int d;
-                row((sel ? b1 : b0)[i], o, d);
-                for (int j = 32 * wid; j < d; j += kCoreThreads)
-                    visit(j + lane < d, j + lane < d ? __ldg(adj + o + j + lane) : 0);
             }
-            __syncthreads();
-            sel = to;
-            nf = s_nf[sel];
-            nb = s_nb[sel];
-            removed += (int)(nf + nb);
+            take = __shfl_sync(0xffffffffu, take, 0);
+            h = __shfl_sync(0xffffffffu, h, 0);
+            if (take < 0) break;
+            if (take == 0) continue;
+            int32_t v = 0;
+            if (lane < take)
+                for (int i = 0; i < kCoreSpins && (v = queue[h + lane]) == 0; i++) __nanosleep(20);   // being written
+            if (__any_sync(0xffffffffu, lane < take && v == 0)) {
+                if (lane == 0) s_fail = 1;
+                break;
+            }
+            if (lane < take) queue[h + lane] = 0;
+            if (take == 1) one_row(__shfl_sync(0xffffffffu, v, 0) - 1);
+            else core_rows(adj, (unsigned)take, 0, 1, [&](unsigned) { return v - 1; }, row, visit);   // entry i: lane i
+            __syncwarp();
+            if (lane == 0) {
+                __threadfence_block();
+                atomicAdd(&s_done, (unsigned)take);
+            }
+        }
+        if (lane == 0 && taken) atomicAdd(&s_removed, taken);
+        __syncthreads();
+        const int removed = s_removed, lowest = s_low;
+        const bool again = s_again != 0, failed = s_fail != 0;
+        __syncthreads();
+        if (threadIdx.x == 0) {
+            s_head = s_tail = s_done = s_scanned = 0;
+            s_low = INT_MAX;
+            s_again = 0;
         }
         __syncthreads();
-        level++;
+        if (removed >= n || failed) break;
+        if (!again) level = removed == before ? max(level + 1, lowest) : level + 1;
+        before = removed;
     }
     int top = 0;
     for (int v = threadIdx.x; v < n - 1; v += kCoreThreads) top = max(top, core[v]);
@@ -1249,7 +1317,7 @@ k_core_block(const int64_t *off, const int32_t *adj, const int32_t *deg, int n, 
     __syncthreads();
     if (threadIdx.x == 0) {
         S->max_core = s_max;
-        S->failed = 0;
+        S->failed = s_fail;
     }
 }
 
@@ -1258,15 +1326,16 @@ k_core_block(const int64_t *off, const int32_t *adj, const int32_t *deg, int n, 
 cudaError_t pgd_build_limits() {
     constexpr cudaFuncAttribute kDyn = cudaFuncAttributeMaxDynamicSharedMemorySize;
     constexpr int kSort = 2 * (int)kSmallPairs * 8;
-    cudaError_t e = cudaFuncSetAttribute(k_core_block<false>, kDyn, kCoreSmallBytes);
-    if (e == cudaSuccess) e = cudaFuncSetAttribute(k_core_block<true>, kDyn, kCoreSmallBytes);
+    cudaError_t e = cudaFuncSetAttribute(k_core_block, kDyn, kCoreSmallBytes);
+    if (e == cudaSuccess) e = cudaFuncSetAttribute(k_core_cluster, cudaFuncAttributeNonPortableClusterSizeAllowed, 1);
     if (e == cudaSuccess) e = cudaFuncSetAttribute(k_small_build, kDyn, kSort);
     if (e == cudaSuccess) e = cudaFuncSetAttribute(k_small_edges, kDyn, kSort);
     if (e == cudaSuccess) e = cudaFuncSetAttribute(k_small_order, kDyn, kSort);
     return e;
 }
 
-static pgd_status cores_by_cluster(pgd_graph *g) {
+// *launched false: the device has no room for the cluster, nothing was done
+static pgd_status cores_by_cluster(pgd_graph *g, bool *launched) {
     pgd_ctx *ctx = g->ctx;
     cudaStream_t s = ctx->stream;
     const int64_t n = g->n;
@@ -1275,20 +1344,17 @@ static pgd_status cores_by_cluster(pgd_graph *g) {
     const size_t lists = (7 * (size_t)n * sizeof(int32_t) + 15) & ~(size_t)15;
     if ((st = pgd_tmp_alloc(ctx, (void **)&work, lists + sizeof(CoreShared)))) return st;
     CoreShared *S = (CoreShared *)((uint8_t *)work + lists);
-    const bool small = g->max_degree < 65536 && 2 * g->m <= kCoreSmallEntries;
-    if (small && core_small_bytes_off(n) <= (size_t)kCoreSmallBytes)
-        PGD_LAUNCH(ctx, k_core_block<true>, 1, kCoreThreads, core_small_bytes_off(n), g->off, g->adj, g->deg, (int)n,
-                   g->core, work, work + n, work + 2 * n, work + 3 * n, S);
-    else if (small && core_small_bytes(n) <= (size_t)kCoreSmallBytes)
-        PGD_LAUNCH(ctx, k_core_block<false>, 1, kCoreThreads, core_small_bytes(n), g->off, g->adj, g->deg, (int)n, g->core, work,
-                   work + n, work + 2 * n, work + 3 * n, S);
+    if (g->max_degree < 65536 && 2 * g->m <= kCoreSmallEntries && core_small_bytes(n) <= (size_t)kCoreSmallBytes)
+        PGD_LAUNCH(ctx, k_core_block, 1, kCoreThreads, core_small_bytes(n), g->off, g->adj, g->deg, (int)n, g->core, S);
     else
         PGD_LAUNCH(ctx, k_core_cluster, kCoreBlocks, kCoreThreads, 0, g->off, g->adj, g->deg, (int)n, work, g->core,
                work + n, work + 2 * n, work + 3 * n, work + 4 * n, work + 5 * n, work + 6 * n, S, g->max_degree);
     cudaError_t e = cudaGetLastError();
+    *launched = e != cudaErrorLaunchOutOfResources && e != cudaErrorInvalidClusterSize;
     if (e == cudaSuccess) e = pgd_fetch(ctx, 0, S, sizeof(CoreShared));
     if (e == cudaSuccess) e = cudaStreamSynchronize(s);
     pgd_tmp_free(ctx, work);
+    if (!*launched) return PGD_OK;
     if (e != cudaSuccess) return pgd_cuda_fail(ctx, e, "k-core peeling");
     const CoreShared h = pgd_pinned<CoreShared>(ctx, 0);
     if (h.failed) return pgd_fail(ctx, PGD_EINVAL, "k-core peeling did not converge");
@@ -1418,7 +1484,11 @@ pgd_status pgd_dev_cores(pgd_graph *g) {
         if ((st = pgd_graph_alloc(g, (void **)&g->core, (n + 1) * sizeof(int32_t)))) return st;
     }
     if (n == 0) { g->has_cores = true; g->max_core = 0; return PGD_OK; }
-    if (2 * g->m <= kCoreClusterEntries) return cores_by_cluster(g);
+    if (2 * g->m <= (g->max_degree <= kCoreEvenDegree ? kCoreEvenEntries : kCoreClusterEntries)) {
+        bool launched = false;
+        const pgd_status st = cores_by_cluster(g, &launched);
+        if (launched || st) return st;
+    }
     int32_t *cur = nullptr, *fa = nullptr, *fb = nullptr, *aa = nullptr, *ab = nullptr;
     CoreState *d_st = nullptr;
     if ((st = pgd_tmp_alloc(ctx, (void **)&cur, n * sizeof(int32_t)))) return st;

@@ -81,3 +81,19 @@ def test_core_numbers_around_the_one_block_size(ctx, n):
     o = ol.OracleGraph.from_pairs(src, dst, dedup=True)
     o.prepare(order="kcore")
     assert (np.asarray(core) == np.asarray(o.kcore())).all()
+
+
+@pytest.mark.parametrize("kind", ["path", "star", "ladder", "matching", "ba"])
+def test_core_numbers_by_chain_and_width(ctx, kind):
+    """One link per step, one step of every vertex, and more vertices than the
+    one block's queue and its 32,000 or so vertices hold."""
+    p = np.arange(9000, dtype=np.int32)
+    src, dst = {"path": (p[:-1], p[1:]), "star": (np.zeros(8999, np.int32), p[1:]),
+                "ladder": (np.r_[p[:-1], p[:-100]], np.r_[p[1:], p[100:]]),
+                "matching": (2 * p[:8000], 2 * p[:8000] + 1), "ba": pgd.barabasi_albert(40000, 3, seed=1)}[kind]
+    g = ctx.graph_from_edges(src, dst, dedup=True)
+    core = g.kcore()
+    g.destroy()
+    o = ol.OracleGraph.from_pairs(src, dst, dedup=True)
+    o.prepare(order="kcore")
+    assert (np.asarray(core) == np.asarray(o.kcore())).all()
