@@ -39,13 +39,13 @@ METRIC = "edges/s full 4-node counts (bit-exact)"
 UNIT = "edges/s"
 RMAT = dict(a=0.57, b=0.19, c=0.19)
 
-# ncu figures of one k_hub launch (the dominant kernel) on this workload, read
-# from the committed summary: a `bench-figures:` line holding JSON with the
-# DRAM traffic, the L2 request bytes, issue activity and the SHA-256 of the
-# decompose.cu the capture ran.  A summary whose source hash differs from
+# ncu figures of one k_cycle_direct launch (the dominant kernel) on this
+# workload, read from the committed summary: a `bench-figures:` line holding JSON
+# with the DRAM traffic, the L2 request bytes, issue activity and the SHA-256 of
+# the rank_path.cu the capture ran.  A summary whose source hash differs from
 # the current file is reported as stale.
-PROFILE = os.path.join(ROOT, "profiles", "k_hub_rmat20_dram.md")
-KERNEL_SRC = os.path.join(ROOT, "pgd_gb300", "csrc", "decompose.cu")
+PROFILE = os.path.join(ROOT, "profiles", "k_cycle_direct_rmat20_dram.md")
+KERNEL_SRC = os.path.join(ROOT, "pgd_gb300", "csrc", "rank_path.cu")
 GOLDEN = os.path.join(ROOT, "tests", "golden")
 
 
@@ -126,30 +126,22 @@ class ClockSampler:
                 "samples": len(sm)}
 
 
-def algorithmic_bytes(ev, eu, n, micro=True, anchor_hub=None, ids=None):
+def algorithmic_bytes(ev, eu, n, micro=True, ids=None):
     """Bytes an edge-centric decomposition must stream: per edge both
     endpoint lists plus the 2-hop lists of the cheaper endpoint, 4 B per
-    adjacency entry, plus 64 B of per-edge output (micro).  With anchor_hub,
-    only the edges whose anchor (the endpoint of higher (degree, id)) has at
-    least that degree: the units of the hub-anchored kernel.  With ids, only
+    adjacency entry, plus 64 B of per-edge output (micro).  With ids, only
     those edges (a rank's span).  Returns (bytes, edges counted)."""
     deg = np.bincount(ev, minlength=n) + np.bincount(eu, minlength=n)
     vol2 = np.bincount(ev, weights=deg[eu], minlength=n) + np.bincount(eu, weights=deg[ev], minlength=n)
     if ids is not None:
         ev, eu = ev[ids], eu[ids]
-    sel = slice(None)
-    if anchor_hub is not None:
-        dv, du = deg[ev], deg[eu]
-        dp = np.where((dv > du) | ((dv == du) & (ev > eu)), dv, du)
-        sel = dp >= anchor_hub
-    a, b = ev[sel], eu[sel]
-    entries = (deg[a] + deg[b]).sum(dtype=np.float64) + np.minimum(vol2[a], vol2[b]).sum(dtype=np.float64)
-    return 4.0 * entries + (64.0 * len(a) if micro else 0.0), int(len(a))
+    entries = (deg[ev] + deg[eu]).sum(dtype=np.float64) + np.minimum(vol2[ev], vol2[eu]).sum(dtype=np.float64)
+    return 4.0 * entries + (64.0 * len(ev) if micro else 0.0), int(len(ev))
 
 
 def profile_figures():
-    """The bench-figures JSON of the committed k_hub summary, with whether it
-    was taken on the current kernel source."""
+    """The bench-figures JSON of the committed k_cycle_direct summary, with
+    whether it was taken on the current kernel source."""
     import hashlib
 
     out = {}
@@ -389,7 +381,7 @@ def main():
     clocks = ClockSampler(local)
     ev0 = torch.cuda.Event(enable_timing=True)
     ev1 = torch.cuda.Event(enable_timing=True)
-    kernel_ms, hub_ms = [], []
+    kernel_ms, cycle_ms = [], []
     launches0 = ctx.kernel_launches
     clocks.start()
     barrier()
@@ -400,7 +392,7 @@ def main():
             flush.zero_()
         r = step()
         kernel_ms.append(r.kernel_ms)
-        hub_ms.append(r.hub_ms)
+        cycle_ms.append(r.hub_ms)      # the 4-cycle pass
         if ref_totals is not None:
             assert (r.totals == ref_totals).all(), "decomposition not repeatable"
     ev1.record(stream)
@@ -412,31 +404,30 @@ def main():
     units = m if sharded else world * m     # edges decomposed by all ranks together
     value = units * args.steps / (window_ms / 1000.0)
     ms_per_step = window_ms / args.steps
-    log("rank %d: %.1f ms/step, decomposition kernels %.1f ms (k_hub %.1f ms), %.3g edges/s"
-        % (rank, ms_per_step, np.mean(kernel_ms), np.mean(hub_ms), value))
+    log("rank %d: %.1f ms/step, decomposition kernels %.1f ms (4-cycle pass %.1f ms), %.3g edges/s"
+        % (rank, ms_per_step, np.mean(kernel_ms), np.mean(cycle_ms), value))
 
-    # ---- roofline of the dominant kernel (k_hub) ----------------------------
-    # achieved = the per-edge algorithmic bytes of the edges k_hub decomposes
-    # (hub-anchored edges) over k_hub's own mean duration (CUDA events on the
-    # launching stream); traffic, L2 bytes and issue activity come from the
-    # committed ncu summary of the same launch on this workload.
+    # ---- roofline of the dominant pass (4-cycles) ---------------------------
+    # achieved = the per-edge algorithmic bytes of the edges decomposed over the
+    # 4-cycle pass's own mean duration (CUDA events on its stream; its largest
+    # kernel is k_cycle_direct); traffic, L2 bytes and issue activity come from the
+    # committed ncu summary of a k_cycle_direct launch on this workload.
     ev, eu, _ = g.edges(with_order=False)
-    anchor_hub = ctx.thresholds()[0]
-    b_alg, hub_units = algorithmic_bytes(ev, eu, n, micro=True, anchor_hub=anchor_hub, ids=span_ids)
-    hub_s = float(np.mean(hub_ms)) / 1000.0
+    b_alg, cycle_units = algorithmic_bytes(ev, eu, n, micro=True, ids=span_ids)
+    cycle_s = float(np.mean(cycle_ms)) / 1000.0
     peak, peak_src = peaks()
-    achieved = b_alg / hub_s / 1e9
+    achieved = b_alg / cycle_s / 1e9
     prof = profile_figures() if (args.scale, args.order) == (20, "kcore") else {}
     traffic = prof.get("traffic_bytes")
     l2_bytes = prof.get("l2_bytes")
     roofline = {
         "bound": "hbm", "achieved": achieved, "peak": peak, "unit": "GB/s", "frac": achieved / peak,
-        "traffic": traffic, "kernel": "k_hub", "kernel_ms": 1000.0 * hub_s, "units": hub_units,
-        "unit_name": "hub-anchored edges (anchor degree >= %d)" % anchor_hub,
+        "traffic": traffic, "kernel": "k_cycle_direct", "kernel_ms": 1000.0 * cycle_s, "units": cycle_units,
+        "unit_name": "edges",
         "algorithmic_bytes": b_alg,
-        "dram_frac": (traffic / hub_s / 1e9 / peak) if traffic else None,
+        "dram_frac": (traffic / cycle_s / 1e9 / peak) if traffic else None,
         "model_bytes": l2_bytes,
-        "frac_model": (l2_bytes / hub_s / 1e9 / peak) if l2_bytes else None,
+        "frac_model": (l2_bytes / cycle_s / 1e9 / peak) if l2_bytes else None,
         "issue_active": prof.get("issue_active"),
         "profile_on_current_source": prof.get("current_source"),
         "decomposition_kernels_ms": float(np.mean(kernel_ms)),

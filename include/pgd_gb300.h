@@ -277,20 +277,21 @@ pgd_status pgd_server_stats(pgd_server *sv, pgd_server_stat *st);
 pgd_status pgd_server_destroy(pgd_server *sv);
 
 /* ---- thresholds and autotuning (no reference counterpart) --------------
- * Three thresholds steer how the decomposition kernels split work; counts
- * never depend on them.  Until the caller sets them (here or through
- * pgd_autotune), graphs of more than 1.5·2^20 vertices are decomposed with
- * anchor_hub 128 and cache_hub 40, the faster pair on large power-law
- * graphs.  anchor_hub (2..256, default 64): anchors of degree
- * >= it are processed one CTA per anchor with N(p) as a bitmap, below it one
- * warp per edge with N(p) staged and searched.  cache_hub (>= 2, default
- * 32): W(w,p) comes from the anchor's histogram for neighbours of degree >=
- * it (16-bit counters from degree 256, 8-bit below), below it N(w) is
- * scanned per edge.  dense_max (0..2048, default 2048): in a batch,
- * graphs of at most this many vertices are decomposed with whole adjacency
- * rows as bitsets (one 2048-bit row per warp), larger ones with sorted
- * lists; those of average degree >= n/16 also get a 16-bit common-neighbour
- * matrix (about 2·n² bytes of device memory while the batch runs).
+ * Thresholds steer how the decomposition kernels split work; counts never
+ * depend on them.  anchor_hub and cache_hub act on the edge-by-edge kernels,
+ * which decompose samples of fewer than 1/2048 of a graph's edges and the
+ * allocation-free entry point; whole graphs are decomposed by passes that have
+ * no thresholds.  Until the caller sets them (here or through pgd_autotune),
+ * samples of graphs of more than 1.5·2^20 vertices use anchor_hub 128 and
+ * cache_hub 40.  anchor_hub (2..256, default 64): anchors of degree >= it are
+ * processed one CTA per anchor with N(p) as a bitmap, below it one warp per
+ * edge with N(p) staged and searched.  cache_hub (>= 2, default 32): W(w,p)
+ * comes from the anchor's histogram for neighbours of degree >= it (16-bit
+ * counters from degree 256, 8-bit below), below it N(w) is scanned per edge.
+ * dense_max (0..2048, default 2048): in a batch, graphs of at most this many
+ * vertices and of average degree >= n/16 are decomposed with whole adjacency
+ * rows as bitsets and a 16-bit common-neighbour matrix (about 2·n² bytes of
+ * device memory while the batch runs), all others with sorted lists.
  * A fourth, tensor_min_degree (0 or 2..1088, default 64): in those
  * common-neighbour graphs, the edges (p, q) whose lower-degree endpoint q has
  * degree in [tensor_min_degree, 1088] get their 4-clique count from a

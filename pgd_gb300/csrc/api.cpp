@@ -373,12 +373,12 @@ extern "C" pgd_status pgd_decompose(pgd_graph *g, uint32_t flags, pgd_counts *ou
     memset(out, 0, sizeof(*out));
     if (!g->preprocessed && (st = pgd_preprocess(g, "deg", 0))) return st;
     if (!g->sorted && (st = pgd_sort_edges(g, "deg", 0))) return st;
-    // Default thresholds by graph size (counts never depend on them): while the
-    // caller has set none (directly or through pgd_autotune), graphs of more
-    // than kLargeGraph vertices take hub anchors from degree 128 and cached W
-    // from degree 40.  Measured on RMAT scales 21 to 24 (2.1 M to 16.8 M
-    // vertices): 0.3 %, 1.2 %, 1.0 % and 5.7 % faster than the 64 / 32
-    // defaults, which stay the fastest on RMAT scale 20 (1.05 M vertices).
+    // Default thresholds of the edge-by-edge kernels (small samples) by graph size:
+    // while the caller has set none (directly or through pgd_autotune), graphs of
+    // more than kLargeGraph vertices take hub anchors from degree 128 and cached W
+    // from degree 40.  Measured with those kernels on the whole of RMAT scales 21 to
+    // 24: 0.3 %, 1.2 %, 1.0 % and 5.7 % faster than the 64 / 32 defaults, which stay
+    // the fastest on RMAT scale 20 (1.05 M vertices).
     pgd_ctx *ctx = g->ctx;
     constexpr int64_t kLargeGraph = 3ll << 19;   // 1.5 * 2^20
     if (!ctx->thresholds_set && g->n > kLargeGraph) {

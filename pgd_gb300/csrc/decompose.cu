@@ -40,6 +40,11 @@
 // are reproduced with explicitly rounded double intrinsics.  Partial sums
 // are uint64 and wrap exactly like the reference's (addition mod 2^64 is
 // order independent, so the reduction order does not matter).
+//
+// What runs where: whole graphs, samples of at least 1/2048 of the edges and the
+// sparse graphs of a batch go through the passes of rank_path.cu, dense graphs of
+// a batch through the common-neighbour and tensor-core kernels below; the anchor
+// kernels described above take smaller samples and the allocation-free entry point.
 #include <string.h>
 
 #include <cub/cub.cuh>

@@ -126,7 +126,7 @@ __device__ __forceinline__ int pgd_block_excl_scan(int x, int *sh, int *total) {
 // Graphs of at most this many pairs and vertices are built, ordered and ranked by
 // one block per stage, with their sorts in shared memory: what bounds them is the
 // number of launches and waits, not the work.  Build, order and counts of
-// G(96, 0.08) take 145 us against 270 us with the grid-wide stages; 2,048 pairs of
+// G(96, 0.06) take 145 us against 270 us with the grid-wide stages; 2,048 pairs of
 // 300 vertices 230 us against 320 us for 2,049; 2,048 of 8,192 vertices 307 us
 // against 381 us for 8,193.  At 4,096 pairs one SM sorts as long as the launches
 // take (369 against 347 us), so the line lies below that.
