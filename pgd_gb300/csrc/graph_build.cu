@@ -823,6 +823,8 @@ pgd_status pgd_dev_preprocess(pgd_graph *g, int neigh_kind, int s2l) {
         if ((st = pgd_graph_alloc(g, (void **)&g->eu, (g->m + 1) * sizeof(int32_t)))) return st;
     }
     if (nnz == 0) { g->preprocessed = true; return PGD_OK; }
+    // The rank-ordered copy knows the edges by their ids (eslot), which change here.
+    pgd_rank_drop(g);
     // One sort of the m entries above the diagonal by (row, key, rank) where a
     // 64-bit word holds them (32-bit where that does); else the rows' segments of
     // all 2m entries are sorted.

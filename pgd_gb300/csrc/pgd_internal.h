@@ -87,7 +87,7 @@ struct pgd_graph {
     int64_t top_words = 0;
     int32_t *vrank = nullptr;         // n: rank by (degree desc, id)
     int32_t *adjp_rank = nullptr;     // m: vrank of each adjp entry
-    struct pgd_rank_graph *ranked = nullptr;   // rank-ordered copy (rank_path.cu), built on first use
+    struct pgd_rank_graph *ranked = nullptr;   // rank-ordered copy (rank_path.cu), built on first use of these edge ids
     void *slot = nullptr;             // 2m * 16 B: per adjacency slot {w, vrank(w) | row flag, hubid(w), t}
 };
 
