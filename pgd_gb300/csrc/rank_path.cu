@@ -263,7 +263,7 @@ __global__ void k_rank_bounds(const uint32_t *roff, int ranges, RankMeta *M) {
 // its first entry of degree 1 (those come last); and, from the side of the lower
 // end, the slots of the two directions.
 __global__ void k_rank_slots(const uint32_t *roff, const int32_t *radj, int64_t n, int64_t nnz, RankMeta *M,
-                             uint32_t *wcode, int32_t *tw, int32_t *rup, uint32_t *bend) {
+                             uint32_t *wcode, uint32_t *tw, int32_t *rup, uint32_t *bend) {
     const int lane = threadIdx.x & 31;
     const int64_t stride = (int64_t)gridDim.x * blockDim.x;
     // where each tier's counters end, from the tiers (then kept for the others)
@@ -292,8 +292,8 @@ __global__ void k_rank_slots(const uint32_t *roff, const int32_t *radj, int64_t 
         if (x >= n2 ? first || radj[p - 1] < n2 : last) bend[r] = (uint32_t)(x >= n2 ? p : p + 1);
         if (x < r) {
             const uint32_t s = lower_bound_u(radj, roff[x], roff[x + 1], r);
-            tw[p] = (int32_t)s;
-            tw[s] = (int32_t)p;
+            tw[p] = s;
+            tw[s] = (uint32_t)p;
             if (last || radj[p + 1] > r) {
                 const uint32_t up = (uint32_t)p + 1 - roff[r];
                 rup[r] = (int32_t)up;
@@ -305,16 +305,16 @@ __global__ void k_rank_slots(const uint32_t *roff, const int32_t *radj, int64_t 
 
 __global__ void k_rank_eslot(const int32_t *ev, const int32_t *eu, const int32_t *vrank, const uint32_t *roff,
                              const int32_t *rup, const int32_t *radj, const int32_t *vgraph, const uint8_t *vmask,
-                             int64_t m, int32_t *eslot) {
+                             int64_t m, uint32_t *eslot) {
     for (int64_t e = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; e < m; e += (int64_t)gridDim.x * blockDim.x) {
         const int32_t v = ev[e];
         if (vmask && vmask[vgraph[v]]) {
-            eslot[e] = -1;
+            eslot[e] = kFull;   // not read
             continue;
         }
         const int32_t a = vrank[v], b = vrank[eu[e]];
         const int32_t r = max(a, b), x = min(a, b);
-        eslot[e] = (int32_t)lower_bound_u(radj, roff[r], roff[r] + (uint32_t)rup[r], x);
+        eslot[e] = lower_bound_u(radj, roff[r], roff[r] + (uint32_t)rup[r], x);
     }
 }
 
@@ -330,7 +330,7 @@ __global__ void k_rank_bpos(const uint32_t *roff, const int32_t *radj, int n2, i
 
 // Wedges of every top vertex u (its lower neighbours' entries below u), with
 // one atomic per warp where its slots belong to one row.
-__global__ void k_rank_wedges(const uint32_t *roff, const int32_t *radj, const int32_t *tw, const uint32_t *bend,
+__global__ void k_rank_wedges(const uint32_t *roff, const int32_t *radj, const uint32_t *tw, const uint32_t *bend,
                               int64_t n, const RankMeta *M, uint32_t *wd) {
     const int lane = threadIdx.x & 31;
     const int32_t n2 = (int32_t)M->tier[4];
@@ -341,7 +341,7 @@ __global__ void k_rank_wedges(const uint32_t *roff, const int32_t *radj, const i
         const int u = rows_of_warp(roff, n, (uint32_t)p0, (uint32_t)p, lane);
         uint32_t c = 0;
         const int32_t v = radj[p];
-        if (p0 + lane < nnz2 && v > u && v < n2) c = bend[v] - (uint32_t)tw[p] - 1;
+        if (p0 + lane < nnz2 && v > u && v < n2) c = bend[v] - tw[p] - 1;
         const int u0 = __shfl_sync(kFull, u, 0);
         if (__all_sync(kFull, u == u0)) {
             c = __reduce_add_sync(kFull, c);
@@ -412,7 +412,8 @@ struct RankSmallArgs {
     uint32_t *bend;
     int32_t *radj;
     uint32_t *wcode;
-    int32_t *tw, *eslot, *lists;
+    uint32_t *tw, *eslot;
+    int32_t *lists;
     unsigned long long *hbase;
     uint32_t *wd;
     RankMeta *M, *host;       // the sizes, on the device and in page-locked memory
@@ -524,8 +525,8 @@ __global__ void __launch_bounds__(kSmallThreads) k_rank_small(RankSmallArgs A) {
         if (x >= n2 ? first || rad[p - 1] < n2 : last) A.bend[r] = (uint32_t)(x >= n2 ? p : p + 1);
         if (x < r) {
             const uint32_t s = find(x, r);
-            A.tw[p] = (int32_t)s;
-            A.tw[s] = p;
+            A.tw[p] = s;
+            A.tw[s] = (uint32_t)p;
             if (last || rad[p + 1] > r) {
                 const uint32_t up = (uint32_t)p + 1 - roff[r];
                 A.rup[r] = (int32_t)up;
@@ -535,13 +536,13 @@ __global__ void __launch_bounds__(kSmallThreads) k_rank_small(RankSmallArgs A) {
     }
     for (int e = tid; e < A.m; e += kSmallThreads) {
         const uint32_t a = vr[A.ev[e]], b = vr[A.eu[e]];
-        A.eslot[e] = (int32_t)find(max(a, b), min(a, b));
+        A.eslot[e] = find(max(a, b), min(a, b));
     }
     __syncthreads();
     // wedges below each vertex, and the lists
     for (int p = tid; p < nnz; p += kSmallThreads) {
         const uint32_t u = (uint32_t)(w[p] >> kSmallIdBits), v = rad[p];
-        if (v > u && v < n2) atomicAdd(wd + u, A.bend[v] - (uint32_t)A.tw[p] - 1);
+        if (v > u && v < n2) atomicAdd(wd + u, A.bend[v] - A.tw[p] - 1);
     }
     __syncthreads();
     for (int x = tid; x < (int)n2; x += kSmallThreads) {
@@ -609,7 +610,7 @@ struct CycArgs {
     const int32_t *rup;
     const int32_t *radj;
     const uint32_t *wcode;
-    const int32_t *tw;
+    const uint32_t *tw;
     const uint32_t *bend;
     const uint32_t *bpos;
     int n2;
@@ -656,7 +657,7 @@ __device__ __forceinline__ void walk_wedges(const CycArgs &A, Walk<NT> &W, uint3
         uint32_t s0 = 0;
         if (j < j1) {
             const int32_t v = __ldg(A.radj + j);
-            s0 = (uint32_t)__ldg(A.tw + j) + 1;
+            s0 = __ldg(A.tw + j) + 1;
             len = (int)(__ldg(A.bend + v) - s0);
         }
         const int incl = pgd_warp_incl_scan(len);
@@ -782,7 +783,7 @@ __device__ __forceinline__ void walk_rows(const CycArgs &A, uint32_t u, int k0, 
     // the part of row radj[j] that ends wedges of u in the ranges: start and length
     auto row_of = [&](uint32_t j, uint32_t &s0) {
         const int32_t v = __ldg(A.radj + j);
-        s0 = (uint32_t)__ldg(A.tw + j) + 1;
+        s0 = __ldg(A.tw + j) + 1;
         uint32_t e0 = __ldg(A.bend + v);
         if (A.bpos) {
             if (k1 < A.ranges) e0 = __ldg(A.bpos + (int64_t)(k1 - 1) * A.n2 + v);
@@ -1022,7 +1023,7 @@ __global__ void __launch_bounds__(kWarpThreads) k_cycle_warp(CycArgs A) {
                     int len = 0;
                     uint32_t s0 = 0;
                     if (j < j1) {
-                        s0 = (uint32_t)__ldg(A.tw + j) + 1;
+                        s0 = __ldg(A.tw + j) + 1;
                         len = (int)(__ldg(bend + __ldg(A.radj + j)) - s0);
                     }
                     FlatRows F(len, lane);
@@ -1503,8 +1504,8 @@ __global__ void __launch_bounds__(kWarpThreads) k_clique_warp(EgoArgs A) {
 
 struct CloseArgs {
     pgd_rank_out o;
-    const int32_t *eslot;
-    const int32_t *tw;
+    const uint32_t *eslot;
+    const uint32_t *tw;
     const uint32_t *t;
     const unsigned long long *dk;
     const uint32_t *cyc;
@@ -1545,7 +1546,7 @@ __global__ void __launch_bounds__(kThreads) k_rank_close(CloseArgs A) {
         unsigned long long t = 0, k4 = 0, c4 = 0;
         if (act) {
             const int32_t id = o.order[e];
-            const int32_t j = __ldg(A.eslot + id);
+            const uint32_t j = __ldg(A.eslot + id);
             dv = __ldg(o.deg + __ldg(o.ev + id));
             du = __ldg(o.deg + __ldg(o.eu + id));
             const uint32_t tt = __ldg(A.t + j);
@@ -1746,8 +1747,8 @@ pgd_status pgd_rank_build(pgd_graph *g, int64_t nnz, const int32_t *vgraph, cons
     R->bend = K.take<uint32_t>(nb);
     R->radj = K.take<int32_t>(eb);
     R->wcode = K.take<uint32_t>(eb);
-    R->tw = K.take<int32_t>(eb);
-    R->eslot = K.take<int32_t>(mb);
+    R->tw = K.take<uint32_t>(eb);
+    R->eslot = K.take<uint32_t>(mb);
     R->lists = K.take<int32_t>(lb);
     R->hbase = K.take<unsigned long long>(hb);
     Tmp tg(ctx);

@@ -15,8 +15,8 @@ struct pgd_rank_graph {
     int32_t *rup = nullptr;      // n: entries of the row that are ranked above it (its first ones)
     int32_t *radj = nullptr;     // nnz: ranks, ascending in each row
     uint32_t *wcode = nullptr;   // nnz: bit address of the entry's counter
-    int32_t *tw = nullptr;       // nnz: slot of the reversed edge
-    int32_t *eslot = nullptr;    // per edge id: slot of the edge in the row of its lower-ranked end (or -1)
+    uint32_t *tw = nullptr;      // nnz: slot of the reversed edge (slots take all 32 bits: up to 2^31 - 1 edges)
+    uint32_t *eslot = nullptr;   // per edge id: slot of the edge in the row of its lower-ranked end (all ones: none)
     uint32_t *bend = nullptr;    // n: first entry of the row whose vertex has degree 1
     uint32_t *bpos = nullptr;    // (nranges - 1) x n2: first entry of the row at or beyond an inner range
                                  // boundary (null: searched when needed)
