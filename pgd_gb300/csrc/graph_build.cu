@@ -19,6 +19,7 @@
 #include "cluster_ptx.cuh"
 #include "pgd_internal.h"
 #include "pgd_kernels.cuh"
+#include "size_rules.h"
 
 namespace {
 
@@ -360,12 +361,6 @@ __global__ void k_keys_to_ids(const uint64_t *keys, int64_t m, int s2l, int idb,
     }
 }
 
-int bit_length(uint64_t x) {
-    int b = 0;
-    while (x) { b++; x >>= 1; }
-    return b;
-}
-
 }  // namespace
 
 // ---------------------------------------------------------------------------
@@ -587,7 +582,7 @@ static pgd_status build_small(pgd_graph *g, const int32_t *h_src, const int32_t 
     }
     g->adj = adj;
     g->rank = rank;
-    const int cb = std::max(1, bit_length((uint64_t)n)), ib = std::max(1, bit_length((uint64_t)k));
+    const int cb = std::max(1, pgd_bit_length((uint64_t)n)), ib = std::max(1, pgd_bit_length((uint64_t)k));
     const int P = pgd_small_words(2 * k);
     PGD_LAUNCH(ctx, k_small_build, 1, kSmallThreads, P * sizeof(uint64_t), p_src, p_dst, (int)k, (int)n, cb, ib, P, g->off,
                adj, rank, g->deg, (SmallResult *)ctx->pin);
@@ -680,14 +675,14 @@ pgd_status pgd_build_from_device_pairs(pgd_graph *g, const int32_t *d_src, const
                    d_src, d_dst, k, (int *)stats, stats + 1, stats + 2);
     PGD_CUDA(ctx, pgd_fetch(ctx, 0, stats, 3 * sizeof(unsigned long long)));
     PGD_CUDA(ctx, cudaStreamSynchronize(s));
-    const int max_id = pgd_pinned<int>(ctx, 0);
+    const int64_t max_id = pgd_pinned<int>(ctx, 0);
     if (pgd_pinned<unsigned long long>(ctx, 16)) return pgd_fail(ctx, PGD_EINVAL, "negative vertex id in edge list");
     g->self_loops = pgd_pinned<int64_t>(ctx, 8);
-    g->n = std::max<int64_t>(n_min, (int64_t)max_id + 1);
+    g->n = std::max<int64_t>(n_min, max_id + 1);
     const int64_t valid = 2 * (k - g->self_loops), ne = 2 * k;
     // a word holds row and column on the bits that ids up to max_id + 1 need
-    const int cb = std::max(1, bit_length((uint64_t)(max_id + 1)));
-    const uint64_t sentinel = (uint64_t)(uint32_t)(max_id + 1) << cb;
+    const int cb = pgd_id_bits(max_id);
+    const uint64_t sentinel = (uint64_t)(max_id + 1) << cb;
     uint64_t *keys = nullptr, *keys2 = nullptr;
     uint32_t *vals = nullptr, *vals2 = nullptr;
     size_t tb = 0;
@@ -749,7 +744,7 @@ pgd_status pgd_build_from_csr(pgd_graph *g, const int64_t *h_off, const int32_t 
     if ((st = pgd_tmp_alloc(ctx, (void **)&vals2, nz1 * sizeof(uint32_t)))) return st;
     unsigned long long *bad = ctx->d_ctr;
     PGD_CUDA(ctx, cudaMemsetAsync(bad, 0, sizeof(unsigned long long), s));
-    const int cb = std::max(1, bit_length((uint64_t)n));
+    const int cb = std::max(1, pgd_bit_length((uint64_t)n));
     if (nnz) PGD_LAUNCH(ctx, k_csr_entries, grid_for(nnz), kThreads, 0, d_off, d_adj, n, nnz, cb, keys, vals, bad);
     unsigned long long h_bad = 0;
     PGD_CUDA(ctx, cudaMemcpyAsync(&h_bad, bad, sizeof(h_bad), cudaMemcpyDeviceToHost, s));
@@ -829,9 +824,9 @@ pgd_status pgd_dev_preprocess(pgd_graph *g, int neigh_kind, int s2l) {
     // 64-bit word holds them (32-bit where that does); else the rows' segments of
     // all 2m entries are sorted.
     const bool descend = (neigh_kind != PGD_NEIGH_ASREAD) && !s2l;
-    const int rb = std::max(1, bit_length((uint64_t)g->n)), kb = std::max(1, bit_length((uint64_t)g->rank_limit));
+    const int rb = std::max(1, pgd_bit_length((uint64_t)g->n)), kb = std::max(1, pgd_bit_length((uint64_t)g->rank_limit));
     const int db = neigh_kind == PGD_NEIGH_ASREAD ? 0
-                   : std::max(1, bit_length((uint64_t)(neigh_kind == PGD_NEIGH_DEG ? g->max_degree : g->max_core)));
+                   : std::max(1, pgd_bit_length((uint64_t)(neigh_kind == PGD_NEIGH_DEG ? g->max_degree : g->max_core)));
     if (g->m <= kSmallPairs && g->n <= kSmallVertices && 2 * rb + db + kb <= 63) {
         const int P = pgd_small_words(g->m);
         PGD_LAUNCH(ctx, k_small_edges, 1, kSmallThreads, P * sizeof(uint64_t), g->off, g->adj, g->rank, g->deg, g->core,
@@ -1638,7 +1633,7 @@ static pgd_status sort_edges_impl(pgd_graph *g, int kind, int s2l, const int32_t
     default: top = (uint64_t)count; break;
     }
     const bool small = top < 0x80000000ull;
-    const int kb = small ? std::max(1, bit_length(top)) : 32;
+    const int kb = small ? std::max(1, pgd_bit_length(top)) : 32;
     const uint32_t flip = small ? 0u : 0x80000000u;
     size_t tb = 0;
     void *tmp = nullptr;
@@ -1670,7 +1665,7 @@ static pgd_status sort_edges_impl(pgd_graph *g, int kind, int s2l, const int32_t
         uint64_t *keys = nullptr, *keys2 = nullptr;
         if ((st = pgd_tmp_alloc(ctx, (void **)&keys, count * sizeof(uint64_t)))) return st;
         if ((st = pgd_tmp_alloc(ctx, (void **)&keys2, count * sizeof(uint64_t)))) return st;
-        const int idb = std::max(1, bit_length((uint64_t)m));
+        const int idb = std::max(1, pgd_bit_length((uint64_t)m));
         PGD_LAUNCH(ctx, k_sample_keys, grid_for(count), kThreads, 0, g->ev, g->eu, g->deg, g->core, vsum, d_ids, count,
                    kind, s2l, flip, idb, keys);
         if (s2l) cub::DeviceRadixSort::SortKeys(nullptr, tb, keys, keys2, count, 0, kb + idb, s);

@@ -11,7 +11,7 @@ from pgd_gb300 import build as b
 def compiled(tmp_path, body):
     """Output of a program whose main is `body`."""
     src, exe = tmp_path / "t.cpp", tmp_path / "t"
-    src.write_text('#include <stdio.h>\n#include <type_traits>\n#include "rank_path.h"\n'
+    src.write_text('#include <stdio.h>\n#include <type_traits>\n#include "rank_path.h"\n#include "size_rules.h"\n'
                    "int main() {\n%s\nreturn 0;\n}\n" % body)
     r = subprocess.run(["g++", "-std=c++17", "-I" + b.INCLUDE, "-I" + b.CSRC, "-I" + os.path.join(b.CUDA, "include"),
                         "-o", str(exe), str(src)], stdout=subprocess.PIPE, stderr=subprocess.STDOUT, text=True)
@@ -24,3 +24,12 @@ def test_slots_are_unsigned(tmp_path, field):
     """A graph of more than 2^30 edges has slots of 2^31 and more: read as signed
     they would index before the arrays."""
     compiled(tmp_path, "static_assert(std::is_same<decltype(pgd_rank_graph::%s), uint32_t *>::value, \"\");" % field)
+
+
+@pytest.mark.parametrize("max_id", [-1, 0, 1, 6, 7, 2 ** 20 - 1, 2 ** 30, 2 ** 31 - 2, 2 ** 31 - 1])
+def test_packed_words_hold_every_id(tmp_path, max_id):
+    """A word of row and column takes every id up to the largest and the row behind
+    them, in at most 64 bits."""
+    out = compiled(tmp_path, 'printf("%%d", pgd_id_bits((int32_t)%dll));' % max_id)
+    bits = int(out)
+    assert max_id + 1 < 2 ** bits and bits <= 32 and bits == max(1, (max_id + 1).bit_length())
