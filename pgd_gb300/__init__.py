@@ -14,6 +14,7 @@ importing works but every call raises: there is no Python or CPU fallback.
 """
 import ctypes
 import os
+from functools import cached_property
 
 import numpy as np
 
@@ -187,38 +188,38 @@ def close_counts(sums, n, m):
 
 
 class Counts:
-    """Result of one decomposition: views of the 36 words of a pgd_counts."""
-
-    __slots__ = ("_w",)
+    """Result of one decomposition.  The fields are read from the 36 words of a
+    pgd_counts when they are first asked for (a batch has thousands of results,
+    of which a program reads a few fields) and are the result's own from then on."""
 
     def __init__(self, c):
-        self._w = np.frombuffer(c, np.uint64, _WORDS) if isinstance(c, pgd_counts) else c
+        self._w = np.frombuffer(c, np.uint64, _WORDS).copy() if isinstance(c, pgd_counts) else c
 
-    @property
+    @cached_property
     def totals(self):
         return self._w[:NTOTALS]
 
-    @property
+    @cached_property
     def sums(self):
         return self._w[NTOTALS:NTOTALS + NSUMS]
 
-    @property
+    @cached_property
     def n(self):
         return int(self._w[NTOTALS + NSUMS])
 
-    @property
+    @cached_property
     def m(self):
         return int(self._w[NTOTALS + NSUMS + 1])
 
-    @property
+    @cached_property
     def kernel_ms(self):
         return float(self._w[-2:].view(np.float32)[0])
 
-    @property
+    @cached_property
     def hub_ms(self):
         return float(self._w[-2:].view(np.float32)[1])
 
-    @property
+    @cached_property
     def tri_ms(self):
         return float(self._w[-2:].view(np.float32)[2])
 
