@@ -14,7 +14,6 @@ importing works but every call raises: there is no Python or CPU fallback.
 """
 import ctypes
 import os
-from functools import cached_property
 
 import numpy as np
 
@@ -187,41 +186,36 @@ def close_counts(sums, n, m):
     return out
 
 
+def _field(name, part, read=None):
+    """A field of Counts: words `part` (or read() of them) until it is replaced."""
+    def get(self):
+        own = self._own
+        if own is not None and name in own:
+            return own[name]
+        return self._w[part] if read is None else read(self._w[part])
+
+    def put(self, value):
+        self._own = {**(self._own or {}), name: value}
+    return property(get, put)
+
+
 class Counts:
-    """Result of one decomposition.  The fields are read from the 36 words of a
-    pgd_counts when they are first asked for (a batch has thousands of results,
-    of which a program reads a few fields) and are the result's own from then on."""
+    """Result of one decomposition: views of the 36 words of a pgd_counts, read
+    when a field is asked for (a batch has thousands of results, of which a
+    program reads a few fields).  Fields can be replaced."""
+
+    _own = None   # replaced fields
 
     def __init__(self, c):
         self._w = np.frombuffer(c, np.uint64, _WORDS).copy() if isinstance(c, pgd_counts) else c
 
-    @cached_property
-    def totals(self):
-        return self._w[:NTOTALS]
-
-    @cached_property
-    def sums(self):
-        return self._w[NTOTALS:NTOTALS + NSUMS]
-
-    @cached_property
-    def n(self):
-        return int(self._w[NTOTALS + NSUMS])
-
-    @cached_property
-    def m(self):
-        return int(self._w[NTOTALS + NSUMS + 1])
-
-    @cached_property
-    def kernel_ms(self):
-        return float(self._w[-2:].view(np.float32)[0])
-
-    @cached_property
-    def hub_ms(self):
-        return float(self._w[-2:].view(np.float32)[1])
-
-    @cached_property
-    def tri_ms(self):
-        return float(self._w[-2:].view(np.float32)[2])
+    totals = _field("totals", slice(NTOTALS))
+    sums = _field("sums", slice(NTOTALS, NTOTALS + NSUMS))
+    n = _field("n", NTOTALS + NSUMS, int)
+    m = _field("m", NTOTALS + NSUMS + 1, int)
+    kernel_ms = _field("kernel_ms", slice(-2, None), lambda w: float(w.view(np.float32)[0]))
+    hub_ms = _field("hub_ms", slice(-2, None), lambda w: float(w.view(np.float32)[1]))
+    tri_ms = _field("tri_ms", slice(-2, None), lambda w: float(w.view(np.float32)[2]))
 
     def as_dict(self):
         return {k: int(v) for k, v in zip(TOTAL_NAMES, self.totals)}
