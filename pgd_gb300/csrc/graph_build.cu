@@ -894,23 +894,20 @@ pgd_status pgd_dev_preprocess(pgd_graph *g, int neigh_kind, int s2l) {
     return PGD_OK;
 }
 
-// k-core of graphs of up to kCoreClusterEntries adjacency entries: one cluster of
-// sixteen blocks peels the whole graph in one launch.  What bounds it is the chain
-// of steps (832 on R-MAT 20, 448 on R-MAT 16), each a few dependent L2 accesses
-// and a barrier: the cluster's hardware barrier replaces two graph nodes per step
-// (k_core_work and k_core_ctrl below, about 8 us together with their gaps), and
-// no graph is captured and instantiated for the call (180 us).  Sixteen blocks
-// rather than the portable eight for the graphs of few wide steps: milliseconds of
-// the call with 8 / 16 / the whole device, R-MAT 16 2.2 / 2.25 / 3.2, R-MAT 20 12.1 /
-// 8.0 / 12.2, BA of 400,000 2.8 / 2.0 / 2.4 and of 1M vertices 3.2 / 1.7 / 2.0,
-// geometric with 1M vertices 12.1 / 6.7 / 6.4, G(6000, 0.5) 1.8 / 1.0 / 2.0.
+// k-core of light graphs (pgd_core_light), and of others once their steps have
+// become narrow (pgd_core_narrow): one cluster of sixteen blocks peels the graph in
+// one launch.  What bounds it is the chain of steps (832 on R-MAT 20, 448 on R-MAT
+// 16), each a few dependent L2 accesses and a barrier: the cluster's hardware
+// barrier replaces two graph nodes per step (k_core_work and k_core_ctrl below,
+// about 8 us together with their gaps), and no graph is captured and instantiated
+// for the call (180 us).  Sixteen blocks rather than the portable eight for the
+// steps that are not narrow: milliseconds of the whole call in the cluster with 8 /
+// 16, R-MAT 20 12.1 / 8.0, BA of 400,000 2.8 / 2.0.
 namespace {
 
 constexpr int kCoreBlocks = 16;             // the largest cluster (beyond the portable eight)
 constexpr int kCoreThreads = 1024;
-constexpr int64_t kCoreClusterEntries = 64ll << 20;
-constexpr int64_t kCoreEvenEntries = 16ll << 20;   // the same for graphs of small largest degree:
-constexpr int kCoreEvenDegree = 64;                // few levels, wide steps (the geometric graph above)
+static_assert(kCoreBlocks * kCoreThreads <= kCoreIndexRoom, "thread-strided loops over vertices stay below 2^31");
 constexpr int kCoreLong = 1024;             // rows at least this long are shared by all warps
 
 struct CoreSlot {
@@ -985,32 +982,40 @@ __device__ __forceinline__ void core_rows(const int32_t *adj, unsigned nf, int w
     }
 }
 
-// f and b: two buffers each (n entries) of the frontier's short and long rows;
-// a0, a1: vertices alive.  A level scan moves every alive vertex of count <=
-// level to the frontier and the others to the other alive list; a peel round
-// takes one off the count of the frontier's neighbours.
+// Where the cluster starts: at the beginning (na 0), or where the whole device
+// left off: vertices alive, a frontier of nf vertices in f0 not yet peeled.
+struct CoreStart {
+    int level, removed;
+    unsigned int na, nf;
+};
+
+// f and b: two buffers each of the frontier's short and long rows; a0, a1:
+// vertices alive.  A level scan moves every alive vertex of count <= level to the
+// frontier and the others to the other alive list; a peel round takes one off the
+// count of the frontier's neighbours.
 __global__ void __cluster_dims__(kCoreBlocks, 1, 1) __launch_bounds__(kCoreThreads, 1)
 k_core_cluster(const int64_t *off, const int32_t *adj, const int32_t *deg, int n, int32_t *cur, int32_t *core,
                int32_t *f0, int32_t *f1, int32_t *b0, int32_t *b1, int32_t *a0, int32_t *a1, CoreShared *S,
-               int max_degree) {
+               int max_degree, CoreStart at) {
     const int lane = threadIdx.x & 31;
     const int rank = (int)pgd_cl::cluster_rank();
     constexpr int kAll = kCoreBlocks * kCoreThreads;
     const int t = rank * kCoreThreads + (int)threadIdx.x, w = t >> 5;
     const int t0 = t - lane;
-    for (int v = t; v < n; v += kAll) {
-        cur[v] = deg[v];
-        core[v] = -1;
-        a0[v] = v;
-    }
+    if (at.na == 0)
+        for (int v = t; v < n; v += kAll) {
+            cur[v] = deg[v];
+            core[v] = -1;
+            a0[v] = v;
+        }
     if (t == 0) {
         for (int i = 0; i < 3; i++) S->slot[i] = CoreSlot{0, 0, 0, INT_MAX};
         S->max_core = 0;
         S->failed = 0;
     }
     pgd_cl::cluster_sync();
-    int level = 0, removed = 0;
-    unsigned na = (unsigned)n;
+    int level = at.level, removed = at.removed;
+    unsigned na = at.na ? at.na : (unsigned)n, nf = at.nf, nb = 0;
     long long step = 0;
     const long long max_steps = 2ll * n + max_degree + 8;   // every step removes a vertex or raises the level
     int32_t *ain = a0, *aout = a1, *fin = f0, *fout = f1, *bin = b0, *bout = b1;
@@ -1020,47 +1025,50 @@ k_core_cluster(const int64_t *off, const int32_t *adj, const int32_t *deg, int n
         step++;
         return s;
     };
-    while (removed < n && step < max_steps) {
-        CoreSlot *s = next_slot();
-        int low = INT_MAX;
-        for (unsigned i0 = (unsigned)t0; i0 < na; i0 += kAll) {
-            const unsigned i = i0 + lane;
-            bool leaves = false, stays = false;
-            int32_t v = 0;
-            int d = 0;
-            if (i < na) {
-                v = __ldcg(ain + i);
-                if (__ldcg(core + v) == -1) {
-                    const int c = __ldcg(cur + v);
-                    leaves = c <= level;
-                    stays = !leaves;
-                    if (leaves) {
-                        __stcg(core + v, level);
-                        d = deg[v];
-                    } else {
-                        low = min(low, c);
+    while ((removed < n || nf > 0) && step < max_steps) {
+        if (nf == 0) {   // no frontier left over: a level scan
+            CoreSlot *s = next_slot();
+            int low = INT_MAX;
+            for (unsigned i0 = (unsigned)t0; i0 < na; i0 += kAll) {
+                const unsigned i = i0 + lane;
+                bool leaves = false, stays = false;
+                int32_t v = 0;
+                int d = 0;
+                if (i < na) {
+                    v = __ldcg(ain + i);
+                    if (__ldcg(core + v) == -1) {
+                        const int c = __ldcg(cur + v);
+                        leaves = c <= level;
+                        stays = !leaves;
+                        if (leaves) {
+                            __stcg(core + v, level);
+                            d = deg[v];
+                        } else {
+                            low = min(low, c);
+                        }
                     }
                 }
+                core_append(leaves && d < kCoreLong, v, fin, &s->front, lane);
+                core_append(leaves && d >= kCoreLong, v, bin, &s->lng, lane);
+                core_append(stays, v, aout, &s->alive, lane);
             }
-            core_append(leaves && d < kCoreLong, v, fin, &s->front, lane);
-            core_append(leaves && d >= kCoreLong, v, bin, &s->lng, lane);
-            core_append(stays, v, aout, &s->alive, lane);
+            low = __reduce_min_sync(0xffffffffu, low);
+            if (lane == 0 && low != INT_MAX) atomicMin(&s->min_rest, low);
+            pgd_cl::cluster_sync();
+            nf = __ldcg(&s->front);
+            nb = __ldcg(&s->lng);
+            na = __ldcg(&s->alive);
+            int32_t *x = ain;
+            ain = aout;
+            aout = x;
+            if (nf + nb == 0) {
+                level = max(level + 1, __ldcg(&s->min_rest));   // nobody at this level: on to the smallest count
+                continue;
+            }
+            removed += (int)(nf + nb);
         }
-        low = __reduce_min_sync(0xffffffffu, low);
-        if (lane == 0 && low != INT_MAX) atomicMin(&s->min_rest, low);
-        pgd_cl::cluster_sync();
-        unsigned nf = __ldcg(&s->front), nb = __ldcg(&s->lng);
-        na = __ldcg(&s->alive);
-        int32_t *x = ain;
-        ain = aout;
-        aout = x;
-        if (nf + nb == 0) {
-            level = max(level + 1, __ldcg(&s->min_rest));   // nobody at this level: on to the smallest count
-            continue;
-        }
-        removed += (int)(nf + nb);
         while (nf + nb > 0 && step < max_steps) {
-            s = next_slot();
+            CoreSlot *s = next_slot();
             // one off the count of neighbour y; it leaves when that drops to the level
             auto visit = [&](bool act, int32_t y) {
                 bool leaves = false;
@@ -1095,7 +1103,7 @@ k_core_cluster(const int64_t *off, const int32_t *adj, const int32_t *deg, int n
             nf = __ldcg(&s->front);
             nb = __ldcg(&s->lng);
             removed += (int)(nf + nb);
-            x = fin;
+            int32_t *x = fin;
             fin = fout;
             fout = x;
             x = bin;
@@ -1331,25 +1339,14 @@ cudaError_t pgd_build_limits() {
     return e;
 }
 
-// *launched false: the device has no room for the cluster, nothing was done
-static pgd_status cores_by_cluster(pgd_graph *g, bool *launched) {
+// Waits for a peeling by one block or the cluster, whose work array it frees.
+// *launched false: the device has no room for the cluster, nothing was done.
+static pgd_status cores_result(pgd_graph *g, void *work, const CoreShared *S, bool *launched) {
     pgd_ctx *ctx = g->ctx;
-    cudaStream_t s = ctx->stream;
-    const int64_t n = g->n;
-    int32_t *work = nullptr;
-    pgd_status st;
-    const size_t lists = (7 * (size_t)n * sizeof(int32_t) + 15) & ~(size_t)15;
-    if ((st = pgd_tmp_alloc(ctx, (void **)&work, lists + sizeof(CoreShared)))) return st;
-    CoreShared *S = (CoreShared *)((uint8_t *)work + lists);
-    if (g->max_degree < 65536 && 2 * g->m <= kCoreSmallEntries && core_small_bytes(n) <= (size_t)kCoreSmallBytes)
-        PGD_LAUNCH(ctx, k_core_block, 1, kCoreThreads, core_small_bytes(n), g->off, g->adj, g->deg, (int)n, g->core, S);
-    else
-        PGD_LAUNCH(ctx, k_core_cluster, kCoreBlocks, kCoreThreads, 0, g->off, g->adj, g->deg, (int)n, work, g->core,
-               work + n, work + 2 * n, work + 3 * n, work + 4 * n, work + 5 * n, work + 6 * n, S, g->max_degree);
     cudaError_t e = cudaGetLastError();
     *launched = e != cudaErrorLaunchOutOfResources && e != cudaErrorInvalidClusterSize;
     if (e == cudaSuccess) e = pgd_fetch(ctx, 0, S, sizeof(CoreShared));
-    if (e == cudaSuccess) e = cudaStreamSynchronize(s);
+    if (e == cudaSuccess) e = cudaStreamSynchronize(ctx->stream);
     pgd_tmp_free(ctx, work);
     if (!*launched) return PGD_OK;
     if (e != cudaSuccess) return pgd_cuda_fail(ctx, e, "k-core peeling");
@@ -1360,13 +1357,31 @@ static pgd_status cores_by_cluster(pgd_graph *g, bool *launched) {
     return PGD_OK;
 }
 
-// Larger graphs, on the whole device.
+// A light graph, by one block or the cluster.
+static pgd_status cores_light(pgd_graph *g, bool *launched) {
+    pgd_ctx *ctx = g->ctx;
+    const int64_t n = g->n;
+    int32_t *work = nullptr;
+    pgd_status st;
+    const size_t lists = (7 * (size_t)n * sizeof(int32_t) + 15) & ~(size_t)15;
+    if ((st = pgd_tmp_alloc(ctx, (void **)&work, lists + sizeof(CoreShared)))) return st;
+    CoreShared *S = (CoreShared *)((uint8_t *)work + lists);
+    if (g->max_degree < 65536 && 2 * g->m <= kCoreSmallEntries && core_small_bytes(n) <= (size_t)kCoreSmallBytes)
+        PGD_LAUNCH(ctx, k_core_block, 1, kCoreThreads, core_small_bytes(n), g->off, g->adj, g->deg, (int)n, g->core, S);
+    else
+        PGD_LAUNCH(ctx, k_core_cluster, kCoreBlocks, kCoreThreads, 0, g->off, g->adj, g->deg, (int)n, work, g->core,
+               work + n, work + 2 * n, work + 3 * n, work + 4 * n, work + 5 * n, work + 6 * n, S, g->max_degree,
+               CoreStart{0, 0, 0, 0});
+    return cores_result(g, work, S, launched);
+}
+
+// Other graphs: on the whole device, until their steps are narrow.
 // Device-driven peeling: the state machine below replaces a host loop with
 // one round trip per level and per peel round.  Each step is a work kernel
 // (a level scan or a peel round, chosen from the state) and a one-thread
 // control kernel that applies the transition; a block of kCoreSteps steps is
 // captured once as a CUDA graph and replayed until the control kernel
-// reports that every vertex has a core number.  A level scan reads only the
+// reports that every vertex has a core number or the steps are narrow.  A level scan reads only the
 // vertices still alive at the previous scan (a compacted list, rewritten by
 // each scan), so the scans shrink as the peeling goes inward.
 namespace {
@@ -1375,6 +1390,7 @@ struct CoreState {
     int level, mode, sel, done, failed, min_rest;
     unsigned int cnt[2];          // frontier sizes of buffers 0 and 1
     long long removed, steps, max_steps;
+    long long scanned;            // vertices that the scans have read
     int asel;                     // alive list read by the next scan
     unsigned int acnt[2];         // alive list sizes
 };
@@ -1437,6 +1453,7 @@ __global__ void k_core_ctrl(CoreState *st, int64_t n) {
     const int sel = st->sel;
     if (st->mode == kCoreScan) {
         // the scan's survivors are the next alive list
+        st->scanned += st->acnt[st->asel];
         st->asel ^= 1;
         st->acnt[st->asel ^ 1] = 0;
         const unsigned int f = st->cnt[sel];
@@ -1481,9 +1498,9 @@ pgd_status pgd_dev_cores(pgd_graph *g) {
         if ((st = pgd_graph_alloc(g, (void **)&g->core, (n + 1) * sizeof(int32_t)))) return st;
     }
     if (n == 0) { g->has_cores = true; g->max_core = 0; return PGD_OK; }
-    if (2 * g->m <= (g->max_degree <= kCoreEvenDegree ? kCoreEvenEntries : kCoreClusterEntries)) {
+    if (pgd_core_light(n, 2 * g->m)) {
         bool launched = false;
-        const pgd_status st = cores_by_cluster(g, &launched);
+        const pgd_status st = cores_light(g, &launched);
         if (launched || st) return st;
     }
     int32_t *cur = nullptr, *fa = nullptr, *fb = nullptr, *aa = nullptr, *ab = nullptr;
@@ -1531,13 +1548,32 @@ pgd_status pgd_dev_cores(pgd_graph *g) {
         release();
         return pgd_cuda_fail(ctx, e, "k-core step graph");
     }
-    int done = 0;
-    while (!done) {
+    bool narrow = false, room = true;   // room: the device takes the cluster
+    while (!h.done && !narrow) {
+        const CoreState was = h;
         e = cudaGraphLaunch(exec, s);
-        if (e == cudaSuccess) e = cudaMemcpyAsync(&done, &d_st->done, sizeof(int), cudaMemcpyDeviceToHost, s);
+        if (e == cudaSuccess) e = pgd_fetch(ctx, 0, d_st, sizeof(h));
         if (e == cudaSuccess) e = cudaStreamSynchronize(s);
         if (e != cudaSuccess) break;
+        h = pgd_pinned<CoreState>(ctx, 0);
         ctx->launches += 2 * kCoreSteps;
+        narrow = room && !h.done &&
+                 pgd_core_narrow(n, 2 * g->m, kCoreSteps, h.scanned - was.scanned, h.removed - was.removed);
+        if (!narrow) continue;
+        // the steps are narrow: the rest in the cluster, from the state between two steps
+        int32_t *work = nullptr;
+        const size_t lists = (2 * (size_t)n * sizeof(int32_t) + 15) & ~(size_t)15;
+        if (pgd_tmp_alloc(ctx, (void **)&work, lists + sizeof(CoreShared))) {
+            room = narrow = false;
+            continue;
+        }
+        CoreShared *S = (CoreShared *)((uint8_t *)work + lists);
+        const bool peel = h.mode == kCorePeel;
+        PGD_LAUNCH(ctx, k_core_cluster, kCoreBlocks, kCoreThreads, 0, g->off, g->adj, g->deg, (int)n, cur, g->core,
+                   h.sel ? fb : fa, h.sel ? fa : fb, work, work + n, h.asel ? ab : aa, h.asel ? aa : ab, S,
+                   g->max_degree, CoreStart{h.level, (int)h.removed, h.acnt[h.asel], peel ? h.cnt[h.sel] : 0u});
+        st = cores_result(g, work, S, &room);
+        narrow = room;
     }
     cudaGraphExecDestroy(exec);
     cudaGraphDestroy(graph);
@@ -1545,9 +1581,11 @@ pgd_status pgd_dev_cores(pgd_graph *g) {
         release();
         return pgd_cuda_fail(ctx, e, "k-core peeling");
     }
-    PGD_CUDA(ctx, cudaMemcpyAsync(&h, d_st, sizeof(h), cudaMemcpyDeviceToHost, s));
+    if (narrow) {
+        release();
+        return st;
+    }
     int *d_mc = (int *)d_st;
-    PGD_CUDA(ctx, cudaStreamSynchronize(s));
     if (h.failed) {
         release();
         return pgd_fail(ctx, PGD_EINVAL, "k-core peeling did not converge");

@@ -16,3 +16,36 @@ inline int pgd_id_bits(int64_t max_id) {
     const int b = pgd_bit_length((uint64_t)(max_id + 1));
     return b > 0 ? b : 1;
 }
+
+// k-core: by one block or a cluster of sixteen in one launch, or by steps of the
+// whole device.  The cluster saves a captured graph (0.33 ms with its read-backs)
+// and 3 us a step, and has a tenth of the device's bandwidth: about 65 ps more per
+// row entry, and three quarters of that per vertex scanned.  A step of 46,000
+// entries costs the same on both; the line lies lower because steps may widen
+// again (a random graph of 65,536 vertices and 16.7 M entries 1.55 ms at 16,000,
+// 2.2 ms from 24,000 on, 1.56 ms without the cluster).
+constexpr int64_t kCoreLightWeight = 6000000;   // entries and vertices that cost what the captured graph does
+constexpr int64_t kCoreNarrowWeight = 16000;    // entries and vertices of a narrow step, on average
+constexpr int64_t kCoreIndexRoom = 1 << 16;     // vertices are counted in 32 bits, with strides of at most this
+
+inline bool pgd_core_fits(int64_t n) { return n <= 0x7fffffffll - kCoreIndexRoom; }
+
+// Graphs that the cluster takes from the start.  Milliseconds, cluster / device, on
+// both sides of the line: G(n, p) of 2^18 vertices with 5.24 M entries 1.04 / 1.13,
+// 6.29 M 1.10 / 0.94; of 2^20 with 4.19 M 1.07 / 1.18, 7.34 M 1.60 / 1.30; half a
+// million pairs among 4 M vertices 1.03 / 1.27, among 16 M 4.08 / 3.47.
+inline bool pgd_core_light(int64_t n, int64_t entries) {
+    return pgd_core_fits(n) && entries + n / 4 * 3 <= kCoreLightWeight;
+}
+
+// Whether `steps` steps of the whole device, which scanned and removed so many
+// vertices, were narrow: the cluster then takes the rest.  Milliseconds, device
+// alone / with the cluster: R-MAT 20 13.5 / 9.1, R-MAT 22 with 2 edges per vertex
+// 7.1 / 5.5, a 2000 x 2000 grid 11.2 / 9.0, geometric graphs of 500,000 vertices
+// and degree 60 and 100 10.2 / 9.7 and 15.8 / 14.7, BA of 400,000 2.85 / 2.20; a
+// random graph of 1M vertices and degree 50 and other wide ones stay: 2.46 / 2.46
+// (5.4 in the cluster from the start).
+inline bool pgd_core_narrow(int64_t n, int64_t entries, int64_t steps, int64_t scanned, int64_t removed) {
+    return pgd_core_fits(n) &&
+           0.75 * (double)scanned + (double)removed * ((double)entries / (double)n) <= (double)(steps * kCoreNarrowWeight);
+}

@@ -33,3 +33,23 @@ def test_packed_words_hold_every_id(tmp_path, max_id):
     out = compiled(tmp_path, 'printf("%%d", pgd_id_bits((int32_t)%dll));' % max_id)
     bits = int(out)
     assert max_id + 1 < 2 ** bits and bits <= 32 and bits == max(1, (max_id + 1).bit_length())
+
+
+@pytest.mark.parametrize("n,entries", [(2 ** 31 - 2 ** 16, 2), (2 ** 31 - 16385, 2 ** 20), (2 ** 31 - 1, 2), (2 ** 31, 0),
+                                       (2 ** 31, 2 ** 32 - 2)])
+def test_core_kernels_that_count_in_32_bits_take_no_such_graph(tmp_path, n, entries):
+    """Few edges on large ids: the cluster's loops over vertices would pass 2^31."""
+    out = compiled(tmp_path, 'printf("%%d %%d", pgd_core_light(%dll, %dll), pgd_core_narrow(%dll, %dll, 64, 0, 0));'
+                   % (n, entries, n, entries))
+    assert out == "0 0"
+
+
+def test_core_choice_follows_the_measured_sides(tmp_path):
+    """Light graphs by the cluster, wide ones by the device until their steps are narrow."""
+    light = [(1, 0), (65473, 1818884), (262144, 5242608), (4194304, 999926), (1048576, 4194282)]
+    heavy = [(262144, 6291128), (16777216, 999926), (4194305, 8388608), (1048576, 52427448), (100, 2 ** 32 - 2)]
+    body = "".join('printf("%%d", pgd_core_light(%dll, %dll));' % x for x in light + heavy)
+    # steps of a path (two vertices leave), and of a random graph (every vertex scanned again and again)
+    body += 'printf("%d%d", pgd_core_narrow(4000000, 8000000, 64, 0, 128), ' \
+            'pgd_core_narrow(1048576, 52427448, 64, 20000000, 1000));'
+    assert compiled(tmp_path, body) == "1" * len(light) + "0" * len(heavy) + "10"
