@@ -78,6 +78,9 @@ constexpr int kCycWarpMax = 512;
 constexpr int kCycHashMax = 4096;
 constexpr int kMaxRanges = 8192;
 constexpr int64_t kKeepBytes = 16ll << 30;     // largest bound of the triangle lists kept between the passes
+constexpr int64_t kTableBytes = 8ll << 30;     // largest lists and tables of the blocks of kEgoGlobal
+constexpr int64_t kListFloor = 256ll << 20;    // lists and tables that are taken without asking for the room (about what
+                                               // the edge-by-edge kernels take)
 constexpr int64_t kBposBytes = 4ll << 30;      // largest table of range boundaries per row
 constexpr uint32_t kDirectWords = 50 * 1024;   // counter words of one item: 200 KB of shared memory
 
@@ -1806,8 +1809,14 @@ pgd_status pgd_rank_build(pgd_graph *g, int64_t nnz, const int32_t *vgraph, cons
     R->nranges = (int32_t)std::min<int64_t>(kMaxRanges, std::max<int64_t>(16, 2 * (2 * words / kDirectWords + 1)));
     PGD_LAUNCH(ctx, k_rank_bounds, 1, 128, 0, R->roff, R->nranges, M);
     const int64_t bpos_bytes = (int64_t)(R->nranges - 1) * n2 * (int64_t)sizeof(uint32_t);
-    if (bpos_bytes <= kBposBytes) {
-        RB_TRY(keep(&R->bpos, (size_t)bpos_bytes));
+    // the table is left out where the budget or the device has no room for it
+    const std::string err = ctx->err;
+    st = bpos_bytes <= kBposBytes ? keep(&R->bpos, (size_t)bpos_bytes) : PGD_ENOMEM;
+    if (st == PGD_ENOMEM) {
+        R->bpos = nullptr;
+        ctx->err = err;
+    } else {
+        RB_TRY(st);
         PGD_LAUNCH(ctx, k_rank_bpos, grid_for((int64_t)n2 * (R->nranges - 1)), kThreads, 0, R->roff, R->radj, n2,
                    R->nranges, M, R->bpos);
     }
@@ -1848,11 +1857,66 @@ static int ego_grid(const pgd_ctx *ctx, const pgd_rank_graph &R, int c) {
     return (int)std::min<int64_t>(R.nlist[c], (int64_t)(ego_wide(ctx, R, c) ? 2 : ego_blocks_per_sm(c)) * ctx->num_sms);
 }
 
+// What the ego classes hold beside the counts per slot: every triangle of pass 1
+// kept for pass 2, or a list of each block of pass 2, which then lists them again;
+// and the tables of the largest neighbourhoods.
+struct EgoMemory {
+    bool keep = false;
+    int64_t hits = 0;             // triangles in the lists
+    int grid[kEgoGlobal] = {0};   // blocks of pass 2 where they are not kept, by class
+    int gblocks = 0;              // blocks of kEgoGlobal
+    int64_t table_bytes = 0;      // each one's tables
+    int64_t bytes() const { return hits * (int64_t)sizeof(uint2) + gblocks * table_bytes; }
+};
+
+// The fastest choice of at most `limit` bytes, and at least a block per class.
+static EgoMemory ego_memory(const pgd_ctx *ctx, const pgd_rank_graph &R, int64_t limit) {
+    EgoMemory E;
+    const int64_t hit = sizeof(uint2);
+    auto blocks_in = [](int64_t bytes, int64_t each, int64_t most) {
+        return (int)std::max<int64_t>(1, std::min(most, bytes / each));
+    };
+    if (R.nlist[kEgoGlobal]) {
+        const int64_t per = (int64_t)R.max_up * (R.max_up - 1) / 2;
+        E.table_bytes = ego_table_bytes(R.max_up, true, true);
+        E.gblocks = blocks_in(std::min(kTableBytes, limit), per * hit + E.table_bytes,
+                              std::min<int64_t>(ctx->num_sms, R.nlist[kEgoGlobal]));
+        E.hits = per * E.gblocks;
+    }
+    const int64_t left = limit - E.gblocks * E.table_bytes;
+    for (int c : {kEgoA, kEgoB, kEgoC}) {
+        if (!R.nlist[c]) continue;
+        const int64_t dmax = std::min(kEgoMax[c], (int)R.max_up), per = dmax * (dmax - 1) / 2;
+        E.grid[c] = blocks_in(left, per * hit, ego_grid(ctx, R, c));
+        E.hits = std::max(E.hits, per * E.grid[c]);
+    }
+    E.keep = R.pairs * hit <= std::min(kKeepBytes, left);
+    if (E.keep) E.hits = R.pairs;
+    return E;
+}
+
+// Bytes that lists and tables may take beyond kListFloor: at most what the context
+// was given, what is left of its budget and half of the device's free memory.
+static int64_t ego_room(const pgd_ctx *ctx) {
+    size_t free_b = 0, total_b = 0;
+    uint64_t reserved = 0, used = 0;   // the pool's: what it holds and does not use is free as well
+    cudaMemPool_t pool;
+    if (cudaMemGetInfo(&free_b, &total_b) != cudaSuccess) free_b = 0;
+    if (cudaDeviceGetDefaultMemPool(&pool, ctx->device) != cudaSuccess ||
+        cudaMemPoolGetAttribute(pool, cudaMemPoolAttrReservedMemCurrent, &reserved) != cudaSuccess ||
+        cudaMemPoolGetAttribute(pool, cudaMemPoolAttrUsedMemCurrent, &used) != cudaSuccess)
+        reserved = used = 0;
+    cudaGetLastError();
+    const uint64_t left = ctx->budget > ctx->resident ? ctx->budget - ctx->resident : 0;
+    const uint64_t room = std::min<uint64_t>(left, (free_b + (reserved - used)) / 2);
+    return std::max<int64_t>(kListFloor, (int64_t)std::min<uint64_t>(room, INT64_MAX / 2));
+}
+
 // The ego classes' launches: pass 1, pass 2 that lists the triangles again, or
 // (kept) pass 2 from the triangles of pass 1.
 static void ego_pass(pgd_ctx *ctx, const pgd_rank_graph &R, EgoArgs A, int pass, unsigned long long *ctr,
-                     uint8_t *tables, int gblocks, int64_t table_bytes) {
-    const bool kept = pass == 2 && A.hcount;
+                     uint8_t *tables, const EgoMemory &mem) {
+    const bool kept = pass == 2 && mem.keep;
     auto args = [&](int c) {
         EgoArgs B = A;
         B.list = R.lists + (int64_t)c * R.n;
@@ -1871,15 +1935,15 @@ static void ego_pass(pgd_ctx *ctx, const pgd_rank_graph &R, EgoArgs A, int pass,
         EgoArgs B = args(kEgoGlobal);
         B.hits_stride = (int64_t)R.max_up * (R.max_up - 1) / 2;
         B.tables = tables;
-        B.tables_stride = table_bytes;
-        EGO_BLOCK(1024, true, gblocks, 0, B, R.max_up);
+        B.tables_stride = mem.table_bytes;
+        EGO_BLOCK(1024, true, mem.gblocks, 0, B, R.max_up);
     }
     for (int c : {kEgoC, kEgoB, kEgoA}) {
         if (!R.nlist[c]) continue;
         EgoArgs B = args(c);
         const int dmax = std::min(kEgoMax[c], (int)R.max_up);
         B.hits_stride = (int64_t)dmax * (dmax - 1) / 2;
-        const int blocks = ego_grid(ctx, R, c);
+        const int blocks = pass == 2 && !kept ? mem.grid[c] : ego_grid(ctx, R, c);
         const size_t smem = (size_t)ego_table_bytes(dmax, !kept, pass == 2);
         if (c == kEgoC || ego_wide(ctx, R, c)) EGO_BLOCK(1024, false, blocks, smem, B, dmax);
         else if (c == kEgoB) EGO_BLOCK(512, false, blocks, smem, B, dmax);
@@ -1981,34 +2045,26 @@ pgd_status pgd_rank_decompose(pgd_ctx *ctx, const pgd_rank_graph &R, const pgd_r
     pgd_status st;
     if (out.npos == 0 || R.nnz == 0) return PGD_OK;
     const int nsm = ctx->num_sms;
-    // triangle lists (pass 2) and the tables of the largest neighbourhoods
-    int64_t hit_count = 0, table_bytes = 0;
-    int gblocks = 0;
-    for (int c : {kEgoA, kEgoB, kEgoC}) {
-        const int64_t dmax = std::min(kEgoMax[c], (int)R.max_up);
-        hit_count = std::max(hit_count, ego_grid(ctx, R, c) * (dmax * (dmax - 1) / 2));
-    }
-    if (R.nlist[kEgoGlobal]) {
-        const int64_t per = (int64_t)R.max_up * (R.max_up - 1) / 2;
-        table_bytes = ego_table_bytes(R.max_up, true, true);
-        // at most about 8 GB of tables and lists, at least one block's
-        gblocks = (int)std::max<int64_t>(1, std::min<int64_t>(std::min<int64_t>(nsm, R.nlist[kEgoGlobal]),
-                                                              (8ll << 30) / (per * 8 + table_bytes)));
-        hit_count = std::max(hit_count, per * gblocks);
-    }
-    // Every triangle of pass 1 is kept for pass 2 where the lists' bound (every
-    // pair of every N+) is at most kKeepBytes; else pass 2 lists them again.
-    const bool keep = R.pairs * (int64_t)sizeof(uint2) <= kKeepBytes;
-    if (keep) hit_count = R.pairs;
-    // one allocation: counters, dk, t, cyc (zeroed), then the lists and tables
+    // one allocation: counters, dk, t, cyc (zeroed), then the lists and tables, in
+    // smaller ones where there is no room
     constexpr int kCounters = 16;   // [0..5) pass 1, [5..10) pass 2, [10..13) 4-cycles
     auto up128 = [](int64_t x) { return (x + 127) & ~(int64_t)127; };
-    const int64_t zeroed = kCounters * 8 + R.nnz * 16;
-    const int64_t at_count = up128(zeroed), at_hits = at_count + up128(keep ? (int64_t)R.n2 * 4 : 0),
-                  at_tables = at_hits + up128(hit_count * (int64_t)sizeof(uint2));
+    const int64_t zeroed = kCounters * 8 + R.nnz * 16, at_count = up128(zeroed);
+    int64_t at_hits = 0, at_tables = 0;
+    EgoMemory mem = ego_memory(ctx, R, INT64_MAX / 2);
+    if (mem.bytes() > kListFloor) mem = ego_memory(ctx, R, ego_room(ctx));
     Tmp tg(ctx);
     uint8_t *work = nullptr;
-    if ((st = tg.alloc(&work, (size_t)(at_tables + gblocks * table_bytes)))) return st;
+    const std::string err = ctx->err;
+    while (true) {
+        at_hits = at_count + up128(mem.keep ? (int64_t)R.n2 * 4 : 0);
+        at_tables = at_hits + up128(mem.hits * (int64_t)sizeof(uint2));
+        st = tg.alloc(&work, (size_t)(at_tables + mem.gblocks * mem.table_bytes));
+        const int64_t had = mem.bytes();
+        if (st != PGD_ENOMEM || (mem = ego_memory(ctx, R, had / 4)).bytes() >= had) break;
+        ctx->err = err;
+    }
+    if (st) return st;
     unsigned long long *ctr = (unsigned long long *)work, *dk = ctr + kCounters;
     uint32_t *t = (uint32_t *)(dk + R.nnz), *cyc = t + R.nnz;
     PGD_CUDA(ctx, cudaMemsetAsync(work, 0, zeroed, s));
@@ -2038,10 +2094,10 @@ pgd_status pgd_rank_decompose(pgd_ctx *ctx, const pgd_rank_graph &R, const pgd_r
     E.dk = dk;
     E.hits = (uint2 *)(work + at_hits);
     E.hbase = R.hbase;
-    E.hcount = keep ? (uint32_t *)(work + at_count) : nullptr;
+    E.hcount = mem.keep ? (uint32_t *)(work + at_count) : nullptr;
     PGD_CUDA(ctx, cudaEventRecord(ctx->evt0, s));
-    ego_pass(ctx, R, E, 1, ctr, work + at_tables, gblocks, table_bytes);
-    ego_pass(ctx, R, E, 2, ctr + 5, work + at_tables, gblocks, table_bytes);
+    ego_pass(ctx, R, E, 1, ctr, work + at_tables, mem);
+    ego_pass(ctx, R, E, 2, ctr + 5, work + at_tables, mem);
     PGD_CUDA(ctx, cudaEventRecord(ctx->evt1, s));
     PGD_CUDA(ctx, side.join());
     CloseArgs Z;

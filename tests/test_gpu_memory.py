@@ -1,0 +1,89 @@
+"""Memory that a decomposition can do without: the triangles kept between the
+passes and the table of range positions of the 4-cycle pass.  Where the budget
+has no room for them the counts are the same, and every class of the passes that
+list the triangles again is run.  All counts are exact."""
+import ctypes
+
+import numpy as np
+import pytest
+
+import pgd_gb300 as pgd
+
+pytestmark = pytest.mark.gpu
+
+MB = 1 << 20
+
+
+def decomposed(budget, src, dst, micro=True):
+    """Counts, rows and resident bytes of a graph in a context of `budget` bytes."""
+    c = pgd.Context(hbm_budget=budget)
+    g = c.graph_from_edges(src, dst, dedup=True)
+    g.sort_edges("deg")
+    r = g.decompose(micro=micro)
+    rows = g.micro() if micro else None
+    held = g.resident_bytes
+    g.destroy()
+    c.close()
+    return r, rows, held
+
+
+def complete(n):
+    a, b = np.triu_indices(n, 1)
+    return a.astype(np.int32), b.astype(np.int32)
+
+
+@pytest.mark.parametrize("kind", ["complete", "dense", "rmat", "geometric"])
+def test_triangles_listed_again(kind):
+    """Lists of more than 256 MB in a context without room for them."""
+    src, dst = {"complete": lambda: complete(1100), "dense": lambda: pgd.erdos_renyi(1300, 0.9, seed=1),
+                "rmat": lambda: pgd.rmat(17, 16, seed=2), "geometric": lambda: pgd.rgg3d(20000, 0.17, seed=3)}[kind]()
+    r, rows, held = decomposed(0, src, dst)
+    w, wrows, _ = decomposed(held + MB, src, dst)
+    assert (r.sums == w.sums).all() and (r.totals == w.totals).all()
+    for a, b in zip(rows, wrows):
+        assert (a == b).all()
+    if kind == "complete":
+        t = 1098
+        assert (wrows[2][:, 0] == t).all() and (wrows[2][:, 2] == t * (t - 1) // 2).all()
+        assert (wrows[2][:, 5] == 0).all()
+
+
+def test_range_positions_searched():
+    """A budget that holds everything but the table of range positions."""
+    src, dst = pgd.rmat(14, 16, seed=4)
+    r, _, held = decomposed(0, src, dst, micro=False)
+    n2 = int((np.bincount(np.concatenate(pgd_edges(src, dst))) >= 2).sum())
+    w, _, small = decomposed(held - 15 * 4 * n2 // 2, src, dst, micro=False)   # half of at least 15 positions a vertex
+    assert small < held
+    assert (r.sums == w.sums).all() and (r.totals == w.totals).all()
+
+
+def pgd_edges(src, dst):
+    lo, hi = np.minimum(src, dst), np.maximum(src, dst)
+    return np.unique(np.stack([lo, hi])[:, lo != hi], axis=1)
+
+
+class Pool:
+    """The device's default memory pool, as the CUDA runtime reports it."""
+
+    def __init__(self):
+        self.rt = ctypes.CDLL("libcudart.so.13")
+        self.pool = ctypes.c_void_p()
+        assert self.rt.cudaDeviceGetDefaultMemPool(ctypes.byref(self.pool), 0) == 0
+
+    def restart(self):
+        assert self.rt.cudaMemPoolSetAttribute(self.pool, 8, ctypes.byref(ctypes.c_uint64(0))) == 0   # UsedMemHigh
+
+    def high(self):
+        v = ctypes.c_uint64()
+        assert self.rt.cudaMemPoolGetAttribute(self.pool, 8, ctypes.byref(v)) == 0
+        return v.value
+
+
+def test_a_small_budget_bounds_the_lists():
+    """1.8 GB of triangles of a complete graph: not where 100 MB are asked for."""
+    src, dst = complete(1100)
+    p = Pool()
+    p.restart()
+    decomposed(100 * MB, src, dst, micro=False)
+    assert p.high() < 700 * MB   # 256 MB of lists, the graph, 16 bytes per entry, sort buffers
