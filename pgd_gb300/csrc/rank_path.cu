@@ -92,8 +92,10 @@ struct RankMeta {
     uint32_t nlist[kClasses];
     unsigned long long direct_wedges;   // wedges of the vertices beyond the lists
     unsigned long long pairs;           // sum of |N+(a)| (|N+(a)| - 1) / 2
-    uint32_t bound[kMaxRanges + 1];   // range boundaries (ranks)
+    uint32_t bound[kMaxRanges + 1];   // range boundaries (ranks); not there where no vertex has items
 };
+constexpr size_t kMetaHead = offsetof(RankMeta, bound);
+static_assert(kMetaHead <= kPinBytes, "the sizes fit the read-back buffer");
 
 // Bit address of the counter of rank r.  A counter of w never exceeds deg(w):
 // 32, 16, 8, 4 or 2 bits by degree (wide ones first, so none straddles a word).
@@ -1712,7 +1714,7 @@ static pgd_status rank_build_large(pgd_graph *g, int64_t nnz, const int32_t *vgr
     PGD_LAUNCH(ctx, k_rank_wedges, grid_for(nnz), kThreads, 0, R->roff, R->radj, R->tw, R->bend, n, M, wd);
     PGD_LAUNCH(ctx, k_rank_lists, grid_for(n), kThreads, 0, R->rup, wd, n, R->lists, R->hbase, M);
     PGD_CUDA(ctx, cudaGetLastError());
-    PGD_CUDA(ctx, pgd_fetch(ctx, 0, M, offsetof(RankMeta, bound)));
+    PGD_CUDA(ctx, pgd_fetch(ctx, 0, M, kMetaHead));
     PGD_CUDA(ctx, cudaStreamSynchronize(s));
     return PGD_OK;
 }
@@ -1741,9 +1743,9 @@ pgd_status pgd_rank_build(pgd_graph *g, int64_t nnz, const int32_t *vgraph, cons
     pgd_pieces K;
     const size_t nb = (n + 1) * sizeof(uint32_t), eb = nnz * sizeof(uint32_t), mb = m * sizeof(int32_t),
                  lb = (size_t)kClasses * n * sizeof(int32_t), hb = n * sizeof(unsigned long long);
-    K.add(sizeof(RankMeta)); K.add(nb); K.add(nb); K.add(nb); K.add(eb); K.add(eb); K.add(eb); K.add(mb); K.add(lb); K.add(hb);
+    K.add(kMetaHead); K.add(nb); K.add(nb); K.add(nb); K.add(eb); K.add(eb); K.add(eb); K.add(mb); K.add(lb); K.add(hb);
     RB_TRY(keep(&K.base, K.bytes));
-    RankMeta *M = K.take<RankMeta>(sizeof(RankMeta));
+    RankMeta *M = K.take<RankMeta>(kMetaHead);
     R->meta = M;
     R->roff = K.take<uint32_t>(nb);
     R->rup = K.take<int32_t>(nb);
@@ -1794,10 +1796,8 @@ pgd_status pgd_rank_build(pgd_graph *g, int64_t nnz, const int32_t *vgraph, cons
     } else {
         RB_TRY(rank_build_large(g, nnz, vgraph, vmask, R, M, tg, &wd, &tmp, &tb));
     }
-    constexpr size_t kHead = offsetof(RankMeta, bound);
-    static_assert(kHead <= kPinBytes, "the sizes fit the read-back buffer");
     RankMeta h;
-    memcpy((void *)&h, ctx->pin, kHead);
+    memcpy((void *)&h, ctx->pin, kMetaHead);
     const int n2 = R->n2 = (int32_t)h.tier[4];
     R->max_up = (int32_t)std::max((uint32_t)kEgoMax[kEgoWarp], h.max_up);
     for (int i = 0; i < kClasses; i++) R->nlist[i] = h.nlist[i];
@@ -1807,6 +1807,12 @@ pgd_status pgd_rank_build(pgd_graph *g, int64_t nnz, const int32_t *vgraph, cons
     // fine enough to balance the items, and at most half an item's counters each
     const int64_t words = R->words = ((int64_t)h.tcode[4] + 31) / 32;
     R->nranges = (int32_t)std::min<int64_t>(kMaxRanges, std::max<int64_t>(16, 2 * (2 * words / kDirectWords + 1)));
+    // the sizes again, with the boundaries behind them
+    const size_t meta_bytes = kMetaHead + ((size_t)R->nranges + 1) * sizeof(uint32_t);
+    RankMeta *full = nullptr;
+    RB_TRY(keep(&full, meta_bytes));
+    RB_CUDA(cudaMemcpyAsync(full, M, kMetaHead, cudaMemcpyDeviceToDevice, s));
+    R->meta = M = full;
     PGD_LAUNCH(ctx, k_rank_bounds, 1, 128, 0, R->roff, R->nranges, M);
     const int64_t bpos_bytes = (int64_t)(R->nranges - 1) * n2 * (int64_t)sizeof(uint32_t);
     // the table is left out where the budget or the device has no room for it

@@ -87,3 +87,10 @@ def test_a_small_budget_bounds_the_lists():
     p.restart()
     decomposed(100 * MB, src, dst, micro=False)
     assert p.high() < 700 * MB   # 256 MB of lists, the graph, 16 bytes per entry, sort buffers
+
+
+def test_small_graphs_hold_little():
+    """A program may keep thousands of them: 96 vertices and 239 edges in less than
+    the 28,532 bytes of the edge-by-edge structures."""
+    _, _, held = decomposed(0, *pgd.erdos_renyi(96, 0.06, seed=1), micro=False)
+    assert held < 28532
