@@ -173,17 +173,7 @@ extern "C" pgd_status pgd_graph_destroy(pgd_graph *g) {
     pgd_graph_free(g, g->core, (g->n + 1) * sizeof(int32_t));
     pgd_graph_free(g, g->order, (g->m + 1) * sizeof(int32_t));
     pgd_graph_free(g, g->micro, (g->m + 1) * PGD_NMICRO * sizeof(uint64_t));
-    pgd_graph_free(g, g->offp, (g->n + 1) * sizeof(int64_t));
-    pgd_graph_free(g, g->adjp, (g->m + 1) * sizeof(int32_t));
-    pgd_graph_free(g, g->hubid, (g->n + 1) * sizeof(int32_t));
-    pgd_graph_free(g, g->vrank, (g->n + 1) * sizeof(int32_t));
-    pgd_graph_free(g, g->adjp_rank, (g->m + 1) * sizeof(int32_t));
-    pgd_graph_free(g, g->slot, (2 * g->m + 1) * 16);
-    pgd_graph_free(g, g->offh, (g->n + 1) * sizeof(int64_t));
-    pgd_graph_free(g, g->adjh, (g->nadjh + 1) * sizeof(int32_t));
-    pgd_graph_free(g, g->toprows, (g->top_words + 1) * sizeof(uint32_t));
-    pgd_graph_free(g, g->vrec, (g->n + 1) * 32);
-    pgd_graph_free(g, g->adj_rank, (2 * g->m + 1) * sizeof(int32_t));
+    pgd_aux_drop(g);
     pgd_rank_drop(g);
     // whatever is left (partial builds) is returned to the budget as well
     g->ctx->resident -= g->bytes;

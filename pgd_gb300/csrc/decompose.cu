@@ -2265,11 +2265,32 @@ cudaError_t pgd_decompose_limits() {
     return e;
 }
 
+void pgd_aux_drop(pgd_graph *g) {
+    const int64_t n = g->n, m = g->m;
+    auto drop = [&](auto *&p, int64_t bytes) {
+        pgd_graph_free(g, p, (size_t)bytes);
+        p = nullptr;
+    };
+    drop(g->offp, (n + 1) * (int64_t)sizeof(int64_t));
+    drop(g->adjp, (m + 1) * (int64_t)sizeof(int32_t));
+    drop(g->hubid, (n + 1) * (int64_t)sizeof(int32_t));
+    drop(g->vrank, (n + 1) * (int64_t)sizeof(int32_t));
+    drop(g->adjp_rank, (m + 1) * (int64_t)sizeof(int32_t));
+    drop(g->slot, (2 * m + 1) * (int64_t)sizeof(int4));
+    drop(g->offh, (n + 1) * (int64_t)sizeof(int64_t));
+    drop(g->adjh, (g->nadjh + 1) * (int64_t)sizeof(int32_t));
+    drop(g->toprows, (g->top_words + 1) * (int64_t)sizeof(uint32_t));
+    drop(g->vrec, (n + 1) * 32);
+    drop(g->adj_rank, (2 * m + 1) * (int64_t)sizeof(int32_t));
+    g->has_aux = false;
+}
+
 static pgd_status build_aux(pgd_graph *g) {
     pgd_ctx *ctx = g->ctx;
     cudaStream_t s = ctx->stream;
     pgd_status st;
     const int64_t n = g->n, nnz = 2 * g->m;
+    g->has_aux = false;   // until the last step
     if (!g->offp) {
         if ((st = pgd_graph_alloc(g, (void **)&g->offp, (n + 1) * sizeof(int64_t)))) return st;
         if ((st = pgd_graph_alloc(g, (void **)&g->adjp, (g->m + 1) * sizeof(int32_t)))) return st;
@@ -2866,17 +2887,31 @@ pgd_status pgd_dev_decompose(pgd_graph *g, bool micro, pgd_counts *out) {
     if (micro && !g->micro) {
         if ((st = pgd_graph_alloc(g, (void **)&g->micro, (g->m + 1) * PGD_NMICRO * sizeof(uint64_t)))) return st;
     }
-    PGD_CUDA(ctx, cudaMemsetAsync(ctx->d_sums, 0, PGD_NSUMS * sizeof(unsigned long long), s));
     StageMs ms;
-    if (g->norder >= g->m / kSampleShare) {
-        if ((st = rank_decompose(g, micro, &ms))) return st;
-    } else {
+    const bool whole = g->norder >= g->m / kSampleShare;
+    auto run = [&]() -> pgd_status {
+        PGD_CUDA(ctx, cudaMemsetAsync(ctx->d_sums, 0, PGD_NSUMS * sizeof(unsigned long long), s));
+        if (whole) return rank_decompose(g, micro, &ms);
         if ((!g->has_aux || g->aux_cache_hub != ctx->cache_hub) && (st = build_aux(g))) return st;
         if ((st = run_decompose(ctx, dev_view(g, micro), (int4 *)g->slot, g->nhubs, g->nhubs_wide, g->max_degree, &ms)))
             return st;
         PGD_CUDA(ctx, pgd_fetch(ctx, 0, ctx->d_sums, PGD_NSUMS * sizeof(unsigned long long)));
         PGD_CUDA(ctx, cudaStreamSynchronize(s));
+        return PGD_OK;
+    };
+    st = run();
+    if (st == PGD_ENOMEM && (whole ? (bool)g->offp : (bool)g->ranked)) {
+        // a graph keeps what either path has built while there is room for both
+        if (whole) {
+            pgd_aux_drop(g);
+        } else {
+            pgd_rank_drop(g);
+            pgd_aux_drop(g);   // built half-way
+        }
+        st = run();
     }
+    if (st && !g->has_aux) pgd_aux_drop(g);
+    if (st) return st;
     memcpy(out->sums, ctx->pin, PGD_NSUMS * sizeof(uint64_t));
     out->n = g->n;
     out->m = g->m;

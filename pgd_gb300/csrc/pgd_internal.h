@@ -112,6 +112,7 @@ pgd_status pgd_cuda_fail(pgd_ctx *ctx, cudaError_t e, const char *what);
 pgd_status pgd_graph_alloc(pgd_graph *g, void **p, size_t bytes);
 void pgd_graph_free(pgd_graph *g, void *p, size_t bytes);
 void pgd_rank_drop(pgd_graph *g);   // frees g's rank-ordered copy, if any
+void pgd_aux_drop(pgd_graph *g);    // frees the edge-by-edge structures, also half-built ones (decompose.cu)
 
 // Stream-ordered temporaries (not counted against the budget).
 pgd_status pgd_tmp_alloc(pgd_ctx *ctx, void **p, size_t bytes);

@@ -94,3 +94,35 @@ def test_small_graphs_hold_little():
     the 28,532 bytes of the edge-by-edge structures."""
     _, _, held = decomposed(0, *pgd.erdos_renyi(96, 0.06, seed=1), micro=False)
     assert held < 28532
+
+
+def test_either_path_makes_room_for_the_other():
+    """A budget that holds the structures of whole graphs or those of small samples,
+    as it held the one set that served both."""
+    src, dst = pgd.rmat(14, 16, seed=5)
+    big = pgd.Context()
+    g = big.graph_from_edges(src, dst, dedup=True)
+    g.sort_edges("deg")
+    ids = np.arange(7, g.m, g.m // 60, dtype=np.int64)     # below 1/2048 of the edges
+    assert len(ids) < g.m // 2048
+    g.sort_edges_sample(ids, "natural", s2l=True)
+    part = g.decompose(micro=True)
+    part_rows, held = g.micro(), g.resident_bytes          # structures of small samples alone
+    g.sort_edges("deg")
+    whole = g.decompose(micro=True)
+    assert g.resident_bytes > held                         # both
+    g.destroy()
+    big.close()
+    c = pgd.Context(hbm_budget=held + MB)
+    g = c.graph_from_edges(src, dst, dedup=True)
+    for _ in range(2):
+        g.sort_edges("deg")
+        assert (g.decompose(micro=True).sums == whole.sums).all()
+        g.sort_edges_sample(ids, "natural", s2l=True)
+        assert (g.decompose(micro=True).sums == part.sums).all()
+        for a, b in zip(g.micro(), part_rows):
+            assert (a == b).all()
+        assert g.resident_bytes <= held + MB
+    g.destroy()
+    assert c.resident_bytes == 0
+    c.close()
