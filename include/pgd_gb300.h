@@ -281,13 +281,13 @@ pgd_status pgd_server_destroy(pgd_server *sv);
  * depend on them.  anchor_hub and cache_hub act on the edge-by-edge kernels,
  * which decompose samples of fewer than 1/2048 of a graph's edges and the
  * allocation-free entry point; whole graphs are decomposed by passes that have
- * no thresholds.  Until the caller sets them (here or through pgd_autotune),
- * samples of graphs of more than 1.5·2^20 vertices use anchor_hub 128 and
- * cache_hub 40.  anchor_hub (2..256, default 64): anchors of degree >= it are
- * processed one CTA per anchor with N(p) as a bitmap, below it one warp per
- * edge with N(p) staged and searched.  cache_hub (>= 2, default 32): W(w,p)
- * comes from the anchor's histogram for neighbours of degree >= it (16-bit
- * counters from degree 256, 8-bit below), below it N(w) is scanned per edge.
+ * no thresholds.  Until the caller sets them, samples of graphs of more than
+ * 1.5·2^20 vertices use anchor_hub 128 and cache_hub 40.  anchor_hub (2..256,
+ * default 64): anchors of degree >= it are processed one CTA per anchor with
+ * N(p) as a bitmap, below it one warp per edge with N(p) staged and searched.
+ * cache_hub (>= 2, default 32): W(w,p) comes from the anchor's histogram for
+ * neighbours of degree >= it (16-bit counters from degree 256, 8-bit below),
+ * below it N(w) is scanned per edge.
  * dense_max (0..2048, default 2048): in a batch, graphs of at most this many
  * vertices and of average degree >= n/16 are decomposed with whole adjacency
  * rows as bitsets and a 16-bit common-neighbour matrix (about 2·n² bytes of
@@ -297,11 +297,13 @@ pgd_status pgd_server_destroy(pgd_server *sv);
  * degree in [tensor_min_degree, 1088] get their 4-clique count from a
  * product of q's ego network on the tensor cores (e4m3 0/1 operands, fp32
  * sums, exact); 0 keeps every edge on the integer path.
- * pgd_autotune decomposes the given graphs `reps` times per
- * candidate -- first dense_max in {0, 256, 1024, 2048}, then
- * tensor_min_degree in {0, 64, 128, 256}, then 16 (anchor_hub, cache_hub)
- * pairs -- checks that every candidate gives identical counts, keeps the
- * fastest on the context and reports it. */
+ * pgd_autotune decomposes the given graphs as a batch `reps` times per
+ * candidate -- first the values of {the context's own, 0, 256, 1024, 2048} for
+ * dense_max that differ in the graphs they give to the matrix kernels, then, if
+ * there are such graphs, tensor_min_degree in {0, 64, 128, 256} -- checks that
+ * every candidate gives identical counts, keeps the fastest on the context and
+ * reports it.  anchor_hub and cache_hub act on no batch: they stay, and the
+ * context's are reported. */
 pgd_status pgd_set_thresholds(pgd_ctx *ctx, int anchor_hub, int cache_hub, int dense_max);
 pgd_status pgd_get_thresholds(const pgd_ctx *ctx, int *anchor_hub, int *cache_hub, int *dense_max);
 pgd_status pgd_set_tensor_min_degree(pgd_ctx *ctx, int tensor_min_degree);

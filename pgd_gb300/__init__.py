@@ -306,7 +306,8 @@ class Context:
         return d.value
 
     def autotune(self, graphs, reps=1):
-        """Pick the fastest thresholds for these graphs; returns (anchor_hub, cache_hub, dense_max, ms)."""
+        """Pick the fastest dense_max and tensor_min_degree for a batch of these graphs;
+        returns (anchor_hub, cache_hub, dense_max, ms), the first two as they were."""
         arr = (ctypes.c_void_p * len(graphs))(*[g.h.value for g in graphs])
         a, c, d, ms = ctypes.c_int(), ctypes.c_int(), ctypes.c_int(), ctypes.c_float()
         self._check(lib().pgd_autotune(self.h, arr, len(graphs), reps, ctypes.byref(a), ctypes.byref(c),

@@ -9,6 +9,7 @@
 #include <vector>
 
 #include "pgd_internal.h"
+#include "size_rules.h"
 
 // ---------------------------------------------------------------------------
 // errors and memory
@@ -364,8 +365,7 @@ extern "C" pgd_status pgd_decompose(pgd_graph *g, uint32_t flags, pgd_counts *ou
     if (!g->preprocessed && (st = pgd_preprocess(g, "deg", 0))) return st;
     if (!g->sorted && (st = pgd_sort_edges(g, "deg", 0))) return st;
     // Default thresholds of the edge-by-edge kernels (small samples) by graph size:
-    // while the caller has set none (directly or through pgd_autotune), graphs of
-    // more than kLargeGraph vertices take hub anchors from degree 128 and cached W
+    // while the caller has set none, graphs of more than kLargeGraph vertices take hub anchors from degree 128 and cached W
     // from degree 40.  Measured with those kernels on the whole of RMAT scales 21 to
     // 24: 0.3 %, 1.2 %, 1.0 % and 5.7 % faster than the 64 / 32 defaults, which stay
     // the fastest on RMAT scale 20 (1.05 M vertices).
@@ -504,6 +504,9 @@ extern "C" pgd_status pgd_get_tensor_min_degree(const pgd_ctx *ctx, int *tensor_
 extern "C" pgd_status pgd_autotune(pgd_ctx *ctx, pgd_graph *const *graphs, int k, int reps, int *anchor_hub,
                                    int *cache_hub, int *dense_max, float *best_ms) {
     if (!ctx || k <= 0 || !graphs) return pgd_fail(ctx, PGD_EINVAL, "bad arguments");
+    for (int i = 0; i < k; i++)
+        if (!graphs[i] || graphs[i]->ctx != ctx)
+            return pgd_fail(ctx, PGD_EINVAL, "batch graph is null or from another context");
     if (reps < 1) reps = 1;
     std::vector<pgd_counts> out((size_t)k);
     std::vector<uint64_t> first;
@@ -522,43 +525,42 @@ extern "C" pgd_status pgd_autotune(pgd_ctx *ctx, pgd_graph *const *graphs, int k
         *ms = total / reps;
         return PGD_OK;
     };
-    // 1. the bitset/list crossover for small graphs
+    // Two values of dense_max that give as many graphs to the matrix kernels do the
+    // same work: the first of them stands, the context's own choice before all.
+    auto dense_graphs = [&](int d) {
+        int c = 0;
+        for (int i = 0; i < k; i++) c += pgd_dense_member(graphs[i]->n, graphs[i]->m, d);
+        return c;
+    };
+    // 1. which graphs take the matrix kernels
     float best = -1, ms = 0;
     int bd = ctx->dense_max;
-    for (int d : {0, 256, 1024, 2048}) {
+    std::vector<int> tried;
+    for (int d : {ctx->dense_max, 0, 256, 1024, 2048}) {
+        const int c = dense_graphs(d);
+        if (std::find(tried.begin(), tried.end(), c) != tried.end()) continue;
+        tried.push_back(c);
         ctx->dense_max = d;
         pgd_status st = trial(&ms);
         if (st) return st;
         if (best < 0 || ms < best) { best = ms; bd = d; }
     }
     ctx->dense_max = bd;
-    // 2. which runs of the dense graphs go to the tensor cores
-    best = -1;
-    int bt = ctx->tc_min_deg;
-    for (int t : {0, 64, 128, 256}) {
-        ctx->tc_min_deg = t;
-        pgd_status st = trial(&ms);
-        if (st) return st;
-        if (best < 0 || ms < best) { best = ms; bt = t; }
-    }
-    ctx->tc_min_deg = bt;
-    // 3. the two hub thresholds
-    best = -1;
-    int ba = ctx->anchor_hub, bc = ctx->cache_hub;
-    for (int a : {32, 64, 128, 256}) {
-        for (int c : {32, 64, 128, 512}) {
-            ctx->anchor_hub = a;
-            ctx->cache_hub = c;
+    // 2. which runs of the dense graphs go to the tensor cores, if there are any
+    if (dense_graphs(bd)) {
+        best = -1;
+        int bt = ctx->tc_min_deg;
+        for (int t : {0, 64, 128, 256}) {
+            ctx->tc_min_deg = t;
             pgd_status st = trial(&ms);
             if (st) return st;
-            if (best < 0 || ms < best) { best = ms; ba = a; bc = c; }
+            if (best < 0 || ms < best) { best = ms; bt = t; }
         }
+        ctx->tc_min_deg = bt;
     }
-    ctx->anchor_hub = ba;
-    ctx->cache_hub = bc;
-    ctx->thresholds_set = true;
-    if (anchor_hub) *anchor_hub = ba;
-    if (cache_hub) *cache_hub = bc;
+    // the hub thresholds steer kernels that no batch runs: not tuned here
+    if (anchor_hub) *anchor_hub = ctx->anchor_hub;
+    if (cache_hub) *cache_hub = ctx->cache_hub;
     if (dense_max) *dense_max = bd;
     if (best_ms) *best_ms = best;
     return PGD_OK;

@@ -55,6 +55,7 @@
 #include "pgd_internal.h"
 #include "pgd_kernels.cuh"
 #include "rank_path.h"
+#include "size_rules.h"
 #include "tc_ptx.cuh"
 
 namespace {
@@ -2994,7 +2995,7 @@ static BatchSplit split_batch(int k, const std::vector<long long> &gnm, int dens
         before[g] = B.sparse_edges;
         ctile[g] = B.tiles;
         const int64_t e = n * (((n + 63) / 64) * 64);   // a multiple of 64: every matrix is 128-byte aligned
-        if (m == 0 || n > dense_max || 32 * m < n * n || B.entries + e > kCnMaxEntries) {
+        if (!pgd_dense_member(n, m, dense_max) || B.entries + e > kCnMaxEntries) {
             B.sparse_edges += m;
             continue;
         }

@@ -27,12 +27,12 @@ struct pgd_ctx {
     // stage events of a decomposition: triangle pass [evt0, evt1), k_hub [evh0, evh1)
     cudaEvent_t evt0 = nullptr, evt1 = nullptr, evh0 = nullptr, evh1 = nullptr;
     unsigned long long launches = 0;        // kernels of this library launched
-    // decomposition thresholds (results never depend on them; pgd_autotune sets them)
+    // decomposition thresholds (results never depend on them; pgd_autotune sets the last two)
     int anchor_hub = 64;     // anchors of degree >= this take the bitmap (block) path
     int cache_hub = 32;      // W(w,p) taken from the per-anchor histogram for neighbours of degree >= this
     int dense_max = 2048;    // batched graphs with at most this many vertices use row bitsets
     int tc_min_deg = 64;     // batched CN-graph runs with d_q >= this count k4 on the tensor cores (0: never)
-    bool thresholds_set = false;   // anchor_hub / cache_hub chosen by the caller or pgd_autotune
+    bool thresholds_set = false;   // anchor_hub / cache_hub chosen by the caller
 };
 
 struct pgd_graph {

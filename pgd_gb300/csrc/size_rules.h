@@ -49,3 +49,7 @@ inline bool pgd_core_narrow(int64_t n, int64_t entries, int64_t steps, int64_t s
     return pgd_core_fits(n) &&
            0.75 * (double)scanned + (double)removed * ((double)entries / (double)n) <= (double)(steps * kCoreNarrowWeight);
 }
+
+// Whether a batch decomposes a graph with whole adjacency rows as bits and a
+// common-neighbour matrix: at most dense_max vertices, average degree at least n/16.
+inline bool pgd_dense_member(int64_t n, int64_t m, int dense_max) { return m > 0 && n <= dense_max && 32 * m >= n * n; }
