@@ -635,6 +635,9 @@ pgd_status pgd_build_from_pairs(pgd_graph *g, const int32_t *h_src, const int32_
     if (k < 0 || k > (int64_t)0x7fffffff) return pgd_fail(ctx, PGD_EINVAL, "pair count out of range (0..2^31-1)");
     pgd_status st;
     if (k > 0 && k <= kSmallPairs) {
+        // the host reads the pairs here: after what the caller's own stream still has
+        // to do, which may be what fills them (page-locked memory)
+        if (!ctx->own_stream) PGD_CUDA(ctx, cudaStreamSynchronize(ctx->stream));
         int32_t top = -1;   // largest id of an edge
         bool bad = false;
         for (int64_t i = 0; i < k; i++) {
