@@ -18,6 +18,8 @@ struct pgd_ctx {
     cudaEvent_t ev_fork = nullptr, ev_join = nullptr;
     uint64_t budget = 0;     // bytes graphs of this context may hold
     uint64_t resident = 0;   // bytes currently held
+    uint64_t list_limit = UINT64_MAX;   // bytes a decomposition may take for what it can do without (kept triangles,
+                                        // range positions); the server's workers: what their batch was given
     std::string err;
     // decomposition scratch: per-launch counters and sums
     unsigned long long *d_sums = nullptr;   // PGD_NSUMS

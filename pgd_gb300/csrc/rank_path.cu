@@ -1817,7 +1817,8 @@ pgd_status pgd_rank_build(pgd_graph *g, int64_t nnz, const int32_t *vgraph, cons
     const int64_t bpos_bytes = (int64_t)(R->nranges - 1) * n2 * (int64_t)sizeof(uint32_t);
     // the table is left out where the budget or the device has no room for it
     const std::string err = ctx->err;
-    st = bpos_bytes <= kBposBytes ? keep(&R->bpos, (size_t)bpos_bytes) : PGD_ENOMEM;
+    const int64_t bpos_most = (int64_t)std::min<uint64_t>(kBposBytes, ctx->list_limit / 4);
+    st = bpos_bytes <= bpos_most ? keep(&R->bpos, (size_t)bpos_bytes) : PGD_ENOMEM;
     if (st == PGD_ENOMEM) {
         R->bpos = nullptr;
         ctx->err = err;
@@ -1901,9 +1902,11 @@ static EgoMemory ego_memory(const pgd_ctx *ctx, const pgd_rank_graph &R, int64_t
     return E;
 }
 
-// Bytes that lists and tables may take beyond kListFloor: at most what the context
-// was given, what is left of its budget and half of the device's free memory.
+// Bytes that lists and tables may take: what the context was given (a quarter of it
+// is for the range positions), else kListFloor and beyond it at most what is left
+// of its budget and half of the device's free memory.
 static int64_t ego_room(const pgd_ctx *ctx) {
+    if (ctx->list_limit != UINT64_MAX) return (int64_t)std::min<uint64_t>(ctx->list_limit / 4 * 3, INT64_MAX / 2);
     size_t free_b = 0, total_b = 0;
     uint64_t reserved = 0, used = 0;   // the pool's: what it holds and does not use is free as well
     cudaMemPool_t pool;
@@ -2058,7 +2061,7 @@ pgd_status pgd_rank_decompose(pgd_ctx *ctx, const pgd_rank_graph &R, const pgd_r
     const int64_t zeroed = kCounters * 8 + R.nnz * 16, at_count = up128(zeroed);
     int64_t at_hits = 0, at_tables = 0;
     EgoMemory mem = ego_memory(ctx, R, INT64_MAX / 2);
-    if (mem.bytes() > kListFloor) mem = ego_memory(ctx, R, ego_room(ctx));
+    if (mem.bytes() > kListFloor || ctx->list_limit != UINT64_MAX) mem = ego_memory(ctx, R, ego_room(ctx));
     Tmp tg(ctx);
     uint8_t *work = nullptr;
     const std::string err = ctx->err;

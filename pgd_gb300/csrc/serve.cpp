@@ -31,6 +31,7 @@
 #include <cmath>
 
 #include "pgd_internal.h"
+#include "size_rules.h"
 
 namespace {
 
@@ -40,7 +41,7 @@ struct Request {
     uint64_t ticket = 0;
     std::vector<int32_t> src, dst;
     int64_t n_min = 0;
-    uint64_t est_bytes = 0;
+    uint64_t est_bytes = 0, opt_bytes = 0;
     Clock::time_point t_submit, t_admit, t_done;
     pgd_counts result{};
     pgd_status status = PGD_OK;
@@ -59,6 +60,19 @@ uint64_t estimate_bytes(int64_t pairs, int64_t n) {
     if (v <= 2048) bytes += 2 * v * (v + 64) + 8 * v * ((v + 63) / 64) + 24 * p;
     return bytes;
 }
+
+// Bytes that a request's decomposition can use beside that, and can do without: the
+// triangles kept between its passes (8 bytes for every pair of every up-neighbourhood,
+// at most 4 p sqrt(2 p) bytes) and range positions.  It gets a share of what the
+// budget has left, and of its estimate what the arrays above leave.  Graphs for the
+// matrix kernels need neither.
+uint64_t optional_bytes(int64_t pairs, int64_t n, int dense_max) {
+    if (pgd_dense_member(n, pairs, dense_max)) return 0;
+    const double p = (double)std::max<int64_t>(pairs, 1);
+    return (uint64_t)std::min(6 * p * std::sqrt(2 * p), 1e18) + 256 * (uint64_t)std::max<int64_t>(n, 1);
+}
+constexpr uint64_t kMaxOptional = 20ull << 30;   // what the passes take at most
+constexpr uint64_t kSparePerPair = 16;           // of the 160 bytes per pair of the estimate
 
 // A batch is closed once it holds this many pairs (it always takes at least
 // one request): long batches make every request that arrives meanwhile wait.
@@ -118,7 +132,7 @@ struct pgd_server {
         std::vector<pgd_counts> out;
         while (true) {
             batch.clear();
-            uint64_t bytes = 0;
+            uint64_t bytes = 0, optional = 0, lists = 0;
             {
                 std::unique_lock<std::mutex> lock(mu);
                 cv_work.wait(lock, [&] { return stop || !pending.empty(); });
@@ -151,6 +165,7 @@ struct pgd_server {
                     if (skipped) skipped_ahead++;
                     it = pending.erase(it);
                     bytes += r->est_bytes;
+                    optional += r->opt_bytes;
                     pairs += (int64_t)r->src.size();
                     r->t_admit = now;
                     batch.push_back(r);
@@ -160,6 +175,10 @@ struct pgd_server {
                     cv_work.wait_for(lock, std::chrono::milliseconds(1));
                     continue;
                 }
+                // the batch's share of what is left: each worker takes a part of the rest
+                lists = std::min({optional, kMaxOptional, (opts.hbm_budget - inflight - bytes) / (uint64_t)opts.workers});
+                ctx->list_limit = lists + kSparePerPair * (uint64_t)pairs;
+                bytes += lists;
                 inflight += bytes;
                 peak = std::max(peak, inflight);
                 batches++;
@@ -241,6 +260,7 @@ extern "C" pgd_status pgd_server_submit(pgd_server *sv, const int32_t *src, cons
     int64_t n = n_min;
     for (int64_t i = 0; i < k; i++) n = std::max<int64_t>(n, (int64_t)std::max(src[i], dst[i]) + 1);
     r->est_bytes = estimate_bytes(k, n);
+    r->opt_bytes = std::min(optional_bytes(k, n, sv->ctxs[0]->dense_max), kMaxOptional);
     r->t_submit = Clock::now();
     {
         std::lock_guard<std::mutex> lock(sv->mu);

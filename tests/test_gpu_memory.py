@@ -74,6 +74,11 @@ class Pool:
     def restart(self):
         assert self.rt.cudaMemPoolSetAttribute(self.pool, 8, ctypes.byref(ctypes.c_uint64(0))) == 0   # UsedMemHigh
 
+    def used(self):
+        v = ctypes.c_uint64()
+        assert self.rt.cudaMemPoolGetAttribute(self.pool, 7, ctypes.byref(v)) == 0   # UsedMemCurrent
+        return v.value
+
     def high(self):
         v = ctypes.c_uint64()
         assert self.rt.cudaMemPoolGetAttribute(self.pool, 8, ctypes.byref(v)) == 0
@@ -126,3 +131,21 @@ def test_either_path_makes_room_for_the_other():
     g.destroy()
     assert c.resident_bytes == 0
     c.close()
+
+
+@pytest.mark.parametrize("workers,budget", [(1, 400), (2, 800)])
+def test_a_servers_budget_bounds_what_its_requests_take(workers, budget):
+    """3 GB of triangles in each request, estimated at 180 MB."""
+    graphs = [pgd.erdos_renyi(2100, 0.5, seed=i) for i in range(4)]
+    want = [decomposed(0, *g, micro=False)[0].totals for g in graphs]
+    p = Pool()
+    before = p.used()
+    p.restart()
+    sv = pgd.Server(workers=workers, hbm_budget=budget * MB)
+    tickets = [sv.submit(*g) for g in graphs]
+    for t, w in zip(tickets, want):
+        st, r = sv.wait(t, 120000)
+        assert st == 0 and (r.totals == w).all()
+    assert sv.stats()["peak_bytes"] <= budget * MB
+    sv.close()
+    assert p.high() - before <= budget * MB
