@@ -41,10 +41,10 @@
 // are uint64 and wrap exactly like the reference's (addition mod 2^64 is
 // order independent, so the reduction order does not matter).
 //
-// What runs where: whole graphs, samples of at least 1/2048 of the edges and the
+// What runs where: whole graphs, all but small samples (pgd_sample_edgewise) and the
 // sparse graphs of a batch go through the passes of rank_path.cu, dense graphs of
 // a batch through the common-neighbour and tensor-core kernels below; the anchor
-// kernels described above take smaller samples and the allocation-free entry point.
+// kernels described above take small samples and the allocation-free entry point.
 #include <string.h>
 
 #include <cub/cub.cuh>
@@ -2574,16 +2574,6 @@ static size_t hub_layout(int64_t n, int32_t nhubs, int32_t nwide, int32_t max_de
     return (size_t)((H->smem_hist ? H->hstride : 0) + bm_words) * 4;
 }
 
-// A sample of fewer than one edge in kSampleShare is decomposed edge by edge
-// (run_decompose), everything else by the passes of rank_path.cu, whose cost
-// does not depend on the number of edges asked for.  Microseconds for order and
-// counts of 1/2000, 1/500 and 1/66 of the edges, edge by edge against whole-graph:
-// RMAT-16 2151, 2298, 2609 / 699, 702, 771; RMAT-20 39110, 55900, 83642 / 32673,
-// 32721, 32978; 1M-vertex BA 3257, 3452, 3909 / 1315, 1334, 1422; rgg-20 4345,
-// 4368, 4714 / 3333, 3336, 3466; dense G(1000, 0.5) 636, 790, 1107 / 992, 926,
-// 968.  At 1/10000 RMAT-20 takes 27447 / 32621.
-constexpr int64_t kSampleShare = 2048;
-
 // Device times of one decomposition: all kernels, the triangle pass, k_hub.
 struct StageMs {
     float total = 0, tri = 0, hub = 0;
@@ -2889,7 +2879,7 @@ pgd_status pgd_dev_decompose(pgd_graph *g, bool micro, pgd_counts *out) {
         if ((st = pgd_graph_alloc(g, (void **)&g->micro, (g->m + 1) * PGD_NMICRO * sizeof(uint64_t)))) return st;
     }
     StageMs ms;
-    const bool whole = g->norder >= g->m / kSampleShare;
+    bool whole = !pgd_sample_edgewise(g->n, g->m, g->norder);
     auto run = [&]() -> pgd_status {
         PGD_CUDA(ctx, cudaMemsetAsync(ctx->d_sums, 0, PGD_NSUMS * sizeof(unsigned long long), s));
         if (whole) return rank_decompose(g, micro, &ms);
@@ -2909,6 +2899,11 @@ pgd_status pgd_dev_decompose(pgd_graph *g, bool micro, pgd_counts *out) {
             pgd_rank_drop(g);
             pgd_aux_drop(g);   // built half-way
         }
+        st = run();
+    }
+    if (st == PGD_ENOMEM && !whole) {   // the passes hold less
+        pgd_aux_drop(g);
+        whole = true;
         st = run();
     }
     if (st && !g->has_aux) pgd_aux_drop(g);

@@ -2,6 +2,7 @@
 // functions of numbers, so that tests reach sizes that no graph of theirs has.
 #pragma once
 
+#include <math.h>
 #include <stdint.h>
 
 inline int pgd_bit_length(uint64_t x) {
@@ -53,3 +54,34 @@ inline bool pgd_core_narrow(int64_t n, int64_t entries, int64_t steps, int64_t s
 // Whether a batch decomposes a graph with whole adjacency rows as bits and a
 // common-neighbour matrix: at most dense_max vertices, average degree at least n/16.
 inline bool pgd_dense_member(int64_t n, int64_t m, int dense_max) { return m > 0 && n <= dense_max && 32 * m >= n * n; }
+
+// Whether k of a graph's m edges are decomposed edge by edge (decompose.cu), or by
+// the passes over the whole graph (rank_path.cu), whose cost hardly depends on k.
+//
+// Below 1/2048 of the edges always edge by edge: microseconds for order and counts
+// of 1/10000 of RMAT-20 27447 edge by edge, 32621 by the passes.  From there on the
+// passes, edge by edge against whole-graph for 1/2000, 1/500 and 1/66 of the edges:
+// RMAT-16 2151, 2298, 2609 / 699, 702, 771; RMAT-20 39110, 55900, 83642 / 32673,
+// 32721, 32978; 1M-vertex BA 3257, 3452, 3909 / 1315, 1334, 1422; rgg-20 4345, 4368,
+// 4714 / 3333, 3336, 3466.
+//
+// Dense graphs (average degree d at least 0.15 n) are the exception: their passes
+// are bound by the triangles, of which there are about m d p / 3 with p = d / n, at
+// 20 + d / 60 ps each; edge by edge it is 1.4 ps for each of the m d list entries of
+// the triangle pass, 2.6 ps for those of the anchors met (k edges meet 1 - exp(-k/n)
+// of n), and 38 ps for those of the sampled edges.  Microseconds edge by edge /
+// whole-graph, G(1000, 0.5): 1/2048 638 / 950, 1/256 882 / 961, 1/64 1120 / 947;
+// G(1000, 0.9): 1/2048 1259 / 3427, 1/16 2785 / 3479, 1/4 4763 / 3546; G(2000, 0.5):
+// 1/64 4917 / 5179, 1/16 6033 / 5243; G(3000, 0.5): 1/16 20374 / 27159, 1/8 28133 /
+// 27304; G(5000, 0.2): 1/2048 5602 / 7344, 1/512 8760 / 7396; G(250, 0.9) and
+// G(1000, 0.25): the passes at any share from 1/2048.
+inline bool pgd_sample_edgewise(int64_t n, int64_t m, int64_t k) {
+    if (k < m / 2048) return true;
+    if (k > m / 4) return false;
+    const double d = 2.0 * (double)m / (double)n, p = d / (double)n, md = (double)m * d;
+    if (!(p >= 0.15)) return false;
+    const double f = 1.0 - exp(-(double)k / (double)n), share = (double)k / (double)m;
+    const double edgewise = 300.0 + 1e-6 * md * (1.4 + 2.6 * f + 38.0 * share);
+    const double whole = 150.0 + 1e-6 * md * p / 3.0 * (20.0 + d / 60.0);
+    return edgewise < whole;
+}

@@ -53,3 +53,20 @@ def test_core_choice_follows_the_measured_sides(tmp_path):
     body += 'printf("%d%d", pgd_core_narrow(4000000, 8000000, 64, 0, 128), ' \
             'pgd_core_narrow(1048576, 52427448, 64, 20000000, 1000));'
     assert compiled(tmp_path, body) == "1" * len(light) + "0" * len(heavy) + "10"
+
+
+# n, p, share, edge by edge: clearly faster on its side in the times beside the rule
+SAMPLES = [(1000, 0.5, 1 / 2048, 1), (1000, 0.5, 1 / 512, 1), (1000, 0.5, 1 / 64, 0), (1000, 0.9, 1 / 16, 1),
+           (1000, 0.9, 1 / 4, 0), (2000, 0.5, 1 / 256, 1), (2000, 0.5, 1 / 8, 0), (3000, 0.5, 1 / 16, 1),
+           (5000, 0.2, 1 / 2048, 1), (5000, 0.2, 1 / 512, 0), (250, 0.9, 1 / 2048, 0), (1000, 0.25, 1 / 2048, 0),
+           (3000, 0.1, 1 / 2048, 0), (1 << 20, 3e-5, 1 / 2000, 0), (1 << 20, 3e-5, 1 / 10000, 1), (3000, 0.9, 1, 0),
+           (20000, 1.0, 1, 0), (3, 1.0, 1, 0)]
+
+
+def test_samples_take_the_faster_path(tmp_path):
+    body = ""
+    for n, p, share, _ in SAMPLES:
+        m = int(p * n * (n - 1) / 2)
+        body += 'printf("%%d", pgd_sample_edgewise(%dll, %dll, %dll));' % (n, m, max(1, int(share * m)))
+    body += 'printf("%d%d", pgd_sample_edgewise(5, 0, 0), pgd_sample_edgewise(0, 0, 0));'
+    assert compiled(tmp_path, body) == "".join(str(s[3]) for s in SAMPLES) + "00"
