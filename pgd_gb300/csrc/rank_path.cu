@@ -1283,6 +1283,57 @@ __device__ __forceinline__ void clique_hits(const EgoArgs &A, const uint2 *hits,
     }
 }
 
+// Index in N+(a) of the vertex of rank y, -1 if it is not among them (last: the
+// largest rank asked for).
+__device__ __forceinline__ int ego_find(const EgoTables &T, int32_t y, int32_t last, int shift, uint32_t hmask) {
+    if (y < kTopRanks) return (int)T.top[y] - 1;
+    if (y > last) return -1;
+    uint32_t h = hash_of((uint32_t)y, shift), k;
+    while ((k = T.hkey[h]) != (uint32_t)y && k != kFull) h = (h + 1) & hmask;
+    return k == (uint32_t)y ? (int)T.hidx[h] : -1;
+}
+
+// The same without a list: the rows of N+(a) looked up once more, a warp per row
+// from the counter *next (index of the last row at the start).
+__device__ __forceinline__ void clique_rows(const EgoArgs &A, const EgoTables &T, int W, int WS, int shift,
+                                            uint32_t hmask, int *next) {
+    const int lane = threadIdx.x & 31;
+    while (true) {
+        int i = 0;
+        if (lane == 0) i = atomicSub(next, 1);
+        i = __shfl_sync(kFull, i, 0);
+        if (i < 1) break;
+        const uint32_t r0 = T.rs[i], ti = T.ta[i];
+        const int len = T.ru[i];
+        const int32_t last = T.ls[i - 1];
+        const unsigned long long *fi = T.F + (int64_t)i * WS;
+        uint32_t ci = 0, di = 0;
+        for (int b = 0; b < len; b += 32) {
+            const uint32_t pos = r0 + (uint32_t)(b + lane);
+            const int32_t y = b + lane < len ? __ldg(A.radj + pos) : 0x7fffffff;
+            const int j = ego_find(T, y, last, shift, hmask);
+            if (j >= 0) {
+                const unsigned long long *fj = T.F + (int64_t)j * WS;
+                uint32_t c = 0;
+                for (int w = 0; w < W; w++) c += (uint32_t)__popcll(fi[w] & fj[w]);
+                const uint32_t tij = A.t[pos], tj = T.ta[j];
+                atomicAdd(A.dk + pos, ((unsigned long long)(ti + tj) << 32) + c);
+                if (c) atomicAdd(T.ck + j, c);
+                atomicAdd(T.cd + j, ti + tij);
+                ci += c;
+                di += tj + tij;
+            }
+            if (__shfl_sync(kFull, y, 31) > last) break;   // ascending: nothing more at or below last
+        }
+        ci = __reduce_add_sync(kFull, ci);
+        di = __reduce_add_sync(kFull, di);
+        if (lane == 0) {
+            if (ci) atomicAdd(T.ck + i, ci);
+            if (di) atomicAdd(T.cd + i, di);
+        }
+    }
+}
+
 // |N+(a)| = d in a block's range: a block per vertex.  The indices of N+(a) go
 // into the lookup tables; each warp takes vertices x of N+(a) and looks the
 // entries of N+(x) up (searching N+(a)'s entries in N+(x) where that takes fewer
@@ -1316,7 +1367,7 @@ __global__ void __launch_bounds__(NT) k_ego_block(EgoArgs A, int dmax) {
         const uint32_t ra = A.roff[a];
         const int W = (d + 63) >> 6;
         uint2 *hits = nullptr;
-        if (PASS == 2) hits = A.hits + (int64_t)blockIdx.x * A.hits_stride;
+        if (PASS == 2) hits = A.hits ? A.hits + (int64_t)blockIdx.x * A.hits_stride : nullptr;
         else if (A.hcount) hits = A.hits + A.hbase[a];
         if (threadIdx.x == 0) s_row = d - 1;
         for (int i = threadIdx.x; i <= (int)hmask; i += NT) T.hkey[i] = kFull;
@@ -1351,14 +1402,7 @@ __global__ void __launch_bounds__(NT) k_ego_block(EgoArgs A, int dmax) {
             const int len = T.ru[i];
             uint32_t found = 0;
             const int32_t last = T.ls[i - 1];
-            // index in N+(a) of the vertex of rank y, -1 if it is not among them
-            auto find = [&](int32_t y) {
-                if (y < kTopRanks) return (int)T.top[y] - 1;
-                if (y > last) return -1;
-                uint32_t h = hash_of((uint32_t)y, shift), k;
-                while ((k = T.hkey[h]) != (uint32_t)y && k != kFull) h = (h + 1) & hmask;
-                return k == (uint32_t)y ? (int)T.hidx[h] : -1;
-            };
+            auto find = [&](int32_t y) { return ego_find(T, y, last, shift, hmask); };
             // 64 entries a turn: two loads in flight, one place among the hits for both
             // (R-MAT 20: 5.38 -> 4.68 ms for the smaller class, 2.52 -> 1.74 ms for the
             // next; bound by issue.  Short rows end to end over the lanes instead: 5.72 ms)
@@ -1398,7 +1442,13 @@ __global__ void __launch_bounds__(NT) k_ego_block(EgoArgs A, int dmax) {
         }
         __syncthreads();
         if (PASS == 2) {
-            clique_hits<NT>(A, hits, s_nhit, T, W, WS);
+            if (hits) {
+                clique_hits<NT>(A, hits, s_nhit, T, W, WS);
+            } else {
+                if (threadIdx.x == 0) s_row = d - 1;
+                __syncthreads();
+                clique_rows(A, T, W, WS, shift, hmask, &s_row);
+            }
             __syncthreads();
         } else if (A.hcount && threadIdx.x == 0) {
             A.hcount[a] = s_nhit;
@@ -1864,41 +1914,41 @@ static int ego_grid(const pgd_ctx *ctx, const pgd_rank_graph &R, int c) {
     return (int)std::min<int64_t>(R.nlist[c], (int64_t)(ego_wide(ctx, R, c) ? 2 : ego_blocks_per_sm(c)) * ctx->num_sms);
 }
 
-// What the ego classes hold beside the counts per slot: every triangle of pass 1
-// kept for pass 2, or a list of each block of pass 2, which then lists them again;
-// and the tables of the largest neighbourhoods.
+// What the ego classes hold beside the counts per slot: the tables of the largest
+// neighbourhoods, and every triangle of pass 1, kept for pass 2; or a list of each
+// block of pass 2, which then finds its triangles again; or no list, and it finds
+// them twice.  A request of G(3000, 0.5): 32 ms with its 8.8 GB kept, 32 to 34 ms
+// without a list, 370 ms with a list for as few blocks as 120 MB hold; one of R-MAT
+// 16 3.8 and 4.0 ms.
 struct EgoMemory {
     bool keep = false;
     int64_t hits = 0;             // triangles in the lists
-    int grid[kEgoGlobal] = {0};   // blocks of pass 2 where they are not kept, by class
     int gblocks = 0;              // blocks of kEgoGlobal
     int64_t table_bytes = 0;      // each one's tables
     int64_t bytes() const { return hits * (int64_t)sizeof(uint2) + gblocks * table_bytes; }
 };
 
-// The fastest choice of at most `limit` bytes, and at least a block per class.
+// The fastest of them that takes at most `limit` bytes (and at least one block's tables).
 static EgoMemory ego_memory(const pgd_ctx *ctx, const pgd_rank_graph &R, int64_t limit) {
     EgoMemory E;
-    const int64_t hit = sizeof(uint2);
-    auto blocks_in = [](int64_t bytes, int64_t each, int64_t most) {
-        return (int)std::max<int64_t>(1, std::min(most, bytes / each));
+    const int64_t hit = sizeof(uint2), most = std::min<int64_t>(ctx->num_sms, R.nlist[kEgoGlobal]);
+    auto blocks_in = [&](int64_t bytes, int64_t each) {
+        return most ? (int)std::max<int64_t>(1, std::min(most, bytes / each)) : 0;
     };
-    if (R.nlist[kEgoGlobal]) {
-        const int64_t per = (int64_t)R.max_up * (R.max_up - 1) / 2;
-        E.table_bytes = ego_table_bytes(R.max_up, true, true);
-        E.gblocks = blocks_in(std::min(kTableBytes, limit), per * hit + E.table_bytes,
-                              std::min<int64_t>(ctx->num_sms, R.nlist[kEgoGlobal]));
-        E.hits = per * E.gblocks;
-    }
-    const int64_t left = limit - E.gblocks * E.table_bytes;
+    const int64_t per = (int64_t)R.max_up * (R.max_up - 1) / 2;
+    if (most) E.table_bytes = ego_table_bytes(R.max_up, true, true);
+    E.gblocks = blocks_in(kTableBytes, per * hit + E.table_bytes);
+    E.hits = R.pairs;
+    E.keep = R.pairs * hit <= kKeepBytes && E.bytes() <= limit;
+    if (E.keep) return E;
+    E.hits = per * E.gblocks;
     for (int c : {kEgoA, kEgoB, kEgoC}) {
-        if (!R.nlist[c]) continue;
-        const int64_t dmax = std::min(kEgoMax[c], (int)R.max_up), per = dmax * (dmax - 1) / 2;
-        E.grid[c] = blocks_in(left, per * hit, ego_grid(ctx, R, c));
-        E.hits = std::max(E.hits, per * E.grid[c]);
+        const int64_t dmax = std::min(kEgoMax[c], (int)R.max_up);
+        E.hits = std::max(E.hits, ego_grid(ctx, R, c) * (dmax * (dmax - 1) / 2));
     }
-    E.keep = R.pairs * hit <= std::min(kKeepBytes, left);
-    if (E.keep) E.hits = R.pairs;
+    if (E.bytes() <= limit) return E;
+    E.hits = 0;
+    E.gblocks = blocks_in(std::min(kTableBytes, limit), E.table_bytes);
     return E;
 }
 
@@ -1952,7 +2002,7 @@ static void ego_pass(pgd_ctx *ctx, const pgd_rank_graph &R, EgoArgs A, int pass,
         EgoArgs B = args(c);
         const int dmax = std::min(kEgoMax[c], (int)R.max_up);
         B.hits_stride = (int64_t)dmax * (dmax - 1) / 2;
-        const int blocks = pass == 2 && !kept ? mem.grid[c] : ego_grid(ctx, R, c);
+        const int blocks = ego_grid(ctx, R, c);
         const size_t smem = (size_t)ego_table_bytes(dmax, !kept, pass == 2);
         if (c == kEgoC || ego_wide(ctx, R, c)) EGO_BLOCK(1024, false, blocks, smem, B, dmax);
         else if (c == kEgoB) EGO_BLOCK(512, false, blocks, smem, B, dmax);
@@ -2101,7 +2151,7 @@ pgd_status pgd_rank_decompose(pgd_ctx *ctx, const pgd_rank_graph &R, const pgd_r
     E.radj = R.radj;
     E.t = t;
     E.dk = dk;
-    E.hits = (uint2 *)(work + at_hits);
+    E.hits = mem.hits ? (uint2 *)(work + at_hits) : nullptr;
     E.hbase = R.hbase;
     E.hcount = mem.keep ? (uint32_t *)(work + at_count) : nullptr;
     PGD_CUDA(ctx, cudaEventRecord(ctx->evt0, s));

@@ -32,13 +32,15 @@ def complete(n):
     return a.astype(np.int32), b.astype(np.int32)
 
 
+@pytest.mark.parametrize("room", [1, 1200])
 @pytest.mark.parametrize("kind", ["complete", "dense", "rmat", "geometric"])
-def test_triangles_listed_again(kind):
-    """Lists of more than 256 MB in a context without room for them."""
+def test_triangles_found_again(kind, room):
+    """Triangles of more than 256 MB in a context without room for them: with a list
+    per block, and without any."""
     src, dst = {"complete": lambda: complete(1100), "dense": lambda: pgd.erdos_renyi(1300, 0.9, seed=1),
                 "rmat": lambda: pgd.rmat(17, 16, seed=2), "geometric": lambda: pgd.rgg3d(20000, 0.17, seed=3)}[kind]()
     r, rows, held = decomposed(0, src, dst)
-    w, wrows, _ = decomposed(held + MB, src, dst)
+    w, wrows, _ = decomposed(held + room * MB, src, dst)
     assert (r.sums == w.sums).all() and (r.totals == w.totals).all()
     for a, b in zip(rows, wrows):
         assert (a == b).all()
