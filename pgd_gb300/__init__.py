@@ -186,17 +186,14 @@ def close_counts(sums, n, m):
     return out
 
 
-def _field(name, part, read=None):
-    """A field of Counts: words `part` (or read() of them) until it is replaced."""
-    def get(self):
-        own = self._own
-        if own is not None and name in own:
-            return own[name]
-        return self._w[part] if read is None else read(self._w[part])
-
+def _replace(name):
+    """Setter of a field of Counts: the result then has plain attributes."""
     def put(self, value):
-        self._own = {**(self._own or {}), name: value}
-    return property(get, put)
+        fields = {f: getattr(self, f) for f in _FIELDS}
+        self.__class__ = _OwnCounts
+        self.__dict__.update(fields)
+        self.__dict__[name] = value
+    return put
 
 
 class Counts:
@@ -204,21 +201,31 @@ class Counts:
     when a field is asked for (a batch has thousands of results, of which a
     program reads a few fields).  Fields can be replaced."""
 
-    _own = None   # replaced fields
+    __slots__ = ("_w", "__dict__", "__weakref__")
 
     def __init__(self, c):
         self._w = np.frombuffer(c, np.uint64, _WORDS).copy() if isinstance(c, pgd_counts) else c
 
-    totals = _field("totals", slice(NTOTALS))
-    sums = _field("sums", slice(NTOTALS, NTOTALS + NSUMS))
-    n = _field("n", NTOTALS + NSUMS, int)
-    m = _field("m", NTOTALS + NSUMS + 1, int)
-    kernel_ms = _field("kernel_ms", slice(-2, None), lambda w: float(w.view(np.float32)[0]))
-    hub_ms = _field("hub_ms", slice(-2, None), lambda w: float(w.view(np.float32)[1]))
-    tri_ms = _field("tri_ms", slice(-2, None), lambda w: float(w.view(np.float32)[2]))
+    totals = property(lambda self: self._w[:NTOTALS], _replace("totals"))
+    sums = property(lambda self: self._w[NTOTALS:NTOTALS + NSUMS], _replace("sums"))
+    n = property(lambda self: int(self._w[NTOTALS + NSUMS]), _replace("n"))
+    m = property(lambda self: int(self._w[NTOTALS + NSUMS + 1]), _replace("m"))
+    kernel_ms = property(lambda self: float(self._w[-2:].view(np.float32)[0]), _replace("kernel_ms"))
+    hub_ms = property(lambda self: float(self._w[-2:].view(np.float32)[1]), _replace("hub_ms"))
+    tri_ms = property(lambda self: float(self._w[-2:].view(np.float32)[2]), _replace("tri_ms"))
 
     def as_dict(self):
         return {k: int(v) for k, v in zip(TOTAL_NAMES, self.totals)}
+
+
+_FIELDS = ("totals", "sums", "n", "m", "kernel_ms", "hub_ms", "tri_ms")
+
+
+class _OwnCounts(Counts):
+    """A result with replaced fields."""
+
+    __slots__ = ()
+    totals = sums = n = m = kernel_ms = hub_ms = tri_ms = None
 
 
 def _counts_list(out):
@@ -416,7 +423,7 @@ class Graph:
         c = pgd_counts()
         self.ctx._check(lib().pgd_decompose(self.h, MICRO if micro else 0, ctypes.byref(c)),
                         "pgd_decompose")
-        return Counts(c)
+        return Counts(np.frombuffer(c, np.uint64, _WORDS))
 
     def micro(self, ids=True, out=None):
         m = self.order_length
