@@ -1789,13 +1789,16 @@ pgd_status pgd_rank_build(pgd_graph *g, int64_t nnz, const int32_t *vgraph, cons
         }
         return e;
     };
-    // kept arrays in one allocation
+    // kept arrays in one allocation; the range boundaries behind the sizes only where
+    // vertices are likely to have items
+    const bool one_block = !vgraph && nnz <= 2 * kSmallPairs && n <= kSmallVertices;
+    const size_t meta_bytes = one_block ? kMetaHead : sizeof(RankMeta);
     pgd_pieces K;
     const size_t nb = (n + 1) * sizeof(uint32_t), eb = nnz * sizeof(uint32_t), mb = m * sizeof(int32_t),
                  lb = (size_t)kClasses * n * sizeof(int32_t), hb = n * sizeof(unsigned long long);
-    K.add(kMetaHead); K.add(nb); K.add(nb); K.add(nb); K.add(eb); K.add(eb); K.add(eb); K.add(mb); K.add(lb); K.add(hb);
+    K.add(meta_bytes); K.add(nb); K.add(nb); K.add(nb); K.add(eb); K.add(eb); K.add(eb); K.add(mb); K.add(lb); K.add(hb);
     RB_TRY(keep(&K.base, K.bytes));
-    RankMeta *M = K.take<RankMeta>(kMetaHead);
+    RankMeta *M = K.take<RankMeta>(meta_bytes);
     R->meta = M;
     R->roff = K.take<uint32_t>(nb);
     R->rup = K.take<int32_t>(nb);
@@ -1810,7 +1813,7 @@ pgd_status pgd_rank_build(pgd_graph *g, int64_t nnz, const int32_t *vgraph, cons
     uint32_t *wd = nullptr;
     void *tmp = nullptr;
     size_t tb = 0;
-    if (!vgraph && nnz <= 2 * kSmallPairs && n <= kSmallVertices) {
+    if (one_block) {
         RankSmallArgs A{};
         A.off = g->off;
         A.adj = g->adj;
@@ -1857,12 +1860,12 @@ pgd_status pgd_rank_build(pgd_graph *g, int64_t nnz, const int32_t *vgraph, cons
     // fine enough to balance the items, and at most half an item's counters each
     const int64_t words = R->words = ((int64_t)h.tcode[4] + 31) / 32;
     R->nranges = (int32_t)std::min<int64_t>(kMaxRanges, std::max<int64_t>(16, 2 * (2 * words / kDirectWords + 1)));
-    // the sizes again, with the boundaries behind them
-    const size_t meta_bytes = kMetaHead + ((size_t)R->nranges + 1) * sizeof(uint32_t);
-    RankMeta *full = nullptr;
-    RB_TRY(keep(&full, meta_bytes));
-    RB_CUDA(cudaMemcpyAsync(full, M, kMetaHead, cudaMemcpyDeviceToDevice, s));
-    R->meta = M = full;
+    if (one_block) {   // the sizes again, with room for the boundaries
+        RankMeta *full = nullptr;
+        RB_TRY(keep(&full, sizeof(RankMeta)));
+        RB_CUDA(cudaMemcpyAsync(full, M, kMetaHead, cudaMemcpyDeviceToDevice, s));
+        R->meta = M = full;
+    }
     PGD_LAUNCH(ctx, k_rank_bounds, 1, 128, 0, R->roff, R->nranges, M);
     const int64_t bpos_bytes = (int64_t)(R->nranges - 1) * n2 * (int64_t)sizeof(uint32_t);
     // the table is left out where the budget or the device has no room for it
