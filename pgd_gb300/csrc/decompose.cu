@@ -1418,8 +1418,8 @@ __global__ void __launch_bounds__(256, 3) k_dense_cn(DenseCnArgs A) {
 // are 32 x 32 bit blocks of N(q)'s rows transposed, of which N(q)'s columns are
 // kept.  Then for each pair of 128-edge tiles and each 256-row tile of N(q), every
 // 64-column chunk is expanded to e4m3 tiles (one B tile shared by both edge tiles)
-// by 16 builder warps into one of two alternating stages while the tensor cores
-// run the previous chunk's MMAs, which one thread of the last warp issues into two
+// by 16 builder warps into one of several stages while the tensor cores
+// run the previous chunks' MMAs, which one thread of the last warp issues into two
 // TMEM accumulators.  The builders and the issuing thread meet at per-stage
 // mbarriers only: "full" (every builder warp arrived) and "empty" (tcgen05.commit
 // of the MMAs that read the stage); at the end of a row tile every warp reads back
@@ -1429,9 +1429,8 @@ __global__ void __launch_bounds__(256, 3) k_dense_cn(DenseCnArgs A) {
 // all sums are multiples of 4 below 2^24, exact in fp32.
 //
 // Builders start on the next row tile's stages before they read back the last
-// one's accumulators.  Of the time on 131 graphs of up to 2048 vertices about two
-// thirds go to the stages, a quarter to the compaction and the rest to the
-// read-back; the bound is the integer work of building the operands (the tensor
+// one's accumulators.  Of the time on 131 graphs of up to 2048 vertices about half
+// goes to the stages, three tenths to the compaction and the rest to the read-back; the bound is the integer work of building the operands (the tensor
 // cores are busy for about 0.4 of it), not a memory.  27.5 -> 24.6 ms with the
 // products below the diagonal only, -> 21.9 ms with transposes instead of bit
 // compression and word-wise spreading, the next run fetched in advance and records
@@ -2675,7 +2674,7 @@ __global__ void k_iota(int32_t *a, int64_t n) {
         a[i] = (int32_t)i;
 }
 
-// The edge-by-edge decomposition of G's positions.
+// The edge-by-edge decomposition of G's positions, a sample of its edges.
 static pgd_status run_decompose(pgd_ctx *ctx, const DevGraph &G, int4 *slot, int32_t nhubs, int32_t nwide,
                                 int32_t max_degree, StageMs *ms) {
     cudaStream_t s = ctx->stream;
@@ -2683,8 +2682,6 @@ static pgd_status run_decompose(pgd_ctx *ctx, const DevGraph &G, int4 *slot, int
     const int64_t m = G.npos;   // positions to decompose (E_ordered length)
     *ms = StageMs();
     if (m == 0) return PGD_OK;
-    // a sampled order decomposes some edges but reads t(x, q) of any edge
-    const bool sampled = G.npos < G.m;
     uint32_t *ghist = nullptr;
     uint32_t *gbm = nullptr;
     int32_t *thigh = nullptr;
@@ -2698,9 +2695,9 @@ static pgd_status run_decompose(pgd_ctx *ctx, const DevGraph &G, int4 *slot, int
     }
     PGD_CUDA(ctx, cudaEventRecord(ctx->ev0, s));
     // triangle counts of every edge first: k_hub and k_light read t(x, q) of
-    // other edges.  A sampled order still needs t of all edges: the same
-    // grouped pass runs over a plan of every edge (positions = edge ids).
-    if (sampled) {
+    // other edges than the sample's.  The pass runs over a plan of every edge
+    // (positions = edge ids).
+    {
         int32_t *iota = nullptr;
         if ((st = tg.alloc(&iota, (size_t)G.m * sizeof(int32_t)))) return st;
         PGD_LAUNCH(ctx, k_iota, grid_for(G.m), kThreads, 0, iota, G.m);
@@ -2722,11 +2719,6 @@ static pgd_status run_decompose(pgd_ctx *ctx, const DevGraph &G, int4 *slot, int
     int64_t *items = P.items;
     int2 *hrec = P.hrec;
     unsigned long long *ctr = ctx->d_ctr;
-    if (!sampled) {
-        PGD_CUDA(ctx, cudaEventRecord(ctx->evt0, s));
-        if ((st = triangle_pass(ctx, G, slot, P, H, gbm))) return st;
-        PGD_CUDA(ctx, cudaEventRecord(ctx->evt1, s));
-    }
     if (nitems > 0) {
         if (!H.smem_hist) {
             if ((st = tg.alloc(&ghist, (size_t)nsm * H.hstride * 4))) return st;
