@@ -15,11 +15,12 @@ ordering, k-core, decomposition and the copy of all per-edge rows back.
 
     python bench.py [--gpus N] [--steps K] [--warmup W] [--impl reference]
 
-With N > 1 (torchrun) the graph's ordered edge list is cut into N spans of
-about equal estimated work (pgd_gb300/shard.py): every rank holds the whole
-graph, decomposes its span, and the 15 partial sums are added with one NCCL
-all-reduce before the totals are closed -- strong scaling (`--mode shard`,
-the default).  `--mode replicas` instead decomposes an independent copy per
+With N > 1 (torchrun) the graph's ordered edge list is cut into N spans
+(pgd_gb300/shard.py): every rank holds the whole graph, decomposes its span, and
+the 15 partial sums are added with one NCCL all-reduce before the totals are
+closed (`--mode shard`, the default; the total work is fixed, so the line says
+"strong").  A span of this graph goes through the passes over the whole graph on
+every rank: only the closing and the rows shrink with N.  `--mode replicas` instead decomposes an independent copy per
 rank (no collective on the data path): weak scaling.
 """
 import argparse
@@ -41,8 +42,8 @@ RMAT = dict(a=0.57, b=0.19, c=0.19)
 
 # ncu figures of one k_cycle_direct launch (the dominant kernel) on this
 # workload, read from the committed summary: a `bench-figures:` line holding JSON
-# with the DRAM traffic, the L2 request bytes, issue activity and the SHA-256 of
-# the rank_path.cu the capture ran.  A summary whose source hash differs from
+# with the DRAM traffic, the L2 request bytes, issue activity, the kernel's time and
+# the SHA-256 of the rank_path.cu the capture ran.  A summary whose source hash differs from
 # the current file is reported as stale.
 PROFILE = os.path.join(ROOT, "profiles", "k_cycle_direct_rmat20_dram.md")
 KERNEL_SRC = os.path.join(ROOT, "pgd_gb300", "csrc", "rank_path.cu")
@@ -126,17 +127,19 @@ class ClockSampler:
                 "samples": len(sm)}
 
 
-def algorithmic_bytes(ev, eu, n, micro=True, ids=None):
-    """Bytes an edge-centric decomposition must stream: per edge both
-    endpoint lists plus the 2-hop lists of the cheaper endpoint, 4 B per
-    adjacency entry, plus 64 B of per-edge output (micro).  With ids, only
-    those edges (a rank's span).  Returns (bytes, edges counted)."""
+def cycle_bytes(ev, eu, n):
+    """Bytes the 4-cycle pass must touch: each wedge u - v - w below its highest
+    vertex u (rank_path.cu) reads a 4-byte counter address in both walks, and
+    each slot (an edge from either end) has a 4-byte count.  Returns (bytes,
+    wedges)."""
     deg = np.bincount(ev, minlength=n) + np.bincount(eu, minlength=n)
-    vol2 = np.bincount(ev, weights=deg[eu], minlength=n) + np.bincount(eu, weights=deg[ev], minlength=n)
-    if ids is not None:
-        ev, eu = ev[ids], eu[ids]
-    entries = (deg[ev] + deg[eu]).sum(dtype=np.float64) + np.minimum(vol2[ev], vol2[eu]).sum(dtype=np.float64)
-    return 4.0 * entries + (64.0 * len(ev) if micro else 0.0), int(len(ev))
+    above = (deg[ev] > deg[eu]) | ((deg[ev] == deg[eu]) & (ev > eu))   # ranks: (degree, id) descending
+    up = np.bincount(np.where(above, eu, ev), minlength=n)             # neighbours above each vertex
+    d2 = np.bincount(ev[deg[eu] >= 2], minlength=n) + np.bincount(eu[deg[ev] >= 2], minlength=n)
+    up, d2 = up.astype(np.float64), d2.astype(np.float64)
+    inner = deg >= 2
+    wedges = float((up * (d2 - 1) - up * (up - 1) / 2)[inner].sum())   # sum over i < up of d2 - 1 - i
+    return 8.0 * wedges + 8.0 * len(ev), wedges
 
 
 def profile_figures():
@@ -408,26 +411,25 @@ def main():
         % (rank, ms_per_step, np.mean(kernel_ms), np.mean(cycle_ms), value))
 
     # ---- roofline of the dominant pass (4-cycles) ---------------------------
-    # achieved = the per-edge algorithmic bytes of the edges decomposed over the
-    # 4-cycle pass's own mean duration (CUDA events on its stream; its largest
-    # kernel is k_cycle_direct); traffic, L2 bytes and issue activity come from the
-    # committed ncu summary of a k_cycle_direct launch on this workload.
+    # achieved = what the pass must touch (cycle_bytes, mostly from L2) over its own
+    # mean duration (CUDA events on its stream), against the HBM copy rate; traffic,
+    # L2 bytes, issue activity and kernel time come from the committed ncu summary
+    # of a k_cycle_direct launch, its largest kernel, on this workload.  What bounds
+    # that kernel is its shared-memory accesses, as the summary says.
     ev, eu, _ = g.edges(with_order=False)
-    b_alg, cycle_units = algorithmic_bytes(ev, eu, n, micro=True, ids=span_ids)
+    b_pass, wedges = cycle_bytes(ev, eu, n)
     cycle_s = float(np.mean(cycle_ms)) / 1000.0
     peak, peak_src = peaks()
-    achieved = b_alg / cycle_s / 1e9
+    achieved = b_pass / cycle_s / 1e9
     prof = profile_figures() if (args.scale, args.order) == (20, "kcore") else {}
-    traffic = prof.get("traffic_bytes")
-    l2_bytes = prof.get("l2_bytes")
+    traffic, direct_ms = prof.get("traffic_bytes"), prof.get("kernel_ms")
     roofline = {
-        "bound": "hbm", "achieved": achieved, "peak": peak, "unit": "GB/s", "frac": achieved / peak,
-        "traffic": traffic, "kernel": "k_cycle_direct", "kernel_ms": 1000.0 * cycle_s, "units": cycle_units,
-        "unit_name": "edges",
-        "algorithmic_bytes": b_alg,
-        "dram_frac": (traffic / cycle_s / 1e9 / peak) if traffic else None,
-        "model_bytes": l2_bytes,
-        "frac_model": (l2_bytes / cycle_s / 1e9 / peak) if l2_bytes else None,
+        "bound": "shared memory", "achieved": achieved, "peak": peak, "unit": "GB/s", "frac": achieved / peak,
+        "peak_of": "hbm copy", "pass_ms": 1000.0 * cycle_s, "units": wedges, "unit_name": "wedges",
+        "pass_bytes": b_pass,
+        "kernel": "k_cycle_direct", "kernel_ms": direct_ms, "traffic": traffic,
+        "dram_frac": (traffic / direct_ms / 1e6 / peak) if traffic and direct_ms else None,
+        "l2_bytes": prof.get("l2_bytes"),
         "issue_active": prof.get("issue_active"),
         "profile_on_current_source": prof.get("current_source"),
         "decomposition_kernels_ms": float(np.mean(kernel_ms)),
