@@ -279,9 +279,9 @@ pgd_status pgd_server_destroy(pgd_server *sv);
 /* ---- thresholds and autotuning (no reference counterpart) --------------
  * Thresholds steer how the decomposition kernels split work; counts never
  * depend on them.  anchor_hub and cache_hub act on the edge-by-edge kernels,
- * which decompose samples of fewer than 1/2048 of a graph's edges and the
- * allocation-free entry point; whole graphs are decomposed by passes that have
- * no thresholds.  Until the caller sets them, samples of graphs of more than
+ * which decompose small samples (fewer than 1/2048 of a graph's edges, more of
+ * dense graphs) and the allocation-free entry point; whole graphs are
+ * decomposed by passes that have no thresholds.  Until the caller sets them, samples of graphs of more than
  * 1.5·2^20 vertices use anchor_hub 128 and cache_hub 40.  anchor_hub (2..256,
  * default 64): anchors of degree >= it are processed one CTA per anchor with
  * N(p) as a bitmap, below it one warp per edge with N(p) staged and searched.

@@ -1337,9 +1337,10 @@ __device__ __forceinline__ void clique_rows(const EgoArgs &A, const EgoTables &T
 // |N+(a)| = d in a block's range: a block per vertex.  The indices of N+(a) go
 // into the lookup tables; each warp takes vertices x of N+(a) and looks the
 // entries of N+(x) up (searching N+(a)'s entries in N+(x) where that takes fewer
-// instructions is bound by the searches' latency: 5.0 against 5.4 ms for the
-// smaller class on R-MAT 20, 2.9 against 2.1 ms for the next).  PASS 1 counts the triangles and, where there is room,
-// keeps them for k_clique_block; PASS 2 (else) lists them again, with F.
+// instructions is bound by the searches' latency: with 32 entries a turn 5.0 against
+// 5.4 ms for the smaller class on R-MAT 20, 2.9 against 2.1 ms for the next).  PASS 1
+// counts the triangles and, where there is room, keeps them for k_clique_block;
+// PASS 2 (else) lists them again, with F, or only finds them again (clique_rows).
 template <int PASS, int NT, bool GLOBAL>
 __global__ void __launch_bounds__(NT) k_ego_block(EgoArgs A, int dmax) {
     extern __shared__ __align__(16) uint32_t s_dyn[];
@@ -1404,7 +1405,7 @@ __global__ void __launch_bounds__(NT) k_ego_block(EgoArgs A, int dmax) {
             const int32_t last = T.ls[i - 1];
             auto find = [&](int32_t y) { return ego_find(T, y, last, shift, hmask); };
             // 64 entries a turn: two loads in flight, one place among the hits for both
-            // (R-MAT 20: 5.38 -> 4.68 ms for the smaller class, 2.52 -> 1.74 ms for the
+            // (R-MAT 20: 5.42 -> 4.70 ms for the smaller class, 2.12 -> 1.64 ms for the
             // next; bound by issue.  Short rows end to end over the lanes instead: 5.72 ms)
             for (int b = 0; b < len; b += 64) {
                 const uint32_t pos = r0 + (uint32_t)(b + lane);

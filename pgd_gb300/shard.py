@@ -1,14 +1,15 @@
 """Decomposition of one graph sharded over ranks.
 
 Edges are independent given the CSR, so every rank holds the whole graph and
-decomposes a contiguous span of the ordered edge list (E_ordered).  The spans
-are weighted by an estimate of each edge's work in the decomposition kernels:
-the scan of the non-anchor endpoint q's list plus the lists of its
-low-degree neighbours, which are scanned per edge (see edge_cost).  Every
-rank also computes the triangle count of every edge (the c4 identity reads
-t of edges outside the span) and the graph's per-vertex structures: that
-O(m) part is repeated on each rank and bounds strong scaling.  Each rank orders and decomposes its span with the sampled edge
-order (`Graph.sort_edges_sample`, the reference's sort_edges with E_s,
+decomposes a contiguous span of the ordered edge list (E_ordered).  A span of
+1/2048 of the edges or more goes through the passes over the whole graph on
+every rank (dense graphs take larger spans edge by edge): the identities read
+the counts of edges outside the span, and only the closing and the per-edge rows
+shrink with it.  So a split divides the rows of one graph, not its time; many
+graphs shard by graph.  The spans are weighted by an estimate of the work of
+edge-by-edge decomposition (see edge_cost), which smaller spans take.  Each rank
+orders and decomposes its span with the sampled edge order
+(`Graph.sort_edges_sample`, the reference's sort_edges with E_s,
 graphlet_core.cpp:836-851).  The only exchange is a sum of the 15 uint64
 partial sums, which wraps mod 2^64 exactly like the device sums.  The 17
 totals are then closed on every rank from the summed partials
@@ -41,10 +42,10 @@ def edge_spans(cost, world):
 
 
 def edge_cost(ev, eu, deg, order, cache_hub=40):
-    """Work estimate of each ordered edge (p, q), p the endpoint of higher
-    (degree, id): deg(q) slot records, plus the lists of q's neighbours of
-    degree below cache_hub (their W(w, p) is counted per edge, the higher
-    ones come from the anchor's histogram), plus one."""
+    """Work estimate of each ordered edge (p, q) decomposed edge by edge, p the
+    endpoint of higher (degree, id): deg(q) slot records, plus the lists of q's
+    neighbours of degree below cache_hub (their W(w, p) is counted per edge, the
+    higher ones come from the anchor's histogram), plus one."""
     ev = np.asarray(ev, np.int64)
     eu = np.asarray(eu, np.int64)
     deg = np.asarray(deg, np.int64)
