@@ -121,7 +121,7 @@ pgd_status pgd_graph_from_file(pgd_ctx *ctx, const char *path, pgd_graph **out);
  * PGD_EDGES_DEDUP) removes duplicates, keeping each pair's first position
  * as its insertion rank, as the reader's adjacency map does
  * (graphlet_core.cpp:410-411, 448-455).  n = max(n_min, 1 + largest id with
- * an edge).  Without PGD_EDGES_DEDUP a repeated pair is an error, since the
+ * an edge), at most 2^31.  Without PGD_EDGES_DEDUP a repeated pair is an error, since the
  * reference's marking is ill-defined on multigraphs. */
 pgd_status pgd_graph_from_edges(pgd_ctx *ctx, const int32_t *src, const int32_t *dst, int64_t k,
                                 int64_t n_min, uint32_t flags, pgd_graph **out);

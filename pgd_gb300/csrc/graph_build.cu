@@ -682,6 +682,11 @@ pgd_status pgd_build_from_device_pairs(pgd_graph *g, const int32_t *d_src, const
     if (pgd_pinned<unsigned long long>(ctx, 16)) return pgd_fail(ctx, PGD_EINVAL, "negative vertex id in edge list");
     g->self_loops = pgd_pinned<int64_t>(ctx, 8);
     g->n = std::max<int64_t>(n_min, max_id + 1);
+    // vertices are kept as 32-bit numbers from 0
+    if (g->n > (int64_t)1 << 31) {
+        g->n = 0;
+        return pgd_fail(ctx, PGD_EINVAL, "vertex count out of range (0..2^31)");
+    }
     const int64_t valid = 2 * (k - g->self_loops), ne = 2 * k;
     // a word holds row and column on the bits that ids up to max_id + 1 need
     const int cb = pgd_id_bits(max_id);

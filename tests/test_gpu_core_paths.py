@@ -58,3 +58,13 @@ def test_largest_vertex_ids():
     assert (got == want).all()
     g.destroy()
     c.close()
+
+
+@pytest.mark.parametrize("k", [3, 3000])
+def test_more_vertices_than_ids_are_refused(ctx, k):
+    """n_min beyond 2^31: the k-core and the ranks would number vertices past 32 bits."""
+    p = np.arange(k, dtype=np.int32)
+    held = ctx.resident_bytes
+    with pytest.raises(pgd.PGDError) as e:
+        ctx.graph_from_edges(p, p + 1, n_min=2 ** 31 + 1)
+    assert e.value.status == 1 and ctx.resident_bytes == held   # PGD_EINVAL
