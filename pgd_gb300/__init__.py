@@ -231,7 +231,12 @@ class _OwnCounts(Counts):
 def _counts_list(out):
     """The results of a ctypes array of pgd_counts, each a view of its words
     (no copy and no per-field conversion: a batch has thousands of them)."""
-    return [Counts(w) for w in np.frombuffer(out, np.uint64).reshape(-1, _WORDS)]
+    new, res = Counts.__new__, []
+    for w in np.frombuffer(out, np.uint64).reshape(-1, _WORDS):
+        r = new(Counts)
+        r._w = w
+        res.append(r)
+    return res
 
 
 class Context:
